@@ -33,7 +33,8 @@ int launch_gen_normal(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, double, do
 int launch_gen_cmatrix(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, int64_t, int64_t,
                        double, double*, cudaStream_t);
 int launch_chi0_fp64(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
-                     int, double2*, cudaStream_t, int);
+                     int, double2*, void* part, size_t part_bytes, cudaStream_t, int*);
+size_t fp64_part_bytes(const spx_ctx*, int64_t P, int N, int nw);
 int split_chi0_slab(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
                     int, double2*, void*, size_t, cudaStream_t, int*, int variant, int slab);
 size_t split_workspace_bytes(int64_t P, int N, int nw);
@@ -146,6 +147,15 @@ int ensure_workspace(spx_ctx* ctx, size_t bytes) {
   return SPX_OK;
 }
 
+int ensure_workspace_opt(spx_ctx* ctx, size_t bytes, size_t* extra) {
+  int rc = ensure_workspace(ctx, bytes + *extra);
+  if (rc == SPX_ENOMEM && *extra > 0) {
+    *extra = 0;
+    rc = ensure_workspace(ctx, bytes);
+  }
+  return rc;
+}
+
 int ensure_pinned(spx_ctx* ctx, size_t bytes) {
   if (bytes <= ctx->pinned_bytes) return SPX_OK;
   if (ctx->pinned) {
@@ -212,7 +222,8 @@ static int check_chi0_args(spx_ctx* ctx, const double* cprod, int64_t ldc, int64
 }
 
 // Accumulates one slab of band pairs already on the device into the device
-// output. `W` is workspace for npair*nw weights (ldw = round_up(npair, 16)).
+// output. `W` is workspace for npair*nw weights (ldw = round_up(npair, 16)); `split_ws`
+// the split path's scratch, or the FP64 path's partial tiles (optional).
 // `plan` (variant, slab, tile), when given, replaces the per-call choice: a caller
 // that streams one array in chunks keeps one kernel and one slab size for all of it.
 static int chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N,
@@ -227,8 +238,7 @@ static int chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
   ++*launches;
   if (precision == SPX_FP64) {
     timing_mark(ctx, s, 1);
-    rc = launch_chi0_fp64(ctx, M, ldc, P, N, W, ldw, nw, out, s, 8);
-    ++*launches;
+    rc = launch_chi0_fp64(ctx, M, ldc, P, N, W, ldw, nw, out, split_ws, split_ws_bytes, s, launches);
   } else {
     // kernel variant and slab from the context's tuning table when the caller left
     // the variant open and the table has this shape (smaller slabs need less scratch)
@@ -425,9 +435,11 @@ extern "C" int spx_chi0_accumulate_dev(spx_ctx* ctx, const double* cprod, int64_
   const int64_t ldw = (int64_t)align_up((size_t)npair, 16);
   size_t wbytes = align_up(sizeof(double) * (size_t)ldw * nw, 256);
   size_t sbytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
-  if ((rc = ensure_workspace(ctx, wbytes + sbytes))) return rc;
+  size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, npair, nbas, nw) : 0;
+  if ((rc = ensure_workspace_opt(ctx, wbytes + sbytes, &part))) return rc;
+  sbytes += part;
   double* W = (double*)ctx->ws;
-  void* sws = (char*)ctx->ws + wbytes;
+  void* sws = sbytes ? (char*)ctx->ws + wbytes : nullptr;
   int launches = 0;
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
@@ -573,9 +585,11 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
   const size_t e_bytes = align_up(sizeof(double) * (size_t)slab, 256);
   const size_t om_bytes = align_up(sizeof(double) * (size_t)nw, 256);
   const size_t w_bytes = align_up(sizeof(double) * (size_t)slab * nw, 256);
-  const size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, slab, nbas, nw) : 0;
+  size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, slab, nbas, nw) : 0;
   size_t total = out_bytes + nslab_buf * (slab_bytes + 2 * e_bytes) + om_bytes + w_bytes + s_bytes;
-  if ((rc = ensure_workspace(ctx, total))) return rc;
+  size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, slab, nbas, nw) : 0;
+  if ((rc = ensure_workspace_opt(ctx, total, &part))) return rc;
+  s_bytes += part;
   char* base = (char*)ctx->ws;
   double2* d_out = (double2*)base;
   base += out_bytes;
@@ -753,9 +767,14 @@ extern "C" int spx_chi0_from_coeffs_dev(spx_ctx* ctx, const spx_mt_desc* mt,
                                      wfprod_pw_workspace(pw, nk, nocc, nunocc, split_products));
   const int64_t ldw = ldc;
   const size_t w_bytes = align_up(sizeof(double) * (size_t)ldw * nw, 256);
-  const size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
-  const size_t scratch = std::max(prod_bytes, w_bytes + s_bytes);
-  if ((rc = ensure_workspace(ctx, m_bytes + scratch))) return rc;
+  size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
+  size_t scratch = std::max(prod_bytes, w_bytes + s_bytes);
+  // the FP64 path's partial tiles follow the weights, in what the products leave free or beyond
+  const size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, npair, nbas, nw) : 0;
+  size_t beyond = w_bytes + part > scratch ? w_bytes + part - scratch : 0;
+  if ((rc = ensure_workspace_opt(ctx, m_bytes + scratch, &beyond))) return rc;
+  scratch += beyond;
+  if (w_bytes + part <= scratch) s_bytes += part;
   double2* M = (double2*)ctx->ws;
   char* sc = (char*)ctx->ws + m_bytes;
   int launches = 0;
@@ -811,6 +830,7 @@ extern "C" int spx_weights_hilbert_dev(spx_ctx* ctx, int64_t npair, int32_t nfrq
 // Adds sum_p M(p,i) conj(M(p,j)) w(p,f) with caller weights (any sign) into the
 // packed `out`, using `scratch` (accumulate_w_scratch bytes) for the padded weight
 // copy and the split path's planes.
+// FP64 calls may pass `part_bytes` of scratch beyond that for their partial tiles.
 static size_t accumulate_w_scratch(int64_t npair, int nbas, int nw, int precision) {
   const int64_t ldi = (int64_t)align_up((size_t)npair, 16);
   return align_up(sizeof(double) * (size_t)ldi * nw, 256) +
@@ -819,7 +839,8 @@ static size_t accumulate_w_scratch(int64_t npair, int nbas, int nw, int precisio
 
 static int accumulate_w_into(spx_ctx* ctx, const double* cprod, int64_t ldc, int64_t npair,
                              int nbas, const double* w, int64_t ldw, int nw, int precision,
-                             double* out, char* scratch, cudaStream_t s, int* launches) {
+                             double* out, char* scratch, size_t part_bytes, cudaStream_t s,
+                             int* launches) {
   // the kernels read the weights with 16-pair bulk copies: an aligned, padded copy
   const int64_t ldi = (int64_t)align_up((size_t)npair, 16);
   const size_t wbytes = align_up(sizeof(double) * (size_t)ldi * nw, 256);
@@ -834,10 +855,9 @@ static int accumulate_w_into(spx_ctx* ctx, const double* cprod, int64_t ldc, int
     return rc;
   if (precision == SPX_FP64) {
     timing_mark(ctx, s, 1);
-    rc = launch_chi0_fp64(ctx, reinterpret_cast<const double2*>(cprod), ldc, npair, nbas, W, ldi, nw,
-                          reinterpret_cast<double2*>(out), s, 8);
-    ++*launches;
-    return rc;
+    return launch_chi0_fp64(ctx, reinterpret_cast<const double2*>(cprod), ldc, npair, nbas, W, ldi, nw,
+                            reinterpret_cast<double2*>(out), part_bytes ? sws : nullptr, part_bytes, s,
+                            launches);
   }
   return split_chi0_slab(ctx, reinterpret_cast<const double2*>(cprod), ldc, npair, nbas, W, ldi, nw,
                          reinterpret_cast<double2*>(out), sws, sbytes, s, launches, 0, 0);
@@ -860,12 +880,13 @@ extern "C" int spx_chi0_accumulate_w_dev(spx_ctx* ctx, const double* cprod, int6
   }
   if (npair == 0 || nbas == 0 || nw == 0) return SPX_OK;
   cudaStream_t s = pick_stream(ctx, stream);
-  if ((rc = ensure_workspace(ctx, accumulate_w_scratch(npair, nbas, nw, precision)))) return rc;
+  size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, npair, nbas, nw) : 0;
+  if ((rc = ensure_workspace_opt(ctx, accumulate_w_scratch(npair, nbas, nw, precision), &part))) return rc;
   int launches = 0;
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
   rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, w, ldw, nw, precision, susceph,
-                         (char*)ctx->ws, s, &launches);
+                         (char*)ctx->ws, part, s, &launches);
   timing_mark(ctx, s, 2);
   ctx->timing = false;
   if (rc) return rc;
@@ -907,7 +928,8 @@ extern "C" int spx_chi0_accumulate_c_dev(spx_ctx* ctx, const double* cprod, int6
   const int64_t npack = (int64_t)nbas * (nbas + 1) / 2;
   const size_t pbytes = align_up(sizeof(double2) * (size_t)npack * nw, 256);
   const size_t sc = accumulate_w_scratch(npair, nbas, nw, precision);
-  if ((rc = ensure_workspace(ctx, 2 * pbytes + sc))) return rc;
+  size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, npair, nbas, nw) : 0;
+  if ((rc = ensure_workspace_opt(ctx, 2 * pbytes + sc, &part))) return rc;
   double* S1 = (double*)ctx->ws;
   double* S2 = (double*)((char*)ctx->ws + pbytes);
   char* scratch = (char*)ctx->ws + 2 * pbytes;
@@ -915,8 +937,11 @@ extern "C" int spx_chi0_accumulate_c_dev(spx_ctx* ctx, const double* cprod, int6
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
   if ((rc = check_cuda(ctx, cudaMemsetAsync(S1, 0, 2 * pbytes, s), "zero partial sums"))) return rc;
-  rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, wr, ldw, nw, precision, S1, scratch, s, &launches);
-  if (!rc) rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, wi, ldw, nw, precision, S2, scratch, s, &launches);
+  rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, wr, ldw, nw, precision, S1, scratch, part, s,
+                         &launches);
+  if (!rc)
+    rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, wi, ldw, nw, precision, S2, scratch, part, s,
+                           &launches);
   if (!rc) {
     timing_mark(ctx, s, 0);
     rc = launch_suscepc_combine(ctx, nbas, nw, (const double2*)S1, (const double2*)S2,

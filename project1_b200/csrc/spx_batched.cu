@@ -31,7 +31,8 @@ namespace spx {
 int launch_weights(spx_ctx*, int64_t, int64_t, const double*, const double*, double, int,
                    const double*, double*, cudaStream_t);
 int launch_chi0_fp64(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
-                     int, double2*, cudaStream_t, int);
+                     int, double2*, void* part, size_t part_bytes, cudaStream_t, int*);
+size_t fp64_part_bytes(const spx_ctx*, int64_t P, int N, int nw);
 int split_chi0_slab(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
                     int, double2*, void*, size_t, cudaStream_t, int*, int, int);
 size_t split_workspace_bytes(int64_t P, int N, int nw, int slab);
@@ -118,10 +119,10 @@ static uint64_t fnv(uint64_t h, const void* p, size_t n) {
   return h;
 }
 
-// Enqueues the whole schedule on `s`.
+// Enqueues the whole schedule on `s`; `part` is scratch for the FP64 path's partial tiles.
 static int enqueue_batch(spx_ctx* ctx, int nq, const spx_q_desc* q, const QPlan* pl, int nw,
-                         const double* omega, int precision, char* ws, cudaStream_t s,
-                         int* launches) {
+                         const double* omega, int precision, char* ws, void* part,
+                         size_t part_bytes, cudaStream_t s, int* launches) {
   for (int i = 0; i < nq; ++i) {
     const spx_q_desc& d = q[i];
     const QPlan& p = pl[i];
@@ -156,8 +157,8 @@ static int enqueue_batch(spx_ctx* ctx, int nq, const spx_q_desc* q, const QPlan*
                              p.variant, p.slab);
       } else {
         rc = launch_chi0_fp64(ctx, M, ldc, len, d.nbas, W, ldw, nw,
-                              reinterpret_cast<double2*>(d.susceph), s, 8);
-        ++*launches;
+                              reinterpret_cast<double2*>(d.susceph), part_bytes ? part : nullptr,
+                              part_bytes, s, launches);
       }
       if (rc) return rc;
     }
@@ -240,7 +241,11 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
     pl[i] = plan_q(ctx, q[i], nw, precision);
     need = std::max(need, pl[i].w_bytes + pl[i].g_bytes + pl[i].s_bytes);
   }
-  if ((rc = ensure_workspace(ctx, need + 1024))) return rc;
+  need = align_up(need + 1024, 256);
+  size_t part = 0;
+  if (precision == SPX_FP64)
+    for (int i = 0; i < nq; ++i) part = std::max(part, fp64_part_bytes(ctx, q[i].npair, q[i].nbas, nw));
+  if ((rc = ensure_workspace_opt(ctx, need, &part))) return rc;
   cudaStream_t s = pick_stream(ctx, stream);
   int launches = 0;
   cudaEvent_t e0 = ctx->ev[8], e1 = ctx->ev[9];
@@ -248,7 +253,8 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
   const bool timing = ctx->timing;
   ctx->timing = false;
   if (flags & SPX_BATCH_NOGRAPH) {
-    rc = enqueue_batch(ctx, nq, q, pl.data(), nw, omega, precision, (char*)ctx->ws, s, &launches);
+    rc = enqueue_batch(ctx, nq, q, pl.data(), nw, omega, precision, (char*)ctx->ws, (char*)ctx->ws + need,
+                       part, s, &launches);
   } else {
     uint64_t key = 1469598103934665603ull;
     key = fnv(key, &nq, sizeof(nq));
@@ -258,6 +264,7 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
     key = fnv(key, &precision, sizeof(precision));
     key = fnv(key, &ctx->ws, sizeof(ctx->ws));
     key = fnv(key, &ctx->ws_bytes, sizeof(ctx->ws_bytes));
+    key = fnv(key, &part, sizeof(part));
     for (const QPlan& p : pl) key = fnv(key, &p, sizeof(p));
     spx_ctx::BatchGraph* hit = nullptr;
     for (auto& g : ctx->graphs)
@@ -273,8 +280,8 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
         return rc;
       }
       int cap_launches = 0;
-      rc = enqueue_batch(ctx, nq, q, pl.data(), nw, omega, precision, (char*)ctx->ws, cs,
-                         &cap_launches);
+      rc = enqueue_batch(ctx, nq, q, pl.data(), nw, omega, precision, (char*)ctx->ws,
+                         (char*)ctx->ws + need, part, cs, &cap_launches);
       cudaError_t ee = cudaStreamEndCapture(cs, &graph);
       if (!rc) rc = check_cuda(ctx, ee, "end capture");
       if (!rc) rc = check_cuda(ctx, cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");

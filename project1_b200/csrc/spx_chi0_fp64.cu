@@ -278,77 +278,486 @@ __global__ void __launch_bounds__(F64_THREADS, 2)
   }
 }
 
+// ---------------------------------------------------------------------------
+// K1p: the product-first form of K1, for calls with several frequencies.
+//
+// The pair products z_p(i, j) = M(p, i) conj(M(p, j)) do not depend on the frequency:
+// the reference forms them once and takes one ddot per frequency
+// (src/susceptibility.f:1194-1205, :1779-1782). Per (p, i, j) that is 4 FP64 operations for
+// z and 2 multiply-adds per frequency, against the 4 per frequency of K1, which
+// folds the weight into one operand and contracts complex numbers. Here the
+// contraction over p runs on DMMA with the products as the A operand (16 rows i of
+// one column j, 8 pairs) and the weights as the B operand (8 pairs, 8 frequencies),
+// re and im separately: 16 NT + 4 units for 8 NT frequencies instead of 32 NT
+// (52 against 96 at 24 frequencies). Every thread forms exactly the products its
+// fragment needs, in registers, so nothing is staged twice.
+//
+// Measured (1200 functions, 128000 pairs, 24 frequencies): 603 ms with K1, 305 ms here,
+// 0.84 of the FP64 pipe at 1965 MHz for the 52 units; the error against 64-bit sums falls
+// from 1.3e-14 to 8.7e-15.
+//
+// Bound: the FP64 pipe (DMMA and the products share it). A CTA of four warps owns
+// 16 x 8 elements (two columns per warp: 32 NT accumulator registers leave three CTAs
+// per SM) for one group of 8 NT frequencies, and streams 16-pair chunks of 16 + 8
+// columns of M and of the weights through F64P_ST TMA stages (SWIZZLE_128B).
+//
+// Work is dealt in whole tiles, one per CTA and round; the tiles of the last,
+// partial round are cut along p into equal ranges, one per CTA, whose partial sums go
+// to `part` and are added in CTA order by chi0_fp64p_reduce_kernel, so the result
+// depends on the sizes only. Without `part` the last round stays whole.
+constexpr int F64P_ST = 4;
+constexpr int F64P_TI = 16, F64P_TJ = 8, F64P_JW = 2;   // tile rows, columns, columns per warp
+constexpr int F64P_CTAS = 3;                            // resident CTAs per SM
+constexpr int F64P_MINCHUNK = 16;                       // shortest p axis (in chunks) worth cutting
+
+template <int NT>
+struct __align__(1024) F64PSmem {
+  double2 a[F64P_ST][2][F64P_TI][F64_KBOX];
+  double2 b[F64P_ST][2][F64P_TJ][F64_KBOX];
+  double w[F64P_ST][8 * NT][F64_KC];   // row f's 16-byte chunk c stored at c ^ (f & 7)
+  uint64_t full[F64P_ST];
+  uint64_t empty[F64P_ST];
+};
+
+struct F64PParams {
+  int N, nw, f0;           // matrix size, frequencies of the call, first frequency of this launch
+  int ntile, nchunk;
+  int64_t items;           // ntile x frequency groups
+  int64_t whole;           // items dealt whole: rounds x grid (all of them without `part`)
+  double2* out;
+  int64_t npack;
+  double2* part;           // [CTA][2 slots][elements] partial tiles, or NULL
+  int* status;
+  uint64_t timeout_ns;
+};
+
+// The segments of one CTA: whole items blockIdx.x, + gridDim.x, ... below `whole`, then
+// its share [u, u1) of the remaining items' chunks, cut at item boundaries.
+struct F64PSeg {
+  int64_t item;   // next whole item
+  int64_t u, u1;
+  int nseg;       // partial-range segments handed out
+  __device__ __forceinline__ void init(const F64PParams& p, int cta, int grid) {
+    item = cta;
+    const int64_t tail = (p.items - p.whole) * (int64_t)p.nchunk;
+    u = tail * cta / grid;
+    u1 = tail * (cta + 1) / grid;
+    nseg = 0;
+  }
+  // Next segment: item, chunks [k0, k1), slot (-1: a whole item). False at the end.
+  __device__ __forceinline__ bool next(const F64PParams& p, int grid, int64_t* it, int* k0, int* k1, int* slot) {
+    if (item < p.whole) {
+      *it = item;
+      *k0 = 0;
+      *k1 = p.nchunk;
+      *slot = -1;
+      item += grid;
+      return true;
+    }
+    if (u >= u1) return false;
+    const int64_t t = u / p.nchunk;
+    *it = p.whole + t;
+    *k0 = (int)(u - t * p.nchunk);
+    const int64_t e = min(u1, (t + 1) * (int64_t)p.nchunk);
+    *k1 = (int)(e - t * p.nchunk);
+    *slot = (*k0 == 0 && *k1 == p.nchunk) ? -1 : min(nseg, 1);
+    ++nseg;
+    u = e;
+    return true;
+  }
+};
+
+// Tile t of the upper triangle in 16-row x 8-column blocks: column block bj has
+// bj / 2 + 1 row blocks, so blocks 2m and 2m + 1 start at m (m + 1) and (m + 1)^2.
+__host__ __device__ __forceinline__ void f64p_decode(int t, int* bi, int* bj) {
+  int m = (int)((sqrtf(4.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+  while (m * (m + 1) > t) --m;
+  while ((m + 1) * (m + 2) <= t) ++m;
+  const int r = t - m * (m + 1);
+  *bj = 2 * m + (r > m ? 1 : 0);
+  *bi = r > m ? r - (m + 1) : r;
+}
+static int f64p_tiles(int N) {
+  const int nbj = (N + F64P_TJ - 1) / F64P_TJ, m = nbj / 2;
+  return m * (m + 1) + (nbj & 1) * (m + 1);
+}
+
+// Adds a tile held as accumulator fragments (row i = g + 8 (r / 2), frequency
+// 8 nt + 2 t + (r & 1)) into the packed output.
+template <int NT>
+__device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item,
+                                           const double (&re)[F64P_JW][NT][4], const double (&im)[F64P_JW][NT][4]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  int bi, bj;
+  f64p_decode((int)(item % prm.ntile), &bi, &bj);
+  const int fb = prm.f0 + (int)(item / prm.ntile) * 8 * NT;
+#pragma unroll
+  for (int jj = 0; jj < F64P_JW; ++jj) {
+    const int j = bj * F64P_TJ + F64P_JW * warp + jj;
+    if (j >= prm.N) continue;
+    double2* oj = prm.out + (int64_t)j * (j + 1) / 2;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int i = bi * F64P_TI + g + 8 * (r >> 1), f = fb + 8 * nt + 2 * t + (r & 1);
+        if (i > j || f >= prm.nw) continue;
+        double2* o = oj + (int64_t)f * prm.npack + i;
+        double2 v = *o;
+        v.x += re[jj][nt][r];
+        v.y += im[jj][nt][r];
+        *o = v;
+      }
+  }
+}
+
+template <int NT>
+__global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
+    chi0_fp64p_kernel(const __grid_constant__ CUtensorMap mapI, const __grid_constant__ CUtensorMap mapJ,
+                      const __grid_constant__ CUtensorMap mapW, F64PParams prm) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  using Smem = F64PSmem<NT>;
+  Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < F64P_ST; ++s) {
+      mbar_init(&sm.full[s], 1);
+      mbar_init(&sm.empty[s], F64_WARPS);
+    }
+    fence_barrier_init();
+  }
+  __syncthreads();
+
+  // warp 0, lane 0 issues the copies, F64P_ST - 2 chunks ahead of the chunk it computes:
+  // a stage is refilled two chunks after it was read, so the issuer rarely waits
+  F64PSeg ps;
+  int64_t p_item = 0;
+  int pk = 0, pk1 = 0, p_slot, py = 0, pyj = 0, pf = 0;
+  bool p_more = false;
+  uint32_t issued = 0;
+  auto enter = [&] {
+    int bi, bj;
+    f64p_decode((int)(p_item % prm.ntile), &bi, &bj);
+    py = bi * F64P_TI;
+    pyj = bj * F64P_TJ;
+    pf = prm.f0 + (int)(p_item / prm.ntile) * 8 * NT;
+  };
+  auto issue = [&] {
+    const int st = (int)(issued % F64P_ST);
+    mbar_arrive_expect_tx(&sm.full[st], (uint32_t)(sizeof(sm.a[0]) + sizeof(sm.b[0]) + sizeof(sm.w[0])));
+    const int x = pk * 2 * F64_KC;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      tma_load_2d(&sm.a[st][h][0][0], &mapI, x + 2 * F64_KBOX * h, py, &sm.full[st]);
+      tma_load_2d(&sm.b[st][h][0][0], &mapJ, x + 2 * F64_KBOX * h, pyj, &sm.full[st]);
+    }
+    tma_load_2d(&sm.w[st][0][0], &mapW, pk * F64_KC, pf, &sm.full[st]);
+    ++issued;
+    if (++pk == pk1) {
+      p_more = ps.next(prm, gridDim.x, &p_item, &pk, &pk1, &p_slot);
+      if (p_more) enter();
+    }
+  };
+  if (threadIdx.x == 0) {
+    ps.init(prm, blockIdx.x, gridDim.x);
+    p_more = ps.next(prm, gridDim.x, &p_item, &pk, &pk1, &p_slot);
+    if (p_more) enter();
+    while (p_more && issued < F64P_ST - 2) issue();
+  }
+
+  F64PSeg seg;
+  seg.init(prm, blockIdx.x, gridDim.x);
+  int64_t item;
+  int k0, k1, slot;
+  uint32_t c = 0;   // chunks computed
+  bool ok = true;
+  while (ok && seg.next(prm, gridDim.x, &item, &k0, &k1, &slot)) {
+    double re[F64P_JW][NT][4], im[F64P_JW][NT][4];
+#pragma unroll
+    for (int jj = 0; jj < F64P_JW; ++jj)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) re[jj][nt][r] = im[jj][nt][r] = 0.0;
+    for (int k = k0; k < k1; ++k, ++c) {
+      const int st = (int)(c % F64P_ST);
+      if (warp == 0) {
+        int good = 1;
+        if (lane == 0 && p_more) {
+          // the next chunk to issue is c + F64P_ST - 2, into the stage of chunk c - 2
+          if (c >= 2)
+            good = mbar_wait(&sm.empty[(c - 2) % F64P_ST], ((c - 2) / F64P_ST) & 1u, prm.timeout_ns, prm.status);
+          if (good) issue();
+        }
+        if (!__shfl_sync(0xffffffffu, good, 0)) {
+          ok = false;
+          break;
+        }
+      }
+      if (!mbar_wait(&sm.full[st], (c / F64P_ST) & 1u, prm.timeout_ns, prm.status)) {
+        ok = false;
+        break;
+      }
+#pragma unroll
+      for (int ks = 0; ks < F64_KC / F64_KBOX; ++ks) {
+        double wf[NT][2];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int p = F64_KBOX * ks + t + 4 * q;
+            wf[nt][q] = sm.w[st][8 * nt + g][(((p >> 1) ^ g) << 1) | (p & 1)];
+          }
+        double2 a[4];   // a[2q + h] = M(pair t + 4q, row g + 8h)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) a[2 * q + h] = sm.a[st][ks][g + 8 * h][(t + 4 * q) ^ g];
+#pragma unroll
+        for (int jj = 0; jj < F64P_JW; ++jj) {
+          const int rj = F64P_JW * warp + jj;
+          const double2 b0 = sm.b[st][ks][rj][t ^ rj], b1 = sm.b[st][ks][rj][(t + 4) ^ rj];
+          double z[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const double2 b = e < 2 ? b0 : b1;
+            z[e] = fma(a[e].x, b.x, a[e].y * b.y);
+          }
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) dmma<8>(re[jj][nt], z, wf[nt]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const double2 b = e < 2 ? b0 : b1;
+            z[e] = fma(a[e].y, b.x, -(a[e].x * b.y));
+          }
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) dmma<8>(im[jj][nt], z, wf[nt]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.empty[st]);
+    }
+    if (!ok) break;
+    if (slot < 0) {
+      f64p_store<NT>(prm, item, re, im);
+    } else {
+      double2* pp = prm.part + ((int64_t)blockIdx.x * 2 + slot) * (F64P_JW * NT * 4 * F64_THREADS) + threadIdx.x;
+#pragma unroll
+      for (int jj = 0; jj < F64P_JW; ++jj)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            pp[((jj * NT + nt) * 4 + r) * F64_THREADS] = make_double2(re[jj][nt][r], im[jj][nt][r]);
+    }
+  }
+  if (!ok && threadIdx.x == 0) {
+    // never leave with copies still landing in this CTA's shared memory
+    for (uint32_t k = c; k < issued; ++k)
+      mbar_drain(&sm.full[k % F64P_ST], (k / F64P_ST) & 1u, prm.timeout_ns);
+  }
+}
+
+// One CTA per boundary b between the ranges of CTAs b and b + 1 of the accumulation
+// (grid `ncta`): when it falls inside an item and is the first to do so, adds the item's
+// partial tiles in CTA order into the output.
+template <int NT>
+__global__ void __launch_bounds__(F64_THREADS) chi0_fp64p_reduce_kernel(F64PParams prm, int ncta) {
+  const int64_t tail = (prm.items - prm.whole) * (int64_t)prm.nchunk;
+  const int c = blockIdx.x + 1;
+  const int64_t u = tail * c / ncta;
+  const int64_t t = u / prm.nchunk;
+  const int64_t t0 = t * prm.nchunk, t1 = t0 + prm.nchunk;
+  if (u == t0 || u >= tail) return;
+  const int64_t up = tail * (c - 1) / ncta;
+  if (up > t0) return;   // an earlier boundary already lies inside this item
+  double re[F64P_JW][NT][4], im[F64P_JW][NT][4];
+#pragma unroll
+  for (int jj = 0; jj < F64P_JW; ++jj)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) re[jj][nt][r] = im[jj][nt][r] = 0.0;
+  for (int k = c - 1; k < ncta; ++k) {
+    const int64_t s = tail * k / ncta;
+    if (s >= t1) break;
+    if (tail * (k + 1) / ncta == s) continue;   // an empty range
+    // the item is a CTA's first segment when its range starts inside it
+    const int slot = s >= t0 ? 0 : 1;
+    const double2* pp = prm.part + ((int64_t)k * 2 + slot) * (F64P_JW * NT * 4 * F64_THREADS) + threadIdx.x;
+#pragma unroll
+    for (int jj = 0; jj < F64P_JW; ++jj)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const double2 v = pp[((jj * NT + nt) * 4 + r) * F64_THREADS];
+          re[jj][nt][r] += v.x;
+          im[jj][nt][r] += v.y;
+        }
+  }
+  f64p_store<NT>(prm, prm.whole + t, re, im);
+}
+
 // Tensor map of M as a 2-D FP64 array: pairs (re, im interleaved) contiguous,
-// columns ldc complex apart; boxes of 8 pairs x 64 columns, SWIZZLE_128B.
-static int f64_map(CUtensorMap* map, const double2* M, int64_t ldc, int64_t P, int N) {
+// columns ldc complex apart; boxes of 8 pairs x `cols` columns, SWIZZLE_128B.
+static int f64_map(CUtensorMap* map, const double2* M, int64_t ldc, int64_t P, int N, int cols) {
   const uint64_t dims[2] = {(uint64_t)(2 * P), (uint64_t)N};
   const uint64_t strides[1] = {(uint64_t)ldc * 16};
-  const uint32_t box[2] = {2 * F64_KBOX, F64_B};
+  const uint32_t box[2] = {2 * F64_KBOX, (uint32_t)cols};
   return encode_tmap(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, M, dims, strides, box,
                      CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-static int f64_launch(int num_sms, const double2* M, int64_t ldc, int64_t P, int N, const double* W,
-                      int64_t ldw, int nw, double2* out, int* status, uint64_t timeout_ns,
-                      cudaStream_t stream) {
-  const int nblk = (N + F64_B - 1) / F64_B;
+// What both launchers share.
+struct F64Call {
+  int num_sms;
+  const double2* M;
+  int64_t ldc, P;
+  int N;
+  const double* W;
+  int64_t ldw;
+  int nw;
+  double2* out;
+  double2* part;
+  size_t part_bytes;
+  int* status;
+  uint64_t timeout_ns;
+  cudaStream_t stream;
+};
+
+// K1 for the `n` frequencies from f0.
+static int f64_launch(const F64Call& q, int f0, int n, int* launches) {
+  const int nblk = (q.N + F64_B - 1) / F64_B;
   F64Params prm;
-  prm.P = P;
-  prm.N = N;
-  prm.W = W;
-  prm.ldw = ldw;
-  prm.nw = nw;
-  prm.out = out;
-  prm.npack = (int64_t)N * (N + 1) / 2;
+  prm.P = q.P;
+  prm.N = q.N;
+  prm.W = q.W + (int64_t)f0 * q.ldw;
+  prm.ldw = q.ldw;
+  prm.nw = n;
+  prm.npack = (int64_t)q.N * (q.N + 1) / 2;
+  prm.out = q.out + (int64_t)f0 * prm.npack;
   prm.ntile = nblk * (nblk + 1) / 2;
-  prm.nitems = (int64_t)prm.ntile * nw;
-  prm.status = status;
-  prm.timeout_ns = timeout_ns;
+  prm.nitems = (int64_t)prm.ntile * n;
+  prm.status = q.status;
+  prm.timeout_ns = q.timeout_ns;
   CUtensorMap map;
-  const int e = f64_map(&map, M, ldc, P, N);
+  const int e = f64_map(&map, q.M, q.ldc, q.P, q.N, F64_B);
   if (e) return e;
   const size_t smem = sizeof(F64Smem) + 1024;
   if (cudaFuncSetAttribute(chi0_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return -2;
-  const int grid = (int)std::min<int64_t>(prm.nitems, (int64_t)2 * num_sms);
-  chi0_fp64_kernel<<<grid, F64_THREADS, smem, stream>>>(map, prm);
+  const int grid = (int)std::min<int64_t>(prm.nitems, (int64_t)2 * q.num_sms);
+  chi0_fp64_kernel<<<grid, F64_THREADS, smem, q.stream>>>(map, prm);
+  ++*launches;
   return 0;
 }
 
-// Enqueues K1 over one slab of band pairs. W holds the weights of exactly these
-// pairs (leading dimension ldw, a multiple of 16, padding zeroed).
+static size_t f64p_part_bytes(int num_sms, int nt) {
+  return sizeof(double2) * (size_t)F64P_CTAS * num_sms * 2 * F64P_JW * nt * 4 * F64_THREADS;
+}
+
+// K1p for `groups` groups of 8 NT frequencies from f0 (the last may be ragged).
+template <int NT>
+static int f64p_launch(const F64Call& q, int f0, int groups, int* launches) {
+  F64PParams prm;
+  prm.N = q.N;
+  prm.nw = q.nw;
+  prm.f0 = f0;
+  prm.ntile = f64p_tiles(q.N);
+  const int64_t nchunk = (q.P + F64_KC - 1) / F64_KC;
+  if (nchunk > 0x7fffffff / (2 * F64_KC)) return -3;   // pair coordinates are 32-bit
+  prm.nchunk = (int)nchunk;
+  prm.items = (int64_t)prm.ntile * groups;
+  prm.out = q.out;
+  prm.npack = (int64_t)q.N * (q.N + 1) / 2;
+  prm.status = q.status;
+  prm.timeout_ns = q.timeout_ns;
+  const int64_t slots = (int64_t)F64P_CTAS * q.num_sms;
+  const bool cut = q.part && q.part_bytes >= f64p_part_bytes(q.num_sms, NT) && prm.nchunk >= F64P_MINCHUNK &&
+                   prm.items % slots != 0;
+  // fewer items than slots: as many CTAs as get half of the shortest cut axis each
+  const int64_t fit = cut ? std::max(prm.items, prm.items * prm.nchunk / (F64P_MINCHUNK / 2)) : prm.items;
+  const int grid = (int)std::min(slots, fit);
+  prm.whole = cut ? prm.items / grid * grid : prm.items;
+  prm.part = cut ? q.part : nullptr;
+  CUtensorMap mi, mj, mw;
+  int e = f64_map(&mi, q.M, q.ldc, q.P, q.N, F64P_TI);
+  if (!e) e = f64_map(&mj, q.M, q.ldc, q.P, q.N, F64P_TJ);
+  if (!e) {
+    const uint64_t dims[2] = {(uint64_t)q.ldw, (uint64_t)q.nw};
+    const uint64_t strides[1] = {(uint64_t)q.ldw * 8};
+    const uint32_t box[2] = {F64_KC, 8 * NT};
+    e = encode_tmap(&mw, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, q.W, dims, strides, box,
+                    CU_TENSOR_MAP_SWIZZLE_128B);
+  }
+  if (e) return e;
+  const size_t smem = sizeof(F64PSmem<NT>) + 1024;
+  if (cudaFuncSetAttribute(chi0_fp64p_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
+    return -2;
+  chi0_fp64p_kernel<NT><<<grid, F64_THREADS, smem, q.stream>>>(mi, mj, mw, prm);
+  ++*launches;
+  if (prm.whole < prm.items && grid > 1) {
+    chi0_fp64p_reduce_kernel<NT><<<grid - 1, F64_THREADS, 0, q.stream>>>(prm, grid);
+    ++*launches;
+  }
+  return 0;
+}
+
+// Frequencies go to K1p in groups of 24 (three DMMA columns blocks); a remainder takes
+// the narrowest form that holds it. Up to four frequencies cost K1 no more than one
+// 8-wide block costs K1p (4 units each against 4 + 16), so those stay with K1.
+static int f64_run(const F64Call& q, int* launches) {
+  int full = q.nw / 24, r = q.nw % 24;
+  if (r > 16) ++full, r = 0;
+  int e = 0;
+  if (full) e = f64p_launch<3>(q, 0, full, launches);
+  const int f0 = 24 * full;
+  if (!e && r > 8) e = f64p_launch<2>(q, f0, 1, launches);
+  else if (!e && r > 4) e = f64p_launch<1>(q, f0, 1, launches);
+  else if (!e && r > 0) e = f64_launch(q, f0, r, launches);
+  return e;
+}
+
+// Scratch for the partial tiles of a call (0 when none are used); optional: without it
+// the tiles of the last round are not cut.
+size_t fp64_part_bytes(const spx_ctx* ctx, int64_t P, int N, int nw) {
+  if (P < (int64_t)F64P_MINCHUNK * F64_KC || N <= 0 || nw <= 4) return 0;
+  return f64p_part_bytes(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
+}
+
+// Enqueues the FP64 accumulation over one slab of band pairs. W holds the weights of
+// exactly these pairs (leading dimension ldw, a multiple of 16, padding zeroed, 16-byte
+// aligned); `part` is fp64_part_bytes of scratch or NULL.
 int launch_chi0_fp64(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N,
-                     const double* W, int64_t ldw, int nw, double2* out, cudaStream_t stream,
-                     int ki) {
-  (void)ki;
+                     const double* W, int64_t ldw, int nw, double2* out, void* part,
+                     size_t part_bytes, cudaStream_t stream, int* launches) {
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
   const uint64_t timeout_ns =
       (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
-  const int e = f64_launch(ctx->num_sms, M, ldc, P, N, W, ldw, nw, out, ctx->d_status, timeout_ns, stream);
-  if (e) return set_error(ctx, SPX_ECUDA, "chi0_fp64_kernel: tensor map or attribute failed (" +
+  const F64Call q{ctx->num_sms, M, ldc, P, N, W, ldw, nw, out, (double2*)part, part_bytes,
+                  ctx->d_status, timeout_ns, stream};
+  const int e = f64_run(q, launches);
+  if (e) return set_error(ctx, SPX_ECUDA, "chi0_fp64 kernels: tensor map or attribute failed (" +
                                               std::to_string(e) + ")");
-  return check_cuda(ctx, cudaGetLastError(), "chi0_fp64_kernel launch");
+  return check_cuda(ctx, cudaGetLastError(), "chi0_fp64 kernel launch");
 }
 
-}  // namespace spx
-
-namespace spx {
-
-// Launches K1 with explicit device resources instead of a context: used by the
+// The same with explicit device resources instead of a context: used by the
 // allocation-free entry point, whose status word and weights live in static
 // device memory.
 int launch_chi0_fp64_noctx(int num_sms, int* status, uint64_t timeout_ns, const double2* M,
                            int64_t ldc, int64_t P, int N, const double* W, int64_t ldw, int nw,
                            double2* out, cudaStream_t stream) {
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
-  if (f64_launch(num_sms, M, ldc, P, N, W, ldw, nw, out, status, timeout_ns, stream)) return SPX_ECUDA;
+  const F64Call q{num_sms, M, ldc, P, N, W, ldw, nw, out, nullptr, 0, status, timeout_ns, stream};
+  int launches = 0;
+  if (f64_run(q, &launches)) return SPX_ECUDA;
   return cudaGetLastError() == cudaSuccess ? SPX_OK : SPX_ECUDA;
 }
-
-}  // namespace spx
-
-namespace spx {
 
 // ---------------------------------------------------------------------------
 // K1r: the -DINV build (MCOMPLEX_dp = real_dp, src/cppmacro.h:53-64), where

@@ -65,6 +65,9 @@ int set_error(spx_ctx* ctx, int code, const std::string& msg);
 int check_cuda(spx_ctx* ctx, cudaError_t e, const char* what);
 // Makes sure the workspace holds `bytes`; returns SPX_OK or SPX_ENOMEM.
 int ensure_workspace(spx_ctx* ctx, size_t bytes);
+// The same for `bytes` and, if they can be had (memory, workspace_limit), `*extra` more;
+// else *extra becomes 0.
+int ensure_workspace_opt(spx_ctx* ctx, size_t bytes, size_t* extra);
 int ensure_pinned(spx_ctx* ctx, size_t bytes);
 // Reads and clears the device status word (synchronises `stream`).
 int collect_status(spx_ctx* ctx, cudaStream_t stream, const char* what);
