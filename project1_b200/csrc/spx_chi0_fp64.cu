@@ -306,13 +306,24 @@ __global__ void __launch_bounds__(F64_THREADS, 2)
 // to `part` and are added in CTA order by chi0_fp64p_reduce_kernel, so the result
 // depends on the sizes only. Without `part` the last round stays whole.
 constexpr int F64P_ST = 4;
-constexpr int F64P_TI = 16, F64P_TJ = 8, F64P_JW = 2;   // tile rows, columns, columns per warp
-constexpr int F64P_CTAS = 3;                            // resident CTAs per SM
+constexpr int F64P_TI = 16, F64P_TJ = 8;                // tile rows and columns of the polarisation
 constexpr int F64P_MINCHUNK = 16;                       // shortest p axis (in chunks) worth cutting
 
-template <int NT>
+// HW, the q -> 0 head and wings (src/susceptibility.f:1092-1157): the same sum for the rows
+// i of [cprod | dcprod] against the three columns of dcprod. A warp owns 16 rows and all
+// three columns, a CTA 64 rows; one more block of rows, dcprod itself, gives the head.
+// Measured at 1100 columns, 48000 pairs, 24 frequencies: 0.64 ms with the cut tiles' sum,
+// against 6.4 ms as a 72-row GEMM (weights folded into 3 x 24 rows, 64-row tiles).
+template <bool HW>
+struct F64PTile {
+  static constexpr int TI = HW ? 64 : F64P_TI;
+  static constexpr int JW = HW ? 3 : 2;     // columns per warp
+  static constexpr int CTAS = HW ? 2 : 3;   // resident CTAs per SM
+};
+
+template <int NT, bool HW>
 struct __align__(1024) F64PSmem {
-  double2 a[F64P_ST][2][F64P_TI][F64_KBOX];
+  double2 a[F64P_ST][2][F64PTile<HW>::TI][F64_KBOX];
   double2 b[F64P_ST][2][F64P_TJ][F64_KBOX];
   double w[F64P_ST][8 * NT][F64_KC];   // row f's 16-byte chunk c stored at c ^ (f & 7)
   uint64_t full[F64P_ST];
@@ -324,7 +335,8 @@ struct F64PParams {
   int ntile, nchunk;
   int64_t items;           // ntile x frequency groups
   int64_t whole;           // items dealt whole: rounds x grid (all of them without `part`)
-  double2* out;
+  double2* out;            // packed polarisation; HW: wing (3, N, nw)
+  double2* head;           // HW: head (6, nw)
   int64_t npack;
   double2* part;           // [CTA][2 slots][elements] partial tiles, or NULL
   int* status;
@@ -382,18 +394,54 @@ static int f64p_tiles(int N) {
   return m * (m + 1) + (nbj & 1) * (m + 1);
 }
 
-// Adds a tile held as accumulator fragments (row i = g + 8 (r / 2), frequency
-// 8 nt + 2 t + (r & 1)) into the packed output.
-template <int NT>
-__device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item,
-                                           const double (&re)[F64P_JW][NT][4], const double (&im)[F64P_JW][NT][4]) {
+template <int NT, bool HW>
+struct F64PAcc {
+  double re[F64PTile<HW>::JW][NT][4], im[F64PTile<HW>::JW][NT][4];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int jj = 0; jj < F64PTile<HW>::JW; ++jj)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) re[jj][nt][r] = im[jj][nt][r] = 0.0;
+  }
+  static constexpr int ELEMS = F64PTile<HW>::JW * NT * 4 * F64_THREADS;   // of a CTA
+};
+
+// Adds a tile held as accumulator fragments (row g + 8 (r / 2), frequency
+// 8 nt + 2 t + (r & 1)) into the output.
+template <int NT, bool HW>
+__device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item, const F64PAcc<NT, HW>& acc) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int fb = prm.f0 + (int)(item / prm.ntile) * 8 * NT;
+  if constexpr (HW) {
+    const int bi = (int)(item % prm.ntile);
+    const bool hd = bi == prm.ntile - 1;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row = 16 * warp + g + 8 * (r >> 1), f = fb + 8 * nt + 2 * t + (r & 1);
+        const int i = hd ? row : bi * F64PTile<HW>::TI + row;
+        if (f >= prm.nw || i >= (hd ? 3 : prm.N)) continue;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          if (hd && i > a) continue;
+          double2* o = hd ? prm.head + a * (a + 1) / 2 + i + 6 * (int64_t)f
+                          : prm.out + a + 3 * ((int64_t)i + (int64_t)prm.N * f);
+          double2 v = *o;
+          v.x += acc.re[a][nt][r];
+          v.y += acc.im[a][nt][r];
+          *o = v;
+        }
+      }
+    return;
+  }
   int bi, bj;
   f64p_decode((int)(item % prm.ntile), &bi, &bj);
-  const int fb = prm.f0 + (int)(item / prm.ntile) * 8 * NT;
 #pragma unroll
-  for (int jj = 0; jj < F64P_JW; ++jj) {
-    const int j = bj * F64P_TJ + F64P_JW * warp + jj;
+  for (int jj = 0; jj < F64PTile<HW>::JW; ++jj) {
+    const int j = bj * F64P_TJ + F64PTile<HW>::JW * warp + jj;
     if (j >= prm.N) continue;
     double2* oj = prm.out + (int64_t)j * (j + 1) / 2;
 #pragma unroll
@@ -404,19 +452,22 @@ __device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item,
         if (i > j || f >= prm.nw) continue;
         double2* o = oj + (int64_t)f * prm.npack + i;
         double2 v = *o;
-        v.x += re[jj][nt][r];
-        v.y += im[jj][nt][r];
+        v.x += acc.re[jj][nt][r];
+        v.y += acc.im[jj][nt][r];
         *o = v;
       }
   }
 }
 
-template <int NT>
-__global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
+// mapI: boxes of the rows i; mapJ: the 8-column boxes of j; mapH (HW): dcprod as rows
+template <int NT, bool HW>
+__global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
     chi0_fp64p_kernel(const __grid_constant__ CUtensorMap mapI, const __grid_constant__ CUtensorMap mapJ,
-                      const __grid_constant__ CUtensorMap mapW, F64PParams prm) {
+                      const __grid_constant__ CUtensorMap mapW, const __grid_constant__ CUtensorMap mapH,
+                      F64PParams prm) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  using Smem = F64PSmem<NT>;
+  using Smem = F64PSmem<NT, HW>;
+  constexpr int JW = F64PTile<HW>::JW;
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -434,13 +485,19 @@ __global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
   F64PSeg ps;
   int64_t p_item = 0;
   int pk = 0, pk1 = 0, p_slot, py = 0, pyj = 0, pf = 0;
-  bool p_more = false;
+  bool p_more = false, p_head = false;
   uint32_t issued = 0;
   auto enter = [&] {
-    int bi, bj;
-    f64p_decode((int)(p_item % prm.ntile), &bi, &bj);
-    py = bi * F64P_TI;
-    pyj = bj * F64P_TJ;
+    if constexpr (HW) {
+      const int bi = (int)(p_item % prm.ntile);
+      p_head = bi == prm.ntile - 1;
+      py = p_head ? 0 : bi * F64PTile<HW>::TI;
+    } else {
+      int bi, bj;
+      f64p_decode((int)(p_item % prm.ntile), &bi, &bj);
+      py = bi * F64P_TI;
+      pyj = bj * F64P_TJ;
+    }
     pf = prm.f0 + (int)(p_item / prm.ntile) * 8 * NT;
   };
   auto issue = [&] {
@@ -449,7 +506,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
     const int x = pk * 2 * F64_KC;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      tma_load_2d(&sm.a[st][h][0][0], &mapI, x + 2 * F64_KBOX * h, py, &sm.full[st]);
+      tma_load_2d(&sm.a[st][h][0][0], HW && p_head ? &mapH : &mapI, x + 2 * F64_KBOX * h, py, &sm.full[st]);
       tma_load_2d(&sm.b[st][h][0][0], &mapJ, x + 2 * F64_KBOX * h, pyj, &sm.full[st]);
     }
     tma_load_2d(&sm.w[st][0][0], &mapW, pk * F64_KC, pf, &sm.full[st]);
@@ -473,13 +530,8 @@ __global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
   uint32_t c = 0;   // chunks computed
   bool ok = true;
   while (ok && seg.next(prm, gridDim.x, &item, &k0, &k1, &slot)) {
-    double re[F64P_JW][NT][4], im[F64P_JW][NT][4];
-#pragma unroll
-    for (int jj = 0; jj < F64P_JW; ++jj)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) re[jj][nt][r] = im[jj][nt][r] = 0.0;
+    F64PAcc<NT, HW> acc;
+    acc.zero();
     for (int k = k0; k < k1; ++k, ++c) {
       const int st = (int)(c % F64P_ST);
       if (warp == 0) {
@@ -513,10 +565,10 @@ __global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
 #pragma unroll
         for (int q = 0; q < 2; ++q)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) a[2 * q + h] = sm.a[st][ks][g + 8 * h][(t + 4 * q) ^ g];
+          for (int h = 0; h < 2; ++h) a[2 * q + h] = sm.a[st][ks][(HW ? 16 * warp : 0) + g + 8 * h][(t + 4 * q) ^ g];
 #pragma unroll
-        for (int jj = 0; jj < F64P_JW; ++jj) {
-          const int rj = F64P_JW * warp + jj;
+        for (int jj = 0; jj < JW; ++jj) {
+          const int rj = HW ? jj : JW * warp + jj;
           const double2 b0 = sm.b[st][ks][rj][t ^ rj], b1 = sm.b[st][ks][rj][(t + 4) ^ rj];
           double z[4];
 #pragma unroll
@@ -525,14 +577,14 @@ __global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
             z[e] = fma(a[e].x, b.x, a[e].y * b.y);
           }
 #pragma unroll
-          for (int nt = 0; nt < NT; ++nt) dmma<8>(re[jj][nt], z, wf[nt]);
+          for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.re[jj][nt], z, wf[nt]);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const double2 b = e < 2 ? b0 : b1;
             z[e] = fma(a[e].y, b.x, -(a[e].x * b.y));
           }
 #pragma unroll
-          for (int nt = 0; nt < NT; ++nt) dmma<8>(im[jj][nt], z, wf[nt]);
+          for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.im[jj][nt], z, wf[nt]);
         }
       }
       __syncwarp();
@@ -540,16 +592,16 @@ __global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
     }
     if (!ok) break;
     if (slot < 0) {
-      f64p_store<NT>(prm, item, re, im);
+      f64p_store<NT, HW>(prm, item, acc);
     } else {
-      double2* pp = prm.part + ((int64_t)blockIdx.x * 2 + slot) * (F64P_JW * NT * 4 * F64_THREADS) + threadIdx.x;
+      double2* pp = prm.part + ((int64_t)blockIdx.x * 2 + slot) * F64PAcc<NT, HW>::ELEMS + threadIdx.x;
 #pragma unroll
-      for (int jj = 0; jj < F64P_JW; ++jj)
+      for (int jj = 0; jj < JW; ++jj)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
           for (int r = 0; r < 4; ++r)
-            pp[((jj * NT + nt) * 4 + r) * F64_THREADS] = make_double2(re[jj][nt][r], im[jj][nt][r]);
+            pp[((jj * NT + nt) * 4 + r) * F64_THREADS] = make_double2(acc.re[jj][nt][r], acc.im[jj][nt][r]);
     }
   }
   if (!ok && threadIdx.x == 0) {
@@ -562,7 +614,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64P_CTAS)
 // One CTA per boundary b between the ranges of CTAs b and b + 1 of the accumulation
 // (grid `ncta`): when it falls inside an item and is the first to do so, adds the item's
 // partial tiles in CTA order into the output.
-template <int NT>
+template <int NT, bool HW>
 __global__ void __launch_bounds__(F64_THREADS) chi0_fp64p_reduce_kernel(F64PParams prm, int ncta) {
   const int64_t tail = (prm.items - prm.whole) * (int64_t)prm.nchunk;
   const int c = blockIdx.x + 1;
@@ -572,32 +624,27 @@ __global__ void __launch_bounds__(F64_THREADS) chi0_fp64p_reduce_kernel(F64PPara
   if (u == t0 || u >= tail) return;
   const int64_t up = tail * (c - 1) / ncta;
   if (up > t0) return;   // an earlier boundary already lies inside this item
-  double re[F64P_JW][NT][4], im[F64P_JW][NT][4];
-#pragma unroll
-  for (int jj = 0; jj < F64P_JW; ++jj)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) re[jj][nt][r] = im[jj][nt][r] = 0.0;
+  F64PAcc<NT, HW> acc;
+  acc.zero();
   for (int k = c - 1; k < ncta; ++k) {
     const int64_t s = tail * k / ncta;
     if (s >= t1) break;
     if (tail * (k + 1) / ncta == s) continue;   // an empty range
     // the item is a CTA's first segment when its range starts inside it
     const int slot = s >= t0 ? 0 : 1;
-    const double2* pp = prm.part + ((int64_t)k * 2 + slot) * (F64P_JW * NT * 4 * F64_THREADS) + threadIdx.x;
+    const double2* pp = prm.part + ((int64_t)k * 2 + slot) * F64PAcc<NT, HW>::ELEMS + threadIdx.x;
 #pragma unroll
-    for (int jj = 0; jj < F64P_JW; ++jj)
+    for (int jj = 0; jj < F64PTile<HW>::JW; ++jj)
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const double2 v = pp[((jj * NT + nt) * 4 + r) * F64_THREADS];
-          re[jj][nt][r] += v.x;
-          im[jj][nt][r] += v.y;
+          acc.re[jj][nt][r] += v.x;
+          acc.im[jj][nt][r] += v.y;
         }
   }
-  f64p_store<NT>(prm, prm.whole + t, re, im);
+  f64p_store<NT, HW>(prm, prm.whole + t, acc);
 }
 
 // Tensor map of M as a 2-D FP64 array: pairs (re, im interleaved) contiguous,
@@ -655,53 +702,73 @@ static int f64_launch(const F64Call& q, int f0, int n, int* launches) {
   return 0;
 }
 
+template <bool HW>
 static size_t f64p_part_bytes(int num_sms, int nt) {
-  return sizeof(double2) * (size_t)F64P_CTAS * num_sms * 2 * F64P_JW * nt * 4 * F64_THREADS;
+  return sizeof(double2) * (size_t)F64PTile<HW>::CTAS * num_sms * 2 * F64PTile<HW>::JW * nt * 4 * F64_THREADS;
 }
 
+// The head and wings' second operand and outputs (HW): dcprod (ldd, 3) and head.
+struct F64Head {
+  const double2* dc;
+  int64_t ldd;
+  double2* head;
+};
+
 // K1p for `groups` groups of 8 NT frequencies from f0 (the last may be ragged).
-template <int NT>
-static int f64p_launch(const F64Call& q, int f0, int groups, int* launches) {
+template <int NT, bool HW>
+static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, int* launches) {
+  using Tile = F64PTile<HW>;
   F64PParams prm;
   prm.N = q.N;
   prm.nw = q.nw;
   prm.f0 = f0;
-  prm.ntile = f64p_tiles(q.N);
+  prm.ntile = HW ? (q.N + Tile::TI - 1) / Tile::TI + 1 : f64p_tiles(q.N);
   const int64_t nchunk = (q.P + F64_KC - 1) / F64_KC;
   if (nchunk > 0x7fffffff / (2 * F64_KC)) return -3;   // pair coordinates are 32-bit
   prm.nchunk = (int)nchunk;
   prm.items = (int64_t)prm.ntile * groups;
   prm.out = q.out;
+  prm.head = hw.head;
   prm.npack = (int64_t)q.N * (q.N + 1) / 2;
   prm.status = q.status;
   prm.timeout_ns = q.timeout_ns;
-  const int64_t slots = (int64_t)F64P_CTAS * q.num_sms;
-  const bool cut = q.part && q.part_bytes >= f64p_part_bytes(q.num_sms, NT) && prm.nchunk >= F64P_MINCHUNK &&
-                   prm.items % slots != 0;
+  const int64_t slots = (int64_t)Tile::CTAS * q.num_sms;
+  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<HW>(q.num_sms, NT) &&
+                   prm.nchunk >= F64P_MINCHUNK && prm.items % slots != 0;
   // fewer items than slots: as many CTAs as get half of the shortest cut axis each
   const int64_t fit = cut ? std::max(prm.items, prm.items * prm.nchunk / (F64P_MINCHUNK / 2)) : prm.items;
   const int grid = (int)std::min(slots, fit);
   prm.whole = cut ? prm.items / grid * grid : prm.items;
   prm.part = cut ? q.part : nullptr;
-  CUtensorMap mi, mj, mw;
-  int e = f64_map(&mi, q.M, q.ldc, q.P, q.N, F64P_TI);
-  if (!e) e = f64_map(&mj, q.M, q.ldc, q.P, q.N, F64P_TJ);
+  CUtensorMap mi, mj, mw, mh;
+  int e;
+  if (HW) {
+    e = f64_map(&mj, hw.dc, hw.ldd, q.P, 3, F64P_TJ);
+    if (!e) e = f64_map(&mh, hw.dc, hw.ldd, q.P, 3, Tile::TI);
+    if (!e && q.N > 0) e = f64_map(&mi, q.M, q.ldc, q.P, q.N, Tile::TI);
+    if (q.N == 0) mi = mh;
+  } else {
+    e = f64_map(&mi, q.M, q.ldc, q.P, q.N, Tile::TI);
+    if (!e) e = f64_map(&mj, q.M, q.ldc, q.P, q.N, F64P_TJ);
+    mh = mi;
+  }
   if (!e) {
-    const uint64_t dims[2] = {(uint64_t)q.ldw, (uint64_t)q.nw};
+    // pairs past the end of the weights read as zeros
+    const uint64_t dims[2] = {(uint64_t)q.P, (uint64_t)q.nw};
     const uint64_t strides[1] = {(uint64_t)q.ldw * 8};
     const uint32_t box[2] = {F64_KC, 8 * NT};
     e = encode_tmap(&mw, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, q.W, dims, strides, box,
                     CU_TENSOR_MAP_SWIZZLE_128B);
   }
   if (e) return e;
-  const size_t smem = sizeof(F64PSmem<NT>) + 1024;
-  if (cudaFuncSetAttribute(chi0_fp64p_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  const size_t smem = sizeof(F64PSmem<NT, HW>) + 1024;
+  if (cudaFuncSetAttribute(chi0_fp64p_kernel<NT, HW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return -2;
-  chi0_fp64p_kernel<NT><<<grid, F64_THREADS, smem, q.stream>>>(mi, mj, mw, prm);
+  chi0_fp64p_kernel<NT, HW><<<grid, F64_THREADS, smem, q.stream>>>(mi, mj, mw, mh, prm);
   ++*launches;
   if (prm.whole < prm.items && grid > 1) {
-    chi0_fp64p_reduce_kernel<NT><<<grid - 1, F64_THREADS, 0, q.stream>>>(prm, grid);
+    chi0_fp64p_reduce_kernel<NT, HW><<<grid - 1, F64_THREADS, 0, q.stream>>>(prm, grid);
     ++*launches;
   }
   return 0;
@@ -714,10 +781,10 @@ static int f64_run(const F64Call& q, int* launches) {
   int full = q.nw / 24, r = q.nw % 24;
   if (r > 16) ++full, r = 0;
   int e = 0;
-  if (full) e = f64p_launch<3>(q, 0, full, launches);
+  if (full) e = f64p_launch<3, false>(q, {}, 0, full, launches);
   const int f0 = 24 * full;
-  if (!e && r > 8) e = f64p_launch<2>(q, f0, 1, launches);
-  else if (!e && r > 4) e = f64p_launch<1>(q, f0, 1, launches);
+  if (!e && r > 8) e = f64p_launch<2, false>(q, {}, f0, 1, launches);
+  else if (!e && r > 4) e = f64p_launch<1, false>(q, {}, f0, 1, launches);
   else if (!e && r > 0) e = f64_launch(q, f0, r, launches);
   return e;
 }
@@ -726,7 +793,7 @@ static int f64_run(const F64Call& q, int* launches) {
 // the tiles of the last round are not cut.
 size_t fp64_part_bytes(const spx_ctx* ctx, int64_t P, int N, int nw) {
   if (P < (int64_t)F64P_MINCHUNK * F64_KC || N <= 0 || nw <= 4) return 0;
-  return f64p_part_bytes(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
+  return f64p_part_bytes<false>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
 }
 
 // Enqueues the FP64 accumulation over one slab of band pairs. W holds the weights of
@@ -746,7 +813,36 @@ int launch_chi0_fp64(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
   return check_cuda(ctx, cudaGetLastError(), "chi0_fp64 kernel launch");
 }
 
-// The same with explicit device resources instead of a context: used by the
+// Scratch for launch_headwings' partial tiles (0 when none are used), optional.
+size_t headwings_part_bytes(const spx_ctx* ctx, int64_t P, int nw) {
+  if (P < (int64_t)F64P_MINCHUNK * F64_KC || nw <= 0) return 0;
+  return f64p_part_bytes<true>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
+}
+
+// head(:, f) += sum_p dc(p, k1) conj(dc(p, k2)) w(p, f), wing(k2, i, f) += sum_p M(p, i)
+// conj(dc(p, k2)) w(p, f): M (ldc, dim), dc (ldd, 3), W (ldw, nw) with ldw even and W 16-byte
+// aligned. P < 2^30.
+int launch_headwings(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int dim,
+                     const double2* dc, int64_t ldd, const double* W, int64_t ldw, int nw,
+                     double2* head, double2* wing, void* part, size_t part_bytes,
+                     cudaStream_t stream) {
+  if (P <= 0 || nw <= 0) return SPX_OK;
+  const uint64_t timeout_ns =
+      (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
+  const F64Call q{ctx->num_sms, M, ldc, P, dim, W, ldw, nw, wing, (double2*)part, part_bytes,
+                  ctx->d_status, timeout_ns, stream};
+  const F64Head hw{dc, ldd, head};
+  int full = nw / 24, r = nw % 24, e = 0, launches = 0;
+  if (r > 16) ++full, r = 0;
+  if (full) e = f64p_launch<3, true>(q, hw, 0, full, &launches);
+  if (!e && r > 8) e = f64p_launch<2, true>(q, hw, 24 * full, 1, &launches);
+  else if (!e && r > 0) e = f64p_launch<1, true>(q, hw, 24 * full, 1, &launches);
+  if (e) return set_error(ctx, SPX_ECUDA, "head and wings: tensor map or attribute failed (" +
+                                              std::to_string(e) + ")");
+  return check_cuda(ctx, cudaGetLastError(), "head and wings launch");
+}
+
+// launch_chi0_fp64 with explicit device resources instead of a context: used by the
 // allocation-free entry point, whose status word and weights live in static
 // device memory.
 int launch_chi0_fp64_noctx(int num_sms, int* status, uint64_t timeout_ns, const double2* M,
