@@ -20,7 +20,7 @@
 //
 // K4c: C(m, col) += alpha * sum_k A(m, k) * conj(B(col, k)), A rows and B rows
 // K-contiguous (B possibly gathered), on the FP64 DMMA path (mma.sync
-// m16n8k8 f64): 64x64 complex tiles, four warps of 32x32, two-stage cp.async
+// m16n8k8 f64): 64x64 complex tiles, four warps of 32x32, three-stage cp.async
 // pipeline with zero fill at the edges, output rows m contiguous in cprod.
 #include <cuda_runtime.h>
 
@@ -40,7 +40,6 @@ namespace spx {
 
 constexpr int ZG_B = 64;             // tile edge (rows m and columns col)
 constexpr int ZG_KC = 16;            // K per pipeline stage
-constexpr int ZG_ROW = ZG_KC + 4;    // padded shared row, double2 units
 constexpr int ZG_THREADS = 128;
 
 // ZgParams: see spx_zgemm.h
@@ -66,148 +65,216 @@ __device__ __forceinline__ void dmma8(double (&d)[4], const double* a, const dou
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
+// Shared rows of 16 complex k (256 bytes); 16-byte chunk k of row r sits at
+// k ^ zg_swz(r): fragment reads (two rows x four k), row-wise and column-wise fills all
+// fall in distinct banks.
+constexpr int ZG_ST = 3;             // pipeline stages
+__device__ __forceinline__ int zg_swz(int r) { return ((r & 1) << 2) | ((r >> 1) & 3); }
+
 struct __align__(16) ZgSmem {
-  double2 a[2][ZG_B][ZG_ROW];
-  double2 b[2][ZG_B][ZG_ROW];
+  double2 a[ZG_ST][ZG_B][ZG_KC];
+  double2 b[ZG_ST][ZG_B][ZG_KC];
+  int64_t boff[8][ZG_THREADS];       // element offsets of the B rows a thread fills
 };
 
-__global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams prm) {
+struct ZgTile {
+  int m0, c0, b1, b2;
+};
+__device__ __forceinline__ ZgTile zg_tile(const ZgParams& prm, int64_t item, int64_t tiles) {
+  const int b = (int)(item / tiles), t = (int)(item - b * tiles);
+  int tm, tn;
+  if (prm.upper) {
+    int j = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while (j * (j + 1) / 2 > t) --j;
+    while ((j + 1) * (j + 2) / 2 <= t) ++j;
+    tn = j;
+    tm = t - j * (j + 1) / 2;
+  } else {
+    tm = t % prm.mtiles;
+    tn = t / prm.mtiles;
+  }
+  return {tm * ZG_B, tn * ZG_B, b % prm.nb1, b / prm.nb1};
+}
+
+// Two persistent CTAs per SM; each walks the tiles (batch by batch, rows fastest) and its
+// chunks of 16 k form one sequence over all its tiles, two chunks in flight, so a tile's
+// first chunks load while the previous tile's last ones compute and its output is written.
+// Bound: the FP64 pipe (DMMA). Fills are 256-byte runs along k, or along m for an
+// m-contiguous A (MC); GATHER reads B's k offsets through kOff. Measured against one CTA
+// per tile with a two-stage pipeline: 48000 x 1014 x 3000 gathered 38.5 -> 36.5 ms (0.86
+// of the DMMA rate), 48000 x 1100 x 1200 m-contiguous 16.8 -> 15.3 ms, K = 243 (muffin
+// tin) 1.9 -> 1.66 ms.
+template <bool MC, bool GATHER>
+__global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams prm, int64_t tiles,
+                                                                    int64_t items) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   ZgSmem& sm = *reinterpret_cast<ZgSmem*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x;
-  const int tm = tile % prm.mtiles, tn = tile / prm.mtiles;
-  const int b = blockIdx.y;
-  const int b1 = b % prm.nb1, b2 = b / prm.nb1;
-  const int m0 = tm * ZG_B, c0 = tn * ZG_B;
-  const int Kb = (prm.K_last > 0 && b == (int)gridDim.y - 1) ? prm.K_last : prm.K;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int nst = (prm.K + ZG_KC - 1) / ZG_KC;
 
-  // loader role: thread -> (row r, 8 consecutive k); rows of A are m, rows of B col
-  const int lr = threadIdx.x >> 1, lk = (threadIdx.x & 1) * 8;
-  const bool a_ok = m0 + lr < prm.M;
-  const int64_t a_mstride = prm.a_mcontig ? 1 : prm.lda, a_kstride = prm.a_mcontig ? prm.lda : 1;
-  const double2* a_row = prm.A + b1 * prm.sA1 + b2 * prm.sA2 + (int64_t)(a_ok ? m0 + lr : 0) * a_mstride;
-  const int col = c0 + lr;
-  const bool b_ok = col < prm.ncol;
-  const double2* b_row;
-  {
-    const int cc = b_ok ? col : 0;
-    const int n = cc / prm.ncin, c = cc - n * prm.ncin;
-    b_row = prm.B + b1 * prm.sB1 + b2 * prm.sB2 + (int64_t)n * prm.sBn +
-            (prm.cOff ? prm.cOff[c] : (int64_t)c * prm.sBc);
-  }
-  auto issue = [&](int st, int k0) {
+  // loader: one k and rows r0, r0 + 8, ... (MC: one row and k0, k0 + 2, ... for A)
+  const int lk = tid & 15, r0 = tid >> 4, mr = tid & 63, mk = tid >> 6;
+  int64_t l_item = blockIdx.x;
+  int l_chunk = 0, a_mask = 0, b_mask = 0, l_stage = 0;
+  const double2* pa = nullptr;
+  const double2* pb = nullptr;
+  auto enter = [&] {
+    const ZgTile q = zg_tile(prm, l_item, tiles);
+    const double2* ab = prm.A + q.b1 * prm.sA1 + q.b2 * prm.sA2;
+    pb = prm.B + q.b1 * prm.sB1 + q.b2 * prm.sB2;
+    a_mask = b_mask = 0;
+    if (MC) {
+      a_mask = q.m0 + mr < prm.M;
+      pa = ab + (a_mask ? q.m0 + mr : 0) + (int64_t)mk * prm.lda;
+    } else {
+      pa = ab + (int64_t)(q.m0 + r0) * prm.lda + lk;
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int k = k0 + lk + j;
-      const bool kin = k < Kb;
-      const int kk = kin ? k : 0;
-      cp_async16(&sm.a[st][lr][lk + j], a_row + kk * a_kstride, a_ok && kin);
-      const int64_t ko = prm.kOff ? (int64_t)__ldg(prm.kOff + kk) : (int64_t)kk;
-      cp_async16(&sm.b[st][lr][lk + j], b_ok && kin ? b_row + ko : prm.B, b_ok && kin);
+      if (!MC) a_mask |= (q.m0 + r0 + 8 * j < prm.M) << j;
+      const int col = q.c0 + r0 + 8 * j;
+      int64_t off = 0;
+      if (col < prm.ncol) {
+        b_mask |= 1 << j;
+        const int n = col / prm.ncin, c = col - n * prm.ncin;
+        off = (int64_t)n * prm.sBn + (prm.cOff ? prm.cOff[c] : (int64_t)c * prm.sBc);
+      }
+      sm.boff[j][tid] = off;
+    }
+  };
+  // copies of the next chunk of the sequence; an empty group past its end
+  auto issue = [&] {
+    if (l_item < items) {
+      if (l_chunk == 0) enter();
+      const int k0 = l_chunk * ZG_KC, k = k0 + lk;
+      const bool kin = k < prm.K;
+      const int64_t ko = GATHER ? (kin ? (int64_t)__ldg(prm.kOff + k) : 0) : (kin ? (int64_t)k : 0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (MC) {
+          const int kj = mk + 2 * j;
+          const bool v = a_mask && k0 + kj < prm.K;
+          cp_async16(&sm.a[l_stage][mr][kj ^ zg_swz(mr)], v ? pa + (int64_t)(k0 + 2 * j) * prm.lda : prm.A, v);
+        } else {
+          const bool v = kin && (a_mask >> j & 1);
+          cp_async16(&sm.a[l_stage][r0 + 8 * j][lk ^ zg_swz(r0 + 8 * j)],
+                     v ? pa + (int64_t)(8 * j) * prm.lda + k0 : prm.A, v);
+        }
+        const bool v = kin && (b_mask >> j & 1);
+        cp_async16(&sm.b[l_stage][r0 + 8 * j][lk ^ zg_swz(r0 + 8 * j)], v ? pb + sm.boff[j][tid] + ko : prm.B, v);
+      }
+      if (++l_chunk == nst) l_chunk = 0, l_item += gridDim.x;
     }
     cp_async_commit();
+    if (++l_stage == ZG_ST) l_stage = 0;
   };
-
-  const int nst = (Kb + ZG_KC - 1) / ZG_KC;
-  issue(0, 0);
+  issue();
+  issue();
 
   const int wi = warp & 1, wj = warp >> 1;
   const int g = lane >> 2, t = lane & 3;
-  double accR[2][4][4], accI[2][4][4];
+  int st = 0;
+  for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+    double accR[2][4][4], accI[2][4][4];
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) accR[mt][nt][r] = accI[mt][nt][r] = 0.0;
+    for (int s = 0; s < nst; ++s) {
+      cp_async_wait<1>();   // this thread's copies of the chunk have landed ...
+      __syncthreads();      // ... everyone's have, and the stage issued next has been read
+      issue();
+#pragma unroll
+      for (int ks = 0; ks < ZG_KC / 8; ++ks) {
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          double ar[4], ai[4];
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const double2 v = sm.a[st][32 * wi + 16 * mt + g + 8 * h][(ks * 8 + t + 4 * q) ^ zg_swz(g)];
+              ar[2 * q + h] = v.x;
+              ai[2 * q + h] = v.y;
+            }
+#pragma unroll
+          for (int np = 0; np < 2; ++np) {
+            double br[2][2], bim[2][2], bneg[2][2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                const double2 v = sm.b[st][32 * wj + 8 * (2 * np + h) + g][(ks * 8 + t + 4 * q) ^ zg_swz(g)];
+                br[h][q] = v.x;
+                bim[h][q] = v.y;
+                bneg[h][q] = -v.y;
+              }
+            // A conj(B): re += ar br + ai bi, im += ai br - ar bi
+            dmma8(accR[mt][2 * np], ar, br[0]);
+            dmma8(accR[mt][2 * np + 1], ar, br[1]);
+            dmma8(accI[mt][2 * np], ai, br[0]);
+            dmma8(accI[mt][2 * np + 1], ai, br[1]);
+            dmma8(accR[mt][2 * np], ai, bim[0]);
+            dmma8(accR[mt][2 * np + 1], ai, bim[1]);
+            dmma8(accI[mt][2 * np], ar, bneg[0]);
+            dmma8(accI[mt][2 * np + 1], ar, bneg[1]);
+          }
+        }
+      }
+      if (++st == ZG_ST) st = 0;
+    }
+
+    const ZgTile q = zg_tile(prm, item, tiles);
+    const double2 al = prm.alpha ? prm.alpha[q.b1] : prm.alpha_v;
+    double2* ob = prm.O + q.b1 * prm.sO1 + q.b2 * prm.sO2;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) accR[mt][nt][r] = accI[mt][nt][r] = 0.0;
-
-  for (int s = 0; s < nst; ++s) {
-    const int st = s & 1;
-    if (s + 1 < nst) {
-      issue(st ^ 1, (s + 1) * ZG_KC);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+      for (int e = 0; e < 2; ++e) {
+        const int cl = q.c0 + 32 * wj + 8 * nt + 2 * t + e;
+        if (cl >= prm.ncol) continue;
+        const int n = cl / prm.ncin, c = cl - n * prm.ncin;
+        double2* oc = ob + (int64_t)n * prm.sOn + (int64_t)c * prm.sOc;
+        double2 v[4];
 #pragma unroll
-    for (int ks = 0; ks < ZG_KC / 8; ++ks) {
+        for (int x = 0; x < 4; ++x) {
+          const int m = q.m0 + 32 * wi + 8 * x + g;
+          v[x] = make_double2(0.0, 0.0);
+          if (!prm.overwrite && m < prm.M) v[x] = oc[m];
+        }
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
-        double ar[4], ai[4];
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const double2 v = sm.a[st][32 * wi + 16 * mt + g + 8 * h][ks * 8 + t + 4 * q];
-            ar[2 * q + h] = v.x;
-            ai[2 * q + h] = v.y;
-          }
-#pragma unroll
-        for (int np = 0; np < 2; ++np) {
-          double br[2][2], bim[2][2], bneg[2][2];
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const double2 v = sm.b[st][32 * wj + 8 * (2 * np + h) + g][ks * 8 + t + 4 * q];
-              br[h][q] = v.x;
-              bim[h][q] = v.y;
-              bneg[h][q] = -v.y;
-            }
-          // A conj(B): re += ar br + ai bi, im += ai br - ar bi
-          dmma8(accR[mt][2 * np], ar, br[0]);
-          dmma8(accR[mt][2 * np + 1], ar, br[1]);
-          dmma8(accI[mt][2 * np], ai, br[0]);
-          dmma8(accI[mt][2 * np + 1], ai, br[1]);
-          dmma8(accR[mt][2 * np], ai, bim[0]);
-          dmma8(accR[mt][2 * np + 1], ai, bim[1]);
-          dmma8(accI[mt][2 * np], ar, bneg[0]);
-          dmma8(accI[mt][2 * np + 1], ar, bneg[1]);
+        for (int x = 0; x < 4; ++x) {
+          const int m = q.m0 + 32 * wi + 8 * x + g;
+          const double re = accR[x >> 1][nt][2 * (x & 1) + e], im = accI[x >> 1][nt][2 * (x & 1) + e];
+          v[x].x += al.x * re - al.y * im;
+          v[x].y += al.x * im + al.y * re;
+          if (m < prm.M) oc[m] = v[x];
         }
       }
-    }
-    __syncthreads();  // stage st is refilled by the next iteration's issue
   }
-
-  const double2 al = prm.alpha ? prm.alpha[b1] : prm.alpha_v;
-  double2* ob = prm.O + b1 * prm.sO1 + b2 * prm.sO2;
-#pragma unroll
-  for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int cl = c0 + 32 * wj + 8 * nt + 2 * t + e;
-      if (cl >= prm.ncol) continue;
-      const int n = cl / prm.ncin, c = cl - n * prm.ncin;
-      double2* oc = ob + (int64_t)n * prm.sOn + (int64_t)c * prm.sOc;
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int m = m0 + 32 * wi + 16 * mt + g + 8 * h;
-          if (m >= prm.M) continue;
-          const int r = 2 * h + e;
-          const double re = accR[mt][nt][r], im = accI[mt][nt][r];
-          double2 v = oc[m];
-          v.x += al.x * re - al.y * im;
-          v.y += al.x * im + al.y * re;
-          oc[m] = v;
-        }
-    }
+  cp_async_wait<0>();
 }
 
 int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s) {
   if (prm.M <= 0 || prm.ncol <= 0 || prm.K <= 0 || nbatch <= 0) return SPX_OK;
   prm.mtiles = (prm.M + ZG_B - 1) / ZG_B;
   prm.ntiles = (prm.ncol + ZG_B - 1) / ZG_B;
-  const int64_t tiles = (int64_t)prm.mtiles * prm.ntiles;
+  const int64_t tiles = prm.upper ? (int64_t)prm.ntiles * (prm.ntiles + 1) / 2 : (int64_t)prm.mtiles * prm.ntiles;
   if (tiles > 0x7fffffff || nbatch > 65535)
     return set_error(ctx, SPX_EINVAL, "product GEMM grid too large");
+  const int64_t items = tiles * nbatch;
   const size_t smem = sizeof(ZgSmem);
-  cudaFuncSetAttribute(zgemm_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 grid((unsigned)tiles, (unsigned)nbatch);
-  zgemm_gather_kernel<<<grid, ZG_THREADS, smem, s>>>(prm);
+  const int grid = (int)std::min<int64_t>(items, (int64_t)2 * ctx->num_sms);
+  auto run = [&](auto kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<grid, ZG_THREADS, smem, s>>>(prm, tiles, items);
+  };
+  if (prm.a_mcontig && prm.kOff) run(zgemm_gather_kernel<true, true>);
+  else if (prm.a_mcontig) run(zgemm_gather_kernel<true, false>);
+  else if (prm.kOff) run(zgemm_gather_kernel<false, true>);
+  else run(zgemm_gather_kernel<false, false>);
   return check_cuda(ctx, cudaGetLastError(), "zgemm_gather_kernel launch");
 }
 
@@ -762,10 +829,9 @@ static int trafo_run(spx_ctx* ctx, const double* cprod, int64_t ldc, int64_t npa
   prm.ncol = dim;
   prm.K = nbas;
   prm.nb1 = 1;
+  prm.overwrite = 1;
   if (out != cprod) {
-    if ((rc = check_cuda(ctx, cudaMemset2DAsync(out, 16 * ldo, 0, 16 * npair, dim, s), "zero out")))
-      return rc;
-    if (nbas == 0) return SPX_OK;
+    if (nbas == 0) return check_cuda(ctx, cudaMemset2DAsync(out, 16 * ldo, 0, 16 * npair, dim, s), "zero out");
     prm.A = reinterpret_cast<const double2*>(cprod);
     prm.O = reinterpret_cast<double2*>(out);
     prm.sOc = ldo;
@@ -779,7 +845,8 @@ static int trafo_run(spx_ctx* ctx, const double* cprod, int64_t ldc, int64_t npa
   double2* tmp = reinterpret_cast<double2*>((char*)ctx->ws + ws_off);
   for (int64_t r0 = 0; r0 < npair; r0 += chunk) {
     const int64_t len = std::min<int64_t>(chunk, npair - r0);
-    if ((rc = check_cuda(ctx, cudaMemsetAsync(tmp, 0, 16 * (size_t)len * dim, s), "zero chunk")))
+    if (nbas == 0 &&
+        (rc = check_cuda(ctx, cudaMemsetAsync(tmp, 0, 16 * (size_t)len * dim, s), "zero chunk")))
       return rc;
     if (nbas > 0) {
       prm.A = reinterpret_cast<const double2*>(cprod) + r0;
@@ -868,9 +935,6 @@ extern "C" int spx_trafo_olap_dev(spx_ctx* ctx, const double* cprod, int64_t ldc
                          "copy step function")) ||
         0)
       return rc;
-    if ((rc = check_cuda(ctx, cudaMemset2DAsync(T1 + nbasp, 16 * (size_t)nbas, 0, 16 * (size_t)ng, dim, s),
-                         "zero PW rows")))
-      return rc;
     olap_conj_kernel<<<std::min<int64_t>(((int64_t)ng * ng + 255) / 256, (int64_t)ctx->num_sms * 16), 256, 0, s>>>(
         G, ng, CS, sr, O);
     if ((rc = check_cuda(ctx, cudaGetLastError(), "olap_conj_kernel launch"))) return rc;
@@ -889,6 +953,7 @@ extern "C" int spx_trafo_olap_dev(spx_ctx* ctx, const double* cprod, int64_t ldc
     prm.ncol = dim;
     prm.K = ng;
     prm.nb1 = 1;
+    prm.overwrite = 1;
     if ((rc = launch_zgemm(ctx, prm, 1, s))) return rc;
     conj_rows_kernel<<<std::min<int64_t>(((int64_t)ng * dim + 255) / 256, (int64_t)ctx->num_sms * 16), 256, 0, s>>>(
         T1 + nbasp, nbas, ng, dim);
@@ -1172,8 +1237,7 @@ extern "C" int spx_dcprod_dev(spx_ctx* ctx, const spx_mom_desc* d, int32_t nk, i
     if ((rc = check_cuda(ctx, cudaMemcpyAsync(G, d->gpt, sizeof(int) * 3 * ng, cudaMemcpyHostToDevice, s), "copy G")) ||
         (rc = check_cuda(ctx, cudaMemcpyAsync(CS, d->cstep, 16 * (size_t)ns * ns * ns, cudaMemcpyHostToDevice, s), "copy cstep")) ||
         (rc = check_cuda(ctx, cudaMemcpyAsync(kc, kch.data(), sizeof(double) * 3 * nk, cudaMemcpyHostToDevice, s), "copy k")) ||
-        (rc = check_cuda(ctx, cudaStreamSynchronize(s), "copy k")) ||
-        (rc = check_cuda(ctx, cudaMemsetAsync(R, 0, sizeof(double2) * (size_t)ng * nkn, s), "zero R")))
+        (rc = check_cuda(ctx, cudaStreamSynchronize(s), "copy k")))
       return rc;
     olap_conj_kernel<<<std::min<int64_t>(((int64_t)ng * ng + 255) / 256, (int64_t)ctx->num_sms * 16), 256, 0, s>>>(
         G, ng, CS, sr, O);
@@ -1193,6 +1257,7 @@ extern "C" int spx_dcprod_dev(spx_ctx* ctx, const spx_mom_desc* d, int32_t nk, i
     p1.ncol = (int)nkn;
     p1.K = ng;
     p1.nb1 = 1;
+    p1.overwrite = 1;
     if ((rc = launch_zgemm(ctx, p1, 1, s))) return rc;
     Mat3 rl;
     for (int i = 0; i < 9; ++i) rl.r[i] = d->rlat[i];

@@ -26,7 +26,8 @@ struct ZgParams {
   const double2* alpha;  // per b1, or null: alpha_v
   double2 alpha_v;
   int M, ncol, ncin, K, nb1;
-  int K_last;  // K of the last batch when > 0 (split-K over batches)
+  int overwrite;  // 1: store, the output holds nothing yet; 0: add
+  int upper;      // 1: only the 64 x 64 tiles on and above the diagonal (M == ncol)
   int mtiles, ntiles;
 };
 
