@@ -37,6 +37,10 @@ int launch_chi0_fp64(spx_ctx*, const double2*, int64_t, int64_t, int, const doub
 size_t fp64_part_bytes(const spx_ctx*, int64_t P, int N, int nw);
 int split_chi0_slab(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
                     int, double2*, void*, size_t, cudaStream_t, int*, int variant, int slab);
+int split_chi0_ediff(spx_ctx*, const double2*, int64_t, int64_t, int, const double* ediff,
+                     const double* wscale, double scale_all, int nw, const double* omega, double2*,
+                     void*, size_t, cudaStream_t, int*, int variant, int slab);
+size_t split_part_bytes(int num_sms, bool real);
 size_t split_workspace_bytes(int64_t P, int N, int nw);
 size_t split_workspace_bytes(int64_t P, int N, int nw, int slab);
 size_t split_workspace_bytes_real(int64_t P, int N, int nw);
@@ -46,7 +50,8 @@ int pb_single(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, con
               int tile, int slab, char* scratch, size_t scratch_bytes, cudaStream_t s, int* launches);
 
 // The split variant and slab a call of this shape runs with: the context's forced
-// variant, else the tuning table's, else one CTA per 64 x 80 tile with 32768-pair slabs.
+// variant, else the tuning table's, else one CTA per tile (variant 0: the tile shape that
+// suits the width) with 32768-pair slabs.
 static void split_choice(spx_ctx* ctx, int N, int64_t P, int nw, int* variant, int* slab, int* tile) {
   *variant = ctx->opt.split_variant;
   *slab = 0;
@@ -79,8 +84,9 @@ static size_t split_scratch_bytes(spx_ctx* ctx, int64_t P, int N, int nw) {
   if (persistent) b = std::max(b, pb_single_bytes(P, N, nw, 32768));
   return b;
 }
-int split_chi0_real_slab(spx_ctx*, const double*, int64_t, int64_t, int, const double*, int64_t,
-                         int, double*, void*, size_t, cudaStream_t, int*);
+int split_chi0_real_ediff(spx_ctx*, const double*, int64_t, int64_t, int, const double* ediff,
+                          const double* wscale, double scale_all, int nw, const double* omega, double*,
+                          void*, size_t, cudaStream_t, int*);
 int launch_chi0_fp64_real(spx_ctx*, const double*, int64_t, int64_t, int, const double*, int64_t,
                           int, double*, cudaStream_t);
 
@@ -221,9 +227,14 @@ static int check_chi0_args(spx_ctx* ctx, const double* cprod, int64_t ldc, int64
   return SPX_OK;
 }
 
+// Optional scratch of an accumulation: the partial tiles of a cut last round.
+static size_t part_bytes_for(const spx_ctx* ctx, int64_t P, int N, int nw, int precision) {
+  return precision == SPX_FP64 ? fp64_part_bytes(ctx, P, N, nw) : split_part_bytes(ctx->num_sms, false);
+}
+
 // Accumulates one slab of band pairs already on the device into the device
-// output. `W` is workspace for npair*nw weights (ldw = round_up(npair, 16)); `split_ws`
-// the split path's scratch, or the FP64 path's partial tiles (optional).
+// output. `W` is workspace for the FP64 path's npair*nw weights (ldw = round_up(npair, 16));
+// `split_ws` the split path's scratch, or the FP64 path's partial tiles (optional).
 // `plan` (variant, slab, tile), when given, replaces the per-call choice: a caller
 // that streams one array in chunks keeps one kernel and one slab size for all of it.
 static int chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N,
@@ -233,10 +244,10 @@ static int chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
                      const int* plan = nullptr) {
   const int64_t ldw = (int64_t)align_up((size_t)std::max<int64_t>(P, 1), 16);
   timing_mark(ctx, s, 0);
-  int rc = launch_weights(ctx, P, ldw, ediff, wscale, scale_all, nw, omega, W, s);
-  if (rc) return rc;
-  ++*launches;
+  int rc;
   if (precision == SPX_FP64) {
+    if ((rc = launch_weights(ctx, P, ldw, ediff, wscale, scale_all, nw, omega, W, s))) return rc;
+    ++*launches;
     timing_mark(ctx, s, 1);
     rc = launch_chi0_fp64(ctx, M, ldc, P, N, W, ldw, nw, out, split_ws, split_ws_bytes, s, launches);
   } else {
@@ -251,9 +262,10 @@ static int chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
       rc = pb_single(ctx, M, ldc, P, N, ediff, wscale, scale_all, nw, omega, out, tile,
                      slab > 0 ? slab : 32768, (char*)split_ws, split_ws_bytes, s, launches);
     } else {
-      // the split path marks its own preparation / accumulation phases
-      rc = split_chi0_slab(ctx, M, ldc, P, N, W, ldw, nw, out, split_ws, split_ws_bytes, s,
-                           launches, variant == 3 ? 0 : variant, slab);
+      // the split path forms its weights beside its column scales and marks its own
+      // preparation / accumulation phases
+      rc = split_chi0_ediff(ctx, M, ldc, P, N, ediff, wscale, scale_all, nw, omega, out, split_ws,
+                            split_ws_bytes, s, launches, variant, slab);
     }
   }
   timing_mark(ctx, s, 2);
@@ -433,9 +445,9 @@ extern "C" int spx_chi0_accumulate_dev(spx_ctx* ctx, const double* cprod, int64_
   if (npair == 0 || nbas == 0 || nw == 0) return SPX_OK;
   cudaStream_t s = pick_stream(ctx, stream);
   const int64_t ldw = (int64_t)align_up((size_t)npair, 16);
-  size_t wbytes = align_up(sizeof(double) * (size_t)ldw * nw, 256);
+  size_t wbytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)ldw * nw, 256) : 0;
   size_t sbytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
-  size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, npair, nbas, nw) : 0;
+  size_t part = part_bytes_for(ctx, npair, nbas, nw, precision);
   if ((rc = ensure_workspace_opt(ctx, wbytes + sbytes, &part))) return rc;
   sbytes += part;
   double* W = (double*)ctx->ws;
@@ -478,14 +490,15 @@ extern "C" int spx_chi0_accumulate_real_dev(spx_ctx* ctx, const double* cprod, i
   if (npair == 0 || nbas == 0 || nw == 0) return SPX_OK;
   cudaStream_t s = pick_stream(ctx, stream);
   const int64_t ldw = (int64_t)align_up((size_t)npair, 16);
-  const size_t wbytes = align_up(sizeof(double) * (size_t)ldw * nw, 256);
-  const size_t sbytes = precision == SPX_SPLIT ? split_workspace_bytes_real(npair, nbas, nw) : 0;
+  const size_t wbytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)ldw * nw, 256) : 0;
+  size_t sbytes = precision == SPX_SPLIT ? split_workspace_bytes_real(npair, nbas, nw) : 0;
   // the FP64 kernel streams M with 2-D tensor copies: columns must start on 16 bytes,
   // otherwise M goes through an aligned copy first
   const bool realign = precision == SPX_FP64 && ((ldc & 1) || ((uintptr_t)cprod & 15));
   const int64_t ldm = realign ? (int64_t)align_up((size_t)npair, 2) : ldc;
   const size_t mbytes = realign ? align_up(sizeof(double) * (size_t)ldm * nbas, 256) : 0;
-  if ((rc = ensure_workspace(ctx, wbytes + sbytes + mbytes))) return rc;
+  size_t part = precision == SPX_SPLIT ? split_part_bytes(ctx->num_sms, true) : 0;
+  if ((rc = ensure_workspace_opt(ctx, wbytes + sbytes + mbytes, &part))) return rc;
   double* W = (double*)ctx->ws;
   void* sws = (char*)ctx->ws + wbytes;
   const double* M = cprod;
@@ -501,16 +514,17 @@ extern "C" int spx_chi0_accumulate_real_dev(spx_ctx* ctx, const double* cprod, i
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
   timing_mark(ctx, s, 0);
-  rc = launch_weights(ctx, npair, ldw, ediff, wscale, scale_all, nw, omega, W, s);
-  ++launches;
-  if (!rc) {
-    if (precision == SPX_FP64) {
+  if (precision == SPX_FP64) {
+    rc = launch_weights(ctx, npair, ldw, ediff, wscale, scale_all, nw, omega, W, s);
+    ++launches;
+    if (!rc) {
       timing_mark(ctx, s, 1);
       rc = launch_chi0_fp64_real(ctx, M, ldm, npair, nbas, W, ldw, nw, susceph, s);
       ++launches;
-    } else {
-      rc = split_chi0_real_slab(ctx, M, ldm, npair, nbas, W, ldw, nw, susceph, sws, sbytes, s, &launches);
     }
+  } else {
+    rc = split_chi0_real_ediff(ctx, M, ldm, npair, nbas, ediff, wscale, scale_all, nw, omega, susceph, sws,
+                               sbytes + part, s, &launches);
   }
   timing_mark(ctx, s, 2);
   ctx->timing = false;
@@ -584,10 +598,10 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
   const size_t slab_bytes = align_up(sizeof(double) * 2 * (size_t)slab * nbas, 256);
   const size_t e_bytes = align_up(sizeof(double) * (size_t)slab, 256);
   const size_t om_bytes = align_up(sizeof(double) * (size_t)nw, 256);
-  const size_t w_bytes = align_up(sizeof(double) * (size_t)slab * nw, 256);
+  const size_t w_bytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)slab * nw, 256) : 0;
   size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, slab, nbas, nw) : 0;
   size_t total = out_bytes + nslab_buf * (slab_bytes + 2 * e_bytes) + om_bytes + w_bytes + s_bytes;
-  size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, slab, nbas, nw) : 0;
+  size_t part = part_bytes_for(ctx, slab, nbas, nw, precision);
   if ((rc = ensure_workspace_opt(ctx, total, &part))) return rc;
   s_bytes += part;
   char* base = (char*)ctx->ws;
@@ -766,15 +780,15 @@ extern "C" int spx_chi0_from_coeffs_dev(spx_ctx* ctx, const spx_mt_desc* mt,
   const size_t prod_bytes = std::max(wfprod_mt_workspace(mt, nk, nocc),
                                      wfprod_pw_workspace(pw, nk, nocc, nunocc, split_products));
   const int64_t ldw = ldc;
-  const size_t w_bytes = align_up(sizeof(double) * (size_t)ldw * nw, 256);
+  const size_t w_bytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)ldw * nw, 256) : 0;
   size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
   size_t scratch = std::max(prod_bytes, w_bytes + s_bytes);
-  // the FP64 path's partial tiles follow the weights, in what the products leave free or beyond
-  const size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, npair, nbas, nw) : 0;
-  size_t beyond = w_bytes + part > scratch ? w_bytes + part - scratch : 0;
+  // partial tiles follow the accumulation's scratch, in what the products leave free or beyond
+  const size_t part = part_bytes_for(ctx, npair, nbas, nw, precision), acc = w_bytes + s_bytes + part;
+  size_t beyond = acc > scratch ? acc - scratch : 0;
   if ((rc = ensure_workspace_opt(ctx, m_bytes + scratch, &beyond))) return rc;
   scratch += beyond;
-  if (w_bytes + part <= scratch) s_bytes += part;
+  if (acc <= scratch) s_bytes += part;
   double2* M = (double2*)ctx->ws;
   char* sc = (char*)ctx->ws + m_bytes;
   int launches = 0;
@@ -830,7 +844,7 @@ extern "C" int spx_weights_hilbert_dev(spx_ctx* ctx, int64_t npair, int32_t nfrq
 // Adds sum_p M(p,i) conj(M(p,j)) w(p,f) with caller weights (any sign) into the
 // packed `out`, using `scratch` (accumulate_w_scratch bytes) for the padded weight
 // copy and the split path's planes.
-// FP64 calls may pass `part_bytes` of scratch beyond that for their partial tiles.
+// A caller may pass `part_bytes` of scratch beyond that for partial tiles.
 static size_t accumulate_w_scratch(int64_t npair, int nbas, int nw, int precision) {
   const int64_t ldi = (int64_t)align_up((size_t)npair, 16);
   return align_up(sizeof(double) * (size_t)ldi * nw, 256) +
@@ -860,7 +874,7 @@ static int accumulate_w_into(spx_ctx* ctx, const double* cprod, int64_t ldc, int
                             launches);
   }
   return split_chi0_slab(ctx, reinterpret_cast<const double2*>(cprod), ldc, npair, nbas, W, ldi, nw,
-                         reinterpret_cast<double2*>(out), sws, sbytes, s, launches, 0, 0);
+                         reinterpret_cast<double2*>(out), sws, sbytes + part_bytes, s, launches, 0, 0);
 }
 
 extern "C" int spx_chi0_accumulate_w_dev(spx_ctx* ctx, const double* cprod, int64_t ldc,
@@ -880,7 +894,7 @@ extern "C" int spx_chi0_accumulate_w_dev(spx_ctx* ctx, const double* cprod, int6
   }
   if (npair == 0 || nbas == 0 || nw == 0) return SPX_OK;
   cudaStream_t s = pick_stream(ctx, stream);
-  size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, npair, nbas, nw) : 0;
+  size_t part = part_bytes_for(ctx, npair, nbas, nw, precision);
   if ((rc = ensure_workspace_opt(ctx, accumulate_w_scratch(npair, nbas, nw, precision), &part))) return rc;
   int launches = 0;
   ctx->timing = stats != nullptr;
@@ -928,7 +942,7 @@ extern "C" int spx_chi0_accumulate_c_dev(spx_ctx* ctx, const double* cprod, int6
   const int64_t npack = (int64_t)nbas * (nbas + 1) / 2;
   const size_t pbytes = align_up(sizeof(double2) * (size_t)npack * nw, 256);
   const size_t sc = accumulate_w_scratch(npair, nbas, nw, precision);
-  size_t part = precision == SPX_FP64 ? fp64_part_bytes(ctx, npair, nbas, nw) : 0;
+  size_t part = part_bytes_for(ctx, npair, nbas, nw, precision);
   if ((rc = ensure_workspace_opt(ctx, 2 * pbytes + sc, &part))) return rc;
   double* S1 = (double*)ctx->ws;
   double* S2 = (double*)((char*)ctx->ws + pbytes);

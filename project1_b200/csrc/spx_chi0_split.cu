@@ -53,6 +53,7 @@ constexpr int SP_THREADS = 192;        // warp 0 TMA, warp 1 MMA + TMEM, warps 2
 constexpr int SP1_EPI = 8;
 constexpr int SP_WIDE_BN = 80;  // complex columns of the wide tile (variant 5): N = 160
 constexpr int SP1_THREADS = 64 + 32 * SP1_EPI;
+constexpr int SP_SMS = 148;   // SMs of the one GPU these kernels are built for
 constexpr int SP1_REGS = 128;  // 40960 registers: two 96-register quantizer blocks fit beside
 
 // BROWS: real rows of the B tile (the MMA's N): 128 for 64 x 64 complex tiles, 160
@@ -80,18 +81,101 @@ struct SplitParams {
   const int* wsgn;        // per frequency: +1 / -1 one-signed weights, 0 both signs
   double* out;            // packed complex output, as doubles
   int64_t npack;
+  int whole;              // items dealt whole (all of them without `part`)
+  double* part;           // partial tiles [CTA][2 slots][elements], or NULL
   int* status;
   uint64_t timeout_ns;
 };
+
+// The items of one CTA of the one-CTA kernels: whole items blockIdx.x, + gridDim.x, ...
+// below `whole`, then its share of the K stages of the items left over. Those would fill
+// a fraction of the SMs for a whole item's time; cut along K they take that fraction of
+// it. A partial sum is an exact integer (below 2^49 in magnitude), so adding the parts
+// before the scale gives the bits of an uncut item (split_gram_finish_kernel). Measured at
+// 403 columns, 12201 pairs, 12 frequencies (336 items on 148 SMs): 375 us uncut with
+// 64 x 80 tiles, 270 us cut with 64 x 64 and 9 us for the sum.
+struct SplitSeg {
+  int item, u, u1, n;
+  __device__ __forceinline__ SplitSeg(const SplitParams& p, int cta, int grid) {
+    item = cta;
+    const int64_t tail = (int64_t)(p.nitems - p.whole) * p.nk;   // < 2^31: fewer than `grid` items
+    u = (int)(tail * cta / grid);
+    u1 = (int)(tail * (cta + 1) / grid);
+    n = 0;
+  }
+  // Next item and its stages [k0, k1); slot -1: the whole item.
+  __device__ __forceinline__ bool next(const SplitParams& p, int grid, int* it, int* k0, int* k1, int* slot) {
+    if (item < p.whole) {
+      *it = item, *k0 = 0, *k1 = p.nk, *slot = -1;
+      item += grid;
+      return true;
+    }
+    if (u >= u1) return false;
+    const int t = u / p.nk;
+    *it = p.whole + t;
+    *k0 = u - t * p.nk;
+    const int e = min(u1 - t * p.nk, p.nk);
+    *k1 = e;
+    *slot = (*k0 == 0 && e == p.nk) ? -1 : (n > 0);
+    ++n;
+    u = t * p.nk + e;
+    return true;
+  }
+};
+
+// Doubles of one partial tile: 64 x BN complex values, or 128 x 2 BN real ones.
+__host__ __device__ constexpr int split_part_elems(bool real, int bn) { return (real ? 256 : 128) * bn; }
+
+// This epilogue thread's first value of its CTA's partial tile `slot`; the next ones follow
+// 32 SP1_EPI apart.
+template <bool REAL, int BN>
+__device__ __forceinline__ double* split_part_of(const SplitParams& prm, int slot) {
+  return prm.part + ((int64_t)blockIdx.x * 2 + slot) * split_part_elems(REAL, BN) + (threadIdx.x - 64);
+}
+
+// Adds a thread's folded values (row bi 64 + 16 q + lane / 2, part lane & 1, NC columns from
+// j0 of column block bj) into the packed output. One add per element per launch: launches
+// are stream-ordered, so the sum is deterministic, and the reduction needs no read
+// round trip.
+template <int NC, int BN>
+__device__ __forceinline__ void fold_add(int q, int lane, int bi, int bj, int f, const SplitParams& prm,
+                                         int j0, const double (&o)[NC]) {
+  const int gil = bi * SP_TILE + 16 * q + lane / 2;
+  if (gil >= prm.N) return;
+  const double fac = fold_row_factor(prm.wsgn[f], prm.sA[gil], prm.wmax[f]);
+  double* ob = prm.out + 2 * (int64_t)f * prm.npack + 2 * gil + (lane & 1);
+#pragma unroll
+  for (int jj = 0; jj < NC; ++jj) {
+    const int gj = bj * BN + j0 + jj;
+    if (gil <= gj && gj < prm.N) atomicAdd(ob + (int64_t)gj * (gj + 1), fac * prm.sA[gj] * o[jj]);
+  }
+}
+
+// Adds 16 columns (from j0 of column block bj) of a thread's row of real chi.
+template <int BROWS>
+__device__ __forceinline__ void real_add16(int q, int lane, int bi, int bj, int f, const SplitParams& prm,
+                                           int j0, const double (&T)[16]) {
+  const int gi = bi * SP_ROWS + 32 * q + lane;
+  if (gi >= prm.N) return;
+  const double fac = fold_row_factor(prm.wsgn[f], prm.sA[gi], prm.wmax[f]);
+  double* of = prm.out + (int64_t)f * prm.npack + gi;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const int gj = bj * BROWS + j0 + k;
+    if (gi <= gj && gj < prm.N) atomicAdd(of + (int64_t)gj * (gj + 1) / 2, fac * prm.sA[gj] * T[k]);
+  }
+}
 
 // The epilogue of one tile (or of NC of its 64 complex columns, from column j0), run
 // by the epilogue warps (warp q reads TMEM lanes 32q..32q+31, i.e. rows
 // i = 16q + lane/2, part c = lane & 1). The warp's part of the accumulator is read
 // into registers first and released to the MMA warp, so the next item's MMAs overlap
 // this tile's reductions into the output.
+// A partial item's values go to its slot of `part` instead.
 template <int NC = SP_TILE, int BN = SP_TILE, class Release>
 __device__ __forceinline__ void fold_epilogue(uint32_t tl, int q, int lane, int bi, int bj, int f,
-                                              const SplitParams& prm, Release release, int j0 = 0) {
+                                              const SplitParams& prm, Release release, int j0 = 0,
+                                              int slot = -1) {
   const int c = lane & 1;
   double o[NC];
 #pragma unroll
@@ -106,17 +190,13 @@ __device__ __forceinline__ void fold_epilogue(uint32_t tl, int q, int lane, int 
     }
   }
   release();
-  const int gil = bi * SP_TILE + 16 * q + lane / 2;
-  if (gil >= prm.N) return;
-  const double fac = fold_row_factor(prm.wsgn[f], prm.sA[gil], prm.wmax[f]);
-  double* ob = prm.out + 2 * (int64_t)f * prm.npack + 2 * gil + c;
+  if (slot >= 0) {
+    double* part = split_part_of<false, BN>(prm, slot);
 #pragma unroll
-  for (int jj = 0; jj < NC; ++jj) {
-    const int gj = bj * BN + j0 + jj;
-    // one add per element per launch: launches are stream-ordered, so the sum is
-    // deterministic, and the reduction needs no read round trip
-    if (gil <= gj && gj < prm.N) atomicAdd(ob + (int64_t)gj * (gj + 1), fac * prm.sA[gj] * o[jj]);
+    for (int jj = 0; jj < NC; ++jj) part[jj * (32 * SP1_EPI)] = o[jj];
+    return;
   }
+  fold_add<NC, BN>(q, lane, bi, bj, f, prm, j0, o);
 }
 
 // The -DINV (real) epilogue: columns [j0, j0 + ncol) of a 128 x BROWS tile of real chi,
@@ -125,19 +205,17 @@ __device__ __forceinline__ void fold_epilogue(uint32_t tl, int q, int lane, int 
 template <int BROWS, class Release>
 __device__ __forceinline__ void real_epilogue(uint32_t tl, int q, int lane, int bi, int bj, int f,
                                               const SplitParams& prm, Release release, int j0,
-                                              int ncol) {
-  const int gi = bi * SP_ROWS + 32 * q + lane;
-  const double fac = gi < prm.N ? fold_row_factor(prm.wsgn[f], prm.sA[gi], prm.wmax[f]) : 0.0;
-  double* of = prm.out + (int64_t)f * prm.npack + gi;
+                                              int ncol, int slot) {
 #pragma unroll 1
   for (int cc = 0; cc < ncol / 16; ++cc) {
     double T[16];
     load_fold16(tl + (uint32_t)(j0 + 16 * cc), (uint32_t)BROWS, T);
+    if (slot >= 0) {
+      double* part = split_part_of<true, BROWS / 2>(prm, slot);
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int gj = bj * BROWS + j0 + 16 * cc + k;
-      if (gi < prm.N && gi <= gj && gj < prm.N)
-        atomicAdd(of + (int64_t)gj * (gj + 1) / 2, fac * prm.sA[gj] * T[k]);
+      for (int k = 0; k < 16; ++k) part[(16 * cc + k) * (32 * SP1_EPI)] = T[k];
+    } else {
+      real_add16<BROWS>(q, lane, bi, bj, f, prm, j0 + 16 * cc, T);
     }
   }
   release();
@@ -184,8 +262,9 @@ __global__ void __maxnreg__(SP1_REGS)
       uint32_t last_ph[SP_ST];
       for (int s = 0; s < SP_ST; ++s) issued[s] = false, last_ph[s] = 0;
       bool ok = true;
-      int j = 0;
-      for (int item = blockIdx.x; item < prm.nitems && ok; item += gridDim.x, ++j) {
+      int item, k0, k1, slot;
+      SplitSeg seg(prm, blockIdx.x, gridDim.x);
+      for (int j = 0; ok && seg.next(prm, gridDim.x, &item, &k0, &k1, &slot); ++j) {
         const int f = item / prm.ntile;
         int bi, bj;
         split_decode_tile_bn<BN>(split_item_tile(item, prm.ntile, gridDim.x), prm.nbr, &bi, &bj);
@@ -193,12 +272,13 @@ __global__ void __maxnreg__(SP1_REGS)
         // a diagonal square tile of a one-signed frequency multiplies A by itself
         const bool same = BN == SP_TILE && sg != 0 && bi == bj;
         const int za = f * SP_SLOT, zb = za + (sg == 0 ? SP_SF : 0);
-        for (int ks = 0; ks < prm.nk; ++ks) {
+        for (int ks = k0; ks < k1; ++ks) {
           if (!mbar_wait(&sm.empty[st], ph ^ 1u, prm.timeout_ns, prm.status)) {
             ok = false;
             break;
           }
-          const int kc = split_k_order(j, ks, prm.nk);
+          // a cut item's stages run forwards in every CTA that has some of them
+          const int kc = slot < 0 ? split_k_order(j, ks, prm.nk) : ks;
           mbar_arrive_expect_tx(&sm.full[st], (uint32_t)(SP_SF * (SP_PLANE + (same ? 0 : BROWS * SP_KB))));
           tma_load_4d(&sm.a[st][0][0], &mapF, 0, bi * SP_ROWS, kc, za, &sm.full[st]);
           if (!same) tma_load_4d(&sm.b[st][0][0], &mapB, 0, bj * BROWS, kc, zb, &sm.full[st]);
@@ -216,9 +296,10 @@ __global__ void __maxnreg__(SP1_REGS)
     if (lane == 0) {
       int st = 0;
       uint32_t ph = 0;
-      int j = 0;
       bool committed = false;
-      for (int item = blockIdx.x; item < prm.nitems; item += gridDim.x, ++j) {
+      int item, k0, k1, slot;
+      SplitSeg seg(prm, blockIdx.x, gridDim.x);
+      for (int j = 0; seg.next(prm, gridDim.x, &item, &k0, &k1, &slot); ++j) {
         const int f = item / prm.ntile;
         int bi, bj;
         split_decode_tile_bn<BN>(split_item_tile(item, prm.ntile, gridDim.x), prm.nbr, &bi, &bj);
@@ -227,14 +308,14 @@ __global__ void __maxnreg__(SP1_REGS)
         if (!mbar_wait(&sm.tempty, (uint32_t)(j & 1) ^ 1u, prm.timeout_ns, prm.status)) break;
         tc_fence_after();
         bool ok = true;
-        for (int ks = 0; ks < prm.nk; ++ks) {
+        for (int ks = k0; ks < k1; ++ks) {
           if (!mbar_wait(&sm.full[st], ph, prm.timeout_ns, prm.status)) {
             ok = false;
             break;
           }
           tc_fence_after();
           // order g = t + u lives at TMEM columns [BROWS g, BROWS g + BROWS); the
-          // first product of every order in a slab (first K step) overwrites it
+          // first product of every order in an item (first K step) overwrites it
 #pragma unroll
           for (int kk = 0; kk < SP_NKS; ++kk) {
             uint64_t da[SP_SF], db[SP_SF];
@@ -243,10 +324,10 @@ __global__ void __maxnreg__(SP1_REGS)
               da[t] = desc_sw64(&sm.a[st][t][0]) + (uint64_t)(kk * 2);
               db[t] = same ? da[t] : desc_sw64(&sm.b[st][t][0]) + (uint64_t)(kk * 2);
             }
-            const uint32_t k0 = (ks > 0 || kk > 0);
-            mma_i8<1>(tmem + 0 * BROWS, da[0], db[0], IDESC, k0);
-            mma_i8<2>(tmem + 1 * BROWS, da[0], db[1], IDESC, k0);
-            mma_i8<3>(tmem + 2 * BROWS, da[0], db[2], IDESC, k0);
+            const uint32_t kacc = (ks > k0 || kk > 0);
+            mma_i8<1>(tmem + 0 * BROWS, da[0], db[0], IDESC, kacc);
+            mma_i8<2>(tmem + 1 * BROWS, da[0], db[1], IDESC, kacc);
+            mma_i8<3>(tmem + 2 * BROWS, da[0], db[2], IDESC, kacc);
             mma_i8<1>(tmem + 1 * BROWS, da[1], db[0], IDESC, 1u);
             mma_i8<3>(tmem + 2 * BROWS, da[1], db[1], IDESC, 1u);
             mma_i8<0>(tmem + 2 * BROWS, da[2], db[0], IDESC, 1u);
@@ -269,8 +350,9 @@ __global__ void __maxnreg__(SP1_REGS)
     // ---- epilogue: SP1_EPI warps, SP1_EPI / 4 per TMEM lane quarter (column ranges) ----
     const int q = warp & 3, h = (warp - 2) >> 2;
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
-    int j = 0;
-    for (int item = blockIdx.x; item < prm.nitems; item += gridDim.x, ++j) {
+    int item, k0, k1, slot;
+    SplitSeg seg(prm, blockIdx.x, gridDim.x);
+    for (int j = 0; seg.next(prm, gridDim.x, &item, &k0, &k1, &slot); ++j) {
       if (!mbar_wait_idle(&sm.tfull, (uint32_t)(j & 1), prm.timeout_ns, prm.status)) break;
       tc_fence_after();
       const int f = item / prm.ntile;
@@ -282,8 +364,8 @@ __global__ void __maxnreg__(SP1_REGS)
         if (lane == 0) mbar_arrive(&sm.tempty);
       };
       constexpr int NC = BN * 4 / SP1_EPI;  // complex columns per epilogue warp
-      if constexpr (REAL) real_epilogue<BROWS>(tl, q, lane, bi, bj, f, prm, release, 2 * NC * h, 2 * NC);
-      else fold_epilogue<NC, BN>(tl, q, lane, bi, bj, f, prm, release, NC * h);
+      if constexpr (REAL) real_epilogue<BROWS>(tl, q, lane, bi, bj, f, prm, release, 2 * NC * h, 2 * NC, slot);
+      else fold_epilogue<NC, BN>(tl, q, lane, bi, bj, f, prm, release, NC * h, slot);
     }
   }
 
@@ -291,6 +373,53 @@ __global__ void __maxnreg__(SP1_REGS)
   __syncthreads();
   tc_fence_after();
   if (warp == 1) tmem_dealloc(tmem, SP_TMEM_COLS);
+}
+
+// One CTA per boundary between the stage ranges of CTAs c - 1 and c (grid.x = CTAs of the
+// accumulation - 1) and 16 or 8 columns of a thread's share (grid.y): the first boundary
+// inside an item adds the item's partial tiles (exact) in CTA order, then the scaled
+// sum into the output as the uncut epilogue does.
+template <bool REAL>
+constexpr int split_finish_step() { return REAL ? 16 : 8; }
+template <bool REAL, int BN>
+__global__ void __launch_bounds__(32 * SP1_EPI) split_gram_finish_kernel(SplitParams prm, int ncta) {
+  const int64_t tail = (int64_t)(prm.nitems - prm.whole) * prm.nk;
+  const int c = blockIdx.x + 1;
+  const int64_t u = tail * c / ncta;
+  const int64_t t0 = u / prm.nk * prm.nk, t1 = t0 + prm.nk;
+  if (u == t0 || u >= tail || tail * (c - 1) / ncta > t0) return;
+  const int item = prm.whole + (int)(t0 / prm.nk);
+  const int f = item / prm.ntile;
+  int bi, bj;
+  split_decode_tile_bn<BN>(split_item_tile(item, prm.ntile, ncta), prm.nbr, &bi, &bj);
+  const int warp = (threadIdx.x >> 5) + 2, lane = threadIdx.x & 31;   // the epilogue's warp numbers
+  const int q = warp & 3, h = (warp - 2) >> 2;
+  constexpr int NC = BN * 4 / SP1_EPI, STEP = split_finish_step<REAL>();
+  const int v0 = blockIdx.y * STEP;
+  double o[STEP];
+#pragma unroll
+  for (int v = 0; v < STEP; ++v) o[v] = 0.0;
+  for (int k = c - 1; k < ncta; ++k) {
+    const int64_t s = tail * k / ncta;
+    if (s >= t1) break;
+    if (tail * (k + 1) / ncta == s) continue;   // an empty range
+    // the item is a CTA's first segment when its range starts inside it
+    const double* pp = prm.part + ((int64_t)k * 2 + (s >= t0 ? 0 : 1)) * split_part_elems(REAL, BN) +
+                       (int64_t)v0 * (32 * SP1_EPI) + threadIdx.x;
+#pragma unroll
+    for (int v = 0; v < STEP; ++v) o[v] += pp[v * (32 * SP1_EPI)];
+  }
+  if constexpr (REAL) real_add16<2 * BN>(q, lane, bi, bj, f, prm, 2 * NC * h + v0, o);
+  else fold_add<STEP, BN>(q, lane, bi, bj, f, prm, NC * h + v0, o);
+}
+
+// Whether cutting the last items of `nitems` pays: it saves this many of the last round's
+// `nk` stages (0.55-0.6 us each) and costs the partial tiles' way through memory and one
+// short launch: 20 us with complex tiles (403 columns, 12 frequencies: 40 of 336 items
+// left), 40 us with the twice as large real ones.
+static bool split_cuts(int nitems, int nk, int num_sms, bool real) {
+  const int left = nitems % num_sms;
+  return left > 0 && nk - (int64_t)left * nk / num_sms >= (real ? 128 : 64);
 }
 
 // ---------------------------------------------------------------------------
@@ -499,79 +628,99 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
 // ---------------------------------------------------------------------------
 // operand preparation
 
-// Column scales of one slab: sA[i] = max_p max(|Re M(p,i)|, |Im M(p,i)|).
-__global__ void split_colmax_kernel(const double2* __restrict__ M, int64_t ldc, int64_t p0,
-                                    int len, double* __restrict__ sA) {
-  const int i = blockIdx.x;
-  const double2* col = M + (int64_t)i * ldc + p0;
-  double m = 0.0;
-  for (int p = threadIdx.x; p < len; p += blockDim.x) {
-    const double2 v = col[p];
-    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
-  }
+// Maximum over the CTA of a non-negative value, for every thread.
+__device__ __forceinline__ double block_max(double m, double* red) {
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __shared__ double red[32];
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0) sA[i] = m;
-  }
+  m = red[0];
+  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
+  return m;
 }
 
-// Per frequency f over the slab: wmax[f] = max_p |w(p, f)|, the sign code wsgn[f]
-// (+1 all weights >= 0, -1 all <= 0, 0 both signs), and the folded factors
-// G[f][p] = sgn(w) sqrt(|w| / wmax) * 127 * 2^16 (0 past the slab's end).
-__global__ void split_wstat_kernel(const double* __restrict__ W, int64_t ldw, int64_t p0, int len,
-                                   int lenp, double* __restrict__ wmax, int* __restrict__ wsgn,
-                                   double* __restrict__ G) {
-  const int f = blockIdx.x;
-  const double* wf = W + (int64_t)f * ldw + p0;
+// Statistics of one slab, one launch of clusters of SPS_CL CTAs:
+//   * the first `ncol` CTAs (N rounded up to whole clusters): the column scales
+//     sA[i] = max_p max(|Re M(p,i)|, |Im M(p,i)|), one column each;
+//   * then one cluster per frequency f: wmax[f] = max_p |w(p, f)|, the sign code wsgn[f]
+//     (+1 all weights >= 0, -1 all <= 0, 0 both signs), and the folded factors
+//     G[f][p] = sgn(w) sqrt(|w| / wmax) * 127 * 2^16 (0 past the slab's end), each CTA an
+//     eighth of the slab, the maximum and signs shared through the cluster's shared memory.
+// The factors cost a division and a square root each, and a frequency's were one CTA's
+// work: 102 us for 32768 pairs x 24 frequencies, on the critical path before the first
+// accumulation. With ediff the weights are formed here (HILBERT NONE), else read from W.
+// Measured at 403 columns, 12201 pairs, 12 frequencies: 18 us, against 70 us in three
+// launches (weights, column scales, frequency statistics).
+constexpr int SPS_CL = 8, SPS_THREADS = 256;
+struct SplitStat {
+  const double* W;       // caller's weights (ldw, nw), or NULL:
+  int64_t ldw;
+  const double* ediff;   // HILBERT NONE weights of these energy differences
+  const double* wscale;
+  double scale_all;
+  const double* omega;
+};
+template <bool REAL>
+__global__ void __launch_bounds__(SPS_THREADS) __cluster_dims__(SPS_CL, 1, 1)
+    split_stat_kernel(const double* __restrict__ M, int64_t ldc, int64_t p0, int len, int lenp, int N,
+                      int ncol, SplitStat src, double* __restrict__ sA, double* __restrict__ wmax,
+                      int* __restrict__ wsgn, double* __restrict__ G) {
+  __shared__ double red[SPS_THREADS / 32];
+  __shared__ double share_m;
+  __shared__ int share_s;
+  if ((int)blockIdx.x < ncol) {
+    const int i = blockIdx.x;
+    if (i >= N) return;   // whole clusters take this branch, and none of it synchronises them
+    double m = 0.0;
+    if constexpr (REAL) {
+      const double* col = M + (int64_t)i * ldc + p0;
+#pragma unroll 4
+      for (int p = threadIdx.x; p < len; p += SPS_THREADS) m = fmax(m, fabs(__ldg(col + p)));
+    } else {
+      const double2* col = reinterpret_cast<const double2*>(M) + (int64_t)i * ldc + p0;
+#pragma unroll 4
+      for (int p = threadIdx.x; p < len; p += SPS_THREADS) {
+        const double2 v = __ldg(col + p);
+        m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+      }
+    }
+    m = block_max(m, red);
+    if (threadIdx.x == 0) sA[i] = m;
+    return;
+  }
+  const int f = ((int)blockIdx.x - ncol) / SPS_CL, r = ((int)blockIdx.x - ncol) % SPS_CL;
+  const double om = src.W ? 0.0 : src.omega[f];
+  auto weight = [&](int p) {
+    if (src.W) return src.W[(int64_t)f * src.ldw + p0 + p];
+    return hilbert_none_weight(src.ediff[p0 + p], om, (src.wscale ? src.wscale[p0 + p] : 1.0) * src.scale_all);
+  };
+  // the CTA's pairs, in whole 64-pair blocks of the slab
+  const int nb = lenp / SP_KB, a = (int)((int64_t)nb * r / SPS_CL) * SP_KB,
+            e = (int)((int64_t)nb * (r + 1) / SPS_CL) * SP_KB;
   double m = 0.0;
-  int pos = 0, neg = 0;
-  for (int p = threadIdx.x; p < len; p += blockDim.x) {
-    const double w = wf[p];
+  int sg = 0;   // bit 0: a positive weight, bit 1: a negative one
+  for (int p = a + threadIdx.x; p < min(e, len); p += SPS_THREADS) {
+    const double w = weight(p);
     m = fmax(m, fabs(w));
-    pos |= w > 0.0;
-    neg |= w < 0.0;
+    sg |= (w > 0.0 ? 1 : 0) | (w < 0.0 ? 2 : 0);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    pos |= __shfl_xor_sync(0xffffffffu, pos, o);
-    neg |= __shfl_xor_sync(0xffffffffu, neg, o);
+  m = block_max(m, red);
+  sg = __syncthreads_or(sg & 1) | (__syncthreads_or(sg & 2) ? 2 : 0);
+  if (threadIdx.x == 0) share_m = m, share_s = sg;
+  cluster_sync();
+  double wm = 0.0;
+  sg = 0;
+#pragma unroll
+  for (int k = 0; k < SPS_CL; ++k) {
+    wm = fmax(wm, ld_cluster_f64(&share_m, k));
+    sg |= ld_cluster_s32(&share_s, k);
   }
-  __shared__ double red[32];
-  __shared__ int rpos[32], rneg[32];
-  __shared__ double wm_s;
-  if ((threadIdx.x & 31) == 0) {
-    red[threadIdx.x >> 5] = m;
-    rpos[threadIdx.x >> 5] = pos;
-    rneg[threadIdx.x >> 5] = neg;
+  if (r == 0 && threadIdx.x == 0) {
+    wmax[f] = wm;
+    wsgn[f] = sg == 3 ? 0 : (sg == 2 ? -1 : 1);
   }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const bool v = threadIdx.x < (blockDim.x >> 5);
-    m = v ? red[threadIdx.x] : 0.0;
-    pos = v ? rpos[threadIdx.x] : 0;
-    neg = v ? rneg[threadIdx.x] : 0;
-    for (int o = 16; o > 0; o >>= 1) {
-      m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-      pos |= __shfl_xor_sync(0xffffffffu, pos, o);
-      neg |= __shfl_xor_sync(0xffffffffu, neg, o);
-    }
-    if (threadIdx.x == 0) {
-      wmax[f] = m;
-      wsgn[f] = (pos && neg) ? 0 : (neg ? -1 : 1);
-      wm_s = m;
-    }
-  }
-  __syncthreads();
-  const double wm = wm_s;
   double* gf = G + (int64_t)f * lenp;
-  for (int p = threadIdx.x; p < lenp; p += blockDim.x) {
-    gf[p] = p < len ? fold_factor(wf[p], wm) : 0.0;
-  }
+  for (int p = a + threadIdx.x; p < e; p += SPS_THREADS) gf[p] = p < len ? fold_factor(weight(p), wm) : 0.0;
+  cluster_sync();   // no CTA leaves while another may still read its maximum
 }
 
 // One thread = one complex column i and 8 consecutive pairs of the slab. Digit
@@ -584,14 +733,18 @@ __global__ void split_wstat_kernel(const double* __restrict__ W, int64_t ldw, in
 // when the frequency's weights have both signs, planes f*6 + 3 + t those of
 // round(x G / s). A block is 16 columns x one 64-pair k-block; the block stages the
 // folded factors of its 64 pairs (SPQ_FCH frequencies at a time) in shared memory,
-// so the frequency loop waits on no L2 round trip. The kernel is bound by the HBM
+// so the frequency loop waits on no L2 round trip. 24 frequencies are 12 KB, which does not
+// fit on an SM beside an accumulation CTA (217 KB with 64 x 80 tiles): the next part's
+// planes are written where the accumulation's last round leaves SMs idle, and after it.
+// Side by side on every SM (8 frequencies at a time) both got slower: real form, 900
+// columns, 8192 pairs, 712 us for both against 420 + 139 us one after the other. The kernel is bound by the HBM
 // writes of the planes; 96 registers keep five blocks per SM.
 constexpr int SPQ_FCH = 24;
 __global__ void __maxnreg__(96)
     split_quantize_kernel(const double2* __restrict__ M, int64_t ldc, int64_t p0, int len,
                           int nchunk, int N, int npad, int64_t R, int64_t Ps, int nw,
                           const double* __restrict__ sA, const int* __restrict__ wsgn,
-                          const double* __restrict__ G, int8_t* __restrict__ F) {
+                          const double* __restrict__ G, int ldg, int8_t* __restrict__ F) {
   __shared__ __align__(16) double gs[SPQ_FCH][SP_KB];
   __shared__ int ss[SPQ_FCH];
   // thread -> (k-block, column group of 4, eighth of the k-block, column in group); the
@@ -604,7 +757,6 @@ __global__ void __maxnreg__(96)
   const int i = (int)(rest % ngroup) * 4 + lane4;
   const int64_t kb = ((blockIdx.x * (int64_t)blockDim.x) >> 5) / ngroup;  // the block's k-block
   const int p = (int)(kb * SP_KB) + eighth * 8;
-  const int lenp = nchunk * 16;
   const int64_t nkb = Ps / SP_KB;
   // planes are nkb * R * 64 bytes apart
   const int64_t pstride = nkb * R * SP_KB;
@@ -631,7 +783,7 @@ __global__ void __maxnreg__(96)
       const int f = e / (SP_KB / 2), c = e - f * (SP_KB / 2);
       const int ce = c >> 2, cj = c & 3;
       reinterpret_cast<double2*>(&gs[f][0])[4 * ce + (cj ^ ((ce >> 1) & 3))] =
-          __ldg(reinterpret_cast<const double2*>(G + (int64_t)(f0 + f) * lenp + kb * SP_KB) + c);
+          __ldg(reinterpret_cast<const double2*>(G + (int64_t)(f0 + f) * ldg + kb * SP_KB) + c);
     }
     for (int f = threadIdx.x; f < nf; f += blockDim.x) ss[f] = wsgn[f0 + f];
     __syncthreads();
@@ -686,42 +838,80 @@ __global__ void __maxnreg__(96)
   }
 }
 
-// -DINV (real M): column scales and digit planes with one plane row per column
-// (rows 128 b .. 128 b + 127 hold the columns of 128-block b).
-__global__ void split_colmax_real_kernel(const double* __restrict__ M, int64_t ldc, int64_t p0,
-                                         int len, double* __restrict__ sA) {
-  const int i = blockIdx.x;
-  const double* col = M + (int64_t)i * ldc + p0;
-  double m = 0.0;
-  for (int p = threadIdx.x; p < len; p += blockDim.x) m = fmax(m, fabs(col[p]));
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __shared__ double red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0) sA[i] = m;
-  }
-}
-
-__global__ void __launch_bounds__(128, 4)
+// -DINV (real M): digit planes with one plane row per column (rows 128 b .. 128 b + 127
+// hold the columns of 128-block b). A thread is one column and 16 pairs, a warp 8 columns
+// x the four quarters of a 64-pair block, a block 32 columns; the factors of the block's
+// 64 pairs are staged in shared memory as in the complex form (16-byte chunk c = 8 q + j
+// of quarter q at 8 q + (j ^ 2 q): the quarters a warp reads at once fall in distinct
+// banks). Bound by the planes' writes: 900 columns, 32768 pairs, 24 frequencies 826 ->
+// 525 us (4.8 TB/s).
+__global__ void __launch_bounds__(128, 5)
     split_quantize_real_kernel(const double* __restrict__ M, int64_t ldc, int64_t p0, int len,
                                int nchunk, int N, int npad, int64_t R, int64_t Ps, int nw,
                                const double* __restrict__ sA, const int* __restrict__ wsgn,
-                               const double* __restrict__ G, int8_t* __restrict__ F) {
-  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (tid >= (int64_t)npad * nchunk) return;
-  const int ngroup = npad / 8;
-  const int lane8 = (int)(tid & 7), quarter = (int)((tid >> 3) & 3);
-  const int64_t rest = tid >> 5;
-  const int i = (int)(rest % ngroup) * 8 + lane8;
-  const int64_t kb = rest / ngroup;
+                               const double* __restrict__ G, int ldg, int8_t* __restrict__ F) {
+  __shared__ __align__(16) double gs[SPQ_FCH][SP_KB];
+  __shared__ int ss[SPQ_FCH];
+  const int ngroup = npad / 8;   // a multiple of 16, so a block's 4 warps share the k-block
+  const int64_t warp0 = blockIdx.x * 4ll;
+  const int64_t kb = warp0 / ngroup;
+  const int lane8 = threadIdx.x & 7, quarter = (threadIdx.x >> 3) & 3;
+  const int i = (int)((warp0 + (threadIdx.x >> 5)) % ngroup) * 8 + lane8;
   const int p = (int)(kb * SP_KB) + quarter * 16;
-  const int64_t pstride = (Ps / SP_KB) * R * SP_KB;
+  const int64_t pstride = (Ps / SP_KB) * R * SP_KB, o = (kb * R + i) * SP_KB + quarter * 16;
   const bool col_ok = i < N;
-  quantize_task_real(M + (int64_t)(col_ok ? i : 0) * ldc + p0, col_ok, len, p, col_ok ? sA[i] : 0.0,
-                     (kb * R + i) * SP_KB + quarter * 16, pstride, nw, wsgn, G, nchunk * 16, F);
+  const double* col = M + (int64_t)(col_ok ? i : 0) * ldc + p0;
+  double x[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) x[k] = (col_ok && p + k < len) ? __ldg(col + p + k) : 0.0;
+  const double s = col_ok ? sA[i] : 0.0;
+  const double inv = s > 0.0 ? 1.0 / s : 0.0;
+  for (int f0 = 0; f0 < nw; f0 += SPQ_FCH) {
+    const int nf = min(SPQ_FCH, nw - f0);
+    __syncthreads();   // the previous chunk's factors are consumed
+    for (int e = threadIdx.x; e < nf * (SP_KB / 2); e += blockDim.x) {
+      const int f = e / (SP_KB / 2), c = e - f * (SP_KB / 2), q = c >> 3, j = c & 7;
+      reinterpret_cast<double2*>(&gs[f][0])[8 * q + (j ^ (2 * q))] =
+          __ldg(reinterpret_cast<const double2*>(G + (int64_t)(f0 + f) * ldg + kb * SP_KB) + c);
+    }
+    for (int f = threadIdx.x; f < nf; f += blockDim.x) ss[f] = wsgn[f0 + f];
+    __syncthreads();
+#pragma unroll 1
+    for (int f = 0; f < nf; ++f) {
+      const bool mixed = ss[f] == 0;
+      const double2* gq = reinterpret_cast<const double2*>(&gs[f][0]) + 8 * quarter;
+      uint32_t a[SP_SF][4], b[SP_SF][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double2 g01 = gq[(2 * q) ^ (2 * quarter)], g23 = gq[(2 * q + 1) ^ (2 * quarter)];
+        const double g[4] = {g01.x * inv, g01.y * inv, g23.x * inv, g23.y * inv};
+        uint32_t y[4], pd[SP_SF];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = round_mul(x[4 * q + e], fabs(g[e]));
+        digit_planes<SP_SF>(y, pd);
+#pragma unroll
+        for (int t = 0; t < SP_SF; ++t) a[t][q] = pd[t];
+        if (mixed) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (g[e] < 0.0) y[e] = 0u - y[e];
+          digit_planes<SP_SF>(y, pd);
+#pragma unroll
+          for (int t = 0; t < SP_SF; ++t) b[t][q] = pd[t];
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < SP_SF; ++t)
+        *reinterpret_cast<uint4*>(F + o + ((int64_t)(f0 + f) * SP_SLOT + t) * pstride) =
+            make_uint4(a[t][0], a[t][1], a[t][2], a[t][3]);
+      if (mixed) {
+#pragma unroll
+        for (int t = 0; t < SP_SF; ++t)
+          *reinterpret_cast<uint4*>(F + o + ((int64_t)(f0 + f) * SP_SLOT + SP_SF + t) * pstride) =
+              make_uint4(b[t][0], b[t][1], b[t][2], b[t][3]);
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -799,29 +989,67 @@ int make_tmap_u8_4d(spx_ctx* ctx, CUtensorMap* map, const void* base, const uint
 }
 
 struct SplitLayout {
-  int64_t Ps, R;
-  int nblk;
+  int64_t Ps, Pp, R;   // pairs of a slab, pairs of one operand buffer, plane rows
+  int nblk, nbuf;
   size_t f_bytes, g_bytes, s_bytes, w_bytes, sg_bytes;
+  size_t bytes() const { return nbuf * (f_bytes + g_bytes + s_bytes + w_bytes + sg_bytes) + 1024; }
 };
 
-// slab: band pairs per exact int32 slab, a multiple of SP_KB in [SP_KB, SP_SLAB]
-static SplitLayout split_layout(int64_t P, int N, int nw, int slab = SP_SLAB) {
+// Tiles of one frequency on 64 x BN complex tiles (the -DINV form: 128 x 2 BN real ones,
+// nbr its 128-row blocks and n the columns in halves).
+static int split_ntile(int n, int bn, int nbr) {
+  int t = 0;
+  for (int bj = 0; bj * bn < n; ++bj) t += split_rows_of(bj, bn, nbr);
+  return t;
+}
+
+// One-CTA tile shape of an untuned call: the shape whose tiles take less tensor-pipe time. An MMA
+// of N = 160 takes 1.10 times the time of one of N = 128 (which is bound by the instruction
+// rate), so 64 x 80 tiles win (1.13 fewer of them at 1200 columns: 739 against 705 TFLOP/s)
+// unless their last column block is nearly empty (403 columns: 28 tiles of either shape).
+static bool split_wide(int n, int nbr) { return split_ntile(n, SP_WIDE_BN, nbr) * 110 < split_ntile(n, SP_TILE, nbr) * 100; }
+
+// Pairs of one operand buffer: a slab's scales and factors hold for all of it, but its planes
+// are written and accumulated in equal parts of at most this many pairs (the parts' FP64
+// adds are the only difference from one pass).
+//   * With more tiles per frequency than SMs, a round of CTAs reads a frequency's planes
+//     while the rest of its tiles wait for the next round: the planes come from L2 again
+//     only if they (3 digits x R rows x pairs) leave room there. Measured at 1200 columns,
+//     full calls of a million pairs, one kernel: 739-747 TFLOP/s with 8192 and 12288 pairs
+//     (60 and 90 MB), 718-723 with 16384 (120 MB), 641 with 32768.
+//   * Otherwise a round's CTAs walk the same pairs together: the whole slab.
+static int64_t split_part_pairs(int64_t Ps, int ntile, int64_t R) {
+  int64_t most = Ps;
+  if (ntile > SP_SMS)
+    most = std::min<int64_t>(most, std::max<int64_t>(4096, (90ll << 20) / (SP_SF * R) / SP_KB * SP_KB));
+  const int64_t n = (Ps + most - 1) / most;
+  return (int64_t)align_up((size_t)((Ps + n - 1) / n), SP_KB);
+}
+
+// slab: band pairs per exact int32 slab, a multiple of SP_KB in [SP_KB, SP_SLAB]; R plane rows.
+// Two operand buffers when there is more than one part: the next part is quantized
+// while one accumulates.
+static SplitLayout split_layout_of(int64_t P, int nblk, int64_t R, int ntile, int ncol, int nw, int slab) {
   SplitLayout L;
   L.Ps = std::min<int64_t>((int64_t)align_up((size_t)std::max<int64_t>(P, 1), SP_KB), slab);
-  L.nblk = (N + SP_TILE - 1) / SP_TILE;
-  // an even number of 64-blocks, so a CTA pair's second A tile always exists
-  L.R = (int64_t)((L.nblk + 1) / 2 * 2) * SP_ROWS;
-  L.f_bytes = align_up((size_t)SP_SLOT * nw * L.R * L.Ps, 1024);
+  L.Pp = split_part_pairs(L.Ps, ntile, R);
+  L.nblk = nblk;
+  L.R = R;
+  L.nbuf = P > L.Pp ? 2 : 1;
+  L.f_bytes = align_up((size_t)SP_SLOT * nw * R * L.Pp, 1024);
   L.g_bytes = align_up(sizeof(double) * (size_t)nw * L.Ps, 256);
-  L.s_bytes = align_up(sizeof(double) * (size_t)std::max(N, 1), 256);
+  L.s_bytes = align_up(sizeof(double) * (size_t)std::max(ncol, 1), 256);
   L.w_bytes = align_up(sizeof(double) * (size_t)std::max(nw, 1), 256);
   L.sg_bytes = align_up(sizeof(int) * (size_t)std::max(nw, 1), 256);
   return L;
 }
 
-// Two operand buffers when there is more than one slab: slab s+1 is quantized
-// while slab s accumulates.
-static int split_nbuf(int64_t P, int slab = SP_SLAB) { return P > slab ? 2 : 1; }
+static SplitLayout split_layout(int64_t P, int N, int nw, int slab) {
+  const int nblk = (N + SP_TILE - 1) / SP_TILE;
+  // an even number of 64-blocks, so a CTA pair's second A tile always exists
+  return split_layout_of(P, nblk, (int64_t)((nblk + 1) / 2 * 2) * SP_ROWS, split_ntile(N, SP_WIDE_BN, nblk), N, nw,
+                         slab);
+}
 
 static int clamp_slab(int slab) {
   if (slab <= 0) return SP_SLAB;
@@ -830,88 +1058,172 @@ static int clamp_slab(int slab) {
 
 size_t split_workspace_bytes(int64_t P, int N, int nw, int slab) {
   slab = clamp_slab(slab);
-  SplitLayout L = split_layout(P, N, nw, slab);
-  return split_nbuf(P, slab) * (L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes + L.sg_bytes) + 1024;
+  return split_layout(P, N, nw, slab).bytes();
 }
+// Scratch for partial tiles beyond split_workspace_bytes, optional.
+size_t split_part_bytes(int num_sms, bool real) {
+  // two partial tiles per CTA
+  return align_up(sizeof(double) * 2 * (size_t)num_sms * split_part_elems(real, SP_WIDE_BN), 256) + 1280;
+}
+
 size_t split_workspace_bytes(int64_t P, int N, int nw) {
   return split_workspace_bytes(P, N, nw, SP_SLAB);
 }
 
 void timing_mark(spx_ctx* ctx, cudaStream_t s, int kind);
 
+// Launches the one-CTA kernel for one slab (prm.nitems, nk and the operands set), with the
+// last items cut over all CTAs when that pays and `part` has room for the partial tiles.
+template <bool REAL, int BN>
+static int split_gram_launch(spx_ctx* ctx, const CUtensorMap& mapA, const CUtensorMap& mapB, SplitParams prm,
+                             double* part, cudaStream_t stream, int* launches) {
+  const size_t smem = sizeof(SplitSmemT<2 * BN>) + 1024;
+  int rc = check_cuda(ctx, cudaFuncSetAttribute(split_gram_kernel<REAL, BN>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                      "split_gram_kernel attribute");
+  if (rc) return rc;
+  const bool cut = part && split_cuts(prm.nitems, prm.nk, ctx->num_sms, REAL);
+  // a cut range is at least 8 stages long
+  const int grid = (int)std::min<int64_t>(
+      cut ? std::max<int64_t>(prm.nitems, (int64_t)prm.nitems * prm.nk / 8) : prm.nitems, ctx->num_sms);
+  prm.whole = cut ? prm.nitems / grid * grid : prm.nitems;
+  prm.part = cut ? part : nullptr;
+  split_gram_kernel<REAL, BN><<<grid, SP1_THREADS, smem, stream>>>(mapA, mapB, prm);
+  if ((rc = check_cuda(ctx, cudaGetLastError(), "split_gram_kernel launch"))) return rc;
+  *launches += 1;
+  if (prm.whole < prm.nitems && grid > 1) {
+    const int ny = (REAL ? 2 : 1) * BN * 4 / SP1_EPI / split_finish_step<REAL>();
+    split_gram_finish_kernel<REAL, BN><<<dim3(grid - 1, ny), 32 * SP1_EPI, 0, stream>>>(prm, grid);
+    if ((rc = check_cuda(ctx, cudaGetLastError(), "split_gram_finish_kernel launch"))) return rc;
+    *launches += 1;
+  }
+  return SPX_OK;
+}
+
+// One operand buffer set of a call.
+struct SplitBuf {
+  int8_t* F;
+  double *G, *sA, *wmax;
+  int* wsgn;
+};
+static void split_buffers(const SplitLayout& L, uint8_t* base, SplitBuf (&buf)[2]) {
+  const size_t set_bytes = L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes + L.sg_bytes;
+  for (int b = 0; b < 2; ++b) {
+    uint8_t* s0 = base + (size_t)(b < L.nbuf ? b : 0) * set_bytes;
+    buf[b] = {(int8_t*)s0, (double*)(s0 + L.f_bytes), (double*)(s0 + L.f_bytes + L.g_bytes),
+              (double*)(s0 + L.f_bytes + L.g_bytes + L.s_bytes),
+              (int*)(s0 + L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes)};
+  }
+}
+
+// One part of a slab: slab pairs [p0, p0 + len), part [off, off + plen) of them.
+struct SplitStep {
+  int64_t p0;
+  int len, off, plen;
+  int sb, b;   // buffer of the slab's statistics, of the part's planes
+  bool last;   // nothing is prepared beside this part's accumulation
+};
+
+// Runs the parts of a call: stat(step, stream) before a slab's first part, then
+// quant(step, stream), on the preparation stream, one part ahead of gram(step) on `stream`. A
+// single part has nothing to run beside and stays on `stream`. The statistics buffer of
+// slab s is reused by slab s + 2, whose first part waits for a part of slab s + 1 at least.
+template <class Stat, class Quant, class Gram>
+static int split_run_steps(spx_ctx* ctx, const SplitLayout& L, int64_t P, cudaStream_t stream, Stat stat,
+                           Quant quant, Gram gram) {
+  std::vector<SplitStep> steps;
+  for (int64_t p0 = 0, s = 0; p0 < P; p0 += L.Ps, ++s) {
+    const int len = (int)std::min<int64_t>(L.Ps, P - p0);
+    for (int off = 0; off < len; off += (int)L.Pp)
+      steps.push_back({p0, len, off, (int)std::min<int64_t>(L.Pp, len - off), (int)(s % 2) * (L.nbuf - 1),
+                       (int)(steps.size() % L.nbuf), false});
+  }
+  steps.back().last = true;
+  const bool two = steps.size() > 1;
+  cudaStream_t ps = two ? ctx->prep_stream : stream;
+  cudaEvent_t prep_done[2] = {ctx->sev[1], ctx->sev[2]};
+  cudaEvent_t gram_done[2] = {ctx->sev[3], ctx->sev[4]};
+  int rc = SPX_OK;
+  auto prep = [&](const SplitStep& t) -> int {
+    if (t.off == 0 && (rc = stat(t, ps))) return rc;
+    if ((rc = quant(t, ps))) return rc;
+    return two ? check_cuda(ctx, cudaEventRecord(prep_done[t.b], ps), "event") : SPX_OK;
+  };
+  // the preparation stream starts after everything already queued on `stream` (whatever
+  // produced cprod and the weights, and the last call's use of the buffers)
+  if (two && ((rc = check_cuda(ctx, cudaEventRecord(ctx->sev[0], stream), "event")) ||
+              (rc = check_cuda(ctx, cudaStreamWaitEvent(ps, ctx->sev[0], 0), "event"))))
+    return rc;
+  timing_mark(ctx, stream, 0);
+  if ((rc = prep(steps[0]))) return rc;
+  for (size_t k = 0; k < steps.size(); ++k) {
+    const SplitStep& t = steps[k];
+    if (two && (rc = check_cuda(ctx, cudaStreamWaitEvent(stream, prep_done[t.b], 0), "event"))) return rc;
+    timing_mark(ctx, stream, 1);
+    if ((rc = gram(t))) return rc;
+    timing_mark(ctx, stream, 2);  // the accumulation interval ends with the kernel
+    if (two && (rc = check_cuda(ctx, cudaEventRecord(gram_done[t.b], stream), "event"))) return rc;
+    if (k + 1 < steps.size()) {
+      // the next part goes into the buffer that part k - 1 accumulated from
+      if (k >= 1 && (rc = check_cuda(ctx, cudaStreamWaitEvent(ps, gram_done[steps[k + 1].b], 0), "event")))
+        return rc;
+      if ((rc = prep(steps[k + 1]))) return rc;
+    }
+  }
+  return SPX_OK;
+}
+
 // variant: 1 one CTA per 64 x 64 tile, 2 CTA pair, 5 one CTA per 64 x 80 tile, 0 the
 // context's choice; slab: pairs per exact int32 slab (0 = 32768).
-int split_chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, const double* W,
-                    int64_t ldw, int nw, double2* out, void* ws, size_t ws_bytes,
-                    cudaStream_t stream, int* launches, int variant, int slab) {
+static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, const SplitStat& src,
+                          int nw, double2* out, void* ws, size_t ws_bytes, cudaStream_t stream,
+                          int* launches, int variant, int slab) {
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
   slab = clamp_slab(slab);
   SplitLayout L = split_layout(P, N, nw, slab);
   if (!ws || ws_bytes < split_workspace_bytes(P, N, nw, slab))
     return set_error(ctx, SPX_EINVAL, "split workspace too small");
   uint8_t* base = (uint8_t*)align_up((size_t)ws, 1024);
-  const int nbuf = split_nbuf(P, slab);
-  const size_t set_bytes = L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes + L.sg_bytes;
-  int8_t* F[2];
-  double* G[2];
-  double* sA[2];
-  double* wmax[2];
-  int* wsgn[2];
-  for (int b = 0; b < 2; ++b) {
-    uint8_t* s0 = base + (size_t)(b < nbuf ? b : 0) * set_bytes;
-    F[b] = (int8_t*)s0;
-    G[b] = (double*)(s0 + L.f_bytes);
-    sA[b] = (double*)(s0 + L.f_bytes + L.g_bytes);
-    wmax[b] = (double*)(s0 + L.f_bytes + L.g_bytes + L.s_bytes);
-    wsgn[b] = (int*)(s0 + L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes);
-  }
+  SplitBuf buf[2];
+  split_buffers(L, base, buf);
 
   // planes in HBM: [plane][k-block][row][K bytes]; TMA dims (K, row, k-block, plane)
   // with increasing strides; a box (K, rows, 1, 3 planes) lands as [plane][row][K]
-  const uint64_t nkb = (uint64_t)(L.Ps / SP_KB);
+  const uint64_t nkb = (uint64_t)(L.Pp / SP_KB);
   if (variant == 0) variant = ctx->opt.split_variant;
-  if (variant == 0) variant = 5;  // untuned: one CTA per 64 x 80 tile
+  if (variant == 0) variant = split_wide(N, L.nblk) ? 5 : 1;  // untuned: one CTA per tile
   const bool pair = variant == 2;
   const bool wide = variant == 5;                  // one CTA per 64 x 80 tile (N = 160)
+  const size_t base_bytes = split_workspace_bytes(P, N, nw, slab);
+  double* part = nullptr;   // partial tiles, where the caller has room for them
+  if (!pair && ws_bytes >= base_bytes + split_part_bytes(ctx->num_sms, false))
+    part = (double*)(base + align_up(base_bytes, 256));
   // only the CTA pair needs an even number of 64-column blocks in the planes (the
   // buffers are sized for it either way)
   if (!pair) L.R = (int64_t)L.nblk * SP_ROWS;
   CUtensorMap mapF[2], mapFh[2], mapW[2];
-  for (int b = 0; b < nbuf; ++b) {
+  for (int b = 0; b < L.nbuf; ++b) {
     const uint64_t st[3] = {SP_KB, (uint64_t)L.R * SP_KB, nkb * L.R * SP_KB};
     const uint64_t d[4] = {SP_KB, (uint64_t)L.R, nkb, (uint64_t)SP_SLOT * nw};
     const uint32_t bx[4] = {SP_KB, SP_ROWS, 1, SP_SF};
-    int rc0 = make_tmap_u8_4d(ctx, &mapF[b], F[b], d, st, bx, CU_TENSOR_MAP_SWIZZLE_64B);
+    int rc0 = make_tmap_u8_4d(ctx, &mapF[b], buf[b].F, d, st, bx, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc0) return rc0;
     const uint32_t bh[4] = {SP_KB, SP2_BROWS, 1, SP_SF};
-    rc0 = make_tmap_u8_4d(ctx, &mapFh[b], F[b], d, st, bh, CU_TENSOR_MAP_SWIZZLE_64B);
+    rc0 = make_tmap_u8_4d(ctx, &mapFh[b], buf[b].F, d, st, bh, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc0) return rc0;
     const uint32_t bw[4] = {SP_KB, 2 * SP_WIDE_BN, 1, SP_SF};
-    rc0 = make_tmap_u8_4d(ctx, &mapW[b], F[b], d, st, bw, CU_TENSOR_MAP_SWIZZLE_64B);
+    rc0 = make_tmap_u8_4d(ctx, &mapW[b], buf[b].F, d, st, bw, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc0) return rc0;
   }
   int rc = SPX_OK;
 
-  const size_t smem = sizeof(SplitSmem) + 1024;
-  const size_t smemw = sizeof(SplitSmemT<2 * SP_WIDE_BN>) + 1024;
   const size_t smem2 = sizeof(Split2Smem) + 1024;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(split_gram_kernel<false, SP_TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(split_gram_kernel<false, SP_WIDE_BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemw);
-    cudaFuncSetAttribute(split_gram_kernel<true, SP_TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(split_gram2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem2);
-    attr_set = true;
-  }
+  if (pair) cudaFuncSetAttribute(split_gram2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
   const int nbr = (N + SP_TILE - 1) / SP_TILE;
-  const int ntile = L.nblk * (L.nblk + 1) / 2;
-  int ntile2 = 0, ntilew = 0;
+  int ntile2 = 0;
   for (int bj = 0; bj < L.nblk; ++bj) ntile2 += bj / 2 + 1;
-  for (int bj = 0; bj * SP_WIDE_BN < N; ++bj) ntilew += split_rows_of(bj, SP_WIDE_BN, nbr);
-  const int ntile_used = pair ? ntile2 : (wide ? ntilew : ntile);
+  const int ntile_used = pair ? ntile2 : split_ntile(N, wide ? SP_WIDE_BN : SP_TILE, nbr);
   const int nitems = ntile_used * nw;
-  const int grid = std::min(nitems, ctx->num_sms);
   const int npad = (int)(L.R / 2);  // columns covered by the stacked rows
   // CTA-pair launch: as many clusters as can be resident at once (persistent)
   cudaLaunchConfig_t cfg = {};
@@ -937,216 +1249,146 @@ int split_chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int 
     cfg.gridDim = dim3(2 * nclusters);
   }
 
-  // Preparation (column scales, weight statistics, digit planes) of slab s+1 runs on
-  // the preparation stream while slab s accumulates on `stream`; buffer b = s % 2.
-  const int64_t nslab = (P + L.Ps - 1) / L.Ps;
-  cudaStream_t ps = ctx->prep_stream;
-  cudaEvent_t ev_start = ctx->sev[0];
-  cudaEvent_t prep_done[2] = {ctx->sev[1], ctx->sev[2]};
-  cudaEvent_t gram_done[2] = {ctx->sev[3], ctx->sev[4]};
-  auto prep = [&](int64_t s) -> int {
-    const int b = (int)(s % nbuf);
-    const int64_t p0 = s * L.Ps;
-    const int len = (int)std::min<int64_t>(L.Ps, P - p0);
-    const int lenp = (int)align_up((size_t)len, SP_KB);
-    const int nchunk = lenp / 16;  // 16-pair chunks; npad is a multiple of 64
-    split_colmax_kernel<<<N, 256, 0, ps>>>(M, ldc, p0, len, sA[b]);
-    split_wstat_kernel<<<nw, 256, 0, ps>>>(W, ldw, p0, len, lenp, wmax[b], wsgn[b], G[b]);
-    const int64_t nthr = (int64_t)npad * nchunk * 2;  // 8-pair tasks
-    split_quantize_kernel<<<(unsigned)((nthr + 127) / 128), 128, 0, ps>>>(
-        M, ldc, p0, len, nchunk, N, npad, L.R, L.Ps, nw, sA[b], wsgn[b], G[b], F[b]);
-    int r = check_cuda(ctx, cudaGetLastError(), "split operand preparation");
-    if (r) return r;
-    *launches += 3;
-    return check_cuda(ctx, cudaEventRecord(prep_done[b], ps), "event");
+  auto stat = [&](const SplitStep& t, cudaStream_t ps) -> int {
+    const int ncol = (int)align_up((size_t)N, SPS_CL);
+    split_stat_kernel<false><<<ncol + nw * SPS_CL, SPS_THREADS, 0, ps>>>(
+        reinterpret_cast<const double*>(M), ldc, t.p0, t.len, (int)align_up((size_t)t.len, SP_KB), N, ncol, src,
+        buf[t.sb].sA, buf[t.sb].wmax, buf[t.sb].wsgn, buf[t.sb].G);
+    ++*launches;
+    return check_cuda(ctx, cudaGetLastError(), "split_stat_kernel launch");
   };
-  // the preparation stream starts after everything already queued on `stream`
-  // (the weights, and whatever produced cprod)
-  if ((rc = check_cuda(ctx, cudaEventRecord(ev_start, stream), "event")) ||
-      (rc = check_cuda(ctx, cudaStreamWaitEvent(ps, ev_start, 0), "event")))
-    return rc;
-  timing_mark(ctx, stream, 0);
-  if ((rc = prep(0))) return rc;
-  for (int64_t s = 0; s < nslab; ++s) {
-    const int b = (int)(s % nbuf);
-    const int len = (int)std::min<int64_t>(L.Ps, P - s * L.Ps);
-    const int lenp = (int)align_up((size_t)len, SP_KB);
-    if ((rc = check_cuda(ctx, cudaStreamWaitEvent(stream, prep_done[b], 0), "event"))) return rc;
-    // with two buffers, slab s+1 goes into the buffer that slab s-1 accumulated from
-    if (nbuf == 2 && s >= 1 && s + 1 < nslab &&
-        (rc = check_cuda(ctx, cudaStreamWaitEvent(ps, gram_done[(s + 1) % 2], 0), "event")))
-      return rc;
-    timing_mark(ctx, stream, 1);
+  auto quant = [&](const SplitStep& t, cudaStream_t ps) -> int {
+    const int nchunk = (int)align_up((size_t)t.plen, SP_KB) / 16;  // 16-pair chunks; npad is a multiple of 64
+    const int64_t nthr = (int64_t)npad * nchunk * 2;                // 8-pair tasks
+    split_quantize_kernel<<<(unsigned)((nthr + 127) / 128), 128, 0, ps>>>(
+        M, ldc, t.p0 + t.off, t.plen, nchunk, N, npad, L.R, L.Pp, nw, buf[t.sb].sA, buf[t.sb].wsgn,
+        buf[t.sb].G + t.off, (int)align_up((size_t)t.len, SP_KB), buf[t.b].F);
+    ++*launches;
+    return check_cuda(ctx, cudaGetLastError(), "split_quantize_kernel launch");
+  };
+  auto gram = [&](const SplitStep& t) -> int {
     SplitParams prm;
     prm.N = N;
     prm.nbr = nbr;
     prm.ntile = ntile_used;
     prm.nw = nw;
     prm.nitems = nitems;
-    prm.nk = lenp / SP_KB;
-    prm.sA = sA[b];
-    prm.wmax = wmax[b];
-    prm.wsgn = wsgn[b];
+    prm.nk = (int)align_up((size_t)t.plen, SP_KB) / SP_KB;
+    prm.sA = buf[t.sb].sA;
+    prm.wmax = buf[t.sb].wmax;
+    prm.wsgn = buf[t.sb].wsgn;
     prm.out = reinterpret_cast<double*>(out);
     prm.npack = (int64_t)N * (N + 1) / 2;
     prm.status = ctx->d_status;
     prm.timeout_ns =
         (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
     if (pair) {
-      rc = check_cuda(ctx, cudaLaunchKernelEx(&cfg, split_gram2_kernel, mapF[b], mapFh[b], prm),
-                      "split_gram2_kernel launch");
-    } else if (wide) {
-      split_gram_kernel<false, SP_WIDE_BN><<<grid, SP1_THREADS, smemw, stream>>>(mapF[b], mapW[b], prm);
-      rc = check_cuda(ctx, cudaGetLastError(), "split_gram_kernel (64 x 80) launch");
-    } else {
-      split_gram_kernel<false, SP_TILE><<<grid, SP1_THREADS, smem, stream>>>(mapF[b], mapF[b], prm);
-      rc = check_cuda(ctx, cudaGetLastError(), "split_gram_kernel launch");
+      ++*launches;
+      return check_cuda(ctx, cudaLaunchKernelEx(&cfg, split_gram2_kernel, mapF[t.b], mapFh[t.b], prm),
+                        "split_gram2_kernel launch");
     }
-    if (rc) return rc;
-    *launches += 1;
-    timing_mark(ctx, stream, 2);  // the accumulation interval ends with the kernel
-    if ((rc = check_cuda(ctx, cudaEventRecord(gram_done[b], stream), "event"))) return rc;
-    if (s + 1 < nslab) {
-      // with one buffer, the next preparation waits for this accumulation
-      if (nbuf == 1 &&
-          (rc = check_cuda(ctx, cudaStreamWaitEvent(ps, gram_done[0], 0), "event")))
-        return rc;
-      if ((rc = prep(s + 1))) return rc;
-    }
-  }
-  return SPX_OK;
+    if (wide) return split_gram_launch<false, SP_WIDE_BN>(ctx, mapF[t.b], mapW[t.b], prm, t.last ? part : nullptr, stream, launches);
+    return split_gram_launch<false, SP_TILE>(ctx, mapF[t.b], mapF[t.b], prm, t.last ? part : nullptr, stream, launches);
+  };
+  return split_run_steps(ctx, L, P, stream, stat, quant, gram);
+}
+
+// The accumulation with given weights W (ldw, nw).
+int split_chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, const double* W,
+                    int64_t ldw, int nw, double2* out, void* ws, size_t ws_bytes,
+                    cudaStream_t stream, int* launches, int variant, int slab) {
+  return split_chi0_run(ctx, M, ldc, P, N, SplitStat{W, ldw, nullptr, nullptr, 0.0, nullptr}, nw, out, ws,
+                        ws_bytes, stream, launches, variant, slab);
+}
+
+// The accumulation with the HILBERT NONE weights of ediff (the same bits as K6's).
+int split_chi0_ediff(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, const double* ediff,
+                     const double* wscale, double scale_all, int nw, const double* omega, double2* out,
+                     void* ws, size_t ws_bytes, cudaStream_t stream, int* launches, int variant, int slab) {
+  return split_chi0_run(ctx, M, ldc, P, N, SplitStat{nullptr, 0, ediff, wscale, scale_all, omega}, nw, out, ws,
+                        ws_bytes, stream, launches, variant, slab);
 }
 
 // Real layout: 128 columns per block, one plane row per column.
-static SplitLayout split_layout_real(int64_t P, int N, int nw, int slab) {
-  SplitLayout L = split_layout(P, 1, nw, slab);
-  L.nblk = (N + SP_ROWS - 1) / SP_ROWS;
-  L.R = (int64_t)L.nblk * SP_ROWS;
-  L.f_bytes = align_up((size_t)SP_SLOT * nw * L.R * L.Ps, 1024);
-  L.s_bytes = align_up(sizeof(double) * (size_t)std::max(N, 1), 256);
-  return L;
+static SplitLayout split_layout_real(int64_t P, int N, int nw) {
+  const int nblk = (N + SP_ROWS - 1) / SP_ROWS;
+  return split_layout_of(P, nblk, (int64_t)nblk * SP_ROWS, split_ntile((N + 1) / 2, SP_WIDE_BN, nblk), N, nw, SP_SLAB);
 }
 
-size_t split_workspace_bytes_real(int64_t P, int N, int nw) {
-  SplitLayout L = split_layout_real(P, N, nw, SP_SLAB);
-  return split_nbuf(P, SP_SLAB) * (L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes + L.sg_bytes) + 1024;
-}
+size_t split_workspace_bytes_real(int64_t P, int N, int nw) { return split_layout_real(P, N, nw).bytes(); }
 
 // The -DINV accumulation (src/susceptibility.f:1197, re(k) = cprod(k,i) * cprod(k,j)):
 // real M (ldc, N), real packed out (npack, nw), the folded 6-product int8 contraction
-// on 128 x 160 real tiles (N = 160 MMAs; 128 x 128 when the context's split variant is
-// 1), one CTA per tile.
-int split_chi0_real_slab(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P, int N,
-                         const double* W, int64_t ldw, int nw, double* out, void* ws,
-                         size_t ws_bytes, cudaStream_t stream, int* launches) {
+// on 128 x 160 real tiles (N = 160 MMAs) or 128 x 128 (when those take less time, or the
+// context's split variant is 1), one CTA per tile. HILBERT NONE weights of ediff.
+int split_chi0_real_ediff(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P, int N, const double* ediff,
+                          const double* wscale, double scale_all, int nw, const double* omega, double* out,
+                          void* ws, size_t ws_bytes, cudaStream_t stream, int* launches) {
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
-  SplitLayout L = split_layout_real(P, N, nw, SP_SLAB);
-  if (!ws || ws_bytes < split_workspace_bytes_real(P, N, nw))
-    return set_error(ctx, SPX_EINVAL, "split workspace too small");
+  const SplitStat src{nullptr, 0, ediff, wscale, scale_all, omega};
+  const SplitLayout L = split_layout_real(P, N, nw);
+  const size_t base_bytes = L.bytes();
+  if (!ws || ws_bytes < base_bytes) return set_error(ctx, SPX_EINVAL, "split workspace too small");
   uint8_t* base = (uint8_t*)align_up((size_t)ws, 1024);
-  const int nbuf = split_nbuf(P, SP_SLAB);
-  const size_t set_bytes = L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes + L.sg_bytes;
-  int8_t* F[2];
-  double *G[2], *sA[2], *wmax[2];
-  int* wsgn[2];
-  for (int b = 0; b < 2; ++b) {
-    uint8_t* s0 = base + (size_t)(b < nbuf ? b : 0) * set_bytes;
-    F[b] = (int8_t*)s0;
-    G[b] = (double*)(s0 + L.f_bytes);
-    sA[b] = (double*)(s0 + L.f_bytes + L.g_bytes);
-    wmax[b] = (double*)(s0 + L.f_bytes + L.g_bytes + L.s_bytes);
-    wsgn[b] = (int*)(s0 + L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes);
-  }
-  const uint64_t nkb = (uint64_t)(L.Ps / SP_KB);
-  const bool wide = ctx->opt.split_variant != 1;
+  SplitBuf buf[2];
+  split_buffers(L, base, buf);
+  double* part = ws_bytes >= base_bytes + split_part_bytes(ctx->num_sms, true)
+                     ? (double*)(base + align_up(base_bytes, 256))
+                     : nullptr;
+  const uint64_t nkb = (uint64_t)(L.Pp / SP_KB);
+  const bool wide = ctx->opt.split_variant != 1 && (ctx->opt.split_variant != 0 || split_wide((N + 1) / 2, L.nblk));
   CUtensorMap mapF[2], mapW[2];
-  for (int b = 0; b < nbuf; ++b) {
+  for (int b = 0; b < L.nbuf; ++b) {
     const uint64_t st[3] = {SP_KB, (uint64_t)L.R * SP_KB, nkb * L.R * SP_KB};
     const uint64_t d[4] = {SP_KB, (uint64_t)L.R, nkb, (uint64_t)SP_SLOT * nw};
     const uint32_t bx[4] = {SP_KB, SP_ROWS, 1, SP_SF};
-    int rc0 = make_tmap_u8_4d(ctx, &mapF[b], F[b], d, st, bx, CU_TENSOR_MAP_SWIZZLE_64B);
+    int rc0 = make_tmap_u8_4d(ctx, &mapF[b], buf[b].F, d, st, bx, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc0) return rc0;
     const uint32_t bw[4] = {SP_KB, 2 * SP_WIDE_BN, 1, SP_SF};
-    rc0 = make_tmap_u8_4d(ctx, &mapW[b], F[b], d, st, bw, CU_TENSOR_MAP_SWIZZLE_64B);
+    rc0 = make_tmap_u8_4d(ctx, &mapW[b], buf[b].F, d, st, bw, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc0) return rc0;
   }
-  const size_t smem = sizeof(SplitSmem) + 1024;
-  const size_t smemw = sizeof(SplitSmemT<2 * SP_WIDE_BN>) + 1024;
-  cudaFuncSetAttribute(split_gram_kernel<true, SP_TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaFuncSetAttribute(split_gram_kernel<true, SP_WIDE_BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemw);
   // tiles in 128-row blocks of the real rows; wide tiles in 160-column blocks
   const int nbr = L.nblk;
-  int ntilew = 0;
-  for (int bj = 0; bj * 2 * SP_WIDE_BN < N; ++bj) ntilew += split_rows_of(bj, SP_WIDE_BN, nbr);
-  const int ntile = wide ? ntilew : L.nblk * (L.nblk + 1) / 2;
+  const int ntile = split_ntile((N + 1) / 2, wide ? SP_WIDE_BN : SP_TILE, nbr);
   const int nitems = ntile * nw;
-  const int grid = std::min(nitems, ctx->num_sms);
   const int npad = (int)L.R;
-  const int64_t nslab = (P + L.Ps - 1) / L.Ps;
-  cudaStream_t ps = ctx->prep_stream;
-  cudaEvent_t ev_start = ctx->sev[0];
-  cudaEvent_t prep_done[2] = {ctx->sev[1], ctx->sev[2]};
-  cudaEvent_t gram_done[2] = {ctx->sev[3], ctx->sev[4]};
-  int rc;
-  auto prep = [&](int64_t s) -> int {
-    const int b = (int)(s % nbuf);
-    const int64_t p0 = s * L.Ps;
-    const int len = (int)std::min<int64_t>(L.Ps, P - p0);
-    const int lenp = (int)align_up((size_t)len, SP_KB);
-    const int nchunk = lenp / 16;
-    split_colmax_real_kernel<<<N, 256, 0, ps>>>(M, ldc, p0, len, sA[b]);
-    split_wstat_kernel<<<nw, 256, 0, ps>>>(W, ldw, p0, len, lenp, wmax[b], wsgn[b], G[b]);
-    const int64_t nthr = (int64_t)npad * nchunk;
-    split_quantize_real_kernel<<<(unsigned)((nthr + 127) / 128), 128, 0, ps>>>(
-        M, ldc, p0, len, nchunk, N, npad, L.R, L.Ps, nw, sA[b], wsgn[b], G[b], F[b]);
-    int r = check_cuda(ctx, cudaGetLastError(), "split operand preparation (real)");
-    if (r) return r;
-    *launches += 3;
-    return check_cuda(ctx, cudaEventRecord(prep_done[b], ps), "event");
+  auto stat = [&](const SplitStep& t, cudaStream_t ps) -> int {
+    const int ncol = (int)align_up((size_t)N, SPS_CL);
+    split_stat_kernel<true><<<ncol + nw * SPS_CL, SPS_THREADS, 0, ps>>>(
+        M, ldc, t.p0, t.len, (int)align_up((size_t)t.len, SP_KB), N, ncol, src, buf[t.sb].sA, buf[t.sb].wmax,
+        buf[t.sb].wsgn, buf[t.sb].G);
+    ++*launches;
+    return check_cuda(ctx, cudaGetLastError(), "split_stat_kernel (real) launch");
   };
-  if ((rc = check_cuda(ctx, cudaEventRecord(ev_start, stream), "event")) ||
-      (rc = check_cuda(ctx, cudaStreamWaitEvent(ps, ev_start, 0), "event")))
-    return rc;
-  timing_mark(ctx, stream, 0);
-  if ((rc = prep(0))) return rc;
-  for (int64_t s = 0; s < nslab; ++s) {
-    const int b = (int)(s % nbuf);
-    const int len = (int)std::min<int64_t>(L.Ps, P - s * L.Ps);
-    const int lenp = (int)align_up((size_t)len, SP_KB);
-    if ((rc = check_cuda(ctx, cudaStreamWaitEvent(stream, prep_done[b], 0), "event"))) return rc;
-    if (nbuf == 2 && s >= 1 && s + 1 < nslab &&
-        (rc = check_cuda(ctx, cudaStreamWaitEvent(ps, gram_done[(s + 1) % 2], 0), "event")))
-      return rc;
-    timing_mark(ctx, stream, 1);
+  auto quant = [&](const SplitStep& t, cudaStream_t ps) -> int {
+    const int nchunk = (int)align_up((size_t)t.plen, SP_KB) / 16;
+    // npad columns (a multiple of 128) x 16-pair chunks, 128 threads a block
+    split_quantize_real_kernel<<<(unsigned)((int64_t)npad * nchunk / 128), 128, 0, ps>>>(
+        M, ldc, t.p0 + t.off, t.plen, nchunk, N, npad, L.R, L.Pp, nw, buf[t.sb].sA, buf[t.sb].wsgn,
+        buf[t.sb].G + t.off, (int)align_up((size_t)t.len, SP_KB), buf[t.b].F);
+    ++*launches;
+    return check_cuda(ctx, cudaGetLastError(), "split_quantize_real_kernel launch");
+  };
+  auto gram = [&](const SplitStep& t) -> int {
     SplitParams prm;
     prm.N = N;
     prm.nbr = nbr;
     prm.ntile = ntile;
     prm.nw = nw;
     prm.nitems = nitems;
-    prm.nk = lenp / SP_KB;
-    prm.sA = sA[b];
-    prm.wmax = wmax[b];
-    prm.wsgn = wsgn[b];
+    prm.nk = (int)align_up((size_t)t.plen, SP_KB) / SP_KB;
+    prm.sA = buf[t.sb].sA;
+    prm.wmax = buf[t.sb].wmax;
+    prm.wsgn = buf[t.sb].wsgn;
     prm.out = out;
     prm.npack = (int64_t)N * (N + 1) / 2;
     prm.status = ctx->d_status;
     prm.timeout_ns = (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
-    if (wide)
-      split_gram_kernel<true, SP_WIDE_BN><<<grid, SP1_THREADS, smemw, stream>>>(mapF[b], mapW[b], prm);
-    else
-      split_gram_kernel<true, SP_TILE><<<grid, SP1_THREADS, smem, stream>>>(mapF[b], mapF[b], prm);
-    if ((rc = check_cuda(ctx, cudaGetLastError(), "split_gram_kernel (real) launch"))) return rc;
-    *launches += 1;
-    timing_mark(ctx, stream, 2);
-    if ((rc = check_cuda(ctx, cudaEventRecord(gram_done[b], stream), "event"))) return rc;
-    if (s + 1 < nslab) {
-      if (nbuf == 1 && (rc = check_cuda(ctx, cudaStreamWaitEvent(ps, gram_done[0], 0), "event")))
-        return rc;
-      if ((rc = prep(s + 1))) return rc;
-    }
-  }
-  return SPX_OK;
+    if (wide) return split_gram_launch<true, SP_WIDE_BN>(ctx, mapF[t.b], mapW[t.b], prm, t.last ? part : nullptr, stream, launches);
+    return split_gram_launch<true, SP_TILE>(ctx, mapF[t.b], mapF[t.b], prm, t.last ? part : nullptr, stream, launches);
+  };
+  return split_run_steps(ctx, L, P, stream, stat, quant, gram);
 }
 
 }  // namespace spx
