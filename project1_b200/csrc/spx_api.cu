@@ -13,6 +13,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstring>
 #include <string>
@@ -540,20 +541,89 @@ extern "C" int spx_chi0_accumulate_real_dev(spx_ctx* ctx, const double* cprod, i
   return SPX_OK;
 }
 
-// Copies columns [0, nbas) of rows [p0, p0+len) of a host cprod(ldc, nbas) into a
-// dense pinned slab (len, nbas), using `nthr` host threads.
-static void gather_slab(const double* cprod, int64_t ldc, int64_t p0, int64_t len, int nbas,
-                        double* dst, int nthr) {
-  auto work = [&](int t) {
-    for (int c = t; c < nbas; c += nthr)
-      std::memcpy(dst + 2 * (int64_t)c * len, cprod + 2 * ((int64_t)c * ldc + p0),
-                  sizeof(double) * 2 * (size_t)len);
+// The host threads of one host-pointer call: they gather the chunks of a pageable cprod into
+// pinned staging while earlier chunks are copied and accumulated, touch the output's pages
+// meanwhile, and add the sums at the end. One set per call (a thread costs about as much to
+// start as a megabyte to copy, so not one per chunk).
+struct HostCrew {
+  struct Chunk {
+    int64_t p0, len;
   };
-  std::vector<std::thread> th;
-  for (int t = 1; t < nthr; ++t) th.emplace_back(work, t);
-  work(0);
-  for (auto& x : th) x.join();
-}
+  const double* cprod = nullptr;   // NULL: nothing to gather
+  int64_t ldc = 0;
+  int nbas = 0;
+  std::vector<Chunk> chunks;
+  double* stage[3] = {};           // chunk k goes to stage[k % 3] as (len, nbas)
+  double* out = nullptr;           // susceph, `n` doubles in `pieces` parts
+  const double* sums = nullptr;
+  int64_t n = 0;
+  int pieces = 1;
+
+  std::atomic<int64_t> gather_to{-1};   // chunks up to this one may be gathered
+  std::atomic<int64_t> gathered{0};     // finished shares of chunks
+  std::atomic<int> touched{0}, add_to{-1}, added{0};
+  std::atomic<bool> stop{false};
+  std::atomic<int> size{0};             // threads and the caller; 0 until all have started
+  std::vector<std::thread> threads;
+
+  ~HostCrew() {
+    stop = true;
+    for (auto& t : threads) t.join();
+  }
+  void start(int want) {
+    try {
+      for (int t = 1; t < want; ++t) threads.emplace_back([this, t] { work(t); });
+    } catch (...) {
+      // fewer threads than wanted: the ones that started share the work
+    }
+    size = (int)threads.size() + 1;
+  }
+  // Columns t, t + size, ... of chunk k.
+  void gather(int t, int64_t k) {
+    const Chunk c = chunks[(size_t)k];
+    double* dst = stage[k % 3];
+    for (int i = t; i < nbas; i += size.load())
+      std::memcpy(dst + 2 * (int64_t)i * c.len, cprod + 2 * ((int64_t)i * ldc + c.p0),
+                  sizeof(double) * 2 * (size_t)c.len);
+    gathered.fetch_add(1);
+  }
+  void add(int t, int piece) {
+    const int64_t a0 = n * piece / pieces, a1 = n * (piece + 1) / pieces, w = size.load();
+    for (int64_t i = a0 + (a1 - a0) * t / w, e = a0 + (a1 - a0) * (t + 1) / w; i < e; ++i) out[i] += sums[i];
+    added.fetch_add(1);
+  }
+  // Maps this thread's share of a fresh output's pages before they are needed.
+  void touch(int t) {
+    const int64_t w = size.load();
+    for (int64_t i = n * t / w, e = n * (t + 1) / w; i < e; i += 512) {
+      volatile double* p = out + i;
+      *p = *p;
+    }
+    touched.fetch_add(1);
+  }
+  template <class Cond>
+  bool wait(Cond cond) {
+    for (int spin = 0; !cond(); ++spin) {
+      if (stop) return false;
+      if (spin < 64) std::this_thread::yield();
+      else std::this_thread::sleep_for(std::chrono::microseconds(20));
+    }
+    return true;
+  }
+  void work(int t) {
+    if (!wait([&] { return size.load() > 0; })) return;
+    if (cprod)
+      for (int64_t k = 0; k < (int64_t)chunks.size(); ++k) {
+        if (!wait([&] { return gather_to.load() >= k; })) return;
+        gather(t, k);
+      }
+    touch(t);
+    for (int p = 0; p < pieces; ++p) {
+      if (!wait([&] { return add_to.load() >= p; })) return;
+      add(t, p);
+    }
+  }
+};
 
 extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ldc,
                                    int64_t npair, int32_t nbas, const double* ediff,
@@ -579,19 +649,45 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
   // multiples of that slab and the result equals the device call's bit for bit.
   int plan[3] = {0, 0, kPbDefaultTile};
   if (precision == SPX_SPLIT) split_choice(ctx, nbas, npair, nw, &plan[0], &plan[1], &plan[2]);
-  const int64_t align = precision == SPX_SPLIT ? (plan[1] > 0 ? plan[1] : 32768) : 16384;
+  const int64_t align = precision == SPX_SPLIT ? (plan[1] > 0 ? plan[1] : 32768) : 256;
   // slab size: band pairs per streamed chunk
-  // By default the first chunk is short, since its copy overlaps nothing; the
-  // chunks then grow by an eighth each time, up to 262144 pairs (a chunk's copy, about
-  // 0.35-0.4 us per pair at N = 1200 over PCIe 5, against about 0.32-0.38 us of
-  // accumulation), and halve again over the last quarter or so, so that little
-  // accumulation is left once the last copy has landed. Pageable arrays keep
-  // 65536-pair chunks so that their pinned staging stays small.
+  // By default the first chunk is short, since its copy overlaps nothing.
+  //   * FP64 chunks start at 8 MB and double: the accumulation is the slower stream, and its
+  //     kernels need no particular boundary. Measured from pageable arrays at 400 functions,
+  //     12800 pairs, 12 frequencies: 8-10 ms as one chunk gathered before its copy, 4.6 ms in
+  //     chunks gathered beside the copies and the accumulation (2.8 ms of it).
+  //   * Split chunks grow by an eighth each time, up to 262144 pairs (a chunk's copy, about
+  //     0.35-0.4 us per pair at N = 1200 over PCIe 5, against about 0.32-0.38 us of
+  //     accumulation).
+  // They halve again over the last quarter or so, so that little accumulation is left once
+  // the last copy has landed. Pageable arrays keep 65536-pair chunks at most so that their
+  // pinned staging stays small.
   const bool ramp = ctx->opt.chunk_pairs <= 0;
   int64_t slab = ctx->opt.chunk_pairs > 0 ? ctx->opt.chunk_pairs : (pinned ? 262144 : 65536);
   slab = std::min<int64_t>(slab, npair);
   slab = (int64_t)align_up((size_t)slab, 16);
-  const int64_t first = ramp ? std::min<int64_t>(slab, (int64_t)align_up(16384, (size_t)align)) : slab;
+  const int64_t first_pairs =
+      precision == SPX_FP64
+          ? (int64_t)align_up((size_t)std::min<int64_t>(16384, std::max<int64_t>(256, (8 << 20) / (16 * (int64_t)nbas))), 256)
+          : (int64_t)align_up(16384, (size_t)align);
+  const int64_t first = ramp ? std::min<int64_t>(slab, first_pairs) : slab;
+  HostCrew crew;
+  int64_t longest = 0;
+  for (int64_t p0 = 0, len = 0; p0 < npair; p0 += len) {
+    int64_t want = first;
+    if (p0 > 0 && ramp)
+      want = std::min<int64_t>(slab, (int64_t)align_up((size_t)(precision == SPX_FP64 ? 2 * len : len + len / 8),
+                                                       (size_t)align));
+    // near the end the chunks halve: the accumulation left after the last copy lands
+    // is that of a short chunk (the copies are the slower stream over PCIe)
+    const int64_t left = npair - p0;
+    if (ramp && p0 > 0 && left <= 2 * want)
+      want = std::max<int64_t>(align, (int64_t)align_up((size_t)((left + 1) / 2), (size_t)align));
+    len = std::min<int64_t>(want, left);
+    crew.chunks.push_back({p0, len});
+    longest = std::max(longest, len);
+  }
+  slab = (int64_t)align_up((size_t)longest, 16);   // the buffers hold the longest chunk
   const int nslab_buf = 3;  // chunk k's copy waits only for chunk k-3's accumulation
   const int64_t npack = (int64_t)nbas * (nbas + 1) / 2;
   const size_t out_bytes = align_up(sizeof(double) * 2 * (size_t)npack * nw, 256);
@@ -647,35 +743,37 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
   // rest of the call waits for the host copies
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
-  const int nthr = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-  int64_t k = 0;
-  int64_t len = 0;
-  for (int64_t p0 = 0; p0 < npair; p0 += len, ++k) {
+  if (!pinned) {
+    crew.cprod = cprod;
+    crew.ldc = ldc;
+    crew.nbas = nbas;
+    for (int b = 0; b < nslab_buf; ++b) crew.stage[b] = stage + (size_t)b * (slab_bytes / sizeof(double));
+  }
+  crew.out = susceph;
+  crew.sums = (const double*)ctx->pinned;
+  crew.n = 2 * npack * nw;
+  // the sums come back and are added in pieces (not worth it below a few megabytes)
+  crew.pieces = out_host_bytes > ((size_t)4 << 20) ? 4 : 1;
+  crew.start((int)std::max(1u, std::min(8u, std::thread::hardware_concurrency())));
+  for (int64_t k = 0; k < (int64_t)crew.chunks.size(); ++k) {
     const int b = (int)(k % nslab_buf);
-    int64_t want =
-        k == 0 ? first
-               : (ramp ? std::min<int64_t>(slab, (int64_t)align_up((size_t)(len + len / 8), (size_t)align))
-                       : slab);
-    // near the end the chunks halve: the accumulation left after the last copy lands
-    // is that of a short chunk (the copies are the slower stream over PCIe)
-    const int64_t left = npair - p0;
-    if (ramp && k > 0 && left <= 2 * want)
-      want = std::max<int64_t>(align, (int64_t)align_up((size_t)((left + 1) / 2), (size_t)align));
-    len = std::min<int64_t>(want, left);
-    cudaStreamWaitEvent(xs, ev_free[b], 0);
+    const int64_t p0 = crew.chunks[(size_t)k].p0, len = crew.chunks[(size_t)k].len;
     const size_t bytes = sizeof(double) * 2 * (size_t)len;
-    if (pinned) {
+    if (!pinned) {
+      // the staging part `b` is free once the copy of chunk k - 3 out of it has finished
+      if (k >= nslab_buf) cudaEventSynchronize(ev_copied[b]);
+      crew.gather_to = k;
+      crew.gather(0, k);
+      crew.wait([&] { return crew.gathered.load() >= (k + 1) * crew.size.load(); });
+    }
+    cudaStreamWaitEvent(xs, ev_free[b], 0);
+    if (pinned)
       rc = check_cuda(ctx, cudaMemcpy2DAsync(d_slab[b], bytes, cprod + 2 * p0, sizeof(double) * 2 * ldc,
                                              bytes, nbas, cudaMemcpyHostToDevice, xs),
                       "copy cprod slab");
-    } else {
-      // the staging part `b` is free once the previous copy out of it finished
-      cudaEventSynchronize(ev_free[b]);
-      double* st = stage + (size_t)b * (slab_bytes / sizeof(double));
-      gather_slab(cprod, ldc, p0, len, nbas, st, nthr);
-      rc = check_cuda(ctx, cudaMemcpyAsync(d_slab[b], st, bytes * nbas, cudaMemcpyHostToDevice, xs),
+    else
+      rc = check_cuda(ctx, cudaMemcpyAsync(d_slab[b], crew.stage[b], bytes * nbas, cudaMemcpyHostToDevice, xs),
                       "copy cprod slab");
-    }
     if (rc) {
       ctx->timing = false;
       return rc;
@@ -699,25 +797,27 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
     cudaEventRecord(ev_free[b], cs);
   }
   ctx->timing = false;
-  double* sums = (double*)ctx->pinned;
-  if ((rc = check_cuda(ctx, cudaMemcpyAsync(sums, d_out, out_host_bytes, cudaMemcpyDeviceToHost, cs),
-                       "copy the sums back")))
-    return rc;
-  d2h += out_host_bytes;
-  rc = collect_status(ctx, cs, "chi0_accumulate");
+  crew.touch(0);
+  rc = collect_status(ctx, cs, "chi0_accumulate");   // nothing is added after a failure
   if (rc) return rc;
-  {
-    // susceph += sums, on the host threads
-    const int64_t n = 2 * npack * nw;
-    auto add = [&](int t) {
-      const int64_t a = n * t / nthr, e = n * (t + 1) / nthr;
-      for (int64_t i = a; i < e; ++i) susceph[i] += sums[i];
-    };
-    std::vector<std::thread> th;
-    for (int t = 1; t < nthr; ++t) th.emplace_back(add, t);
-    add(0);
-    for (auto& x : th) x.join();
+  cudaEvent_t ev_piece[4] = {ctx->ev[8], ctx->ev[9], ctx->ev[10], ctx->ev[11]};
+  double* sums = (double*)ctx->pinned;
+  for (int i = 0; i < crew.pieces; ++i) {
+    const int64_t a0 = crew.n * i / crew.pieces, a1 = crew.n * (i + 1) / crew.pieces;
+    if ((rc = check_cuda(ctx, cudaMemcpyAsync(sums + a0, (const double*)d_out + a0, sizeof(double) * (a1 - a0),
+                                              cudaMemcpyDeviceToHost, cs),
+                         "copy the sums back")) ||
+        (rc = check_cuda(ctx, cudaEventRecord(ev_piece[i], cs), "event")))
+      return rc;
   }
+  d2h += out_host_bytes;
+  crew.wait([&] { return crew.touched.load() >= crew.size.load(); });   // no page is being touched any more
+  for (int i = 0; i < crew.pieces; ++i) {
+    if ((rc = check_cuda(ctx, cudaEventSynchronize(ev_piece[i]), "copy the sums back"))) return rc;
+    crew.add_to = i;   // susceph += sums
+    crew.add(0, i);
+  }
+  crew.wait([&] { return crew.added.load() >= crew.pieces * crew.size.load(); });
   if (stats) {
     timing_collect(ctx, &stats->ms_prep, &stats->ms_gram);
     stats->h2d_bytes = h2d;

@@ -424,11 +424,11 @@ def susceptibility(ctx: Context, cprod: np.ndarray, ediff: np.ndarray, frqh: np.
     nw = omega.shape[0]
     susceph = np.zeros((npack(nbas), nw), dtype=np.complex128, order="F")   # intent(out), zeroed
     wscale = None if nkpts is None else np.asarray(nkpts, dtype=np.float64)
-    scale_all = 1.0 / nkpt / nsym1
+    # the spin factor 2 (src/susceptibility.f:1336) goes into the pair weights: a power of two,
+    # so every sum is the doubled one bit for bit, without a pass over the output
+    scale_all = (1.0 if l_soc or nspin != 1 else 2.0) * (1.0 / nkpt / nsym1)
     for (b, e) in (packets or [(0, npair)]):
         ctx.chi0_accumulate(np.asfortranarray(cprod[b:e]), ediff[b:e], omega, susceph,
                             wscale=None if wscale is None else wscale[b:e], scale_all=scale_all,
                             precision=precision)
-    if not l_soc and nspin == 1:
-        susceph *= 2.0                                                        # :1336
     return susceph
