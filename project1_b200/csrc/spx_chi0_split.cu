@@ -1403,11 +1403,10 @@ int split_chi0_real_ediff(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P,
 // products with t + u <= 3 are summed exactly in int32 (k <= 32768 per launch),
 // so the only rounding is the slicing: 2^-17/127 of A's row scale per value, so
 // |error of C(m, col)| <= 2^-17/127 * crest(A_m) * ||A_m|| ||B_col||.
-// Items are rectangular (batch, column tile, row tile), row tiles fastest so that
-// concurrent CTAs share the large B tile through L2. The epilogue stages alpha times
-// the tile in shared memory and writes (or adds) it into cprod's columns as runs of
-// 32 consecutive complex values.
-
+// Items are rectangular (batch, column tile, row tile) of 64 x 64 complex values, row tiles
+// fastest so that concurrent CTAs share the large B tile through L2. Both operands use K2's
+// interleaved rows, so the fragments of a row's two parts meet in neighbouring lanes and a
+// warp's values of one column are 256 contiguous bytes of cprod.
 namespace spx {
 
 struct SgParams {
@@ -1424,47 +1423,36 @@ struct SgParams {
   uint64_t timeout_ns;
 };
 
-// The same GEMM with 32-column tiles (N = 64 real rows of B, stacked in 32-blocks)
-// and two TMEM buffers of 4 orders x 64 columns: the MMAs of item j+1 run while the
-// epilogue drains item j, which the short K of the product GEMM needs (47 stages at
-// 3000 plane waves, against 512 for K2).
-constexpr int SG_TB = 32;                        // complex B rows per tile
+// One CTA per tile: MMAs of N = 128 (an MMA of N = 64 takes the same time, bound by the
+// instruction rate: 32-column tiles with two TMEM buffers took 40 ms of the 27 x 300 x 40560 x
+// 3000 products, this form 24 ms). The four orders of 128 columns fill TMEM, so the next
+// tile's MMAs wait while eight epilogue warps read it into registers (about 3 % of a tile's 47
+// stages); scaling and stores run beside them.
 constexpr int SG_ST = 4;
-constexpr int SG_BPLANE = 2 * SG_TB * SP_KB;     // 4096 bytes
-constexpr uint32_t SG_IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(2 * SG_TB / 8) << 17) |
-                              ((uint32_t)(SP_ROWS / 16) << 24);
 
 struct __align__(1024) SgSmem {
   uint8_t a[SG_ST][SP_SA][SP_PLANE];
-  uint8_t b[SG_ST][SP_SB][SG_BPLANE];
-  long long xchg[2][SP_TILE][SG_TB];   // the Re-row and Im-row products, column k ^ (row & 15)
-  double2 stage[SP_TILE][SG_TB];       // the output tile, column k ^ (row & 31)
+  uint8_t b[SG_ST][SP_SB][SP_PLANE];
   uint64_t full[SG_ST];
   uint64_t empty[SG_ST];
-  uint64_t tfull[2], tempty[2];
-  uint64_t xfull, xstage, xfree, mdone;
+  uint64_t tfull, tempty, mdone;
   uint32_t tmem_base;
 };
 
-// T = ((D0*256 + D1)*256 + D2)*256 + D3 for 32 columns, orders 64 columns apart.
-__device__ __forceinline__ void load_orders64(uint32_t taddr, long long (&T)[32]) {
-  int32_t r[32];
-  tmem_ld32(taddr, r);
+// T = ((D0*256 + D1)*256 + D2)*256 + D3 for 16 columns, orders 128 columns apart.
+__device__ __forceinline__ void load_orders16(uint32_t taddr, long long (&T)[16]) {
+  int32_t r[4][16];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) tmem_ld16(taddr + (uint32_t)(g * SP_ROWS), r[g]);
   tmem_wait_ld();
 #pragma unroll
-  for (int k = 0; k < 32; ++k) T[k] = r[k];
-#pragma unroll
-  for (int g = 1; g < 4; ++g) {
-    tmem_ld32(taddr + (uint32_t)(g * 64), r);
-    tmem_wait_ld();
-#pragma unroll
-    for (int k = 0; k < 32; ++k) T[k] = T[k] * 256 + r[k];
-  }
+  for (int k = 0; k < 16; ++k)
+    T[k] = (((long long)r[0][k] * 256 + r[1][k]) * 256 + r[2][k]) * 256 + r[3][k];
 }
 
-__global__ void __launch_bounds__(SP_THREADS, 1)
-    split_gemm2_kernel(const __grid_constant__ CUtensorMap mapA,
-                       const __grid_constant__ CUtensorMap mapB, SgParams prm) {
+__global__ void __launch_bounds__(SP1_THREADS, 1)
+    split_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                      SgParams prm) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   SgSmem& sm = *reinterpret_cast<SgSmem*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -1474,13 +1462,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
       mbar_init(&sm.full[s], 1);
       mbar_init(&sm.empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&sm.tfull[b], 1);
-      mbar_init(&sm.tempty[b], 4);
-    }
-    mbar_init(&sm.xfull, 4);
-    mbar_init(&sm.xstage, 4);
-    mbar_init(&sm.xfree, 4);
+    mbar_init(&sm.tfull, 1);
+    mbar_init(&sm.tempty, SP1_EPI);
     mbar_init(&sm.mdone, 1);
     fence_barrier_init();
   }
@@ -1492,6 +1475,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
   const int mtiles = prm.mtiles, ntiles = prm.ntiles;
 
   if (warp == 0) {
+    // ---------------- TMA producer ----------------
     if (lane == 0) {
       int st = 0;
       uint32_t ph = 0;
@@ -1501,13 +1485,13 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
       bool ok = true;
       for (int item = blockIdx.x; item < prm.nitems && ok; item += gridDim.x) {
         const int mt = item % mtiles, r = item / mtiles, ct = r % ntiles, b = r / ntiles;
-        const int ra = (int)(b * prm.RA) + mt * SP_ROWS, rb = (int)(b * prm.RB) + ct * (2 * SG_TB);
+        const int ra = (int)(b * prm.RA) + mt * SP_ROWS, rb = (int)(b * prm.RB) + ct * SP_ROWS;
         for (int ks = 0; ks < prm.nk; ++ks) {
           if (!mbar_wait(&sm.empty[st], ph ^ 1u, prm.timeout_ns, prm.status)) {
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(&sm.full[st], (uint32_t)(SP_SA * SP_PLANE + SP_SB * SG_BPLANE));
+          mbar_arrive_expect_tx(&sm.full[st], (uint32_t)((SP_SA + SP_SB) * SP_PLANE));
           tma_load_4d(&sm.a[st][0][0], &mapA, 0, ra, ks, 0, &sm.full[st]);
           tma_load_4d(&sm.b[st][0][0], &mapB, 0, rb, ks, 0, &sm.full[st]);
           issued[st] = true;
@@ -1519,17 +1503,16 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
         if (issued[s]) mbar_drain(&sm.full[s], last_ph[s], prm.timeout_ns);
     }
   } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
     if (lane == 0) {
       int st = 0;
       uint32_t ph = 0;
       int j = 0;
       bool committed = false;
       for (int item = blockIdx.x; item < prm.nitems; item += gridDim.x, ++j) {
-        const int buf = j & 1;
-        // this buffer's previous item (j - 2) has been drained (first use: immediately)
-        if (!mbar_wait(&sm.tempty[buf], (uint32_t)((j >> 1) & 1) ^ 1u, prm.timeout_ns, prm.status)) break;
+        // the previous item's accumulators have been read (first item: immediately)
+        if (!mbar_wait(&sm.tempty, (uint32_t)(j & 1) ^ 1u, prm.timeout_ns, prm.status)) break;
         tc_fence_after();
-        const uint32_t tb = tmem + (uint32_t)(buf * 256);
         bool ok = true;
         for (int ks = 0; ks < prm.nk; ++ks) {
           if (!mbar_wait(&sm.full[st], ph, prm.timeout_ns, prm.status)) {
@@ -1545,22 +1528,22 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
 #pragma unroll
             for (int u = 0; u < SP_SB; ++u) db[u] = desc_sw64(&sm.b[st][u][0]) + (uint64_t)(kk * 2);
             const uint32_t k0 = (ks > 0 || kk > 0);
-            mma_i8<1>(tb + 0 * 64, da[0], db[0], SG_IDESC, k0);
-            mma_i8<2>(tb + 1 * 64, da[0], db[1], SG_IDESC, k0);
-            mma_i8<2>(tb + 2 * 64, da[0], db[2], SG_IDESC, k0);
-            mma_i8<3>(tb + 3 * 64, da[0], db[3], SG_IDESC, k0);
-            mma_i8<1>(tb + 1 * 64, da[1], db[0], SG_IDESC, 1u);
-            mma_i8<2>(tb + 2 * 64, da[1], db[1], SG_IDESC, 1u);
-            mma_i8<3>(tb + 3 * 64, da[1], db[2], SG_IDESC, 1u);
-            mma_i8<1>(tb + 2 * 64, da[2], db[0], SG_IDESC, 1u);
-            mma_i8<3>(tb + 3 * 64, da[2], db[1], SG_IDESC, 1u);
+            mma_i8<1>(tmem + 0 * SP_ROWS, da[0], db[0], SP_IDESC, k0);
+            mma_i8<2>(tmem + 1 * SP_ROWS, da[0], db[1], SP_IDESC, k0);
+            mma_i8<2>(tmem + 2 * SP_ROWS, da[0], db[2], SP_IDESC, k0);
+            mma_i8<3>(tmem + 3 * SP_ROWS, da[0], db[3], SP_IDESC, k0);
+            mma_i8<1>(tmem + 1 * SP_ROWS, da[1], db[0], SP_IDESC, 1u);
+            mma_i8<2>(tmem + 2 * SP_ROWS, da[1], db[1], SP_IDESC, 1u);
+            mma_i8<3>(tmem + 3 * SP_ROWS, da[1], db[2], SP_IDESC, 1u);
+            mma_i8<1>(tmem + 2 * SP_ROWS, da[2], db[0], SP_IDESC, 1u);
+            mma_i8<3>(tmem + 3 * SP_ROWS, da[2], db[1], SP_IDESC, 1u);
           }
           tc_commit(&sm.empty[st]);
           committed = true;
           if (++st == SG_ST) st = 0, ph ^= 1u;
         }
         if (!ok) break;
-        tc_commit(&sm.tfull[buf]);
+        tc_commit(&sm.tfull);
       }
       if (committed) {
         tc_commit(&sm.mdone);
@@ -1568,73 +1551,45 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
       }
     }
   } else {
-    const int q = warp & 3;
-    const bool is_re = q < 2;
-    const int ii = (q & 1) * 32 + lane;
-    const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+    // ---- epilogue: two warps per TMEM lane quarter, 32 complex columns each ----
+    const int q = warp & 3, h = (warp - 2) >> 2, c = lane & 1;
+    const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(SP_TILE * h);
     int j = 0;
-    uint32_t xseq = 0;
-    for (int item = blockIdx.x; item < prm.nitems; item += gridDim.x, ++j, ++xseq) {
-      const int buf = j & 1;
-      if (!mbar_wait_idle(&sm.tfull[buf], (uint32_t)((j >> 1) & 1), prm.timeout_ns, prm.status)) break;
+    for (int item = blockIdx.x; item < prm.nitems; item += gridDim.x, ++j) {
+      if (!mbar_wait_idle(&sm.tfull, (uint32_t)(j & 1), prm.timeout_ns, prm.status)) break;
       tc_fence_after();
       const int mt = item % mtiles, r = item / mtiles, ct = r % ntiles, b = r / ntiles;
-      long long tre[32], tim[32];
-      load_orders64(tl + (uint32_t)(buf * 256), tre);
-      load_orders64(tl + (uint32_t)(buf * 256 + SG_TB), tim);
-      // the buffer is read: the MMAs of item j + 2 may overwrite it
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.tempty[buf]);
-      const int gm = mt * SP_TILE + ii;
-      const double fac = prm.alpha * prm.sA[(int64_t)b * mtiles * SP_TILE + gm] *
-                         (1.0 / (127.0 * 127.0 * 16777216.0));
-      const double* sbb = prm.sB + (int64_t)b * ntiles * SG_TB;
-      // the previous tile's staged values have been written out
-      if (!mbar_wait(&sm.xfree, (xseq & 1u) ^ 1u, prm.timeout_ns, prm.status)) break;
+      long long o[SP_TILE / 2];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) sm.xchg[is_re ? 0 : 1][ii][k ^ (ii & 15)] = tim[k];
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.xfull);
-      if (!mbar_wait(&sm.xfull, xseq & 1u, prm.timeout_ns, prm.status)) break;
-      // this thread's part (Re or Im) of row ii, 32 columns, into the staged tile
-      double* st = reinterpret_cast<double*>(&sm.stage[ii][0]) + (is_re ? 0 : 1);
+      for (int cc = 0; cc < SP_TILE / 16; ++cc) {
+        long long T[16];
+        load_orders16(tl + (uint32_t)(16 * cc), T);
 #pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        const long long partner = sm.xchg[is_re ? 1 : 0][ii][k ^ (ii & 15)];
-        const long long v = is_re ? tre[k] + partner : tre[k] - partner;
-        st[2 * (k ^ lane)] = fac * sbb[ct * SG_TB + k] * (double)v;
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.xstage);
-      if (!mbar_wait(&sm.xstage, xseq & 1u, prm.timeout_ns, prm.status)) break;
-      // write out: warp q takes columns q, q + 4, ...; a lane one row of the two 32-row
-      // halves, so each store is 32 consecutive complex values of one cprod column
-      // (whole 32-byte sectors). Each element belongs to one thread of one launch.
-      double2* ob = reinterpret_cast<double2*>(prm.out) + b * prm.sO2 + mt * SP_TILE;
-#pragma unroll 2
-      for (int k = q; k < SG_TB; k += 4) {
-        const int gc = ct * SG_TB + k;
-        if (gc >= prm.ncol) break;
-        const int n = gc / prm.ncin, c = gc - n * prm.ncin;
-        double2* oc = ob + n * prm.sOn + c * prm.sOc;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int row = 32 * h + lane;
-          if (mt * SP_TILE + row >= prm.M) continue;
-          const double2 v = sm.stage[row][k ^ lane];
-          if (prm.overwrite) {
-            oc[row] = v;
-          } else {
-            double2 o = oc[row];
-            o.x += v.x;
-            o.y += v.y;
-            oc[row] = o;
-          }
+        for (int jj = 0; jj < 8; ++jj) {
+          // A conj(B): re = ArBr + AiBi (even lanes), im = AiBr - ArBi
+          const long long pb = __shfl_xor_sync(0xffffffffu, T[2 * jj + 1], 1);
+          o[8 * cc + jj] = c == 0 ? T[2 * jj] + pb : T[2 * jj] - pb;
         }
       }
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.xfree);
+      if (lane == 0) mbar_arrive(&sm.tempty);
+      const int gm = mt * SP_TILE + 16 * q + lane / 2;
+      if (gm >= prm.M) continue;
+      const double fac = prm.alpha * prm.sA[(int64_t)b * mtiles * SP_TILE + gm] *
+                         (1.0 / (127.0 * 127.0 * 16777216.0));
+      const int gc0 = ct * SP_TILE + 32 * h;
+      const double* sbb = prm.sB + (int64_t)b * ntiles * SP_TILE + gc0;
+      int n = gc0 / prm.ncin, cin = gc0 - n * prm.ncin;
+      double* ob = prm.out + 2 * (b * prm.sO2 + gm) + c;
+#pragma unroll
+      for (int k = 0; k < SP_TILE / 2; ++k) {
+        if (gc0 + k >= prm.ncol) break;
+        double* oc = ob + 2 * (n * prm.sOn + cin * prm.sOc);
+        const double v = fac * sbb[k] * (double)o[k];
+        *oc = prm.overwrite ? v : *oc + v;
+        if (++cin == prm.ncin) cin = 0, ++n;
+      }
     }
   }
   tc_fence_before();
@@ -1643,26 +1598,78 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
   if (warp == 1) tmem_dealloc(tmem, SP_TMEM_COLS);
 }
 
-// Row sources of the two operands: A rows are contiguous in k, B rows are gathered.
+// Row sources of the two operands, k running through the caller's order of the plane
+// waves (the box order of their G vectors, so that a row's gather walks the convolved grid
+// upwards; the integer sums do not depend on it): A rows of cpw, B rows of the grid.
 struct SgSrcRows {
   const double2* base;
   int64_t ld, bstride;
+  const int* kperm;         // plane wave of the k-th position
   __device__ __forceinline__ double2 get(int b, int r, int k) const {
-    return base[b * bstride + (int64_t)r * ld + k];
+    return __ldg(base + b * bstride + (int64_t)r * ld + kperm[k]);
   }
 };
 struct SgSrcGather {
   const double2* grid;      // [batch][n][box]
   int64_t bstride, nstride;
   const int64_t* coff;      // per c
-  const int* koff;          // per k
+  const int* koff;          // per position k
   int ncin;
   __device__ __forceinline__ double2 get(int b, int r, int k) const {
     const int n = r / ncin, c = r - n * ncin;
-    return grid[b * bstride + n * nstride + coff[c] + koff[k]];
+    return __ldg(grid + b * bstride + n * nstride + coff[c] + koff[k]);
   }
 };
 
+// One CTA per row of up to SGP_K values: the row's scale max_k max(|Re|, |Im|) (0 for padding
+// rows) and its S digits in one pass over its (gathered) values, kept in registers between.
+// A thread holds four runs of four consecutive k; planes [t][k-block][row][64 B] as below.
+// Bound by the gather through L2 (53 GB in 16-byte pieces for the 27 x 40560 rows of 3000):
+// 17 ms, against 26 ms as a pass for the scales and one for the digits, plane waves in the
+// caller's order.
+constexpr int SGP_T = 256, SGP_K = 16 * SGP_T;
+template <int S, class Src>
+__global__ void __launch_bounds__(SGP_T)
+    sgemm_prep_kernel(Src src, int rows, int rows_pad, int K, int nkb, int nbatch, int64_t R,
+                      double* __restrict__ s, int8_t* __restrict__ planes) {
+  __shared__ double red[SGP_T / 32];
+  const int r = blockIdx.x, b = blockIdx.y;
+  double2 v[16];
+  double m = 0.0;
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const int k = 4 * (threadIdx.x + SGP_T * (e >> 2)) + (e & 3);
+    v[e] = r < rows && k < K ? src.get(b, r, k) : make_double2(0.0, 0.0);
+    m = fmax(m, fmax(fabs(v[e].x), fabs(v[e].y)));
+  }
+  m = block_max(m, red);
+  if (threadIdx.x == 0) s[(int64_t)b * rows_pad + r] = m;
+  const double inv = m > 0.0 ? 127.0 * (S == 4 ? 16777216.0 : 65536.0) / m : 0.0;
+  const int64_t rows_total = (int64_t)nbatch * R;
+  const int64_t pstride = (int64_t)nkb * rows_total * SP_KB;
+  const int64_t row = ((int64_t)b * R + split_row_re(r)) * SP_KB;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k = 4 * (threadIdx.x + SGP_T * q);
+    if (k >= nkb * SP_KB) break;
+    uint32_t yr[4], yi[4], pr[S], pi[S];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      yr[e] = round_mul(v[4 * q + e].x, inv);
+      yi[e] = round_mul(v[4 * q + e].y, inv);
+    }
+    digit_planes<S>(yr, pr);
+    digit_planes<S>(yi, pi);
+    const int64_t o = (int64_t)(k / SP_KB) * rows_total * SP_KB + row + k % SP_KB;
+#pragma unroll
+    for (int t = 0; t < S; ++t) {
+      *reinterpret_cast<uint32_t*>(planes + o + t * pstride) = pr[t];
+      *reinterpret_cast<uint32_t*>(planes + o + SP_KB + t * pstride) = pi[t];
+    }
+  }
+}
+
+// Longer rows take two passes:
 // s[b*rows_pad + r] = max_k max(|Re|, |Im|) of row r of batch b (0 for padding rows).
 template <class Src>
 __global__ void sgemm_rowmax_kernel(Src src, int rows, int rows_pad, int K, double* s) {
@@ -1684,10 +1691,10 @@ __global__ void sgemm_rowmax_kernel(Src src, int rows, int rows_pad, int K, doub
   }
 }
 
-// S digits of round(x * 127/s * 2^(8(S-1))) into planes [t][k-block][row][64 B] with
-// real-stacked rows b*R + 2 TB (r/TB) + {r%TB Re, TB + r%TB Im}. One thread = one row
-// and 16 consecutive k; a warp = 8 consecutive rows x the 4 quarters of a k-block.
-template <int S, int TB, class Src>
+// S digits of round(x * 127/s * 2^(8(S-1))) into planes [t][k-block][row][64 B] with K2's
+// interleaved rows (split_row_re). One thread = one row and 16 consecutive k; a warp = 8
+// consecutive rows x the 4 quarters of a k-block.
+template <int S, class Src>
 __global__ void __launch_bounds__(128)
     sgemm_quant_kernel(Src src, int rows, int rows_pad, int K, int nkb, int nbatch, int64_t R,
                        const double* __restrict__ s, int8_t* __restrict__ planes) {
@@ -1701,10 +1708,10 @@ __global__ void __launch_bounds__(128)
   const int kb = (int)(kbb % nkb), b = (int)(kbb / nkb);
   const int k0 = kb * SP_KB + quarter * 16;
   const int64_t rows_total = (int64_t)nbatch * R;
-  const int64_t rr = (int64_t)b * R + (r / TB) * (2 * TB) + (r % TB);
+  const int64_t rr = (int64_t)b * R + split_row_re(r);
   const int64_t pstride = (int64_t)nkb * rows_total * SP_KB;
   const int64_t o_re = ((int64_t)kb * rows_total + rr) * SP_KB + quarter * 16;
-  const int64_t o_im = o_re + (int64_t)TB * SP_KB;
+  const int64_t o_im = o_re + SP_KB;
   const double sc = r < rows ? s[(int64_t)b * rows_pad + r] : 0.0;
   const double inv = sc > 0.0 ? 127.0 * (S == 4 ? 16777216.0 : 65536.0) / sc : 0.0;
   uint32_t wr[S][4], wi[S][4];
@@ -1733,8 +1740,7 @@ __global__ void __launch_bounds__(128)
 
 // Bytes of scratch for one launch group of `nbatch` batches (planes and scales).
 size_t sgemm_workspace_bytes(int nbatch, int M, int ncol, int K) {
-  const int64_t mt = (M + SP_TILE - 1) / SP_TILE, nt2 = (ncol + SG_TB - 1) / SG_TB;
-  const int64_t nt = (nt2 + 1) / 2;  // in 64-row units: B has 2 SG_TB rows per tile
+  const int64_t mt = (M + SP_TILE - 1) / SP_TILE, nt = (ncol + SP_TILE - 1) / SP_TILE;
   const int64_t kp = (int64_t)align_up((size_t)std::min(std::max(K, 1), SP_SLAB), SP_KB);
   return align_up((size_t)SP_SA * kp * nbatch * mt * SP_ROWS, 1024) +
          align_up((size_t)SP_SB * kp * nbatch * nt * SP_ROWS, 1024) +
@@ -1743,26 +1749,23 @@ size_t sgemm_workspace_bytes(int nbatch, int M, int ncol, int K) {
 }
 
 // The interstitial product GEMM on int8 slices for `nbatch` k points: A rows from
-// cpw_unocc (contiguous), B rows gathered from the convolved grids.
+// cpw_unocc (plane waves in the order kperm), B rows gathered from the convolved grids at
+// the offsets koff of the same order.
 int sgemm_products(spx_ctx* ctx, int nbatch, int M, int ncol, int K, const double2* A,
-                   int64_t lda, int64_t a_bstride, const double2* grid, int64_t g_bstride,
-                   int64_t g_nstride, const int64_t* coff, const int* koff, int ncin,
-                   double2* out, int64_t sO2, int64_t sOn, int64_t sOc, double alpha, void* ws,
-                   size_t ws_bytes, cudaStream_t s, int* launches, bool overwrite) {
+                   int64_t lda, int64_t a_bstride, const int* kperm, const double2* grid,
+                   int64_t g_bstride, int64_t g_nstride, const int64_t* coff, const int* koff,
+                   int ncin, double2* out, int64_t sO2, int64_t sOn, int64_t sOc, double alpha,
+                   void* ws, size_t ws_bytes, cudaStream_t s, int* launches, bool overwrite) {
   if (nbatch <= 0 || M <= 0 || ncol <= 0 || K <= 0) return SPX_OK;
-  const int mt = (M + SP_TILE - 1) / SP_TILE, nt = (ncol + SG_TB - 1) / SG_TB;
-  const int64_t RA = (int64_t)mt * SP_ROWS, RB = (int64_t)nt * 2 * SG_TB;
+  const int mt = (M + SP_TILE - 1) / SP_TILE, nt = (ncol + SP_TILE - 1) / SP_TILE;
+  const int64_t RA = (int64_t)mt * SP_ROWS, RB = (int64_t)nt * SP_ROWS;
   if ((int64_t)nbatch * RB > 2147483647LL || (int64_t)nbatch * mt * nt > 2147483647LL)
     return set_error(ctx, SPX_EINVAL, "product GEMM too large for one launch group");
   uint8_t* base = (uint8_t*)align_up((size_t)ws, 1024);
   const size_t need = sgemm_workspace_bytes(nbatch, M, ncol, K);
   if (!ws || ws_bytes < need + 1024) return set_error(ctx, SPX_ENOMEM, "split product scratch too small");
   const size_t smem = sizeof(SgSmem) + 1024;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(split_gemm2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
-  }
+  cudaFuncSetAttribute(split_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int rc;
   // k is cut into exact int32 slabs of at most 32768; each slab adds into the output
   for (int kbeg = 0; kbeg < K; kbeg += SP_SLAB) {
@@ -1773,17 +1776,22 @@ int sgemm_products(spx_ctx* ctx, int nbatch, int M, int ncol, int K, const doubl
     int8_t* PB = (int8_t*)(base + align_up((size_t)SP_SA * kp * nbatch * RA, 1024));
     double* sA = (double*)((uint8_t*)PB + align_up((size_t)SP_SB * kp * nbatch * RB, 1024));
     double* sB = (double*)((uint8_t*)sA + align_up(sizeof(double) * nbatch * mt * SP_TILE, 256));
-    const int rows_b = nt * SG_TB;  // padded B rows (complex) per batch
-    SgSrcRows sa{A + kbeg, lda, a_bstride};
+    const int rows_a = mt * SP_TILE, rows_b = nt * SP_TILE;  // padded rows (complex) per batch
+    SgSrcRows sa{A, lda, a_bstride, kperm + kbeg};
     SgSrcGather sb{grid, g_bstride, g_nstride, coff, koff + kbeg, ncin};
-    sgemm_rowmax_kernel<<<dim3(mt * SP_TILE, nbatch), 256, 0, s>>>(sa, M, mt * SP_TILE, Ks, sA);
-    sgemm_rowmax_kernel<<<dim3(rows_b, nbatch), 256, 0, s>>>(sb, ncol, rows_b, Ks, sB);
-    const int64_t ta = (int64_t)mt * SP_TILE / 8 * 32 * nkb * nbatch;
-    const int64_t tb = (int64_t)rows_b / 8 * 32 * nkb * nbatch;
-    sgemm_quant_kernel<SP_SA, SP_TILE><<<(unsigned)((ta + 127) / 128), 128, 0, s>>>(sa, M, mt * SP_TILE, Ks, nkb, nbatch, RA, sA, PA);
-    sgemm_quant_kernel<SP_SB, SG_TB><<<(unsigned)((tb + 127) / 128), 128, 0, s>>>(sb, ncol, rows_b, Ks, nkb, nbatch, RB, sB, PB);
+    if (Ks <= SGP_K) {
+      sgemm_prep_kernel<SP_SA><<<dim3(rows_a, nbatch), SGP_T, 0, s>>>(sa, M, rows_a, Ks, nkb, nbatch, RA, sA, PA);
+      sgemm_prep_kernel<SP_SB><<<dim3(rows_b, nbatch), SGP_T, 0, s>>>(sb, ncol, rows_b, Ks, nkb, nbatch, RB, sB, PB);
+      *launches += 2;
+    } else {
+      sgemm_rowmax_kernel<<<dim3(rows_a, nbatch), 256, 0, s>>>(sa, M, rows_a, Ks, sA);
+      sgemm_rowmax_kernel<<<dim3(rows_b, nbatch), 256, 0, s>>>(sb, ncol, rows_b, Ks, sB);
+      const int64_t ta = (int64_t)rows_a / 8 * 32 * nkb * nbatch, tb = (int64_t)rows_b / 8 * 32 * nkb * nbatch;
+      sgemm_quant_kernel<SP_SA><<<(unsigned)((ta + 127) / 128), 128, 0, s>>>(sa, M, rows_a, Ks, nkb, nbatch, RA, sA, PA);
+      sgemm_quant_kernel<SP_SB><<<(unsigned)((tb + 127) / 128), 128, 0, s>>>(sb, ncol, rows_b, Ks, nkb, nbatch, RB, sB, PB);
+      *launches += 4;
+    }
     if ((rc = check_cuda(ctx, cudaGetLastError(), "split product operand preparation"))) return rc;
-    *launches += 4;
     CUtensorMap mapA, mapB;
     const uint64_t rta = (uint64_t)nbatch * RA, rtb = (uint64_t)nbatch * RB;
     const uint64_t da[4] = {SP_KB, rta, (uint64_t)nkb, SP_SA};
@@ -1792,7 +1800,7 @@ int sgemm_products(spx_ctx* ctx, int nbatch, int M, int ncol, int K, const doubl
     if ((rc = make_tmap_u8_4d(ctx, &mapA, PA, da, sta, ba, CU_TENSOR_MAP_SWIZZLE_64B))) return rc;
     const uint64_t db[4] = {SP_KB, rtb, (uint64_t)nkb, SP_SB};
     const uint64_t stb[3] = {SP_KB, rtb * SP_KB, (uint64_t)nkb * rtb * SP_KB};
-    const uint32_t bb[4] = {SP_KB, 2 * SG_TB, 1, SP_SB};
+    const uint32_t bb[4] = {SP_KB, SP_ROWS, 1, SP_SB};
     if ((rc = make_tmap_u8_4d(ctx, &mapB, PB, db, stb, bb, CU_TENSOR_MAP_SWIZZLE_64B))) return rc;
     SgParams prm;
     prm.nbatch = nbatch;
@@ -1816,8 +1824,8 @@ int sgemm_products(spx_ctx* ctx, int nbatch, int M, int ncol, int K, const doubl
     prm.status = ctx->d_status;
     prm.timeout_ns = (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
     const int grid_n = std::min(prm.nitems, ctx->num_sms);
-    split_gemm2_kernel<<<grid_n, SP_THREADS, smem, s>>>(mapA, mapB, prm);
-    if ((rc = check_cuda(ctx, cudaGetLastError(), "split_gemm2_kernel launch"))) return rc;
+    split_gemm_kernel<<<grid_n, SP1_THREADS, smem, s>>>(mapA, mapB, prm);
+    if ((rc = check_cuda(ctx, cudaGetLastError(), "split_gemm_kernel launch"))) return rc;
     *launches += 1;
   }
   return SPX_OK;

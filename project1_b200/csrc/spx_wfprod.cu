@@ -605,10 +605,10 @@ static int plan_pw(spx_ctx* ctx, const spx_pw_desc* d, PwPlan* pl) {
 size_t wfprod_pw_fft_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc);
 size_t sgemm_workspace_bytes(int nbatch, int M, int ncol, int K);
 int sgemm_products(spx_ctx* ctx, int nbatch, int M, int ncol, int K, const double2* A,
-                   int64_t lda, int64_t a_bstride, const double2* grid, int64_t g_bstride,
-                   int64_t g_nstride, const int64_t* coff, const int* koff, int ncin,
-                   double2* out, int64_t sO2, int64_t sOn, int64_t sOc, double alpha, void* ws,
-                   size_t ws_bytes, cudaStream_t s, int* launches, bool overwrite);
+                   int64_t lda, int64_t a_bstride, const int* kperm, const double2* grid,
+                   int64_t g_bstride, int64_t g_nstride, const int64_t* coff, const int* koff,
+                   int ncin, double2* out, int64_t sO2, int64_t sOn, int64_t sOc, double alpha,
+                   void* ws, size_t ws_bytes, cudaStream_t s, int* launches, bool overwrite);
 int wfprod_pw_fft_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int nunocc,
                       const double2* c1, const double2* c2, double2* cprod, int64_t ldc, int col0,
                       void* ws, size_t ws_bytes, cudaStream_t s, int* launches);
@@ -621,7 +621,7 @@ size_t wfprod_pw_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc, b
   size_t perk = align_up(sizeof(double2) * nocc * (size_t)(pl.b1.size() + pl.b0.size()), 256);
   if (split) perk += sgemm_workspace_bytes(1, nunocc, nocc * d->ngptm, d->ngpt2);
   const size_t fixed = align_up(sizeof(int) * std::max(d->ngpt1, 1), 256) +
-                       align_up(sizeof(int) * std::max(d->ngpt2, 1), 256) +
+                       (split ? 2 : 1) * align_up(sizeof(int) * std::max(d->ngpt2, 1), 256) +
                        align_up(sizeof(int64_t) * std::max(d->ngptm, 1), 256) + 4096;
   const size_t budget = (size_t)2 << 30;
   const size_t kchunk = std::max<size_t>(1, std::min<size_t>((size_t)nk, budget / perk));
@@ -648,6 +648,7 @@ int wfprod_pw_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int nuno
   Carve cv{(char*)ws, ws_bytes};
   int* d_gidx = cv.take<int>(d->ngpt1);
   int* d_koff = cv.take<int>(d->ngpt2);
+  int* d_kperm = split ? cv.take<int>(d->ngpt2) : nullptr;
   int64_t* d_coff = cv.take<int64_t>(d->ngptm);
   double2* d_cstep = cv.take<double2>((size_t)pl.ns * pl.ns * pl.ns);
   double2* d_alpha = cv.take<double2>(1);
@@ -661,6 +662,21 @@ int wfprod_pw_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int nuno
   void* sg_ws = split ? (void*)cv.take<uint8_t>(sg_bytes) : nullptr;
   if (!cv.ok) return set_error(ctx, SPX_ENOMEM, "plane-wave scratch too small");
   const double2 alpha = make_double2(1.0 / std::sqrt(d->vol), 0.0);
+  // split: the plane waves of each exact slab in box order, so that a row of the gathered
+  // operand walks the grid upwards in runs along x
+  std::vector<int> kperm;
+  if (split) {
+    kperm.resize(d->ngpt2);
+    for (int i = 0; i < d->ngpt2; ++i) kperm[i] = i;
+    for (int k0 = 0; k0 < d->ngpt2; k0 += 32768)
+      std::sort(kperm.begin() + k0, kperm.begin() + std::min(d->ngpt2, k0 + 32768),
+                [&](int a, int b) { return pl.koff[a] < pl.koff[b]; });
+    std::vector<int> ko(d->ngpt2);
+    for (int i = 0; i < d->ngpt2; ++i) ko[i] = pl.koff[kperm[i]];
+    pl.koff.swap(ko);
+    if (d->ngpt2 && (rc = check_cuda(ctx, cudaMemcpyAsync(d_kperm, kperm.data(), sizeof(int) * d->ngpt2, cudaMemcpyHostToDevice, s), "copy plan")))
+      return rc;
+  }
   if ((d->ngpt1 && (rc = check_cuda(ctx, cudaMemcpyAsync(d_gidx, pl.gidx1.data(), sizeof(int) * d->ngpt1, cudaMemcpyHostToDevice, s), "copy plan"))) ||
       (d->ngpt2 && (rc = check_cuda(ctx, cudaMemcpyAsync(d_koff, pl.koff.data(), sizeof(int) * d->ngpt2, cudaMemcpyHostToDevice, s), "copy plan"))) ||
       (rc = check_cuda(ctx, cudaMemcpyAsync(d_coff, pl.coff.data(), sizeof(int64_t) * d->ngptm, cudaMemcpyHostToDevice, s), "copy plan")) ||
@@ -691,7 +707,7 @@ int wfprod_pw_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int nuno
     if (split) {
       rc = sgemm_products(ctx, kn, nunocc, nocc * d->ngptm, d->ngpt2,
                           c2 + (int64_t)k0 * nunocc * d->ngpt2, d->ngpt2,
-                          (int64_t)nunocc * d->ngpt2, grid0, (int64_t)nocc * pl.b0.size(),
+                          (int64_t)nunocc * d->ngpt2, d_kperm, grid0, (int64_t)nocc * pl.b0.size(),
                           pl.b0.size(), d_coff, d_koff, d->ngptm,
                           cprod + (int64_t)k0 * nocc * nunocc + ldc * col0,
                           (int64_t)nocc * nunocc, nunocc, ldc, 1.0 / std::sqrt(d->vol), sg_ws,
