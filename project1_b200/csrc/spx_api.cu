@@ -834,7 +834,7 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
 
 namespace spx {
 int wfprod_mt_run(spx_ctx*, const spx_mt_desc*, int, int, int, const double2*, const double2*,
-                  double2*, int64_t, void*, size_t, cudaStream_t, int*);
+                  double2*, int64_t, void*, size_t, cudaStream_t, int*, bool);
 int wfprod_pw_run(spx_ctx*, const spx_pw_desc*, int, int, int, const double2*, const double2*,
                   double2*, int64_t, int, void*, size_t, cudaStream_t, int*, bool, bool);
 size_t wfprod_mt_workspace(const spx_mt_desc*, int, int);
@@ -895,13 +895,13 @@ extern "C" int spx_chi0_from_coeffs_dev(spx_ctx* ctx, const spx_mt_desc* mt,
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
   timing_mark(ctx, s, 0);
-  if ((rc = check_cuda(ctx, cudaMemsetAsync(M, 0, m_bytes, s), "zero cprod"))) return rc;
   rc = wfprod_mt_run(ctx, mt, nk, nocc, nunocc, reinterpret_cast<const double2*>(cmt_occ),
-                     reinterpret_cast<const double2*>(cmt_unocc), M, ldc, sc, scratch, s, &launches);
+                     reinterpret_cast<const double2*>(cmt_unocc), M, ldc, sc, scratch, s, &launches,
+                     /*overwrite: M holds nothing yet*/ true);
   if (!rc)
     rc = wfprod_pw_run(ctx, pw, nk, nocc, nunocc, reinterpret_cast<const double2*>(cpw_occ),
                        reinterpret_cast<const double2*>(cpw_unocc), M, ldc, mt->natom * maxllm,
-                       sc, scratch, s, &launches, split_products, /*overwrite: M was zeroed*/ true);
+                       sc, scratch, s, &launches, split_products, /*overwrite*/ true);
   if (rc) {
     ctx->timing = false;
     return rc;

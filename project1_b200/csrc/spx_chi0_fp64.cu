@@ -774,9 +774,26 @@ static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, 
   return 0;
 }
 
-// Frequencies go to K1p in groups of 24 (three DMMA columns blocks); a remainder takes
-// the narrowest form that holds it. Up to four frequencies cost K1 no more than one
-// 8-wide block costs K1p (4 units each against 4 + 16), so those stay with K1.
+// Whether the last r <= 4 frequencies go to K1 rather than to one 8-wide block of K1p. Per
+// element and pair K1 takes 4 r units against 4 + 16, but on whole 64 x 64 tiles that pad
+// narrow matrices and leave SMs idle when there are few. Time of K1: its tiles per SM, two at
+// once, one alone taking 0.725 of the time of two; of K1p: its units spread over the SMs
+// (uncut: rounds of three tiles), 1.144 times as long per unit. Measured at 12800 pairs, K1
+// against K1p in us: 64 columns, 1 frequency 2828 / 84; 400, 4: 2866 / 1567; 600, 2: 2866 / 3454;
+// 600, 3: 3934 / 3455; 900, 3: 6802 / 7743; 900, 4: 7857 / 7745; 1200, 4: 11727 / 13587.
+static bool f64_takes_k1(const F64Call& q, int r) {
+  const int64_t nblk = (q.N + F64_B - 1) / F64_B, sms = q.num_sms;
+  const int64_t per_sm = (nblk * (nblk + 1) / 2 * r + sms - 1) / sms;
+  const double two = 2.0 * F64_B * F64_B * 4, k1 = (double)(per_sm / 2) * two + (double)(per_sm % 2) * 0.725 * two;
+  const int64_t t2 = f64p_tiles(q.N);
+  const double unit = F64P_TI * F64P_TJ * (4 + 16);
+  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<false>(q.num_sms, 1) && q.P >= F64P_MINCHUNK * F64_KC;
+  const double k1p = cut ? (double)t2 * unit / (double)sms : (double)((t2 + 3 * sms - 1) / (3 * sms)) * 3 * unit;
+  return k1 <= 1.144 * k1p;
+}
+
+// Frequencies go to K1p in groups of 24 (three DMMA column blocks); a remainder takes the
+// narrowest form that holds it, or K1.
 static int f64_run(const F64Call& q, int* launches) {
   int full = q.nw / 24, r = q.nw % 24;
   if (r > 16) ++full, r = 0;
@@ -784,7 +801,7 @@ static int f64_run(const F64Call& q, int* launches) {
   if (full) e = f64p_launch<3, false>(q, {}, 0, full, launches);
   const int f0 = 24 * full;
   if (!e && r > 8) e = f64p_launch<2, false>(q, {}, f0, 1, launches);
-  else if (!e && r > 4) e = f64p_launch<1, false>(q, {}, f0, 1, launches);
+  else if (!e && r > 0 && (r > 4 || !f64_takes_k1(q, r))) e = f64p_launch<1, false>(q, {}, f0, 1, launches);
   else if (!e && r > 0) e = f64_launch(q, f0, r, launches);
   return e;
 }
@@ -792,7 +809,7 @@ static int f64_run(const F64Call& q, int* launches) {
 // Scratch for the partial tiles of a call (0 when none are used); optional: without it
 // the tiles of the last round are not cut.
 size_t fp64_part_bytes(const spx_ctx* ctx, int64_t P, int N, int nw) {
-  if (P < (int64_t)F64P_MINCHUNK * F64_KC || N <= 0 || nw <= 4) return 0;
+  if (P < (int64_t)F64P_MINCHUNK * F64_KC || N <= 0 || nw <= 0) return 0;
   return f64p_part_bytes<false>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
 }
 

@@ -100,11 +100,13 @@ __device__ __forceinline__ ZgTile zg_tile(const ZgParams& prm, int64_t item, int
 // chunks of 16 k form one sequence over all its tiles, two chunks in flight, so a tile's
 // first chunks load while the previous tile's last ones compute and its output is written.
 // Bound: the FP64 pipe (DMMA). Fills are 256-byte runs along k, or along m for an
-// m-contiguous A (MC); GATHER reads B's k offsets through kOff. Measured against one CTA
+// m-contiguous A (MC); GATHER reads B's k offsets through kOff; ADD adds to the output, whose
+// values then come into L2 while the tile computes. Measured against one CTA
 // per tile with a two-stage pipeline: 48000 x 1014 x 3000 gathered 38.5 -> 36.5 ms (0.86
 // of the DMMA rate), 48000 x 1100 x 1200 m-contiguous 16.8 -> 15.3 ms, K = 243 (muffin
-// tin) 1.9 -> 1.66 ms.
-template <bool MC, bool GATHER>
+// tin) 1.9 -> 1.66 ms. With the output fetched ahead the
+// gathered products take 35.7 ms and 24 inverses of 1200 10.5 instead of 11.1.
+template <bool MC, bool GATHER, bool ADD>
 __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams prm, int64_t tiles,
                                                                     int64_t items) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -182,6 +184,22 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int r = 0; r < 4; ++r) accR[mt][nt][r] = accI[mt][nt][r] = 0.0;
+    // (overwrite is 0 whenever ADD; tested here all the same: with the test compiled out the main
+    // loop comes out 2-4 % slower)
+    if (ADD && !prm.overwrite) {
+      // the values this tile adds to come from memory while it computes: thread -> column
+      // tid / 2, 32 rows in four 128-byte lines
+      const ZgTile q = zg_tile(prm, item, tiles);
+      const double2* ob = prm.O + q.b1 * prm.sO1 + q.b2 * prm.sO2;
+      const int cl = q.c0 + (tid >> 1), m = q.m0 + 32 * (tid & 1);
+      if (cl < prm.ncol) {
+        const int n = cl / prm.ncin, c = cl - n * prm.ncin;
+        const double2* o = ob + (int64_t)n * prm.sOn + (int64_t)c * prm.sOc + m;
+#pragma unroll
+        for (int x = 0; x < 32; x += 8)
+          if (m + x < prm.M) asm volatile("prefetch.global.L2 [%0];" ::"l"(o + x));
+      }
+    }
     for (int s = 0; s < nst; ++s) {
       cp_async_wait<1>();   // this thread's copies of the chunk have landed ...
       __syncthreads();      // ... everyone's have, and the stage issued next has been read
@@ -227,8 +245,8 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
     }
 
     const ZgTile q = zg_tile(prm, item, tiles);
-    const double2 al = prm.alpha ? prm.alpha[q.b1] : prm.alpha_v;
     double2* ob = prm.O + q.b1 * prm.sO1 + q.b2 * prm.sO2;
+    const double2 al = prm.alpha ? prm.alpha[q.b1] : prm.alpha_v;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -242,7 +260,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
         for (int x = 0; x < 4; ++x) {
           const int m = q.m0 + 32 * wi + 8 * x + g;
           v[x] = make_double2(0.0, 0.0);
-          if (!prm.overwrite && m < prm.M) v[x] = oc[m];
+          if (ADD && !prm.overwrite && m < prm.M) v[x] = oc[m];
         }
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
@@ -271,10 +289,16 @@ int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kernel<<<grid, ZG_THREADS, smem, s>>>(prm, tiles, items);
   };
-  if (prm.a_mcontig && prm.kOff) run(zgemm_gather_kernel<true, true>);
-  else if (prm.a_mcontig) run(zgemm_gather_kernel<true, false>);
-  else if (prm.kOff) run(zgemm_gather_kernel<false, true>);
-  else run(zgemm_gather_kernel<false, false>);
+  if (prm.a_mcontig && prm.kOff) return set_error(ctx, SPX_EINVAL, "product GEMM: unsupported operand form");
+  if (prm.overwrite) {
+    if (prm.a_mcontig) run(zgemm_gather_kernel<true, false, false>);
+    else if (prm.kOff) run(zgemm_gather_kernel<false, true, false>);
+    else run(zgemm_gather_kernel<false, false, false>);
+  } else {
+    if (prm.a_mcontig) run(zgemm_gather_kernel<true, false, true>);
+    else if (prm.kOff) run(zgemm_gather_kernel<false, true, true>);
+    else run(zgemm_gather_kernel<false, false, true>);
+  }
   return check_cuda(ctx, cudaGetLastError(), "zgemm_gather_kernel launch");
 }
 
@@ -481,10 +505,11 @@ static size_t mt_bytes_per_k(const MtMap& mp, int natom, int nocc) {
   return align_up(sizeof(double2) * (size_t)natom * nocc * mp.maxlm * mp.maxllm, 256);
 }
 
-// Runs the MT products for k points [0, nk) with the scratch [ws, ws+bytes).
+// Runs the MT products for k points [0, nk) with the scratch [ws, ws+bytes); overwrite: the
+// columns hold nothing yet (each is stored once, as there is one batch per atom and k).
 int wfprod_mt_run(spx_ctx* ctx, const spx_mt_desc* d, int nk, int nocc, int nunocc,
                   const double2* c1, const double2* c2, double2* cprod, int64_t ldc, void* ws,
-                  size_t ws_bytes, cudaStream_t s, int* launches) {
+                  size_t ws_bytes, cudaStream_t s, int* launches, bool overwrite) {
   MtMap mp;
   int rc = build_mt_map(ctx, d, &mp);
   if (rc) return rc;
@@ -541,6 +566,7 @@ int wfprod_mt_run(spx_ctx* ctx, const spx_mt_desc* d, int nk, int nocc, int nuno
     prm.ncin = mp.maxllm;
     prm.K = mp.maxlm;
     prm.nb1 = d->natom;
+    prm.overwrite = overwrite;
     if ((rc = launch_zgemm(ctx, prm, d->natom * kn, s))) return rc;
     ++*launches;
   }
@@ -630,17 +656,22 @@ size_t wfprod_pw_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc, b
 
 // Runs the explicit-convolution PW products into cprod columns [col0, col0+ngptm).
 // split: the product GEMM on int8 digit slices (K4s) instead of FP64 (K4c);
-// overwrite: those columns hold nothing yet, so K4s stores instead of adding.
+// overwrite: those columns hold nothing yet, so the GEMM stores instead of adding (what it
+// does not write, without plane waves or on the FFT branch, is zeroed first).
 int wfprod_pw_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int nunocc,
                   const double2* c1, const double2* c2, double2* cprod, int64_t ldc, int col0,
                   void* ws, size_t ws_bytes, cudaStream_t s, int* launches, bool split,
                   bool overwrite) {
+  int rc;
+  if (overwrite && (d->nfft > 0 || d->ngpt2 == 0) && d->ngptm > 0 &&
+      (rc = check_cuda(ctx, cudaMemset2DAsync(cprod + ldc * col0, 16 * ldc, 0, 16 * (size_t)nk * nocc * nunocc,
+                                              d->ngptm, s), "zero cprod")))
+    return rc;
   if (d->nfft > 0)
     return wfprod_pw_fft_run(ctx, d, nk, nocc, nunocc, c1, c2, cprod, ldc, col0, ws, ws_bytes, s,
                              launches);
   PwPlan pl;
-  int rc = plan_pw(ctx, d, &pl);
-  if (rc) return rc;
+  if ((rc = plan_pw(ctx, d, &pl))) return rc;
   if (d->ngptm == 0 || nk == 0 || nocc == 0 || nunocc == 0) return SPX_OK;
   const size_t sg_perk = split ? sgemm_workspace_bytes(1, nunocc, nocc * d->ngptm, d->ngpt2) : 0;
   const size_t perk =
@@ -739,6 +770,7 @@ int wfprod_pw_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int nuno
     prm.ncin = d->ngptm;
     prm.K = d->ngpt2;
     prm.nb1 = 1;
+    prm.overwrite = overwrite;
     if ((rc = launch_zgemm(ctx, prm, kn, s))) return rc;
     ++*launches;
   }
@@ -775,7 +807,7 @@ extern "C" int spx_wfprod_mt_dev(spx_ctx* ctx, const spx_mt_desc* mt, int32_t nk
   cudaStream_t s = pick_stream(ctx, stream);
   return wfprod_mt_run(ctx, mt, nk, nocc, nunocc, reinterpret_cast<const double2*>(cmt_occ),
                        reinterpret_cast<const double2*>(cmt_unocc), reinterpret_cast<double2*>(cprod),
-                       ldc, ctx->ws, ctx->ws_bytes, s, &launches);
+                       ldc, ctx->ws, ctx->ws_bytes, s, &launches, false);
 }
 
 extern "C" int spx_wfprod_pw_dev(spx_ctx* ctx, const spx_pw_desc* pw, int32_t nk, int32_t nocc,
