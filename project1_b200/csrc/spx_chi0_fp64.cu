@@ -292,22 +292,23 @@ __global__ void __launch_bounds__(F64_THREADS, 2)
 // (52 against 96 at 24 frequencies). Every thread forms exactly the products its
 // fragment needs, in registers, so nothing is staged twice.
 //
-// Measured (1200 functions, 128000 pairs, 24 frequencies): 603 ms with K1, 305 ms here,
-// 0.84 of the FP64 pipe at 1965 MHz for the 52 units; the error against 64-bit sums falls
+// Measured (1200 functions, 128000 pairs, 24 frequencies): 603 ms with K1, 295 ms here,
+// 0.88 of the FP64 pipe at 1965 MHz for the 52 units; the error against 64-bit sums falls
 // from 1.3e-14 to 8.7e-15.
 //
 // Bound: the FP64 pipe (DMMA and the products share it). A CTA of four warps owns
-// 16 x 8 elements (two columns per warp: 32 NT accumulator registers leave three CTAs
-// per SM) for one group of 8 NT frequencies, and streams 16-pair chunks of 16 + 8
-// columns of M and of the weights through F64P_ST TMA stages (SWIZZLE_128B).
+// 16 x 8 elements (two columns per warp) for one group of 8 NT frequencies, and streams
+// 64-pair chunks of 16 + 8 columns of M and of the weights through F64P_ST TMA stages
+// (SWIZZLE_128B). Long chunks matter more than resident warps: 16 pairs and three CTAs per
+// SM 306 ms, 32 and three 299, 32 and two 297, 64 and two 295; four columns per warp spill.
 //
 // Work is dealt in whole tiles, one per CTA and round; the tiles of the last,
 // partial round are cut along p into equal ranges, one per CTA, whose partial sums go
 // to `part` and are added in CTA order by chi0_fp64p_reduce_kernel, so the result
 // depends on the sizes only. Without `part` the last round stays whole.
-constexpr int F64P_ST = 4;
+constexpr int F64P_ST = 3;
 constexpr int F64P_TI = 16, F64P_TJ = 8;                // tile rows and columns of the polarisation
-constexpr int F64P_MINCHUNK = 16;                       // shortest p axis (in chunks) worth cutting
+constexpr int F64P_MINPAIR = 256;                       // shortest p axis (pairs) worth cutting
 
 // HW, the q -> 0 head and wings (src/susceptibility.f:1092-1157): the same sum for the rows
 // i of [cprod | dcprod] against the three columns of dcprod. A warp owns 16 rows and all
@@ -317,15 +318,18 @@ constexpr int F64P_MINCHUNK = 16;                       // shortest p axis (in c
 template <bool HW>
 struct F64PTile {
   static constexpr int TI = HW ? 64 : F64P_TI;
-  static constexpr int JW = HW ? 3 : 2;     // columns per warp
-  static constexpr int CTAS = HW ? 2 : 3;   // resident CTAs per SM
+  static constexpr int TJ = HW ? 8 : F64P_TJ;   // columns of a box of j
+  static constexpr int JW = HW ? 3 : 2;         // columns per warp
+  static constexpr int CTAS = 2;                // resident CTAs per SM
+  static constexpr int KC = HW ? 16 : 64;        // band pairs per stage
 };
 
 template <int NT, bool HW>
 struct __align__(1024) F64PSmem {
-  double2 a[F64P_ST][2][F64PTile<HW>::TI][F64_KBOX];
-  double2 b[F64P_ST][2][F64P_TJ][F64_KBOX];
-  double w[F64P_ST][8 * NT][F64_KC];   // row f's 16-byte chunk c stored at c ^ (f & 7)
+  static constexpr int KC = F64PTile<HW>::KC;
+  double2 a[F64P_ST][KC / F64_KBOX][F64PTile<HW>::TI][F64_KBOX];
+  double2 b[F64P_ST][KC / F64_KBOX][F64PTile<HW>::TJ][F64_KBOX];
+  double w[F64P_ST][KC / 16][8 * NT][16];   // row f's 16-byte chunk c stored at c ^ (f & 7)
   uint64_t full[F64P_ST];
   uint64_t empty[F64P_ST];
 };
@@ -467,7 +471,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
                       F64PParams prm) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   using Smem = F64PSmem<NT, HW>;
-  constexpr int JW = F64PTile<HW>::JW;
+  constexpr int JW = F64PTile<HW>::JW, KC = F64PTile<HW>::KC;
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -480,8 +484,8 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
   }
   __syncthreads();
 
-  // warp 0, lane 0 issues the copies, F64P_ST - 2 chunks ahead of the chunk it computes:
-  // a stage is refilled two chunks after it was read, so the issuer rarely waits
+  // warp 0, lane 0 issues the copies, F64P_ST - 2 chunks ahead of the chunk it computes: a
+  // stage is refilled a whole chunk after it was read, so the issuer rarely waits
   F64PSeg ps;
   int64_t p_item = 0;
   int pk = 0, pk1 = 0, p_slot, py = 0, pyj = 0, pf = 0;
@@ -503,13 +507,14 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
   auto issue = [&] {
     const int st = (int)(issued % F64P_ST);
     mbar_arrive_expect_tx(&sm.full[st], (uint32_t)(sizeof(sm.a[0]) + sizeof(sm.b[0]) + sizeof(sm.w[0])));
-    const int x = pk * 2 * F64_KC;
+    const int x = pk * 2 * KC;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < KC / F64_KBOX; ++h) {
       tma_load_2d(&sm.a[st][h][0][0], HW && p_head ? &mapH : &mapI, x + 2 * F64_KBOX * h, py, &sm.full[st]);
       tma_load_2d(&sm.b[st][h][0][0], &mapJ, x + 2 * F64_KBOX * h, pyj, &sm.full[st]);
     }
-    tma_load_2d(&sm.w[st][0][0], &mapW, pk * F64_KC, pf, &sm.full[st]);
+#pragma unroll
+    for (int h = 0; h < KC / 16; ++h) tma_load_2d(&sm.w[st][h][0][0], &mapW, pk * KC + 16 * h, pf, &sm.full[st]);
     ++issued;
     if (++pk == pk1) {
       p_more = ps.next(prm, gridDim.x, &p_item, &pk, &pk1, &p_slot);
@@ -552,14 +557,14 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
         break;
       }
 #pragma unroll
-      for (int ks = 0; ks < F64_KC / F64_KBOX; ++ks) {
+      for (int ks = 0; ks < KC / F64_KBOX; ++ks) {
         double wf[NT][2];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
-            const int p = F64_KBOX * ks + t + 4 * q;
-            wf[nt][q] = sm.w[st][8 * nt + g][(((p >> 1) ^ g) << 1) | (p & 1)];
+            const int p = F64_KBOX * (ks & 1) + t + 4 * q;
+            wf[nt][q] = sm.w[st][ks >> 1][8 * nt + g][(((p >> 1) ^ g) << 1) | (p & 1)];
           }
         double2 a[4];   // a[2q + h] = M(pair t + 4q, row g + 8h)
 #pragma unroll
@@ -569,7 +574,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
 #pragma unroll
         for (int jj = 0; jj < JW; ++jj) {
           const int rj = HW ? jj : JW * warp + jj;
-          const double2 b0 = sm.b[st][ks][rj][t ^ rj], b1 = sm.b[st][ks][rj][(t + 4) ^ rj];
+          const double2 b0 = sm.b[st][ks][rj][t ^ (rj & 7)], b1 = sm.b[st][ks][rj][(t + 4) ^ (rj & 7)];
           double z[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -723,8 +728,8 @@ static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, 
   prm.nw = q.nw;
   prm.f0 = f0;
   prm.ntile = HW ? (q.N + Tile::TI - 1) / Tile::TI + 1 : f64p_tiles(q.N);
-  const int64_t nchunk = (q.P + F64_KC - 1) / F64_KC;
-  if (nchunk > 0x7fffffff / (2 * F64_KC)) return -3;   // pair coordinates are 32-bit
+  const int64_t nchunk = (q.P + Tile::KC - 1) / Tile::KC;
+  if (nchunk > 0x7fffffff / (2 * Tile::KC)) return -3;   // pair coordinates are 32-bit
   prm.nchunk = (int)nchunk;
   prm.items = (int64_t)prm.ntile * groups;
   prm.out = q.out;
@@ -734,29 +739,29 @@ static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, 
   prm.timeout_ns = q.timeout_ns;
   const int64_t slots = (int64_t)Tile::CTAS * q.num_sms;
   const bool cut = q.part && q.part_bytes >= f64p_part_bytes<HW>(q.num_sms, NT) &&
-                   prm.nchunk >= F64P_MINCHUNK && prm.items % slots != 0;
+                   q.P >= F64P_MINPAIR && prm.items % slots != 0;
   // fewer items than slots: as many CTAs as get half of the shortest cut axis each
-  const int64_t fit = cut ? std::max(prm.items, prm.items * prm.nchunk / (F64P_MINCHUNK / 2)) : prm.items;
+  const int64_t fit = cut ? std::max(prm.items, prm.items * prm.nchunk / (F64P_MINPAIR / 2 / Tile::KC)) : prm.items;
   const int grid = (int)std::min(slots, fit);
   prm.whole = cut ? prm.items / grid * grid : prm.items;
   prm.part = cut ? q.part : nullptr;
   CUtensorMap mi, mj, mw, mh;
   int e;
   if (HW) {
-    e = f64_map(&mj, hw.dc, hw.ldd, q.P, 3, F64P_TJ);
+    e = f64_map(&mj, hw.dc, hw.ldd, q.P, 3, Tile::TJ);
     if (!e) e = f64_map(&mh, hw.dc, hw.ldd, q.P, 3, Tile::TI);
     if (!e && q.N > 0) e = f64_map(&mi, q.M, q.ldc, q.P, q.N, Tile::TI);
     if (q.N == 0) mi = mh;
   } else {
     e = f64_map(&mi, q.M, q.ldc, q.P, q.N, Tile::TI);
-    if (!e) e = f64_map(&mj, q.M, q.ldc, q.P, q.N, F64P_TJ);
+    if (!e) e = f64_map(&mj, q.M, q.ldc, q.P, q.N, Tile::TJ);
     mh = mi;
   }
   if (!e) {
     // pairs past the end of the weights read as zeros
     const uint64_t dims[2] = {(uint64_t)q.P, (uint64_t)q.nw};
     const uint64_t strides[1] = {(uint64_t)q.ldw * 8};
-    const uint32_t box[2] = {F64_KC, 8 * NT};
+    const uint32_t box[2] = {16, 8 * NT};
     e = encode_tmap(&mw, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, q.W, dims, strides, box,
                     CU_TENSOR_MAP_SWIZZLE_128B);
   }
@@ -778,18 +783,19 @@ static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, 
 // element and pair K1 takes 4 r units against 4 + 16, but on whole 64 x 64 tiles that pad
 // narrow matrices and leave SMs idle when there are few. Time of K1: its tiles per SM, two at
 // once, one alone taking 0.725 of the time of two; of K1p: its units spread over the SMs
-// (uncut: rounds of three tiles), 1.144 times as long per unit. Measured at 12800 pairs, K1
+// (uncut: rounds of its resident tiles), 1.10 times as long per unit. Measured at 12800 pairs, K1
 // against K1p in us: 64 columns, 1 frequency 2828 / 84; 400, 4: 2866 / 1567; 600, 2: 2866 / 3454;
-// 600, 3: 3934 / 3455; 900, 3: 6802 / 7743; 900, 4: 7857 / 7745; 1200, 4: 11727 / 13587.
+// 600, 3: 3934 / 3455; 900, 3: 6802 / 7743; 900, 4: 7857 / 7745; 1200, 4: 11727 / 13587 (with
+// 16-pair chunks, 1.144; the longer ones take 0.96 of that).
 static bool f64_takes_k1(const F64Call& q, int r) {
   const int64_t nblk = (q.N + F64_B - 1) / F64_B, sms = q.num_sms;
   const int64_t per_sm = (nblk * (nblk + 1) / 2 * r + sms - 1) / sms;
   const double two = 2.0 * F64_B * F64_B * 4, k1 = (double)(per_sm / 2) * two + (double)(per_sm % 2) * 0.725 * two;
   const int64_t t2 = f64p_tiles(q.N);
   const double unit = F64P_TI * F64P_TJ * (4 + 16);
-  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<false>(q.num_sms, 1) && q.P >= F64P_MINCHUNK * F64_KC;
-  const double k1p = cut ? (double)t2 * unit / (double)sms : (double)((t2 + 3 * sms - 1) / (3 * sms)) * 3 * unit;
-  return k1 <= 1.144 * k1p;
+  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<false>(q.num_sms, 1) && q.P >= F64P_MINPAIR;
+  const double k1p = cut ? (double)t2 * unit / (double)sms : (double)((t2 + F64PTile<false>::CTAS * sms - 1) / (F64PTile<false>::CTAS * sms)) * F64PTile<false>::CTAS * unit;
+  return k1 <= 1.10 * k1p;
 }
 
 // Frequencies go to K1p in groups of 24 (three DMMA column blocks); a remainder takes the
@@ -809,7 +815,7 @@ static int f64_run(const F64Call& q, int* launches) {
 // Scratch for the partial tiles of a call (0 when none are used); optional: without it
 // the tiles of the last round are not cut.
 size_t fp64_part_bytes(const spx_ctx* ctx, int64_t P, int N, int nw) {
-  if (P < (int64_t)F64P_MINCHUNK * F64_KC || N <= 0 || nw <= 0) return 0;
+  if (P < F64P_MINPAIR || N <= 0 || nw <= 0) return 0;
   return f64p_part_bytes<false>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
 }
 
@@ -832,7 +838,7 @@ int launch_chi0_fp64(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
 
 // Scratch for launch_headwings' partial tiles (0 when none are used), optional.
 size_t headwings_part_bytes(const spx_ctx* ctx, int64_t P, int nw) {
-  if (P < (int64_t)F64P_MINCHUNK * F64_KC || nw <= 0) return 0;
+  if (P < F64P_MINPAIR || nw <= 0) return 0;
   return f64p_part_bytes<true>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
 }
 
