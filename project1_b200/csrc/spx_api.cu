@@ -89,7 +89,8 @@ int split_chi0_real_ediff(spx_ctx*, const double*, int64_t, int64_t, int, const 
                           const double* wscale, double scale_all, int nw, const double* omega, double*,
                           void*, size_t, cudaStream_t, int*);
 int launch_chi0_fp64_real(spx_ctx*, const double*, int64_t, int64_t, int, const double*, int64_t,
-                          int, double*, cudaStream_t);
+                          int, double*, void* part, size_t part_bytes, cudaStream_t, int*);
+size_t fp64_real_part_bytes(const spx_ctx*, int64_t P, int N, int nw);
 
 void timing_mark(spx_ctx* ctx, cudaStream_t s, int kind) {
   if (!ctx->timing) return;
@@ -498,7 +499,8 @@ extern "C" int spx_chi0_accumulate_real_dev(spx_ctx* ctx, const double* cprod, i
   const bool realign = precision == SPX_FP64 && ((ldc & 1) || ((uintptr_t)cprod & 15));
   const int64_t ldm = realign ? (int64_t)align_up((size_t)npair, 2) : ldc;
   const size_t mbytes = realign ? align_up(sizeof(double) * (size_t)ldm * nbas, 256) : 0;
-  size_t part = precision == SPX_SPLIT ? split_part_bytes(ctx->num_sms, true) : 0;
+  size_t part = precision == SPX_SPLIT ? split_part_bytes(ctx->num_sms, true)
+                                       : fp64_real_part_bytes(ctx, npair, nbas, nw);
   if ((rc = ensure_workspace_opt(ctx, wbytes + sbytes + mbytes, &part))) return rc;
   double* W = (double*)ctx->ws;
   void* sws = (char*)ctx->ws + wbytes;
@@ -520,8 +522,8 @@ extern "C" int spx_chi0_accumulate_real_dev(spx_ctx* ctx, const double* cprod, i
     ++launches;
     if (!rc) {
       timing_mark(ctx, s, 1);
-      rc = launch_chi0_fp64_real(ctx, M, ldm, npair, nbas, W, ldw, nw, susceph, s);
-      ++launches;
+      rc = launch_chi0_fp64_real(ctx, M, ldm, npair, nbas, W, ldw, nw, susceph,
+                                 part ? (char*)ctx->ws + wbytes + mbytes : nullptr, part, s, &launches);
     }
   } else {
     rc = split_chi0_real_ediff(ctx, M, ldm, npair, nbas, ediff, wscale, scale_all, nw, omega, susceph, sws,

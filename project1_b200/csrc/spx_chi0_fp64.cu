@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(F64_THREADS, 2)
 // to `part` and are added in CTA order by chi0_fp64p_reduce_kernel, so the result
 // depends on the sizes only. Without `part` the last round stays whole.
 constexpr int F64P_ST = 3;
-constexpr int F64P_TI = 16, F64P_TJ = 8;                // tile rows and columns of the polarisation
+constexpr int F64P_TI = 16;                              // tile rows of the polarisation
 constexpr int F64P_MINPAIR = 256;                       // shortest p axis (pairs) worth cutting
 
 // HW, the q -> 0 head and wings (src/susceptibility.f:1092-1157): the same sum for the rows
@@ -315,20 +315,29 @@ constexpr int F64P_MINPAIR = 256;                       // shortest p axis (pair
 // three columns, a CTA 64 rows; one more block of rows, dcprod itself, gives the head.
 // Measured at 1100 columns, 48000 pairs, 24 frequencies: 0.64 ms with the cut tiles' sum,
 // against 6.4 ms as a 72-row GEMM (weights folded into 3 x 24 rows, 64-row tiles).
-template <bool HW>
+//
+// REAL, the -DINV build (src/susceptibility.f:1197): real M and chi, one product and one
+// multiply-add per frequency: 1 + 8 NT units of the pipe, four columns per warp, 16 x 16 tiles.
+// N = 1200, P = 10000, 24 frequencies: 19.4 ms on K1r, 11.2 here (0.90 of the FP64 pipe); K1r
+// keeps the shapes of f64r_takes_k1r.
+constexpr int F64P_CPLX = 0, F64P_HW = 1, F64P_REAL = 2;   // MODE
+template <int MODE>
 struct F64PTile {
+  static constexpr bool HW = MODE == F64P_HW, REAL = MODE == F64P_REAL;
   static constexpr int TI = HW ? 64 : F64P_TI;
-  static constexpr int TJ = HW ? 8 : F64P_TJ;   // columns of a box of j
-  static constexpr int JW = HW ? 3 : 2;         // columns per warp
-  static constexpr int CTAS = 2;                // resident CTAs per SM
-  static constexpr int KC = HW ? 16 : 64;        // band pairs per stage
+  static constexpr int JW = HW ? 3 : (REAL ? 4 : 2);           // columns per warp
+  static constexpr int TJ = HW ? 8 : 4 * JW;                   // columns of a box of j
+  static constexpr int CTAS = 2;                               // resident CTAs per SM
+  static constexpr int KC = HW ? 16 : 64;                      // band pairs per stage
+  static constexpr int NBOX = KC / (REAL ? 16 : F64_KBOX);     // 128-byte boxes per stage
+  static constexpr int ELEMS = JW * 4 * F64_THREADS;           // of a CTA, per 8 frequencies
 };
 
-template <int NT, bool HW>
+template <int NT, int MODE>
 struct __align__(1024) F64PSmem {
-  static constexpr int KC = F64PTile<HW>::KC;
-  double2 a[F64P_ST][KC / F64_KBOX][F64PTile<HW>::TI][F64_KBOX];
-  double2 b[F64P_ST][KC / F64_KBOX][F64PTile<HW>::TJ][F64_KBOX];
+  static constexpr int KC = F64PTile<MODE>::KC;
+  double2 a[F64P_ST][F64PTile<MODE>::NBOX][F64PTile<MODE>::TI][F64_KBOX];
+  double2 b[F64P_ST][F64PTile<MODE>::NBOX][F64PTile<MODE>::TJ][F64_KBOX];
   double w[F64P_ST][KC / 16][8 * NT][16];   // row f's 16-byte chunk c stored at c ^ (f & 7)
   uint64_t full[F64P_ST];
   uint64_t empty[F64P_ST];
@@ -339,10 +348,10 @@ struct F64PParams {
   int ntile, nchunk;
   int64_t items;           // ntile x frequency groups
   int64_t whole;           // items dealt whole: rounds x grid (all of them without `part`)
-  double2* out;            // packed polarisation; HW: wing (3, N, nw)
+  double2* out;            // packed polarisation (REAL: as doubles); HW: wing (3, N, nw)
   double2* head;           // HW: head (6, nw)
   int64_t npack;
-  double2* part;           // [CTA][2 slots][elements] partial tiles, or NULL
+  double2* part;           // [CTA][2 slots][elements] partial tiles (REAL: doubles), or NULL
   int* status;
   uint64_t timeout_ns;
 };
@@ -393,32 +402,38 @@ __host__ __device__ __forceinline__ void f64p_decode(int t, int* bi, int* bj) {
   *bj = 2 * m + (r > m ? 1 : 0);
   *bi = r > m ? r - (m + 1) : r;
 }
+template <int MODE>
+__device__ __forceinline__ void f64p_tile(int t, int* bi, int* bj) {
+  if constexpr (MODE == F64P_REAL) decode_tile(t, bi, bj);
+  else f64p_decode(t, bi, bj);
+}
+template <int MODE>
 static int f64p_tiles(int N) {
-  const int nbj = (N + F64P_TJ - 1) / F64P_TJ, m = nbj / 2;
-  return m * (m + 1) + (nbj & 1) * (m + 1);
+  const int nbj = (N + F64PTile<MODE>::TJ - 1) / F64PTile<MODE>::TJ, m = nbj / 2;
+  return MODE == F64P_REAL ? nbj * (nbj + 1) / 2 : m * (m + 1) + (nbj & 1) * (m + 1);
 }
 
-template <int NT, bool HW>
+template <int NT, int MODE>
 struct F64PAcc {
-  double re[F64PTile<HW>::JW][NT][4], im[F64PTile<HW>::JW][NT][4];
+  double re[F64PTile<MODE>::JW][NT][4], im[F64PTile<MODE>::JW][NT][4];
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int jj = 0; jj < F64PTile<HW>::JW; ++jj)
+    for (int jj = 0; jj < F64PTile<MODE>::JW; ++jj)
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int r = 0; r < 4; ++r) re[jj][nt][r] = im[jj][nt][r] = 0.0;
   }
-  static constexpr int ELEMS = F64PTile<HW>::JW * NT * 4 * F64_THREADS;   // of a CTA
+  static constexpr int ELEMS = NT * F64PTile<MODE>::ELEMS;   // of a CTA
 };
 
 // Adds a tile held as accumulator fragments (row g + 8 (r / 2), frequency
 // 8 nt + 2 t + (r & 1)) into the output.
-template <int NT, bool HW>
-__device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item, const F64PAcc<NT, HW>& acc) {
+template <int NT, int MODE>
+__device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item, const F64PAcc<NT, MODE>& acc) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int fb = prm.f0 + (int)(item / prm.ntile) * 8 * NT;
-  if constexpr (HW) {
+  if constexpr (MODE == F64P_HW) {
     const int bi = (int)(item % prm.ntile);
     const bool hd = bi == prm.ntile - 1;
 #pragma unroll
@@ -426,7 +441,7 @@ __device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item, 
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int row = 16 * warp + g + 8 * (r >> 1), f = fb + 8 * nt + 2 * t + (r & 1);
-        const int i = hd ? row : bi * F64PTile<HW>::TI + row;
+        const int i = hd ? row : bi * F64PTile<MODE>::TI + row;
         if (f >= prm.nw || i >= (hd ? 3 : prm.N)) continue;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
@@ -442,10 +457,10 @@ __device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item, 
     return;
   }
   int bi, bj;
-  f64p_decode((int)(item % prm.ntile), &bi, &bj);
+  f64p_tile<MODE>((int)(item % prm.ntile), &bi, &bj);
 #pragma unroll
-  for (int jj = 0; jj < F64PTile<HW>::JW; ++jj) {
-    const int j = bj * F64P_TJ + F64PTile<HW>::JW * warp + jj;
+  for (int jj = 0; jj < F64PTile<MODE>::JW; ++jj) {
+    const int j = bj * F64PTile<MODE>::TJ + F64PTile<MODE>::JW * warp + jj;
     if (j >= prm.N) continue;
     double2* oj = prm.out + (int64_t)j * (j + 1) / 2;
 #pragma unroll
@@ -454,6 +469,10 @@ __device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item, 
       for (int r = 0; r < 4; ++r) {
         const int i = bi * F64P_TI + g + 8 * (r >> 1), f = fb + 8 * nt + 2 * t + (r & 1);
         if (i > j || f >= prm.nw) continue;
+        if constexpr (MODE == F64P_REAL) {
+          reinterpret_cast<double*>(prm.out)[(int64_t)j * (j + 1) / 2 + (int64_t)f * prm.npack + i] += acc.re[jj][nt][r];
+          continue;
+        }
         double2* o = oj + (int64_t)f * prm.npack + i;
         double2 v = *o;
         v.x += acc.re[jj][nt][r];
@@ -464,14 +483,15 @@ __device__ __forceinline__ void f64p_store(const F64PParams& prm, int64_t item, 
 }
 
 // mapI: boxes of the rows i; mapJ: the 8-column boxes of j; mapH (HW): dcprod as rows
-template <int NT, bool HW>
-__global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
+template <int NT, int MODE>
+__global__ void __launch_bounds__(F64_THREADS, F64PTile<MODE>::CTAS)
     chi0_fp64p_kernel(const __grid_constant__ CUtensorMap mapI, const __grid_constant__ CUtensorMap mapJ,
                       const __grid_constant__ CUtensorMap mapW, const __grid_constant__ CUtensorMap mapH,
                       F64PParams prm) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  using Smem = F64PSmem<NT, HW>;
-  constexpr int JW = F64PTile<HW>::JW, KC = F64PTile<HW>::KC;
+  using Smem = F64PSmem<NT, MODE>;
+  constexpr bool HW = F64PTile<MODE>::HW, REAL = F64PTile<MODE>::REAL;
+  constexpr int JW = F64PTile<MODE>::JW, KC = F64PTile<MODE>::KC;
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -495,23 +515,23 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
     if constexpr (HW) {
       const int bi = (int)(p_item % prm.ntile);
       p_head = bi == prm.ntile - 1;
-      py = p_head ? 0 : bi * F64PTile<HW>::TI;
+      py = p_head ? 0 : bi * F64PTile<MODE>::TI;
     } else {
       int bi, bj;
-      f64p_decode((int)(p_item % prm.ntile), &bi, &bj);
+      f64p_tile<MODE>((int)(p_item % prm.ntile), &bi, &bj);
       py = bi * F64P_TI;
-      pyj = bj * F64P_TJ;
+      pyj = bj * F64PTile<MODE>::TJ;
     }
     pf = prm.f0 + (int)(p_item / prm.ntile) * 8 * NT;
   };
   auto issue = [&] {
     const int st = (int)(issued % F64P_ST);
     mbar_arrive_expect_tx(&sm.full[st], (uint32_t)(sizeof(sm.a[0]) + sizeof(sm.b[0]) + sizeof(sm.w[0])));
-    const int x = pk * 2 * KC;
+    const int x = pk * KC * (REAL ? 1 : 2);   // in doubles; a box holds 16
 #pragma unroll
-    for (int h = 0; h < KC / F64_KBOX; ++h) {
-      tma_load_2d(&sm.a[st][h][0][0], HW && p_head ? &mapH : &mapI, x + 2 * F64_KBOX * h, py, &sm.full[st]);
-      tma_load_2d(&sm.b[st][h][0][0], &mapJ, x + 2 * F64_KBOX * h, pyj, &sm.full[st]);
+    for (int h = 0; h < F64PTile<MODE>::NBOX; ++h) {
+      tma_load_2d(&sm.a[st][h][0][0], HW && p_head ? &mapH : &mapI, x + 16 * h, py, &sm.full[st]);
+      tma_load_2d(&sm.b[st][h][0][0], &mapJ, x + 16 * h, pyj, &sm.full[st]);
     }
 #pragma unroll
     for (int h = 0; h < KC / 16; ++h) tma_load_2d(&sm.w[st][h][0][0], &mapW, pk * KC + 16 * h, pf, &sm.full[st]);
@@ -535,7 +555,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
   uint32_t c = 0;   // chunks computed
   bool ok = true;
   while (ok && seg.next(prm, gridDim.x, &item, &k0, &k1, &slot)) {
-    F64PAcc<NT, HW> acc;
+    F64PAcc<NT, MODE> acc;
     acc.zero();
     for (int k = k0; k < k1; ++k, ++c) {
       const int st = (int)(c % F64P_ST);
@@ -566,30 +586,52 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
             const int p = F64_KBOX * (ks & 1) + t + 4 * q;
             wf[nt][q] = sm.w[st][ks >> 1][8 * nt + g][(((p >> 1) ^ g) << 1) | (p & 1)];
           }
-        double2 a[4];   // a[2q + h] = M(pair t + 4q, row g + 8h)
+        if constexpr (REAL) {
+          // pair k of row r sits in 16-byte chunk (k / 2) ^ (r & 7) of its box
+          auto at = [&](const double2 (*box)[F64_KBOX], int r, int q) {
+            const int p = F64_KBOX * (ks & 1) + t + 4 * q;
+            return reinterpret_cast<const double*>(box[r])[(((p >> 1) ^ (r & 7)) << 1) | (p & 1)];
+          };
+          double ar[4];
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+          for (int q = 0; q < 2; ++q)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) a[2 * q + h] = sm.a[st][ks][(HW ? 16 * warp : 0) + g + 8 * h][(t + 4 * q) ^ g];
+            for (int h = 0; h < 2; ++h) ar[2 * q + h] = at(sm.a[st][ks >> 1], g + 8 * h, q);
 #pragma unroll
-        for (int jj = 0; jj < JW; ++jj) {
-          const int rj = HW ? jj : JW * warp + jj;
-          const double2 b0 = sm.b[st][ks][rj][t ^ (rj & 7)], b1 = sm.b[st][ks][rj][(t + 4) ^ (rj & 7)];
-          double z[4];
+          for (int jj = 0; jj < JW; ++jj) {
+            const double b[2] = {at(sm.b[st][ks >> 1], JW * warp + jj, 0), at(sm.b[st][ks >> 1], JW * warp + jj, 1)};
+            const double z[4] = {ar[0] * b[0], ar[1] * b[0], ar[2] * b[1], ar[3] * b[1]};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const double2 b = e < 2 ? b0 : b1;
-            z[e] = fma(a[e].x, b.x, a[e].y * b.y);
+            for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.re[jj][nt], z, wf[nt]);
           }
+        } else {
+          double2 a[4];   // a[2q + h] = M(pair t + 4q, row g + 8h)
 #pragma unroll
-          for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.re[jj][nt], z, wf[nt]);
+          for (int q = 0; q < 2; ++q)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const double2 b = e < 2 ? b0 : b1;
-            z[e] = fma(a[e].y, b.x, -(a[e].x * b.y));
+            for (int h = 0; h < 2; ++h)
+              a[2 * q + h] = sm.a[st][ks][(HW ? 16 * warp : 0) + g + 8 * h][(t + 4 * q) ^ g];
+#pragma unroll
+          for (int jj = 0; jj < JW; ++jj) {
+            const int rj = HW ? jj : JW * warp + jj;
+            const double2 b0 = sm.b[st][ks][rj][t ^ (rj & 7)];
+            const double2 b1 = sm.b[st][ks][rj][(t + 4) ^ (rj & 7)];
+            double z[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const double2 b = e < 2 ? b0 : b1;
+              z[e] = fma(a[e].x, b.x, a[e].y * b.y);
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.re[jj][nt], z, wf[nt]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const double2 b = e < 2 ? b0 : b1;
+              z[e] = fma(a[e].y, b.x, -(a[e].x * b.y));
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.im[jj][nt], z, wf[nt]);
           }
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.im[jj][nt], z, wf[nt]);
         }
       }
       __syncwarp();
@@ -597,16 +639,19 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
     }
     if (!ok) break;
     if (slot < 0) {
-      f64p_store<NT, HW>(prm, item, acc);
+      f64p_store<NT, MODE>(prm, item, acc);
     } else {
-      double2* pp = prm.part + ((int64_t)blockIdx.x * 2 + slot) * F64PAcc<NT, HW>::ELEMS + threadIdx.x;
+      const int64_t at = ((int64_t)blockIdx.x * 2 + slot) * F64PAcc<NT, MODE>::ELEMS + threadIdx.x;
 #pragma unroll
       for (int jj = 0; jj < JW; ++jj)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
           for (int r = 0; r < 4; ++r)
-            pp[((jj * NT + nt) * 4 + r) * F64_THREADS] = make_double2(acc.re[jj][nt][r], acc.im[jj][nt][r]);
+            if constexpr (REAL)
+              reinterpret_cast<double*>(prm.part)[at + ((jj * NT + nt) * 4 + r) * F64_THREADS] = acc.re[jj][nt][r];
+            else
+              prm.part[at + ((jj * NT + nt) * 4 + r) * F64_THREADS] = make_double2(acc.re[jj][nt][r], acc.im[jj][nt][r]);
     }
   }
   if (!ok && threadIdx.x == 0) {
@@ -619,7 +664,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<HW>::CTAS)
 // One CTA per boundary b between the ranges of CTAs b and b + 1 of the accumulation
 // (grid `ncta`): when it falls inside an item and is the first to do so, adds the item's
 // partial tiles in CTA order into the output.
-template <int NT, bool HW>
+template <int NT, int MODE>
 __global__ void __launch_bounds__(F64_THREADS) chi0_fp64p_reduce_kernel(F64PParams prm, int ncta) {
   const int64_t tail = (prm.items - prm.whole) * (int64_t)prm.nchunk;
   const int c = blockIdx.x + 1;
@@ -629,7 +674,7 @@ __global__ void __launch_bounds__(F64_THREADS) chi0_fp64p_reduce_kernel(F64PPara
   if (u == t0 || u >= tail) return;
   const int64_t up = tail * (c - 1) / ncta;
   if (up > t0) return;   // an earlier boundary already lies inside this item
-  F64PAcc<NT, HW> acc;
+  F64PAcc<NT, MODE> acc;
   acc.zero();
   for (int k = c - 1; k < ncta; ++k) {
     const int64_t s = tail * k / ncta;
@@ -637,26 +682,33 @@ __global__ void __launch_bounds__(F64_THREADS) chi0_fp64p_reduce_kernel(F64PPara
     if (tail * (k + 1) / ncta == s) continue;   // an empty range
     // the item is a CTA's first segment when its range starts inside it
     const int slot = s >= t0 ? 0 : 1;
-    const double2* pp = prm.part + ((int64_t)k * 2 + slot) * F64PAcc<NT, HW>::ELEMS + threadIdx.x;
+    const int64_t at = ((int64_t)k * 2 + slot) * F64PAcc<NT, MODE>::ELEMS + threadIdx.x;
 #pragma unroll
-    for (int jj = 0; jj < F64PTile<HW>::JW; ++jj)
+    for (int jj = 0; jj < F64PTile<MODE>::JW; ++jj)
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          const double2 v = pp[((jj * NT + nt) * 4 + r) * F64_THREADS];
+          const int64_t x = at + ((jj * NT + nt) * 4 + r) * F64_THREADS;
+          if constexpr (MODE == F64P_REAL) {
+            acc.re[jj][nt][r] += reinterpret_cast<const double*>(prm.part)[x];
+            continue;
+          }
+          const double2 v = prm.part[x];
           acc.re[jj][nt][r] += v.x;
           acc.im[jj][nt][r] += v.y;
         }
   }
-  f64p_store<NT, HW>(prm, prm.whole + t, acc);
+  f64p_store<NT, MODE>(prm, prm.whole + t, acc);
 }
 
 // Tensor map of M as a 2-D FP64 array: pairs (re, im interleaved) contiguous,
-// columns ldc complex apart; boxes of 8 pairs x `cols` columns, SWIZZLE_128B.
-static int f64_map(CUtensorMap* map, const double2* M, int64_t ldc, int64_t P, int N, int cols) {
-  const uint64_t dims[2] = {(uint64_t)(2 * P), (uint64_t)N};
-  const uint64_t strides[1] = {(uint64_t)ldc * 16};
+// columns ldc complex apart; boxes of 8 pairs x `cols` columns, SWIZZLE_128B. real: M holds
+// doubles, 16 pairs a box.
+static int f64_map(CUtensorMap* map, const double2* M, int64_t ldc, int64_t P, int N, int cols,
+                   bool real = false) {
+  const uint64_t dims[2] = {(uint64_t)((real ? 1 : 2) * P), (uint64_t)N};
+  const uint64_t strides[1] = {(uint64_t)ldc * (real ? 8 : 16)};
   const uint32_t box[2] = {2 * F64_KBOX, (uint32_t)cols};
   return encode_tmap(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, M, dims, strides, box,
                      CU_TENSOR_MAP_SWIZZLE_128B);
@@ -707,9 +759,10 @@ static int f64_launch(const F64Call& q, int f0, int n, int* launches) {
   return 0;
 }
 
-template <bool HW>
+template <int MODE>
 static size_t f64p_part_bytes(int num_sms, int nt) {
-  return sizeof(double2) * (size_t)F64PTile<HW>::CTAS * num_sms * 2 * F64PTile<HW>::JW * nt * 4 * F64_THREADS;
+  return (MODE == F64P_REAL ? sizeof(double) : sizeof(double2)) * (size_t)F64PTile<MODE>::CTAS * num_sms * 2 * nt *
+         F64PTile<MODE>::ELEMS;
 }
 
 // The head and wings' second operand and outputs (HW): dcprod (ldd, 3) and head.
@@ -720,14 +773,15 @@ struct F64Head {
 };
 
 // K1p for `groups` groups of 8 NT frequencies from f0 (the last may be ragged).
-template <int NT, bool HW>
+template <int NT, int MODE>
 static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, int* launches) {
-  using Tile = F64PTile<HW>;
+  using Tile = F64PTile<MODE>;
+  constexpr bool HW = Tile::HW, REAL = Tile::REAL;
   F64PParams prm;
   prm.N = q.N;
   prm.nw = q.nw;
   prm.f0 = f0;
-  prm.ntile = HW ? (q.N + Tile::TI - 1) / Tile::TI + 1 : f64p_tiles(q.N);
+  prm.ntile = HW ? (q.N + Tile::TI - 1) / Tile::TI + 1 : f64p_tiles<MODE>(q.N);
   const int64_t nchunk = (q.P + Tile::KC - 1) / Tile::KC;
   if (nchunk > 0x7fffffff / (2 * Tile::KC)) return -3;   // pair coordinates are 32-bit
   prm.nchunk = (int)nchunk;
@@ -738,7 +792,7 @@ static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, 
   prm.status = q.status;
   prm.timeout_ns = q.timeout_ns;
   const int64_t slots = (int64_t)Tile::CTAS * q.num_sms;
-  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<HW>(q.num_sms, NT) &&
+  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<MODE>(q.num_sms, NT) &&
                    q.P >= F64P_MINPAIR && prm.items % slots != 0;
   // fewer items than slots: as many CTAs as get half of the shortest cut axis each
   const int64_t fit = cut ? std::max(prm.items, prm.items * prm.nchunk / (F64P_MINPAIR / 2 / Tile::KC)) : prm.items;
@@ -753,8 +807,8 @@ static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, 
     if (!e && q.N > 0) e = f64_map(&mi, q.M, q.ldc, q.P, q.N, Tile::TI);
     if (q.N == 0) mi = mh;
   } else {
-    e = f64_map(&mi, q.M, q.ldc, q.P, q.N, Tile::TI);
-    if (!e) e = f64_map(&mj, q.M, q.ldc, q.P, q.N, Tile::TJ);
+    e = f64_map(&mi, q.M, q.ldc, q.P, q.N, Tile::TI, REAL);
+    if (!e) e = f64_map(&mj, q.M, q.ldc, q.P, q.N, Tile::TJ, REAL);
     mh = mi;
   }
   if (!e) {
@@ -766,14 +820,14 @@ static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, 
                     CU_TENSOR_MAP_SWIZZLE_128B);
   }
   if (e) return e;
-  const size_t smem = sizeof(F64PSmem<NT, HW>) + 1024;
-  if (cudaFuncSetAttribute(chi0_fp64p_kernel<NT, HW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  const size_t smem = sizeof(F64PSmem<NT, MODE>) + 1024;
+  if (cudaFuncSetAttribute(chi0_fp64p_kernel<NT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return -2;
-  chi0_fp64p_kernel<NT, HW><<<grid, F64_THREADS, smem, q.stream>>>(mi, mj, mw, mh, prm);
+  chi0_fp64p_kernel<NT, MODE><<<grid, F64_THREADS, smem, q.stream>>>(mi, mj, mw, mh, prm);
   ++*launches;
   if (prm.whole < prm.items && grid > 1) {
-    chi0_fp64p_reduce_kernel<NT, HW><<<grid - 1, F64_THREADS, 0, q.stream>>>(prm, grid);
+    chi0_fp64p_reduce_kernel<NT, MODE><<<grid - 1, F64_THREADS, 0, q.stream>>>(prm, grid);
     ++*launches;
   }
   return 0;
@@ -791,10 +845,10 @@ static bool f64_takes_k1(const F64Call& q, int r) {
   const int64_t nblk = (q.N + F64_B - 1) / F64_B, sms = q.num_sms;
   const int64_t per_sm = (nblk * (nblk + 1) / 2 * r + sms - 1) / sms;
   const double two = 2.0 * F64_B * F64_B * 4, k1 = (double)(per_sm / 2) * two + (double)(per_sm % 2) * 0.725 * two;
-  const int64_t t2 = f64p_tiles(q.N);
-  const double unit = F64P_TI * F64P_TJ * (4 + 16);
-  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<false>(q.num_sms, 1) && q.P >= F64P_MINPAIR;
-  const double k1p = cut ? (double)t2 * unit / (double)sms : (double)((t2 + F64PTile<false>::CTAS * sms - 1) / (F64PTile<false>::CTAS * sms)) * F64PTile<false>::CTAS * unit;
+  const int64_t t2 = f64p_tiles<F64P_CPLX>(q.N);
+  const double unit = F64P_TI * F64PTile<F64P_CPLX>::TJ * (4 + 16);
+  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<F64P_CPLX>(q.num_sms, 1) && q.P >= F64P_MINPAIR;
+  const double k1p = cut ? (double)t2 * unit / (double)sms : (double)((t2 + F64PTile<F64P_CPLX>::CTAS * sms - 1) / (F64PTile<F64P_CPLX>::CTAS * sms)) * F64PTile<F64P_CPLX>::CTAS * unit;
   return k1 <= 1.10 * k1p;
 }
 
@@ -804,10 +858,10 @@ static int f64_run(const F64Call& q, int* launches) {
   int full = q.nw / 24, r = q.nw % 24;
   if (r > 16) ++full, r = 0;
   int e = 0;
-  if (full) e = f64p_launch<3, false>(q, {}, 0, full, launches);
+  if (full) e = f64p_launch<3, F64P_CPLX>(q, {}, 0, full, launches);
   const int f0 = 24 * full;
-  if (!e && r > 8) e = f64p_launch<2, false>(q, {}, f0, 1, launches);
-  else if (!e && r > 0 && (r > 4 || !f64_takes_k1(q, r))) e = f64p_launch<1, false>(q, {}, f0, 1, launches);
+  if (!e && r > 8) e = f64p_launch<2, F64P_CPLX>(q, {}, f0, 1, launches);
+  else if (!e && r > 0 && (r > 4 || !f64_takes_k1(q, r))) e = f64p_launch<1, F64P_CPLX>(q, {}, f0, 1, launches);
   else if (!e && r > 0) e = f64_launch(q, f0, r, launches);
   return e;
 }
@@ -816,7 +870,7 @@ static int f64_run(const F64Call& q, int* launches) {
 // the tiles of the last round are not cut.
 size_t fp64_part_bytes(const spx_ctx* ctx, int64_t P, int N, int nw) {
   if (P < F64P_MINPAIR || N <= 0 || nw <= 0) return 0;
-  return f64p_part_bytes<false>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
+  return f64p_part_bytes<F64P_CPLX>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
 }
 
 // Enqueues the FP64 accumulation over one slab of band pairs. W holds the weights of
@@ -839,7 +893,7 @@ int launch_chi0_fp64(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
 // Scratch for launch_headwings' partial tiles (0 when none are used), optional.
 size_t headwings_part_bytes(const spx_ctx* ctx, int64_t P, int nw) {
   if (P < F64P_MINPAIR || nw <= 0) return 0;
-  return f64p_part_bytes<true>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
+  return f64p_part_bytes<F64P_HW>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
 }
 
 // head(:, f) += sum_p dc(p, k1) conj(dc(p, k2)) w(p, f), wing(k2, i, f) += sum_p M(p, i)
@@ -857,9 +911,9 @@ int launch_headwings(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
   const F64Head hw{dc, ldd, head};
   int full = nw / 24, r = nw % 24, e = 0, launches = 0;
   if (r > 16) ++full, r = 0;
-  if (full) e = f64p_launch<3, true>(q, hw, 0, full, &launches);
-  if (!e && r > 8) e = f64p_launch<2, true>(q, hw, 24 * full, 1, &launches);
-  else if (!e && r > 0) e = f64p_launch<1, true>(q, hw, 24 * full, 1, &launches);
+  if (full) e = f64p_launch<3, F64P_HW>(q, hw, 0, full, &launches);
+  if (!e && r > 8) e = f64p_launch<2, F64P_HW>(q, hw, 24 * full, 1, &launches);
+  else if (!e && r > 0) e = f64p_launch<1, F64P_HW>(q, hw, 24 * full, 1, &launches);
   if (e) return set_error(ctx, SPX_ECUDA, "head and wings: tensor map or attribute failed (" +
                                               std::to_string(e) + ")");
   return check_cuda(ctx, cudaGetLastError(), "head and wings launch");
@@ -1021,35 +1075,81 @@ __global__ void __launch_bounds__(F64_THREADS, 2)
   }
 }
 
-// Enqueues K1r over one slab of real band-pair products M (ldc, N).
-int launch_chi0_fp64_real(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P, int N,
-                          const double* W, int64_t ldw, int nw, double* out, cudaStream_t stream) {
-  if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
-  const int nblk = (N + F64_B - 1) / F64_B;
+// K1r for the `n` frequencies from f0.
+static int f64r_launch(const F64Call& q, int f0, int n) {
+  const int nblk = (q.N + F64_B - 1) / F64_B;
   F64Params prm;
-  prm.P = P;
-  prm.N = N;
-  prm.W = W;
-  prm.ldw = ldw;
-  prm.nw = nw;
+  prm.P = q.P;
+  prm.N = q.N;
+  prm.W = q.W + (int64_t)f0 * q.ldw;
+  prm.ldw = q.ldw;
+  prm.nw = n;
   prm.out = nullptr;
-  prm.npack = (int64_t)N * (N + 1) / 2;
+  prm.npack = (int64_t)q.N * (q.N + 1) / 2;
   prm.ntile = nblk * (nblk + 1) / 2;
-  prm.nitems = (int64_t)prm.ntile * nw;
-  prm.status = ctx->d_status;
-  prm.timeout_ns = (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
+  prm.nitems = (int64_t)prm.ntile * n;
+  prm.status = q.status;
+  prm.timeout_ns = q.timeout_ns;
   CUtensorMap map;
-  const uint64_t dims[2] = {(uint64_t)P, (uint64_t)N};
-  const uint64_t strides[1] = {(uint64_t)ldc * 8};
-  const uint32_t box[2] = {F64_KC, F64_B};
-  const int e = encode_tmap(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, M, dims, strides, box,
-                            CU_TENSOR_MAP_SWIZZLE_128B);
-  if (e) return set_error(ctx, SPX_ECUDA, "chi0_fp64_real_kernel: tensor map (" + std::to_string(e) + ")");
+  const int e = f64_map(&map, q.M, q.ldc, q.P, q.N, F64_B, true);
+  if (e) return e;
   const size_t smem = sizeof(F64RSmem) + 1024;
-  cudaFuncSetAttribute(chi0_fp64_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int grid = (int)std::min<int64_t>(prm.nitems, (int64_t)2 * ctx->num_sms);
-  chi0_fp64_real_kernel<<<grid, F64_THREADS, smem, stream>>>(map, prm, out);
-  return check_cuda(ctx, cudaGetLastError(), "chi0_fp64_real_kernel launch");
+  if (cudaFuncSetAttribute(chi0_fp64_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
+    return -2;
+  const int grid = (int)std::min<int64_t>(prm.nitems, (int64_t)2 * q.num_sms);
+  chi0_fp64_real_kernel<<<grid, F64_THREADS, smem, q.stream>>>(map, prm,
+                                                              reinterpret_cast<double*>(q.out) + (int64_t)f0 * prm.npack);
+  return 0;
+}
+
+// Whether n <= 24 frequencies go to K1r rather than to one launch of `nt` 8-wide blocks of
+// K1p, in multiply-adds of the busiest SM: whole 64 x 64 tiles of one frequency, two at a
+// time per SM, against 1 + 8 nt for every 16 x 16 tile, spread evenly. A K1r tile costs 1.55
+// of a K1p multiply-add each (waits for its loads with two CTAs' warps), one alone on its SM
+// 0.95 of two. us, K1r / K1p: N = 300, P = 10000: 2 frequencies 1146 / 329, 24: 2395 / 781;
+// N = 20, P = 2000, 1: 235 / 38; N = 900, P = 10000, 24: 12180 / 6488; N = 1200, 24:
+// 19409 / 11155, 5: 4783 / 4564; the other way round N = 700, 3: 1230 / 1605; N = 1200, 1:
+// 1222 / 4535; N = 1300, P = 6000, 2: 1474 / 3297.
+static bool f64r_takes_k1r(const F64Call& q, int n, int nt) {
+  const int64_t nblk = (q.N + F64_B - 1) / F64_B, sms = q.num_sms;
+  const int64_t per_sm = (nblk * (nblk + 1) / 2 * n + sms - 1) / sms;
+  const double two = 2.0 * F64_B * F64_B, k1 = 1.55 * two * ((double)(per_sm / 2) + (double)(per_sm % 2) * 0.95);
+  using Tile = F64PTile<F64P_REAL>;
+  const int64_t t2 = f64p_tiles<F64P_REAL>(q.N);
+  const double unit = Tile::TI * Tile::TJ * (1 + 8.0 * nt);
+  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<F64P_REAL>(q.num_sms, nt) && q.P >= F64P_MINPAIR;
+  const double k1p = cut ? (double)t2 * unit / (double)sms
+                         : (double)((t2 + Tile::CTAS * sms - 1) / (Tile::CTAS * sms)) * Tile::CTAS * unit;
+  return k1 <= k1p;
+}
+
+// Scratch for the real accumulation's partial tiles (0 when none are used), optional.
+size_t fp64_real_part_bytes(const spx_ctx* ctx, int64_t P, int N, int nw) {
+  if (P < F64P_MINPAIR || N <= 0 || nw <= 0) return 0;
+  return f64p_part_bytes<F64P_REAL>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
+}
+
+// Enqueues the FP64 accumulation over one slab of real band-pair products M (ldc, N): ldc
+// even, M 16-byte aligned; W and `part` as launch_chi0_fp64.
+int launch_chi0_fp64_real(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P, int N,
+                          const double* W, int64_t ldw, int nw, double* out, void* part,
+                          size_t part_bytes, cudaStream_t stream, int* launches) {
+  if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
+  const F64Call q{ctx->num_sms, reinterpret_cast<const double2*>(M), ldc, P, N, W, ldw, nw,
+                  reinterpret_cast<double2*>(out), (double2*)part, part_bytes, ctx->d_status,
+                  (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull, stream};
+  int e = 0;
+  for (int f0 = 0; f0 < nw && !e; f0 += 24) {
+    const int n = std::min(24, nw - f0), nt = (n + 7) / 8;
+    if (f64r_takes_k1r(q, n, nt)) e = f64r_launch(q, f0, n), ++*launches;
+    else if (nt == 3) e = f64p_launch<3, F64P_REAL>(q, {}, f0, 1, launches);
+    else if (nt == 2) e = f64p_launch<2, F64P_REAL>(q, {}, f0, 1, launches);
+    else e = f64p_launch<1, F64P_REAL>(q, {}, f0, 1, launches);
+  }
+  if (e) return set_error(ctx, SPX_ECUDA, "real FP64 accumulation: tensor map or attribute failed (" +
+                                              std::to_string(e) + ")");
+  return check_cuda(ctx, cudaGetLastError(), "real FP64 accumulation launch");
 }
 
 // FP64 tensor-pipe peak: every warp issues back-to-back m16n8k8 DMMAs on register
