@@ -367,6 +367,7 @@ extern "C" int spx_dielec_dev(spx_ctx* ctx, int32_t nbas, int32_t nw, double* su
     h.K = bk;
     h.nb1 = nw;
     h.upper = 1;
+    h.skip = kb / DI_B + 1;   // the panels replace these tiles: 171 of 190 are left at n = 1200
     if ((rc = launch_zgemm(ctx, h, nw, s))) return rc;
     sweep_panels_kernel<<<tgrid, 256, 0, s>>>(full, n, kb, bk, U, Pb);
     if ((rc = check_cuda(ctx, cudaGetLastError(), "sweep panels"))) return rc;

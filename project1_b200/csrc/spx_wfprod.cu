@@ -89,6 +89,10 @@ __device__ __forceinline__ ZgTile zg_tile(const ZgParams& prm, int64_t item, int
     while ((j + 1) * (j + 2) / 2 <= t) ++j;
     tn = j;
     tm = t - j * (j + 1) / 2;
+    if (prm.skip) {
+      tn += tn >= prm.skip - 1;
+      tm += tm >= prm.skip - 1;
+    }
   } else {
     tm = t % prm.mtiles;
     tn = t / prm.mtiles;
@@ -279,7 +283,9 @@ int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s) {
   if (prm.M <= 0 || prm.ncol <= 0 || prm.K <= 0 || nbatch <= 0) return SPX_OK;
   prm.mtiles = (prm.M + ZG_B - 1) / ZG_B;
   prm.ntiles = (prm.ncol + ZG_B - 1) / ZG_B;
-  const int64_t tiles = prm.upper ? (int64_t)prm.ntiles * (prm.ntiles + 1) / 2 : (int64_t)prm.mtiles * prm.ntiles;
+  const int64_t nu = prm.ntiles - (prm.skip ? 1 : 0);
+  const int64_t tiles = prm.upper ? nu * (nu + 1) / 2 : (int64_t)prm.mtiles * prm.ntiles;
+  if (tiles == 0) return SPX_OK;
   if (tiles > 0x7fffffff || nbatch > 65535)
     return set_error(ctx, SPX_EINVAL, "product GEMM grid too large");
   const int64_t items = tiles * nbatch;

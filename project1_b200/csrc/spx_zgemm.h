@@ -28,6 +28,7 @@ struct ZgParams {
   int M, ncol, ncin, K, nb1;
   int overwrite;  // 1: store, the output holds nothing yet; 0: add
   int upper;      // 1: only the 64 x 64 tiles on and above the diagonal (M == ncol)
+  int skip;       // upper: 64-wide block, counted from 1, whose row and column of tiles are left out
   int mtiles, ntiles;
 };
 
