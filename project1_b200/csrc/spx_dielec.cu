@@ -19,8 +19,9 @@
 // the complex FP64 DMMA GEMM (K4c). The matrix stays Hermitian through the sweep, so
 // only the 64 x 64 tiles on and above the diagonal are kept up to date: half of the
 // multiply-adds and of the traffic of the updates. Measured at 24 matrices of 1200: 23.6 ms
-// with full updates and the pivot block swept in shared memory, 11.1 ms here (updates
-// 18.1 -> 8.5 ms, pivot blocks 3.2 -> 0.75 ms).
+// with full updates and the pivot block swept in shared memory, 9.3 ms here (updates
+// 18.1 -> 7.1 ms: 0.64 of the FP64 pipe, a 64-deep tile's epilogue taking the rest; pivot
+// blocks and panels 4.0 -> 0.86 ms).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -90,48 +91,98 @@ __global__ void pack_upper_kernel(const double2* __restrict__ full, int n, doubl
 
 constexpr int DI_B = 64;  // pivot block of the sweep
 
-// For every frequency (grid.y): CpT[j][t] = A(j, kb + t) for all rows j (the pivot
-// block's column panel, stored row by row), and Pb[t][u] = A(kb + t, kb + u). Rows below
-// the pivot block come from its row panel, conjugated.
-__global__ void sweep_extract_kernel(const double2* __restrict__ A, int n, int kb, int bk,
-                                     double2* __restrict__ CpT, double2* __restrict__ Pb) {
-  const double2* Aw = A + (int64_t)blockIdx.y * n * n;
-  double2* Cw = CpT + (int64_t)blockIdx.y * n * DI_B;
-  double2* Pw = Pb + (int64_t)blockIdx.y * DI_B * DI_B;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n * DI_B;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    // above the block, lanes walk the rows of a column; below it, the rows of the block
-    const int64_t up = (int64_t)(kb + bk) * DI_B;
-    int t, j;
-    if (e < up) {
-      t = (int)(e / (kb + bk));
-      j = (int)(e - (int64_t)t * (kb + bk));
-    } else {
-      j = (int)(e / DI_B);
-      t = (int)(e - (int64_t)j * DI_B);
-    }
-    if (t >= bk) continue;
-    double2 v;
-    if (e < up) {
-      v = Aw[(int64_t)(kb + t) * n + j];
-      if (j >= kb) Pw[(j - kb) * DI_B + t] = v;
-    } else {
-      v = Aw[(int64_t)j * n + kb + t];
-      v.y = -v.y;
-    }
-    Cw[(int64_t)j * DI_B + t] = v;
+// The panels of a pivot block move 16 rows x 64 columns t per CTA of 256 threads, four
+// elements each; where rows and columns swap, through this tile, so that both sides move
+// 256-byte runs.
+using SweepTile = double2[4][16][17];
+
+// After the trailing update, in the kept tiles: A(i, kb+t) = U(i, t) for rows i above the
+// block, A(kb+t, j) = conj U(j, t) for columns j after it. Rows i0 .. i0 + 15 of U.
+__device__ __forceinline__ void sweep_panels(SweepTile& tile, double2* Aw, int n, int kb, int bk, const double2* Uw,
+                                             int i0) {
+  const int lx = threadIdx.x & 15, ly = threadIdx.x >> 4, i = i0 + lx;
+  // 16 divides kb, and bk unless the block is the last one
+  if (i0 >= kb && i0 < kb + bk) return;
+  double2 v[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h)
+    if (i < n && 16 * h + ly < bk) v[h] = Uw[(int64_t)(16 * h + ly) * n + i];
+  if (i0 < kb) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (16 * h + ly < bk) Aw[(int64_t)(kb + 16 * h + ly) * n + i] = v[h];
+    return;
+  }
+#pragma unroll
+  for (int h = 0; h < 4; ++h) tile[h][ly][lx] = v[h];
+  __syncthreads();
+  const int j = i0 + ly;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const int t = 16 * h + lx;
+    if (j < n && t < bk) Aw[(int64_t)j * n + kb + t] = make_double2(tile[h][lx][ly].x, -tile[h][lx][ly].y);
   }
 }
+__global__ void __launch_bounds__(256) sweep_panels_kernel(double2* A, int n, int kb, int bk, const double2* U) {
+  __shared__ SweepTile tile;
+  const int64_t f = blockIdx.y;
+  sweep_panels(tile, A + f * n * n, n, kb, bk, U + f * n * DI_B, 16 * blockIdx.x);
+}
 
-// In place: Pb <- inv(Pb) for the bk x bk Hermitian positive-definite block of every
-// frequency (one CTA each), by the sweep of its columns. A pivot that is not positive
-// records (block row + 1) in info[frequency]. The chain of 64 pivots is serial, so a step
-// is kept short: thread (r, c) of 16 x 16 holds rows r + 16 x, columns c + 16 y in
-// registers, the pivot's row and column go through shared memory, two buffers and one
-// barrier per step.
-__global__ void __launch_bounds__(256) sweep_block_inverse_kernel(double2* __restrict__ Pb, int bk,
-                                                                  int kb, int* __restrict__ info) {
+// CpT[j][t] = A(j, kb + t) for the rows j of one frequency outside the pivot block (its
+// column panel, stored row by row; nothing reads the block's own rows of CpT or of U, and
+// its tiles of A are being replaced). Rows below the pivot block come from its row panel,
+// conjugated; rows of the pivot block before it, whose panels are not in A yet, from its U.
+// Rows j0 .. j0 + 15.
+__device__ __forceinline__ void sweep_extract(SweepTile& tile, const double2* Aw, int n, int kb, int bk,
+                                              const double2* Uw, double2* __restrict__ Cw, int j0) {
+  const int lx = threadIdx.x & 15, ly = threadIdx.x >> 4, j = j0 + ly;
+  if (j0 >= kb && j0 < kb + bk) return;
+  double2 v[4];
+  if (j0 < kb - DI_B) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (16 * h + ly < bk) v[h] = Aw[(int64_t)(kb + 16 * h + ly) * n + j0 + lx];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) tile[h][ly][lx] = v[h];
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (16 * h + lx < bk) Cw[(int64_t)j * DI_B + 16 * h + lx] = tile[h][lx][ly];
+    return;
+  }
+  const double2* src = j < kb ? Uw + (int64_t)(j - (kb - DI_B)) * n : Aw + (int64_t)j * n;
+#pragma unroll
+  for (int h = 0; h < 4; ++h)
+    if (j < n && 16 * h + lx < bk) v[h] = src[kb + 16 * h + lx];
+#pragma unroll
+  for (int h = 0; h < 4; ++h)
+    if (j < n && 16 * h + lx < bk) Cw[(int64_t)j * DI_B + 16 * h + lx] = make_double2(v[h].x, -v[h].y);
+}
+
+// Pb <- inv(P) and A's pivot block <- -inv(P) for the bk x bk Hermitian positive-definite
+// pivot block P of every frequency (the first `nw` CTAs, one each), by the sweep of its
+// columns; meanwhile the other CTAs extract the column panels and put the panels of the
+// pivot block before into A from its U: no two touch the same elements. Inverse, extraction and panels took 39 + 14 + 13 us one after the other at 24
+// matrices of 1200, 45 together. A pivot that is not positive records (block row + 1)
+// in info[frequency]. The chain of 64 pivots is serial, so a step is kept short: thread
+// (r, c) of 16 x 16 holds rows r + 16 x, columns c + 16 y in registers, the pivot's row and
+// column go through shared memory, two buffers and one barrier per step.
+__global__ void __launch_bounds__(256) sweep_pivot_kernel(double2* A, int n, int kb, int bk, int nw,
+                                                          const double2* U, double2* __restrict__ CpT,
+                                                          double2* __restrict__ Pb, int* __restrict__ info) {
   __shared__ double2 col[2][DI_B], row[2][DI_B];
+  if ((int)blockIdx.x >= nw) {
+    __shared__ SweepTile tile;
+    const int e = blockIdx.x - nw, nx = (n + 15) / 16, g = e / nx, x = 16 * (e - g * nx);
+    const int64_t f = g < nw ? g : g - nw;
+    double2* Af = A + f * n * n;
+    const double2* Uf = U + f * n * DI_B;
+    if (g < nw) sweep_extract(tile, Af, n, kb, bk, Uf, CpT + f * n * DI_B, x);
+    else sweep_panels(tile, Af, n, kb - DI_B, DI_B, Uf, x);
+    return;
+  }
+  double2* Aw = A + (int64_t)blockIdx.x * n * n + (int64_t)kb * n + kb;
   double2* Pw = Pb + (int64_t)blockIdx.x * DI_B * DI_B;
   const int r = threadIdx.x >> 4, c = threadIdx.x & 15;
   double2 m[4][4];
@@ -140,7 +191,7 @@ __global__ void __launch_bounds__(256) sweep_block_inverse_kernel(double2* __res
 #pragma unroll
     for (int y = 0; y < 4; ++y) {
       const int i = r + 16 * x, j = c + 16 * y;
-      m[x][y] = i < bk && j < bk ? Pw[i * DI_B + j] : make_double2(i == j ? 1.0 : 0.0, 0.0);
+      m[x][y] = i < bk && j < bk ? Aw[(int64_t)j * n + i] : make_double2(i == j ? 1.0 : 0.0, 0.0);
     }
 #pragma unroll
   for (int pq = 0; pq < 4; ++pq) {
@@ -194,42 +245,11 @@ __global__ void __launch_bounds__(256) sweep_block_inverse_kernel(double2* __res
 #pragma unroll
     for (int y = 0; y < 4; ++y) {
       const int i = r + 16 * x, j = c + 16 * y;
-      if (i < bk && j < bk) Pw[i * DI_B + j] = make_double2(-m[x][y].x, -m[x][y].y);
+      if (i < bk && j < bk) {
+        Pw[i * DI_B + j] = make_double2(-m[x][y].x, -m[x][y].y);
+        Aw[(int64_t)j * n + i] = m[x][y];
+      }
     }
-}
-
-// After the trailing update, in the kept tiles: A(i, kb+t) = U(i, t) for rows i above the
-// block, A(kb+t, j) = conj U(j, t) for columns j after it, and A(kb+t, kb+u) = -P(t, u).
-__global__ void sweep_panels_kernel(double2* __restrict__ A, int n, int kb, int bk,
-                                    const double2* __restrict__ U, const double2* __restrict__ Pb) {
-  __shared__ double2 tile[16][17];
-  double2* Aw = A + (int64_t)blockIdx.z * n * n;
-  const double2* Uw = U + (int64_t)blockIdx.z * n * DI_B;
-  const double2* Pw = Pb + (int64_t)blockIdx.z * DI_B * DI_B;
-  // a CTA moves 16 rows i x 16 columns t; after the block the tile is transposed through
-  // shared memory, so both sides move 256-byte runs
-  const int lx = threadIdx.x & 15, ly = threadIdx.x >> 4;
-  const int i0 = blockIdx.x * 16, t0 = blockIdx.y * 16;
-  const int i = i0 + lx, t = t0 + ly;
-  if (i0 < kb + bk) {   // 16 divides kb, and bk unless the block is the last one
-    if (i >= n || t >= bk) return;
-    double2 v;
-    if (i < kb) {
-      v = Uw[(int64_t)t * n + i];
-    } else {
-      v = Pw[(i - kb) * DI_B + t];
-      v = make_double2(-v.x, -v.y);
-    }
-    Aw[(int64_t)(kb + t) * n + i] = v;
-    return;
-  }
-  if (i < n && t < bk) tile[ly][lx] = Uw[(int64_t)t * n + i];
-  __syncthreads();
-  const int j = i0 + ly, u = t0 + lx;
-  if (j < n && u < bk) {
-    const double2 v = tile[lx][ly];
-    Aw[(int64_t)j * n + kb + u] = make_double2(v.x, -v.y);
-  }
 }
 
 // head(:, f) = I3 - 4 pi head(:, f) (packed 3x3), wing(:, i, f) = -sqrt(4 pi) sqrt(v_i) wing
@@ -322,12 +342,10 @@ extern "C" int spx_dielec_dev(spx_ctx* ctx, int32_t nbas, int32_t nw, double* su
                                                                       full + (int64_t)f * n * n);
     if ((rc = check_cuda(ctx, cudaGetLastError(), "dielec_unpack_kernel launch"))) return rc;
   }
-  const dim3 pgrid((unsigned)std::min<int64_t>(((int64_t)n * DI_B + 255) / 256, 4096), (unsigned)nw);
-  const dim3 tgrid((unsigned)((n + 15) / 16), DI_B / 16, (unsigned)nw);
+  const int nx = (n + 15) / 16;
   for (int kb = 0; kb < n; kb += DI_B) {
     const int bk = std::min(DI_B, n - kb);
-    sweep_extract_kernel<<<pgrid, 256, 0, s>>>(full, n, kb, bk, CpT, Pb);
-    sweep_block_inverse_kernel<<<nw, 256, 0, s>>>(Pb, bk, kb, info);
+    sweep_pivot_kernel<<<nw * (1 + nx * (kb ? 2 : 1)), 256, 0, s>>>(full, n, kb, bk, nw, U, CpT, Pb, info);
     if ((rc = check_cuda(ctx, cudaGetLastError(), "sweep pivot block"))) return rc;
     // U = Cp P: U(i, c) = sum_t Cp(i, t) conj(P(c, t))   (P Hermitian)
     ZgParams g{};
@@ -369,7 +387,8 @@ extern "C" int spx_dielec_dev(spx_ctx* ctx, int32_t nbas, int32_t nw, double* su
     h.upper = 1;
     h.skip = kb / DI_B + 1;   // the panels replace these tiles: 171 of 190 are left at n = 1200
     if ((rc = launch_zgemm(ctx, h, nw, s))) return rc;
-    sweep_panels_kernel<<<tgrid, 256, 0, s>>>(full, n, kb, bk, U, Pb);
+    if (kb + bk < n) continue;
+    sweep_panels_kernel<<<dim3(nx, nw), 256, 0, s>>>(full, n, kb, bk, U);
     if ((rc = check_cuda(ctx, cudaGetLastError(), "sweep panels"))) return rc;
   }
   // the sweep leaves -inv(eps)
