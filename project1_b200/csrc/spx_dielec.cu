@@ -163,9 +163,9 @@ __device__ __forceinline__ void sweep_extract(SweepTile& tile, const double2* Aw
 // Pb <- inv(P) and A's pivot block <- -inv(P) for the bk x bk Hermitian positive-definite
 // pivot block P of every frequency (the first `nw` CTAs, one each), by the sweep of its
 // columns; meanwhile the other CTAs extract the column panels and put the panels of the
-// pivot block before into A from its U: no two touch the same elements. Inverse, extraction and panels took 39 + 14 + 13 us one after the other at 24
-// matrices of 1200, 45 together. A pivot that is not positive records (block row + 1)
-// in info[frequency]. The chain of 64 pivots is serial, so a step is kept short: thread
+// pivot block before into A from its U: no two touch the same elements. Inverse,
+// extraction and panels took 39 + 14 + 13 us one after the other at 24 matrices of 1200, 45
+// together. A pivot that is not positive records (block row + 1) in info[frequency]. The chain of 64 pivots is serial, so a step is kept short: thread
 // (r, c) of 16 x 16 holds rows r + 16 x, columns c + 16 y in registers, the pivot's row and
 // column go through shared memory, two buffers and one barrier per step.
 __global__ void __launch_bounds__(256) sweep_pivot_kernel(double2* A, int n, int kb, int bk, int nw,
