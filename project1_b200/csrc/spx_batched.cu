@@ -35,7 +35,11 @@ int launch_chi0_fp64(spx_ctx*, const double2*, int64_t, int64_t, int, const doub
 size_t fp64_part_bytes(const spx_ctx*, int64_t P, int N, int nw);
 int split_chi0_slab(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
                     int, double2*, void*, size_t, cudaStream_t, int*, int, int);
+int split_chi0_ediff(spx_ctx*, const double2*, int64_t, int64_t, int, const double* ediff,
+                     const double* wscale, double scale_all, int nw, const double* omega, double2*, void*,
+                     size_t, cudaStream_t, int*, int variant, int slab);
 size_t split_workspace_bytes(int64_t P, int N, int nw, int slab);
+size_t split_part_bytes(int num_sms, bool real);
 int launch_gen_cmatrix_rows(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, int64_t, int64_t,
                             int64_t, double, double2*, cudaStream_t);
 int launch_gen_normal(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, double, double*,
@@ -48,6 +52,7 @@ struct PbConfig {
 int pb_run(spx_ctx* ctx, int nq, const spx_q_desc* q, int nw, const double* omega, int flags,
            cudaStream_t s, int* launches, const PbConfig* force, int force_slab, char* scratch,
            size_t scratch_bytes);
+int pb_slab_of(const spx_ctx* ctx, const spx_q_desc& q, int nw, int force);
 size_t pb_single_bytes(int64_t P, int N, int nw, int slab);
 int pb_single(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, const double* ediff,
               const double* wscale, double scale_all, int nw, const double* omega, double2* out,
@@ -166,6 +171,53 @@ static int enqueue_batch(spx_ctx* ctx, int nq, const spx_q_desc* q, const QPlan*
   return SPX_OK;
 }
 
+// Whether a split batch runs as each q's own kernels, one q after the other, instead of the
+// persistent schedule: when every M is given (nothing to generate beside the accumulation)
+// and every descriptor leaves kernel and slab open. In the persistent kernel six warps per SM
+// prepare operands beside the MMAs, which slows both; the separate kernels prepare with the
+// whole chip and cut their last tiles over it, but cost 20 us per q at least. ms, persistent /
+// q by q (q points, mean columns, mean pairs, frequencies): 8, 548, 17287, 24: 17.1 / 14.9;
+// 10, 209, 12418, 24: 5.3 / 2.9; 12, 1049, 47189, 24: 199 / 185; 12, 713, 42921, 1: 8.2 / 6.5;
+// 3, 185, 5533, 1: 0.21 / 0.15; 9, 657, 6556, 12: 4.7 / 4.6; the other way round 7, 135, 1439,
+// 1: 0.17 / 0.22; 12, 64, 373, 1: 0.15 / 0.25. The line, a mean of 500000 operand elements
+// (columns x pairs x frequencies) per q, lies between the last of one group (1.0 million)
+// and the first of the other (0.2 million).
+static bool batch_by_q(const spx_ctx* ctx, int nq, const spx_q_desc* q, int nw) {
+  if (ctx->prof_on || ctx->opt.split_variant != 0) return false;
+  double elems = 0.0;
+  int n = 0;
+  for (int i = 0; i < nq; ++i) {
+    if (q[i].npair <= 0 || q[i].nbas <= 0) continue;
+    if (!q[i].cprod || q[i].variant != 0 || q[i].slab_pairs != 0) return false;
+    elems += (double)q[i].nbas * (double)q[i].npair * nw;
+    ++n;
+  }
+  return elems >= 5e5 * n;
+}
+
+// The batch q by q on `s`, with the slabs of the persistent schedule. SPX_ENOTSUP when the
+// workspace limit is too small for the largest q.
+static int run_by_q(spx_ctx* ctx, int nq, const spx_q_desc* q, int nw, const double* omega, cudaStream_t s,
+                    int* launches) {
+  size_t need = 0, part = split_part_bytes(ctx->num_sms, false);
+  for (int i = 0; i < nq; ++i)
+    if (q[i].npair > 0 && q[i].nbas > 0)
+      need = std::max(need, split_workspace_bytes(q[i].npair, q[i].nbas, nw, pb_slab_of(ctx, q[i], nw, 0)));
+  if (need == 0) return SPX_OK;
+  if (ctx->opt.workspace_limit > 0 && need > (size_t)ctx->opt.workspace_limit) return SPX_ENOTSUP;
+  int rc = ensure_workspace_opt(ctx, need, &part);
+  const bool timing = ctx->timing;
+  ctx->timing = false;
+  for (int i = 0; i < nq && !rc; ++i)
+    if (q[i].npair > 0 && q[i].nbas > 0)
+      rc = split_chi0_ediff(ctx, reinterpret_cast<const double2*>(q[i].cprod), q[i].ldc, q[i].npair, q[i].nbas,
+                            q[i].ediff, q[i].wscale, q[i].scale_all, nw, omega,
+                            reinterpret_cast<double2*>(q[i].susceph), ctx->ws, need + part, s, launches, 0,
+                            pb_slab_of(ctx, q[i], nw, 0));
+  ctx->timing = timing;
+  return rc;
+}
+
 }  // namespace spx
 
 using namespace spx;
@@ -215,7 +267,9 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
     cudaEvent_t e0 = ctx->ev[8], e1 = ctx->ev[9];
     if (stats) cudaEventRecord(e0, s);
     int launches = 0;
-    if ((rc = pb_run(ctx, nq, q, nw, omega, flags, s, &launches, nullptr, 0, nullptr, 0))) return rc;
+    rc = batch_by_q(ctx, nq, q, nw) ? run_by_q(ctx, nq, q, nw, omega, s, &launches) : SPX_ENOTSUP;
+    if (rc == SPX_ENOTSUP) rc = pb_run(ctx, nq, q, nw, omega, flags, s, &launches, nullptr, 0, nullptr, 0);
+    if (rc) return rc;
     if (stats) {
       cudaEventRecord(e1, s);
       if ((rc = collect_status(ctx, s, "chi0_batched"))) return rc;

@@ -784,7 +784,7 @@ int pb_build(spx_ctx* ctx, int nq, const spx_q_desc* qd, const int* S, int nw, i
   // tensor maps per (q, slot): planes [6 nw][nkb][R][64 B]
   std::vector<CUtensorMap> maps(2 * (size_t)nq * nslot);
   for (int i = 0; i < nq; ++i) {
-    if (q[i].N <= 0) continue;
+    if (q[i].N <= 0 || q[i].P <= 0) continue;   // no slab uses its maps
     const uint64_t nkb = (uint64_t)(q[i].S / SP_KB);
     const uint64_t st[3] = {SP_KB, (uint64_t)q[i].R * SP_KB, nkb * q[i].R * SP_KB};
     const uint64_t dims[4] = {SP_KB, (uint64_t)q[i].R, nkb, (uint64_t)SP_SLOT * nw};
@@ -889,6 +889,13 @@ static uint64_t pb_fnv(uint64_t h, const void* p, size_t n) {
   return h;
 }
 
+// Slab of a q of the batch: `force`, else the descriptor's, the tuned one, 16384.
+int pb_slab_of(const spx_ctx* ctx, const spx_q_desc& q, int nw, int force) {
+  const spx_tune_entry* t = pb_find_tune(ctx, q.nbas, q.npair, nw);
+  const int sl = force > 0 ? force : (q.slab_pairs > 0 ? q.slab_pairs : (t ? t->slab_pairs : PB_DEFAULT_SLAB));
+  return std::max(SP_KB, std::min(SP_SLAB, sl / SP_KB * SP_KB));
+}
+
 // One persistent launch for the whole batch (split precision). Slab sizes: the
 // descriptor's, else the tuned, else 16384; tile shape: the tuned shape of the q
 // with most work, else 64 x 80 with 3 stages (`force` overrides both when set).
@@ -901,9 +908,7 @@ int pb_run(spx_ctx* ctx, int nq, const spx_q_desc* q, int nw, const double* omeg
   for (int i = 0; i < nq; ++i) {
     if (q[i].nbas <= 0 || q[i].npair <= 0) continue;
     const spx_tune_entry* t = pb_find_tune(ctx, q[i].nbas, q[i].npair, nw);
-    int sl = q[i].slab_pairs > 0 ? q[i].slab_pairs : (t ? t->slab_pairs : PB_DEFAULT_SLAB);
-    if (force_slab > 0) sl = force_slab;
-    S[i] = std::max(SP_KB, std::min(SP_SLAB, sl / SP_KB * SP_KB));
+    S[i] = pb_slab_of(ctx, q[i], nw, force_slab);
     const double work = (double)q[i].nbas * q[i].nbas * (double)q[i].npair;
     if (work > most) {
       most = work;
