@@ -253,17 +253,21 @@ def int8_ops(N: int, P: int, nw: int, variant: int, slab: int) -> float:
     return 2.0 * 6 * 128 * ncols * tiles * pad * nw
 
 
-def fp64_roofline(ctx, N: int, achieved: float) -> dict:
+def fp64_roofline(ctx, N: int, nw: int, achieved: float) -> dict:
     """Roofline of the FP64 accumulation (DMMA) against this GPU's DMMA rate, measured
-    here by the library's own in-register DMMA loop. The kernel computes only the upper
-    64 x 64 tiles, so the rate the pipe executes is the algorithmic rate times the
-    executed share of the full Gram."""
+    here by the library's own in-register DMMA loop. The kernel visits the upper 16 x 8
+    tiles and forms each band-pair product once (four multiply-adds) for up to 24
+    frequencies (two each, in blocks of eight), so the rate the pipe executes is the
+    algorithmic rate of the full Gram, four multiply-adds per element and frequency, times
+    the executed share; `frac` is that rate over the peak."""
     peak = ctx.measure_dmma_peak()
-    nblk = (N + 63) // 64
-    share = nblk * (nblk + 1) / 2 * 64 * 64 / (N * N)
+    nbj = (N + 7) // 8
+    elems = 128 * sum(bj // 2 + 1 for bj in range(nbj))
+    macs = sum(4 + 16 * -(-min(24, nw - f) // 8) for f in range(0, nw, 24))
+    share = elems * macs / (4.0 * N * N * nw)
     return {"bound": "tensor (FP64 DMMA)", "achieved": achieved, "peak": peak, "unit": UNIT,
-            "frac": achieved / peak, "executed_tflops": achieved * share, "executed_frac": achieved * share / peak,
-            "executed_share_of_full_gram": share, "traffic": None,
+            "frac": achieved * share / peak, "executed_tflops": achieved * share,
+            "executed_frac": achieved * share / peak, "executed_share_of_full_gram": share, "traffic": None,
             "peak_source": "measured: spx_measure_dmma_peak (mma.sync m16n8k8 f64 loop, CUDA events)"}
 
 
@@ -501,7 +505,7 @@ def run_ours(args):
         roof = {"bound": "tensor", "achieved": ach, "peak": bf16s, "unit": UNIT, "frac": ach / bf16s,
                 "traffic": None, "peak_source": f"{src} bf16_tflops_sustained (kernel timed inside a long step)"}
         # the same kernel seen from the int8 pipe it runs on, for the variant and slab that ran
-        variant = tuned["variant"] if tuned else (ctx.split_variant if ctx.split_variant in (1, 3, 5) else 2)
+        variant = tuned["variant"] if tuned else (ctx.split_variant or 5)
         slab = tuned["slab_pairs"] if tuned else 32768
         ops = int8_ops(N, Pr, nw, variant, slab)
         i8 = ops / (kernel_ms * 1e-3) / 1e12
@@ -519,9 +523,9 @@ def run_ours(args):
             roof["traffic_detail"] = dict(tr, kernel=kname, unit="bytes per launch (one slab, all frequencies)",
                                           operand_plane_bytes_per_launch=3.0 * nw * R * min(slab, Pr))
     else:
-        roof = fp64_roofline(ctx, N, ach)
+        roof = fp64_roofline(ctx, N, nw, ach)
     if fp64 is not None:
-        fp64["roofline"] = fp64_roofline(ctx, N, w.flops * (Pr / P) / (fp64["kernel_ms"] * 1e-3) / 1e12)
+        fp64["roofline"] = fp64_roofline(ctx, N, nw, w.flops * (Pr / P) / (fp64["kernel_ms"] * 1e-3) / 1e12)
 
     if rank == 0:
         res = {

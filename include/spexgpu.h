@@ -68,8 +68,8 @@ typedef struct spx_options {
   int32_t chunk_pairs;      /* band pairs per streamed chunk, 0 = auto           */
   int32_t timeout_ms;       /* bound on every device-side wait, 0 = 4000 ms      */
   int32_t split_variant;    /* split-path kernel: 0 auto (the tuning table's choice,
-                               else 5), 1 one CTA per 64 x 64
-                               tile, 2 CTA pair (tcgen05 cta_group::2), 3 the
+                               else 1 or 5, whichever covers nbas with less tile
+                               work), 1 one CTA per 64 x 64 tile, 2 CTA pair (tcgen05 cta_group::2), 3 the
                                persistent schedule with its own preparation warps,
                                5 one CTA per 64 x 80 tile (N = 160 MMAs)         */
   int32_t products;         /* interstitial product GEMM: SPX_PRODUCTS_*         */
@@ -345,14 +345,19 @@ int spx_dielec_dev(spx_ctx* ctx, int32_t nbas, int32_t nw, double* susceph,
                    const double* coul, int32_t invert, double* head, double* wing,
                    void* stream);
 
-/* ---- many q points in one launch (K7) ---------------------------------------
+/* ---- many q points in one call (K7) -----------------------------------------
  * The q loop of the reference driver (src/correlation.f:293-339 calls
  * `susceptibility` once per q point) as one call: every q has its own N_MB,
  * band window and output. Each q is accumulated exactly as by
  * spx_chi0_accumulate_dev (same slabs and kernels, so the same bits). Its M is
  * a device array, or is generated on the device slab by slab from the seeded
  * Philox stream (cprod = NULL), so that no q's M is ever held whole.
- * With SPX_SPLIT the whole batch runs as ONE persistent kernel: every SM takes
+ * With SPX_SPLIT, when every M is given, every descriptor leaves variant and slab
+ * open and the batch is large (a mean of half a million nbas x npair x nw elements
+ * per q), each q runs through the kernels of spx_chi0_accumulate_dev in turn, in
+ * the context workspace, with slabs of the tuning table or 16384 pairs and without
+ * a graph. Otherwise, and where workspace_limit is too small for that, the whole
+ * batch runs as ONE persistent kernel: every SM takes
  * accumulation items (slab, tile, frequency) and operand-preparation items
  * (generation of M, weights, digit planes) from two device work queues, the q
  * with most work first, with bounded waits on the slabs' readiness; the tile

@@ -1,14 +1,17 @@
-// K7: the polarisation of many q points in one launch, and the split-path autotuner.
+// K7: the polarisation of many q points in one call, and the split-path autotuner.
 //
 // The reference computes one q point per call of `susceptibility`
 // (src/correlation.f:293-339), each with its own mixed basis and band window.
-// spx_chi0_batched takes the whole list: the schedule of every q (optional
-// on-device generation of M, FP64 weights, digit planes, int8 tensor-core
-// accumulation, slab by slab) is captured once into a CUDA graph and replayed
-// with one launch; the graph is cached in the context under a hash of the
-// batch (shapes, pointers, workspace), so a repeated batch costs one
-// cudaGraphLaunch. Per q the slabs and kernels are exactly those of
-// spx_chi0_accumulate_dev, so results are bit-identical to per-q calls.
+// spx_chi0_batched takes the whole list. A split batch is one persistent kernel, or, when its
+// products are all given and large enough, the one-call kernels q by q (batch_by_q). FP64
+// batches and SPX_BATCH_KERNELS run the schedule of every q (optional on-device generation of
+// M, FP64 weights, digit planes, accumulation, slab by slab). The persistent kernel and that
+// schedule are captured once into a CUDA graph, cached in the context under a hash of the
+// batch (shapes, pointers, workspace), so a repeated batch costs one cudaGraphLaunch. Per q
+// the slabs, scales and digits are those of spx_chi0_accumulate_dev with the same slab size
+// and the integer sums are exact, so results are bit-identical to such calls; above 148
+// tiles per frequency, where separate kernels accumulate a slab in parts, they differ by the
+// rounding of the parts' FP64 adds.
 //
 // The autotuner times the split-kernel variants (one CTA per tile, CTA pair)
 // and slab sizes on a seeded probe of each (N bucket, pair bucket, nw) and keeps

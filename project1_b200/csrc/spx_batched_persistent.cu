@@ -24,7 +24,8 @@
 // hands items out only to CTAs that run), so the schedule cannot deadlock, whether
 // or not all CTAs are resident. The epilogue of slab s of a q adds into an output
 // tile only after slab s-1 has added into it (a per-(q, tile, frequency) counter),
-// so the sums happen in the same order as per-q calls and give the same bits.
+// so the sums happen in the same order as per-q calls and give the same bits (up to the
+// rounding of FP64 adds where those accumulate a slab in parts: above 148 tiles per frequency).
 #include <cuda.h>
 #include <cuda_runtime.h>
 

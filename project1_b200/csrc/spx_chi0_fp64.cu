@@ -1,6 +1,9 @@
-// K1: complex FP64 band-pair accumulation on the DMMA tensor path (the drop-in).
+// K1, K1p, K1r: FP64 band-pair accumulation on the DMMA tensor path (the drop-in).
 //
-// Computes, for every upper-triangle 64x64 tile (I, J) of the mixed-basis
+// Most calls run on the product-first kernels further down (K1p: complex, -DINV and the
+// q -> 0 head and wings); the two that follow the sum frequency by frequency keep calls of
+// one to four frequencies where they are faster (f64_takes_k1, f64r_takes_k1r). K1 computes,
+// for every upper-triangle 64x64 tile (I, J) of the mixed-basis
 // matrix and every frequency f,
 //   chi_f(i, j) += sum_p M(p, i) * conj(M(p, j)) * w(p, f),      i <= j,
 // which is the body loop of src/susceptibility.f:1182-1240 with the HILBERT
@@ -933,7 +936,7 @@ int launch_chi0_fp64_noctx(int num_sms, int* status, uint64_t timeout_ns, const 
 }
 
 // ---------------------------------------------------------------------------
-// K1r: the -DINV build (MCOMPLEX_dp = real_dp, src/cppmacro.h:53-64), where
+// K1r: the -DINV build for few frequencies (MCOMPLEX_dp = real_dp, src/cppmacro.h:53-64), where
 // re(k) = cprod(k,i) * cprod(k,j) (src/susceptibility.f:1197) and chi is real:
 //   chi_f(i, j) += sum_p M(p, i) M(p, j) w(p, f),  i <= j,
 // on the same pipeline as K1 with one 2-D TMA box of 16 pairs x 64 columns per

@@ -30,6 +30,10 @@
 // g >= 3 are of the same size; both enter with the crest factor max|A| sqrt(P)/||A||
 // of the folded columns.
 //
+// A slab runs as statistics (column scales, weights, signs), digit planes, accumulation and,
+// when the last items were cut along the pairs over all CTAs, the exact sum of their partial
+// tiles; a wide slab's planes are written and accumulated in parts that leave room in L2.
+//
 // Tile layout: a 64 x 64 complex tile is a 128 x 128 real-stacked product whose rows
 // interleave the parts of each mixed-basis function: row 2i holds Re A_i and row
 // 2i+1 holds Im A_i (likewise the columns for j). D[2i+c][2j+c'] then holds the four

@@ -285,11 +285,12 @@ class Context:
         self._check(rc, "spx_trafo_olap_dev")
         return o
 
-    # ---- many q points in one launch ---------------------------------------------
+    # ---- many q points in one call -----------------------------------------------
 
     def chi0_batched(self, qs, omega, precision: str = "split", flags: int = 0, stream=None,
                      stats: bool = False) -> Optional[dict]:
-        """Accumulates every q of `qs` (dicts, see below) in one launch of a cached graph.
+        """Accumulates every q of `qs` (dicts, see below): split batches as one persistent kernel
+        or, with given products of some size, q by q; FP64 batches as one graph of kernels.
 
         Each dict: nbas, npair, ediff (device float64), susceph (device complex128
         (nw, npack)), optionally cprod (device (nbas, ldc)) or seed/stream_id/m_scale
