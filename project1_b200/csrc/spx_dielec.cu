@@ -165,9 +165,11 @@ __device__ __forceinline__ void sweep_extract(SweepTile& tile, const double2* Aw
 // columns; meanwhile the other CTAs extract the column panels and put the panels of the
 // pivot block before into A from its U: no two touch the same elements. Inverse,
 // extraction and panels took 39 + 14 + 13 us one after the other at 24 matrices of 1200, 45
-// together. A pivot that is not positive records (block row + 1) in info[frequency]. The chain of 64 pivots is serial, so a step is kept short: thread
-// (r, c) of 16 x 16 holds rows r + 16 x, columns c + 16 y in registers, the pivot's row and
-// column go through shared memory, two buffers and one barrier per step.
+// together. A pivot that is not positive records (block row + 1) in info[frequency]. The
+// chain of 64 pivots is serial, so a step is kept short: thread (r, c) of 16 x 16 holds rows
+// r + 16 x, columns c + 16 y in registers, the pivot's row and column go through shared
+// memory, two buffers and one barrier per step. (Updating and publishing the next pivot's
+// row, column and reciprocal ahead of the rest of a step gained nothing.)
 __global__ void __launch_bounds__(256) sweep_pivot_kernel(double2* A, int n, int kb, int bk, int nw,
                                                           const double2* U, double2* __restrict__ CpT,
                                                           double2* __restrict__ Pb, int* __restrict__ info) {
