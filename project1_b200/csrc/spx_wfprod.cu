@@ -80,8 +80,10 @@ struct __align__(16) ZgSmem {
 struct ZgTile {
   int m0, c0, b1, b2;
 };
+// FLAT: items fit in 32 bits and b2 is always 0.
+template <bool FLAT>
 __device__ __forceinline__ ZgTile zg_tile(const ZgParams& prm, int64_t item, int64_t tiles) {
-  const int b = (int)(item / tiles), t = (int)(item - b * tiles);
+  const int b = FLAT ? (int)item / (int)tiles : (int)(item / tiles), t = (int)(item - b * tiles);
   int tm, tn;
   if (prm.upper) {
     int j = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
@@ -97,6 +99,7 @@ __device__ __forceinline__ ZgTile zg_tile(const ZgParams& prm, int64_t item, int
     tm = t % prm.mtiles;
     tn = t / prm.mtiles;
   }
+  if (FLAT) return {tm * ZG_B, tn * ZG_B, b, 0};
   return {tm * ZG_B, tn * ZG_B, b % prm.nb1, b / prm.nb1};
 }
 
@@ -109,8 +112,14 @@ __device__ __forceinline__ ZgTile zg_tile(const ZgParams& prm, int64_t item, int
 // per tile with a two-stage pipeline: 48000 x 1014 x 3000 gathered 38.5 -> 36.5 ms (0.86
 // of the DMMA rate), 48000 x 1100 x 1200 m-contiguous 16.8 -> 15.3 ms, K = 243 (muffin
 // tin) 1.9 -> 1.66 ms. With the output fetched ahead the
-// gathered products take 35.7 ms and 24 inverses of 1200 10.5 instead of 11.1.
-template <bool MC, bool GATHER, bool ADD>
+// gathered products take 35.7 ms, and 24 inverses of 1200 0.6 ms less.
+//
+// FLAT: one run of columns (ncin == ncol, no cOff) and one level of batches. A tile's
+// addresses then need no divisions and are formed once, by the loader (which is inside the
+// tile when its first chunk computes: at least two chunks, K > 16). With the two warps per
+// scheduler that fit, those chains are exposed: 24 rank-64 updates of 1200 (upper tiles) take
+// 341 us, 370 with them, and 330 with an epilogue of 16 loads at a time instead of four.
+template <bool MC, bool GATHER, bool ADD, bool FLAT = false>
 __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams prm, int64_t tiles,
                                                                     int64_t items) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -124,10 +133,13 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
   int l_chunk = 0, a_mask = 0, b_mask = 0, l_stage = 0;
   const double2* pa = nullptr;
   const double2* pb = nullptr;
+  ZgTile lq{};
   auto enter = [&] {
-    const ZgTile q = zg_tile(prm, l_item, tiles);
+    const ZgTile q = zg_tile<FLAT>(prm, l_item, tiles);
+    if (FLAT) lq = q;
     const double2* ab = prm.A + q.b1 * prm.sA1 + q.b2 * prm.sA2;
     pb = prm.B + q.b1 * prm.sB1 + q.b2 * prm.sB2;
+    if (FLAT) pb += (int64_t)(q.c0 + r0) * prm.sBc;
     a_mask = b_mask = 0;
     if (MC) {
       a_mask = q.m0 + mr < prm.M;
@@ -139,6 +151,10 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
     for (int j = 0; j < 8; ++j) {
       if (!MC) a_mask |= (q.m0 + r0 + 8 * j < prm.M) << j;
       const int col = q.c0 + r0 + 8 * j;
+      if (FLAT) {
+        b_mask |= (col < prm.ncol) << j;
+        continue;
+      }
       int64_t off = 0;
       if (col < prm.ncol) {
         b_mask |= 1 << j;
@@ -167,7 +183,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
                      v ? pa + (int64_t)(8 * j) * prm.lda + k0 : prm.A, v);
         }
         const bool v = kin && (b_mask >> j & 1);
-        cp_async16(&sm.b[l_stage][r0 + 8 * j][lk ^ zg_swz(r0 + 8 * j)], v ? pb + sm.boff[j][tid] + ko : prm.B, v);
+        cp_async16(&sm.b[l_stage][r0 + 8 * j][lk ^ zg_swz(r0 + 8 * j)], v ? pb + (FLAT ? (int64_t)(8 * j) * prm.sBc : sm.boff[j][tid]) + ko : prm.B, v);
       }
       if (++l_chunk == nst) l_chunk = 0, l_item += gridDim.x;
     }
@@ -181,6 +197,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
   const int g = lane >> 2, t = lane & 3;
   int st = 0;
   for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+    const ZgTile cur = lq;   // FLAT
     double accR[2][4][4], accI[2][4][4];
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
@@ -193,11 +210,11 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
     if (ADD && !prm.overwrite) {
       // the values this tile adds to come from memory while it computes: thread -> column
       // tid / 2, 32 rows in four 128-byte lines
-      const ZgTile q = zg_tile(prm, item, tiles);
+      const ZgTile q = FLAT ? cur : zg_tile<FLAT>(prm, item, tiles);
       const double2* ob = prm.O + q.b1 * prm.sO1 + q.b2 * prm.sO2;
       const int cl = q.c0 + (tid >> 1), m = q.m0 + 32 * (tid & 1);
       if (cl < prm.ncol) {
-        const int n = cl / prm.ncin, c = cl - n * prm.ncin;
+        const int n = FLAT ? 0 : cl / prm.ncin, c = cl - n * prm.ncin;
         const double2* o = ob + (int64_t)n * prm.sOn + (int64_t)c * prm.sOc + m;
 #pragma unroll
         for (int x = 0; x < 32; x += 8)
@@ -248,16 +265,44 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
       if (++st == ZG_ST) st = 0;
     }
 
-    const ZgTile q = zg_tile(prm, item, tiles);
+    const ZgTile q = FLAT ? cur : zg_tile<FLAT>(prm, item, tiles);
     double2* ob = prm.O + q.b1 * prm.sO1 + q.b2 * prm.sO2;
     const double2 al = prm.alpha ? prm.alpha[q.b1] : prm.alpha_v;
+    if constexpr (FLAT) {
+      // 16 loads in flight per thread: four columns of four rows
+#pragma unroll
+      for (int nt = 0; nt < 4; nt += 2) {
+        const int m0 = q.m0 + 32 * wi + g, c0 = q.c0 + 32 * wj + 8 * nt + 2 * t;
+        auto in = [&](int z, int x) { return c0 + 8 * (z >> 1) + (z & 1) < prm.ncol && m0 + 8 * x < prm.M; };
+        auto at = [&](int z) { return ob + (int64_t)(c0 + 8 * (z >> 1) + (z & 1)) * prm.sOc + m0; };
+        double2 v[4][4];
+#pragma unroll
+        for (int z = 0; z < 4; ++z)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            v[z][x] = make_double2(0.0, 0.0);
+            if (ADD && in(z, x)) v[z][x] = at(z)[8 * x];
+          }
+#pragma unroll
+        for (int z = 0; z < 4; ++z)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            const double re = accR[x >> 1][nt + (z >> 1)][2 * (x & 1) + (z & 1)];
+            const double im = accI[x >> 1][nt + (z >> 1)][2 * (x & 1) + (z & 1)];
+            v[z][x].x += al.x * re - al.y * im;
+            v[z][x].y += al.x * im + al.y * re;
+            if (in(z, x)) at(z)[8 * x] = v[z][x];
+          }
+      }
+      continue;
+    }
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int cl = q.c0 + 32 * wj + 8 * nt + 2 * t + e;
         if (cl >= prm.ncol) continue;
-        const int n = cl / prm.ncin, c = cl - n * prm.ncin;
+        const int n = FLAT ? 0 : cl / prm.ncin, c = cl - n * prm.ncin;
         double2* oc = ob + (int64_t)n * prm.sOn + (int64_t)c * prm.sOc;
         double2 v[4];
 #pragma unroll
@@ -296,7 +341,17 @@ int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s) {
     kernel<<<grid, ZG_THREADS, smem, s>>>(prm, tiles, items);
   };
   if (prm.a_mcontig && prm.kOff) return set_error(ctx, SPX_EINVAL, "product GEMM: unsupported operand form");
-  if (prm.overwrite) {
+  const bool flat = !prm.kOff && !prm.cOff && prm.ncin == prm.ncol && prm.nb1 >= nbatch && prm.K > ZG_KC &&
+                    items + grid < 0x7fffffff;
+  if (flat) {
+    if (prm.overwrite) {
+      if (prm.a_mcontig) run(zgemm_gather_kernel<true, false, false, true>);
+      else run(zgemm_gather_kernel<false, false, false, true>);
+    } else {
+      if (prm.a_mcontig) run(zgemm_gather_kernel<true, false, true, true>);
+      else run(zgemm_gather_kernel<false, false, true, true>);
+    }
+  } else if (prm.overwrite) {
     if (prm.a_mcontig) run(zgemm_gather_kernel<true, false, false>);
     else if (prm.kOff) run(zgemm_gather_kernel<false, true, false>);
     else run(zgemm_gather_kernel<false, false, false>);
