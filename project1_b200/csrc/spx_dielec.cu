@@ -19,8 +19,8 @@
 // the complex FP64 DMMA GEMM (K4c). The matrix stays Hermitian through the sweep, so
 // only the 64 x 64 tiles on and above the diagonal are kept up to date: half of the
 // multiply-adds and of the traffic of the updates. Measured at 24 matrices of 1200: 23.6 ms
-// with full updates and the pivot block swept in shared memory, 8.6 ms here (updates
-// 18.1 -> 6.5 ms: 0.70 of the FP64 pipe, a 64-deep tile's epilogue taking the rest; pivot
+// with full updates and the pivot block swept in shared memory, 8.4 ms here (updates
+// 18.1 -> 6.3 ms: 0.72 of the FP64 pipe, a 64-deep tile's epilogue taking the rest; pivot
 // blocks and panels 4.0 -> 0.86 ms).
 #include <cuda_runtime.h>
 
