@@ -45,6 +45,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "spx_chain.cuh"
 #include "spx_split.cuh"
 
 namespace spx {
@@ -223,30 +224,6 @@ __device__ __forceinline__ void real_epilogue(uint32_t tl, int q, int lane, int 
     }
   }
   release();
-}
-
-// The kernels of a one-slab call run as a chain: each lets the next one's CTAs start as soon
-// as its own have all started (release_next) and waits, before it reads what the one before
-// wrote, until that has finished (await_previous). The first kernel of the chain is an
-// ordinary launch, so what came before the call is complete by then. Launched otherwise,
-// both do nothing. 96 columns, 160 pairs, 4 frequencies: 24.6 us unchained, 20.5 chained; 403
-// columns, 12201 pairs, 12 frequencies: 447 and 430.
-__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <typename... P, typename... A>
-static cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s,
-                                  bool chained, A&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 // BN: complex columns of a tile (64 or 80; the -DINV form uses 64, i.e. 128 x 128

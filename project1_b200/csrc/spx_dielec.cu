@@ -28,6 +28,7 @@
 #include <string>
 #include <vector>
 
+#include "spx_chain.cuh"
 #include "spx_common.cuh"
 #include "spx_zgemm.h"
 
@@ -125,6 +126,7 @@ __device__ __forceinline__ void sweep_panels(SweepTile& tile, double2* Aw, int n
 }
 __global__ void __launch_bounds__(256) sweep_panels_kernel(double2* A, int n, int kb, int bk, const double2* U) {
   __shared__ SweepTile tile;
+  await_previous();
   const int64_t f = blockIdx.y;
   sweep_panels(tile, A + f * n * n, n, kb, bk, U + f * n * DI_B, 16 * blockIdx.x);
 }
@@ -174,6 +176,7 @@ __global__ void __launch_bounds__(256) sweep_pivot_kernel(double2* A, int n, int
                                                           const double2* U, double2* __restrict__ CpT,
                                                           double2* __restrict__ Pb, int* __restrict__ info) {
   __shared__ double2 col[2][DI_B], row[2][DI_B];
+  release_next();
   if ((int)blockIdx.x >= nw) {
     __shared__ SweepTile tile;
     const int e = blockIdx.x - nw, nx = (n + 15) / 16, g = e / nx, x = 16 * (e - g * nx);
@@ -347,6 +350,8 @@ extern "C" int spx_dielec_dev(spx_ctx* ctx, int32_t nbas, int32_t nw, double* su
   const int nx = (n + 15) / 16;
   for (int kb = 0; kb < n; kb += DI_B) {
     const int bk = std::min(DI_B, n - kb);
+    // the GEMMs follow this kernel as a chain; not it them: its first CTAs, the serial
+    // inverses, would land in pairs on the SMs that drain first (24 of 1200: 8.4 -> 8.7 ms)
     sweep_pivot_kernel<<<nw * (1 + nx * (kb ? 2 : 1)), 256, 0, s>>>(full, n, kb, bk, nw, U, CpT, Pb, info);
     if ((rc = check_cuda(ctx, cudaGetLastError(), "sweep pivot block"))) return rc;
     // U = Cp P: U(i, c) = sum_t Cp(i, t) conj(P(c, t))   (P Hermitian)
@@ -367,7 +372,7 @@ extern "C" int spx_dielec_dev(spx_ctx* ctx, int32_t nbas, int32_t nw, double* su
     g.K = bk;
     g.nb1 = nw;
     g.overwrite = 1;
-    if ((rc = launch_zgemm(ctx, g, nw, s))) return rc;
+    if ((rc = launch_zgemm(ctx, g, nw, s, true))) return rc;
     // A(i, j) -= sum_t U(i, t) conj(Cp(j, t))   (= U_i A_kj, A Hermitian)
     ZgParams h{};
     h.A = U;
@@ -388,10 +393,11 @@ extern "C" int spx_dielec_dev(spx_ctx* ctx, int32_t nbas, int32_t nw, double* su
     h.nb1 = nw;
     h.upper = 1;
     h.skip = kb / DI_B + 1;   // the panels replace these tiles: 171 of 190 are left at n = 1200
-    if ((rc = launch_zgemm(ctx, h, nw, s))) return rc;
+    if ((rc = launch_zgemm(ctx, h, nw, s, true))) return rc;
     if (kb + bk < n) continue;
-    sweep_panels_kernel<<<dim3(nx, nw), 256, 0, s>>>(full, n, kb, bk, U);
-    if ((rc = check_cuda(ctx, cudaGetLastError(), "sweep panels"))) return rc;
+    if ((rc = check_cuda(ctx, launch_chained(sweep_panels_kernel, dim3(nx, nw), 256, 0, s, true, full, n, kb, bk, U),
+                         "sweep panels")))
+      return rc;
   }
   // the sweep leaves -inv(eps)
   pack_upper_kernel<<<dim3(grid, nw), 256, 0, s>>>(full, n, -1.0, P);

@@ -30,6 +30,7 @@
 #include <string>
 #include <vector>
 
+#include "spx_chain.cuh"
 #include "spx_common.cuh"
 #include "spx_zgemm.h"
 
@@ -196,6 +197,8 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
     cp_async_commit();
     if (++l_stage == ZG_ST) l_stage = 0;
   };
+  release_next();
+  await_previous();
   issue();
   issue();
 
@@ -330,7 +333,7 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
   cp_async_wait<0>();
 }
 
-int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s) {
+int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s, bool chained) {
   if (prm.M <= 0 || prm.ncol <= 0 || prm.K <= 0 || nbatch <= 0) return SPX_OK;
   prm.mtiles = (prm.M + ZG_B - 1) / ZG_B;
   prm.ntiles = (prm.ncol + ZG_B - 1) / ZG_B;
@@ -344,7 +347,7 @@ int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s) {
   const int grid = (int)std::min<int64_t>(items, (int64_t)2 * ctx->num_sms);
   auto run = [&](auto kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kernel<<<grid, ZG_THREADS, smem, s>>>(prm, tiles, items);
+    launch_chained(kernel, grid, ZG_THREADS, smem, s, chained, prm, tiles, items);
   };
   if (prm.a_mcontig && prm.kOff) return set_error(ctx, SPX_EINVAL, "product GEMM: unsupported operand form");
   const bool flat = !prm.kOff && !prm.cOff && prm.ncin == prm.ncol && prm.nb1 >= nbatch && prm.K > ZG_KC &&

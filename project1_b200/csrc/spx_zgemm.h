@@ -33,6 +33,7 @@ struct ZgParams {
 };
 
 // Batch b = b1 + nb1 * b2 runs on grid.y; tiles of 64 x 64 on grid.x.
-int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s);
+// chained: follows its predecessor on `s` by a programmatic launch (spx_chain.cuh).
+int launch_zgemm(spx_ctx* ctx, ZgParams prm, int nbatch, cudaStream_t s, bool chained = false);
 
 }  // namespace spx
