@@ -110,6 +110,9 @@ __global__ void __launch_bounds__(256, 3) dft_across_kernel(DftAcross p) {
   for (int i = threadIdx.x; i < p.n; i += blockDim.x) tw[i] = p.tw[i];
   __syncthreads();
   const int nh = p.n / 2 + 1, ng = (nh + DFT_JP - 1) / DFT_JP;
+  // pairs past the last one repeat it and are not stored: a step of the table index
+  // stays below n, so one subtraction keeps it in the table
+  const int last = nh - 1;
   const int64_t total = p.outer * ng * p.n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -125,7 +128,7 @@ __global__ void __launch_bounds__(256, 3) dft_across_kernel(DftAcross p) {
 #pragma unroll
     for (int k = 0; k < DFT_JP; ++k) {
       pc[k] = ps[k] = make_double2(0.0, 0.0);
-      m[k] = ((p.lo * (j0 + k)) % p.n + p.n) % p.n;
+      m[k] = ((p.lo * min(j0 + k, last)) % p.n + p.n) % p.n;
     }
 #pragma unroll 2
     for (int i = 0; i < p.nin; ++i) {
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(256, 3) dft_across_kernel(DftAcross p) {
         pc[k].y = fma(v.y, w.x, pc[k].y);
         ps[k].x = fma(v.x, w.y, ps[k].x);
         ps[k].y = fma(v.y, w.y, ps[k].y);
-        m[k] += j0 + k;
+        m[k] += min(j0 + k, last);
         if (m[k] >= p.n) m[k] -= p.n;
       }
     }
