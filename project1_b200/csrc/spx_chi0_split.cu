@@ -1002,10 +1002,16 @@ int make_tmap_u8_4d(spx_ctx* ctx, CUtensorMap* map, const void* base, const uint
 }
 
 struct SplitLayout {
-  int64_t Ps, Pp, R;   // pairs of a slab, pairs of one operand buffer, plane rows
-  int nblk, nbuf;
+  int64_t Ps, most, R;   // pairs of a slab, the most pairs of a part, plane rows
+  int64_t pairs;         // pairs of planes reserved, for all operand buffers together
+  int nblk, nstat;       // sets of slab statistics
   size_t f_bytes, g_bytes, s_bytes, w_bytes, sg_bytes;
-  size_t bytes() const { return nbuf * (f_bytes + g_bytes + s_bytes + w_bytes + sg_bytes) + 1024; }
+  size_t bytes() const { return f_bytes + nstat * (g_bytes + s_bytes + w_bytes + sg_bytes) + 1024; }
+  // Pairs of a part of a slab of `len` pairs.
+  int64_t part(int64_t len) const {
+    const int64_t n = std::max<int64_t>((len + most - 1) / most, 1);
+    return (int64_t)align_up((size_t)((len + n - 1) / n), SP_KB);
+  }
 };
 
 // Tiles of one frequency on 64 x BN complex tiles (the -DINV form: 128 x 2 BN real ones,
@@ -1022,34 +1028,35 @@ static int split_ntile(int n, int bn, int nbr) {
 // unless their last column block is nearly empty (403 columns: 28 tiles of either shape).
 static bool split_wide(int n, int nbr) { return split_ntile(n, SP_WIDE_BN, nbr) * 110 < split_ntile(n, SP_TILE, nbr) * 100; }
 
-// Pairs of one operand buffer: a slab's scales and factors hold for all of it, but its planes
-// are written and accumulated in equal parts of at most this many pairs (the parts' FP64
-// adds are the only difference from one pass).
+// Most pairs of a part: a slab's scales and factors hold for all of it, but its planes are
+// written and accumulated in equal parts of at most this many pairs (the parts' FP64 adds are
+// the only difference from one pass). The parts depend on the slab's own length only, so a
+// slab gives the same bits in whatever call it lies.
 //   * With more tiles per frequency than SMs, a round of CTAs reads a frequency's planes
 //     while the rest of its tiles wait for the next round: the planes come from L2 again
 //     only if they (3 digits x R rows x pairs) leave room there. Measured at 1200 columns,
 //     full calls of a million pairs, one kernel: 739-747 TFLOP/s with 8192 and 12288 pairs
 //     (60 and 90 MB), 718-723 with 16384 (120 MB), 641 with 32768.
 //   * Otherwise a round's CTAs walk the same pairs together: the whole slab.
-static int64_t split_part_pairs(int64_t Ps, int ntile, int64_t R) {
-  int64_t most = Ps;
-  if (ntile > SP_SMS)
-    most = std::min<int64_t>(most, std::max<int64_t>(4096, (90ll << 20) / (SP_SF * R) / SP_KB * SP_KB));
-  const int64_t n = (Ps + most - 1) / most;
-  return (int64_t)align_up((size_t)((Ps + n - 1) / n), SP_KB);
+static int64_t split_part_most(int64_t slab, int ntile, int64_t R) {
+  if (ntile <= SP_SMS) return slab;
+  return std::min<int64_t>(slab, std::max<int64_t>(4096, (90ll << 20) / (SP_SF * R) / SP_KB * SP_KB));
 }
 
 // slab: band pairs per exact int32 slab, a multiple of SP_KB in [SP_KB, SP_SLAB]; R plane rows.
 // Two operand buffers when there is more than one part: the next part is quantized
-// while one accumulates.
+// while one accumulates. The size never falls with P, so scratch for a call holds every
+// shorter one of its width: the planes of one slab take the slab's pairs at most (two parts
+// share them), those of several slabs two of the longest parts.
 static SplitLayout split_layout_of(int64_t P, int nblk, int64_t R, int ntile, int ncol, int nw, int slab) {
   SplitLayout L;
   L.Ps = std::min<int64_t>((int64_t)align_up((size_t)std::max<int64_t>(P, 1), SP_KB), slab);
-  L.Pp = split_part_pairs(L.Ps, ntile, R);
+  L.most = split_part_most(slab, ntile, R);
+  L.pairs = P > slab ? 2 * L.most : std::min(L.Ps, 2 * L.most);
   L.nblk = nblk;
   L.R = R;
-  L.nbuf = P > L.Pp ? 2 : 1;
-  L.f_bytes = align_up((size_t)SP_SLOT * nw * R * L.Pp, 1024);
+  L.nstat = P > slab ? 2 : 1;
+  L.f_bytes = align_up((size_t)SP_SLOT * nw * R * L.pairs, 1024);
   L.g_bytes = align_up(sizeof(double) * (size_t)nw * L.Ps, 256);
   L.s_bytes = align_up(sizeof(double) * (size_t)std::max(ncol, 1), 256);
   L.w_bytes = align_up(sizeof(double) * (size_t)std::max(nw, 1), 256);
@@ -1117,20 +1124,28 @@ static int split_gram_launch(spx_ctx* ctx, const CUtensorMap& mapA, const CUtens
   return SPX_OK;
 }
 
-// One operand buffer set of a call.
+// The buffers of a call: `n` operand buffers of Pp[b] pairs each, and the statistics of the
+// slabs in turn.
 struct SplitBuf {
   int8_t* F;
+  int64_t Pp;
   double *G, *sA, *wmax;
   int* wsgn;
 };
-static void split_buffers(const SplitLayout& L, uint8_t* base, SplitBuf (&buf)[2]) {
-  const size_t set_bytes = L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes + L.sg_bytes;
+static int split_buffers(const SplitLayout& L, int64_t P, int nw, uint8_t* base, SplitBuf (&buf)[2]) {
+  const int64_t rest = P % L.Ps, p0 = std::max(L.part(L.Ps), rest ? L.part(rest) : 0);
+  buf[0].Pp = p0;
+  buf[1].Pp = L.nstat == 1 ? std::min(p0, L.Ps - p0) : p0;   // one slab: what its first part leaves
+  buf[0].F = (int8_t*)base;
+  buf[1].F = (int8_t*)base + (size_t)SP_SLOT * nw * L.R * p0;
   for (int b = 0; b < 2; ++b) {
-    uint8_t* s0 = base + (size_t)(b < L.nbuf ? b : 0) * set_bytes;
-    buf[b] = {(int8_t*)s0, (double*)(s0 + L.f_bytes), (double*)(s0 + L.f_bytes + L.g_bytes),
-              (double*)(s0 + L.f_bytes + L.g_bytes + L.s_bytes),
-              (int*)(s0 + L.f_bytes + L.g_bytes + L.s_bytes + L.w_bytes)};
+    uint8_t* s0 = base + L.f_bytes + (b < L.nstat ? b : 0) * (L.g_bytes + L.s_bytes + L.w_bytes + L.sg_bytes);
+    buf[b].G = (double*)s0;
+    buf[b].sA = (double*)(s0 + L.g_bytes);
+    buf[b].wmax = (double*)(s0 + L.g_bytes + L.s_bytes);
+    buf[b].wsgn = (int*)(s0 + L.g_bytes + L.s_bytes + L.w_bytes);
   }
+  return buf[1].Pp > 0 ? 2 : 1;
 }
 
 // One part of a slab: slab pairs [p0, p0 + len), part [off, off + plen) of them.
@@ -1146,17 +1161,16 @@ struct SplitStep {
 // single part has nothing to run beside and stays on `stream`. The statistics buffer of
 // slab s is reused by slab s + 2, whose first part waits for a part of slab s + 1 at least.
 template <class Stat, class Quant, class Gram>
-static int split_run_steps(spx_ctx* ctx, const SplitLayout& L, int64_t P, cudaStream_t stream, Stat stat,
+static int split_run_steps(spx_ctx* ctx, const SplitLayout& L, int64_t P, int nbuf, cudaStream_t stream, Stat stat,
                            Quant quant, Gram gram) {
   std::vector<SplitStep> steps;
   for (int64_t p0 = 0, s = 0; p0 < P; p0 += L.Ps, ++s) {
-    const int len = (int)std::min<int64_t>(L.Ps, P - p0);
-    for (int off = 0; off < len; off += (int)L.Pp)
-      steps.push_back({p0, len, off, (int)std::min<int64_t>(L.Pp, len - off), (int)(s % 2) * (L.nbuf - 1),
-                       (int)(steps.size() % L.nbuf), false});
+    const int len = (int)std::min<int64_t>(L.Ps, P - p0), part = (int)L.part(len);
+    for (int off = 0; off < len; off += part)
+      steps.push_back({p0, len, off, std::min(part, len - off), (int)(s % L.nstat), (int)(steps.size() % nbuf), false});
   }
   steps.back().last = true;
-  const bool two = steps.size() > 1;   // L.nbuf == 2: the kernels of a part lie on two streams, unchained
+  const bool two = nbuf == 2;   // the kernels of a part lie on two streams, unchained
   cudaStream_t ps = two ? ctx->prep_stream : stream;
   cudaEvent_t prep_done[2] = {ctx->sev[1], ctx->sev[2]};
   cudaEvent_t gram_done[2] = {ctx->sev[3], ctx->sev[4]};
@@ -1202,11 +1216,10 @@ static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P
     return set_error(ctx, SPX_EINVAL, "split workspace too small");
   uint8_t* base = (uint8_t*)align_up((size_t)ws, 1024);
   SplitBuf buf[2];
-  split_buffers(L, base, buf);
+  const int nbuf = split_buffers(L, P, nw, base, buf);
 
   // planes in HBM: [plane][k-block][row][K bytes]; TMA dims (K, row, k-block, plane)
   // with increasing strides; a box (K, rows, 1, 3 planes) lands as [plane][row][K]
-  const uint64_t nkb = (uint64_t)(L.Pp / SP_KB);
   if (variant == 0) variant = ctx->opt.split_variant;
   if (variant == 0) variant = split_wide(N, L.nblk) ? 5 : 1;  // untuned: one CTA per tile
   const bool pair = variant == 2;
@@ -1219,7 +1232,8 @@ static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P
   // buffers are sized for it either way)
   if (!pair) L.R = (int64_t)L.nblk * SP_ROWS;
   CUtensorMap mapF[2], mapFh[2], mapW[2];
-  for (int b = 0; b < L.nbuf; ++b) {
+  for (int b = 0; b < nbuf; ++b) {
+    const uint64_t nkb = (uint64_t)(buf[b].Pp / SP_KB);
     const uint64_t st[3] = {SP_KB, (uint64_t)L.R * SP_KB, nkb * L.R * SP_KB};
     const uint64_t d[4] = {SP_KB, (uint64_t)L.R, nkb, (uint64_t)SP_SLOT * nw};
     const uint32_t bx[4] = {SP_KB, SP_ROWS, 1, SP_SF};
@@ -1278,8 +1292,8 @@ static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P
     const int nchunk = (int)align_up((size_t)t.plen, SP_KB) / 16;  // 16-pair chunks; npad is a multiple of 64
     const int64_t nthr = (int64_t)npad * nchunk * 2;                // 8-pair tasks
     ++*launches;
-    return check_cuda(ctx, launch_chained(split_quantize_kernel, (unsigned)((nthr + 127) / 128), 128, 0, ps, L.nbuf == 1,
-                                          M, ldc, t.p0 + t.off, t.plen, nchunk, N, npad, L.R, L.Pp, nw, buf[t.sb].sA,
+    return check_cuda(ctx, launch_chained(split_quantize_kernel, (unsigned)((nthr + 127) / 128), 128, 0, ps, nbuf == 1,
+                                          M, ldc, t.p0 + t.off, t.plen, nchunk, N, npad, L.R, buf[t.b].Pp, nw, buf[t.sb].sA,
                                           buf[t.sb].wsgn, buf[t.sb].G + t.off, (int)align_up((size_t)t.len, SP_KB),
                                           buf[t.b].F),
                       "split_quantize_kernel launch");
@@ -1305,10 +1319,10 @@ static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P
       return check_cuda(ctx, cudaLaunchKernelEx(&cfg, split_gram2_kernel, mapF[t.b], mapFh[t.b], prm),
                         "split_gram2_kernel launch");
     }
-    if (wide) return split_gram_launch<false, SP_WIDE_BN>(ctx, mapF[t.b], mapW[t.b], prm, t.last ? part : nullptr, stream, L.nbuf == 1, launches);
-    return split_gram_launch<false, SP_TILE>(ctx, mapF[t.b], mapF[t.b], prm, t.last ? part : nullptr, stream, L.nbuf == 1, launches);
+    if (wide) return split_gram_launch<false, SP_WIDE_BN>(ctx, mapF[t.b], mapW[t.b], prm, t.last ? part : nullptr, stream, nbuf == 1, launches);
+    return split_gram_launch<false, SP_TILE>(ctx, mapF[t.b], mapF[t.b], prm, t.last ? part : nullptr, stream, nbuf == 1, launches);
   };
-  return split_run_steps(ctx, L, P, stream, stat, quant, gram);
+  return split_run_steps(ctx, L, P, nbuf, stream, stat, quant, gram);
 }
 
 // The accumulation with given weights W (ldw, nw).
@@ -1349,14 +1363,14 @@ int split_chi0_real_ediff(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P,
   if (!ws || ws_bytes < base_bytes) return set_error(ctx, SPX_EINVAL, "split workspace too small");
   uint8_t* base = (uint8_t*)align_up((size_t)ws, 1024);
   SplitBuf buf[2];
-  split_buffers(L, base, buf);
+  const int nbuf = split_buffers(L, P, nw, base, buf);
   double* part = ws_bytes >= base_bytes + split_part_bytes(ctx->num_sms, true)
                      ? (double*)(base + align_up(base_bytes, 256))
                      : nullptr;
-  const uint64_t nkb = (uint64_t)(L.Pp / SP_KB);
   const bool wide = ctx->opt.split_variant != 1 && (ctx->opt.split_variant != 0 || split_wide((N + 1) / 2, L.nblk));
   CUtensorMap mapF[2], mapW[2];
-  for (int b = 0; b < L.nbuf; ++b) {
+  for (int b = 0; b < nbuf; ++b) {
+    const uint64_t nkb = (uint64_t)(buf[b].Pp / SP_KB);
     const uint64_t st[3] = {SP_KB, (uint64_t)L.R * SP_KB, nkb * L.R * SP_KB};
     const uint64_t d[4] = {SP_KB, (uint64_t)L.R, nkb, (uint64_t)SP_SLOT * nw};
     const uint32_t bx[4] = {SP_KB, SP_ROWS, 1, SP_SF};
@@ -1384,7 +1398,7 @@ int split_chi0_real_ediff(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P,
     // npad columns (a multiple of 128) x 16-pair chunks, 128 threads a block
     ++*launches;
     return check_cuda(ctx, launch_chained(split_quantize_real_kernel, (unsigned)((int64_t)npad * nchunk / 128), 128, 0, ps,
-                                          L.nbuf == 1, M, ldc, t.p0 + t.off, t.plen, nchunk, N, npad, L.R, L.Pp, nw,
+                                          nbuf == 1, M, ldc, t.p0 + t.off, t.plen, nchunk, N, npad, L.R, buf[t.b].Pp, nw,
                                           buf[t.sb].sA, buf[t.sb].wsgn, buf[t.sb].G + t.off,
                                           (int)align_up((size_t)t.len, SP_KB), buf[t.b].F),
                       "split_quantize_real_kernel launch");
@@ -1404,10 +1418,10 @@ int split_chi0_real_ediff(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P,
     prm.npack = (int64_t)N * (N + 1) / 2;
     prm.status = ctx->d_status;
     prm.timeout_ns = (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
-    if (wide) return split_gram_launch<true, SP_WIDE_BN>(ctx, mapF[t.b], mapW[t.b], prm, t.last ? part : nullptr, stream, L.nbuf == 1, launches);
-    return split_gram_launch<true, SP_TILE>(ctx, mapF[t.b], mapF[t.b], prm, t.last ? part : nullptr, stream, L.nbuf == 1, launches);
+    if (wide) return split_gram_launch<true, SP_WIDE_BN>(ctx, mapF[t.b], mapW[t.b], prm, t.last ? part : nullptr, stream, nbuf == 1, launches);
+    return split_gram_launch<true, SP_TILE>(ctx, mapF[t.b], mapF[t.b], prm, t.last ? part : nullptr, stream, nbuf == 1, launches);
   };
-  return split_run_steps(ctx, L, P, stream, stat, quant, gram);
+  return split_run_steps(ctx, L, P, nbuf, stream, stat, quant, gram);
 }
 
 }  // namespace spx
