@@ -747,13 +747,13 @@ __global__ void __launch_bounds__(SPS_THREADS) __cluster_dims__(SPS_CL, 1, 1)
 // planes are written where the accumulation's last round leaves SMs idle, and after it.
 // Side by side on every SM (8 frequencies at a time) both got slower: real form, 900
 // columns, 8192 pairs, 712 us for both against 420 + 139 us one after the other. The kernel is bound by the HBM
-// writes of the planes; 96 registers keep five blocks per SM.
+// writes of the planes; 96 registers keep five blocks per SM. sA, wsgn and G are still being
+// written when the first blocks start (spx_chain.cuh): ordinary loads after the wait.
 constexpr int SPQ_FCH = 24;
 __global__ void __maxnreg__(96)
     split_quantize_kernel(const double2* __restrict__ M, int64_t ldc, int64_t p0, int len,
                           int nchunk, int N, int npad, int64_t R, int64_t Ps, int nw,
-                          const double* __restrict__ sA, const int* __restrict__ wsgn,
-                          const double* __restrict__ G, int ldg, int8_t* __restrict__ F) {
+                          const double* sA, const int* wsgn, const double* G, int ldg, int8_t* __restrict__ F) {
   __shared__ __align__(16) double gs[SPQ_FCH][SP_KB];
   __shared__ int ss[SPQ_FCH];
   // thread -> (k-block, column group of 4, eighth of the k-block, column in group); the
@@ -794,7 +794,7 @@ __global__ void __maxnreg__(96)
       const int f = e / (SP_KB / 2), c = e - f * (SP_KB / 2);
       const int ce = c >> 2, cj = c & 3;
       reinterpret_cast<double2*>(&gs[f][0])[4 * ce + (cj ^ ((ce >> 1) & 3))] =
-          __ldg(reinterpret_cast<const double2*>(G + (int64_t)(f0 + f) * ldg + kb * SP_KB) + c);
+          reinterpret_cast<const double2*>(G + (int64_t)(f0 + f) * ldg + kb * SP_KB)[c];
     }
     for (int f = threadIdx.x; f < nf; f += blockDim.x) ss[f] = wsgn[f0 + f];
     __syncthreads();
@@ -859,8 +859,7 @@ __global__ void __maxnreg__(96)
 __global__ void __launch_bounds__(128, 5)
     split_quantize_real_kernel(const double* __restrict__ M, int64_t ldc, int64_t p0, int len,
                                int nchunk, int N, int npad, int64_t R, int64_t Ps, int nw,
-                               const double* __restrict__ sA, const int* __restrict__ wsgn,
-                               const double* __restrict__ G, int ldg, int8_t* __restrict__ F) {
+                               const double* sA, const int* wsgn, const double* G, int ldg, int8_t* __restrict__ F) {
   __shared__ __align__(16) double gs[SPQ_FCH][SP_KB];
   __shared__ int ss[SPQ_FCH];
   const int ngroup = npad / 8;   // a multiple of 16, so a block's 4 warps share the k-block
@@ -885,7 +884,7 @@ __global__ void __launch_bounds__(128, 5)
     for (int e = threadIdx.x; e < nf * (SP_KB / 2); e += blockDim.x) {
       const int f = e / (SP_KB / 2), c = e - f * (SP_KB / 2), q = c >> 3, j = c & 7;
       reinterpret_cast<double2*>(&gs[f][0])[8 * q + (j ^ (2 * q))] =
-          __ldg(reinterpret_cast<const double2*>(G + (int64_t)(f0 + f) * ldg + kb * SP_KB) + c);
+          reinterpret_cast<const double2*>(G + (int64_t)(f0 + f) * ldg + kb * SP_KB)[c];
     }
     for (int f = threadIdx.x; f < nf; f += blockDim.x) ss[f] = wsgn[f0 + f];
     __syncthreads();
