@@ -1474,6 +1474,7 @@ struct __align__(1024) SgSmem {
 // T = ((D0*256 + D1)*256 + D2)*256 + D3 for 16 columns, orders 128 columns apart.
 __device__ __forceinline__ void load_orders16(uint32_t taddr, long long (&T)[16]) {
   int32_t r[4][16];
+  __syncwarp();   // the read is warp-wide; lanes of rows past the end skip the stores before it
 #pragma unroll
   for (int g = 0; g < 4; ++g) tmem_ld16(taddr + (uint32_t)(g * SP_ROWS), r[g]);
   tmem_wait_ld();

@@ -265,6 +265,7 @@ __device__ __forceinline__ int split_k_order(int j, int ks, int nk) {
 // order g at TMEM columns [ostride g, ostride g + 16).
 __device__ __forceinline__ void load_fold16(uint32_t taddr, uint32_t ostride, double (&T)[16]) {
   int32_t r0[16], r1[16], r2[16];
+  __syncwarp();   // the read is warp-wide; lanes outside the matrix skip the stores before it
   tmem_ld16(taddr, r0);
   tmem_ld16(taddr + ostride, r1);
   tmem_ld16(taddr + 2 * ostride, r2);
