@@ -34,13 +34,13 @@ int launch_gen_normal(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, double, do
 int launch_gen_cmatrix(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, int64_t, int64_t,
                        double, double*, cudaStream_t);
 int launch_chi0_fp64(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
-                     int, double2*, void* part, size_t part_bytes, cudaStream_t, int*);
-size_t fp64_part_bytes(const spx_ctx*, int64_t P, int N, int nw);
+                     int, double2*, cudaStream_t, int*);
+size_t fp64_part_bytes(int num_sms);
 int split_chi0_slab(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
-                    int, double2*, void*, size_t, cudaStream_t, int*, int variant, int slab);
+                    int, double2*, void*, size_t, void* part, cudaStream_t, int*, int variant, int slab);
 int split_chi0_ediff(spx_ctx*, const double2*, int64_t, int64_t, int, const double* ediff,
                      const double* wscale, double scale_all, int nw, const double* omega, double2*,
-                     void*, size_t, cudaStream_t, int*, int variant, int slab);
+                     void*, size_t, void* part, cudaStream_t, int*, int variant, int slab);
 size_t split_part_bytes(int num_sms, bool real);
 size_t split_workspace_bytes(int64_t P, int N, int nw);
 size_t split_workspace_bytes(int64_t P, int N, int nw, int slab);
@@ -89,8 +89,7 @@ int split_chi0_real_ediff(spx_ctx*, const double*, int64_t, int64_t, int, const 
                           const double* wscale, double scale_all, int nw, const double* omega, double*,
                           void*, size_t, cudaStream_t, int*);
 int launch_chi0_fp64_real(spx_ctx*, const double*, int64_t, int64_t, int, const double*, int64_t,
-                          int, double*, void* part, size_t part_bytes, cudaStream_t, int*);
-size_t fp64_real_part_bytes(const spx_ctx*, int64_t P, int N, int nw);
+                          int, double*, cudaStream_t, int*);
 
 void timing_mark(spx_ctx* ctx, cudaStream_t s, int kind) {
   if (!ctx->timing) return;
@@ -142,8 +141,21 @@ int ensure_workspace(spx_ctx* ctx, size_t bytes) {
     ctx->ws = nullptr;
     ctx->ws_bytes = 0;
   }
+  // the partial tiles give way to a workspace that has no room beside them
+  auto drop_part = [ctx] {
+    cudaFree(ctx->part);
+    ctx->part = nullptr;
+    ctx->part_bytes = 0;
+  };
+  if (ctx->part && ctx->opt.workspace_limit > 0 && bytes + ctx->part_bytes > (size_t)ctx->opt.workspace_limit)
+    drop_part();
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx->part) {
+    cudaGetLastError();
+    drop_part();
+    e = cudaMalloc(&p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(ctx, SPX_ENOMEM,
@@ -153,15 +165,6 @@ int ensure_workspace(spx_ctx* ctx, size_t bytes) {
   ctx->ws = p;
   ctx->ws_bytes = bytes;
   return SPX_OK;
-}
-
-int ensure_workspace_opt(spx_ctx* ctx, size_t bytes, size_t* extra) {
-  int rc = ensure_workspace(ctx, bytes + *extra);
-  if (rc == SPX_ENOMEM && *extra > 0) {
-    *extra = 0;
-    rc = ensure_workspace(ctx, bytes);
-  }
-  return rc;
 }
 
 int ensure_pinned(spx_ctx* ctx, size_t bytes) {
@@ -229,14 +232,9 @@ static int check_chi0_args(spx_ctx* ctx, const double* cprod, int64_t ldc, int64
   return SPX_OK;
 }
 
-// Optional scratch of an accumulation: the partial tiles of a cut last round.
-static size_t part_bytes_for(const spx_ctx* ctx, int64_t P, int N, int nw, int precision) {
-  return precision == SPX_FP64 ? fp64_part_bytes(ctx, P, N, nw) : split_part_bytes(ctx->num_sms, false);
-}
-
 // Accumulates one slab of band pairs already on the device into the device
 // output. `W` is workspace for the FP64 path's npair*nw weights (ldw = round_up(npair, 16));
-// `split_ws` the split path's scratch, or the FP64 path's partial tiles (optional).
+// `split_ws` the split path's scratch.
 // `plan` (variant, slab, tile), when given, replaces the per-call choice: a caller
 // that streams one array in chunks keeps one kernel and one slab size for all of it.
 static int chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N,
@@ -251,7 +249,7 @@ static int chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
     if ((rc = launch_weights(ctx, P, ldw, ediff, wscale, scale_all, nw, omega, W, s))) return rc;
     ++*launches;
     timing_mark(ctx, s, 1);
-    rc = launch_chi0_fp64(ctx, M, ldc, P, N, W, ldw, nw, out, split_ws, split_ws_bytes, s, launches);
+    rc = launch_chi0_fp64(ctx, M, ldc, P, N, W, ldw, nw, out, s, launches);
   } else {
     // kernel variant and slab from the context's tuning table when the caller left
     // the variant open and the table has this shape (smaller slabs need less scratch)
@@ -267,7 +265,7 @@ static int chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
       // the split path forms its weights beside its column scales and marks its own
       // preparation / accumulation phases
       rc = split_chi0_ediff(ctx, M, ldc, P, N, ediff, wscale, scale_all, nw, omega, out, split_ws,
-                            split_ws_bytes, s, launches, variant, slab);
+                            split_ws_bytes, ctx->part, s, launches, variant, slab);
     }
   }
   timing_mark(ctx, s, 2);
@@ -337,6 +335,14 @@ extern "C" int spx_ctx_create(int device, const spx_options* opt, spx_ctx** out)
     spx_ctx_destroy(ctx);
     return rc;
   }
+  ctx->part_bytes = std::max({fp64_part_bytes(ctx->num_sms), split_part_bytes(ctx->num_sms, false),
+                              split_part_bytes(ctx->num_sms, true)});
+  if ((ctx->opt.workspace_limit > 0 && ctx->part_bytes > (size_t)ctx->opt.workspace_limit) ||
+      cudaMalloc(&ctx->part, ctx->part_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->part = nullptr;
+    ctx->part_bytes = 0;
+  }
   for (auto& ev : ctx->ev) cudaEventCreate(&ev);
   for (auto& ev : ctx->sev) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   *out = ctx;
@@ -365,6 +371,7 @@ extern "C" int spx_ctx_destroy(spx_ctx* ctx) {
     if (g.mem) cudaFree(g.mem);
   }
   if (ctx->ws) cudaFree(ctx->ws);
+  if (ctx->part) cudaFree(ctx->part);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->d_prof) cudaFree(ctx->d_prof);
@@ -447,11 +454,9 @@ extern "C" int spx_chi0_accumulate_dev(spx_ctx* ctx, const double* cprod, int64_
   if (npair == 0 || nbas == 0 || nw == 0) return SPX_OK;
   cudaStream_t s = pick_stream(ctx, stream);
   const int64_t ldw = (int64_t)align_up((size_t)npair, 16);
-  size_t wbytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)ldw * nw, 256) : 0;
-  size_t sbytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
-  size_t part = part_bytes_for(ctx, npair, nbas, nw, precision);
-  if ((rc = ensure_workspace_opt(ctx, wbytes + sbytes, &part))) return rc;
-  sbytes += part;
+  const size_t wbytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)ldw * nw, 256) : 0;
+  const size_t sbytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
+  if ((rc = ensure_workspace(ctx, wbytes + sbytes))) return rc;
   double* W = (double*)ctx->ws;
   void* sws = sbytes ? (char*)ctx->ws + wbytes : nullptr;
   int launches = 0;
@@ -493,15 +498,13 @@ extern "C" int spx_chi0_accumulate_real_dev(spx_ctx* ctx, const double* cprod, i
   cudaStream_t s = pick_stream(ctx, stream);
   const int64_t ldw = (int64_t)align_up((size_t)npair, 16);
   const size_t wbytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)ldw * nw, 256) : 0;
-  size_t sbytes = precision == SPX_SPLIT ? split_workspace_bytes_real(npair, nbas, nw) : 0;
+  const size_t sbytes = precision == SPX_SPLIT ? split_workspace_bytes_real(npair, nbas, nw) : 0;
   // the FP64 kernel streams M with 2-D tensor copies: columns must start on 16 bytes,
   // otherwise M goes through an aligned copy first
   const bool realign = precision == SPX_FP64 && ((ldc & 1) || ((uintptr_t)cprod & 15));
   const int64_t ldm = realign ? (int64_t)align_up((size_t)npair, 2) : ldc;
   const size_t mbytes = realign ? align_up(sizeof(double) * (size_t)ldm * nbas, 256) : 0;
-  size_t part = precision == SPX_SPLIT ? split_part_bytes(ctx->num_sms, true)
-                                       : fp64_real_part_bytes(ctx, npair, nbas, nw);
-  if ((rc = ensure_workspace_opt(ctx, wbytes + sbytes + mbytes, &part))) return rc;
+  if ((rc = ensure_workspace(ctx, wbytes + sbytes + mbytes))) return rc;
   double* W = (double*)ctx->ws;
   void* sws = (char*)ctx->ws + wbytes;
   const double* M = cprod;
@@ -522,12 +525,11 @@ extern "C" int spx_chi0_accumulate_real_dev(spx_ctx* ctx, const double* cprod, i
     ++launches;
     if (!rc) {
       timing_mark(ctx, s, 1);
-      rc = launch_chi0_fp64_real(ctx, M, ldm, npair, nbas, W, ldw, nw, susceph,
-                                 part ? (char*)ctx->ws + wbytes + mbytes : nullptr, part, s, &launches);
+      rc = launch_chi0_fp64_real(ctx, M, ldm, npair, nbas, W, ldw, nw, susceph, s, &launches);
     }
   } else {
     rc = split_chi0_real_ediff(ctx, M, ldm, npair, nbas, ediff, wscale, scale_all, nw, omega, susceph, sws,
-                               sbytes + part, s, &launches);
+                               sbytes, s, &launches);
   }
   timing_mark(ctx, s, 2);
   ctx->timing = false;
@@ -697,11 +699,9 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
   const size_t e_bytes = align_up(sizeof(double) * (size_t)slab, 256);
   const size_t om_bytes = align_up(sizeof(double) * (size_t)nw, 256);
   const size_t w_bytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)slab * nw, 256) : 0;
-  size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, slab, nbas, nw) : 0;
-  size_t total = out_bytes + nslab_buf * (slab_bytes + 2 * e_bytes) + om_bytes + w_bytes + s_bytes;
-  size_t part = part_bytes_for(ctx, slab, nbas, nw, precision);
-  if ((rc = ensure_workspace_opt(ctx, total, &part))) return rc;
-  s_bytes += part;
+  const size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, slab, nbas, nw) : 0;
+  const size_t total = out_bytes + nslab_buf * (slab_bytes + 2 * e_bytes) + om_bytes + w_bytes + s_bytes;
+  if ((rc = ensure_workspace(ctx, total))) return rc;
   char* base = (char*)ctx->ws;
   double2* d_out = (double2*)base;
   base += out_bytes;
@@ -883,14 +883,9 @@ extern "C" int spx_chi0_from_coeffs_dev(spx_ctx* ctx, const spx_mt_desc* mt,
                                      wfprod_pw_workspace(pw, nk, nocc, nunocc, split_products));
   const int64_t ldw = ldc;
   const size_t w_bytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)ldw * nw, 256) : 0;
-  size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
-  size_t scratch = std::max(prod_bytes, w_bytes + s_bytes);
-  // partial tiles follow the accumulation's scratch, in what the products leave free or beyond
-  const size_t part = part_bytes_for(ctx, npair, nbas, nw, precision), acc = w_bytes + s_bytes + part;
-  size_t beyond = acc > scratch ? acc - scratch : 0;
-  if ((rc = ensure_workspace_opt(ctx, m_bytes + scratch, &beyond))) return rc;
-  scratch += beyond;
-  if (acc <= scratch) s_bytes += part;
+  const size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;
+  const size_t scratch = std::max(prod_bytes, w_bytes + s_bytes);
+  if ((rc = ensure_workspace(ctx, m_bytes + scratch))) return rc;
   double2* M = (double2*)ctx->ws;
   char* sc = (char*)ctx->ws + m_bytes;
   int launches = 0;
@@ -946,7 +941,6 @@ extern "C" int spx_weights_hilbert_dev(spx_ctx* ctx, int64_t npair, int32_t nfrq
 // Adds sum_p M(p,i) conj(M(p,j)) w(p,f) with caller weights (any sign) into the
 // packed `out`, using `scratch` (accumulate_w_scratch bytes) for the padded weight
 // copy and the split path's planes.
-// A caller may pass `part_bytes` of scratch beyond that for partial tiles.
 static size_t accumulate_w_scratch(int64_t npair, int nbas, int nw, int precision) {
   const int64_t ldi = (int64_t)align_up((size_t)npair, 16);
   return align_up(sizeof(double) * (size_t)ldi * nw, 256) +
@@ -955,8 +949,7 @@ static size_t accumulate_w_scratch(int64_t npair, int nbas, int nw, int precisio
 
 static int accumulate_w_into(spx_ctx* ctx, const double* cprod, int64_t ldc, int64_t npair,
                              int nbas, const double* w, int64_t ldw, int nw, int precision,
-                             double* out, char* scratch, size_t part_bytes, cudaStream_t s,
-                             int* launches) {
+                             double* out, char* scratch, cudaStream_t s, int* launches) {
   // the kernels read the weights with 16-pair bulk copies: an aligned, padded copy
   const int64_t ldi = (int64_t)align_up((size_t)npair, 16);
   const size_t wbytes = align_up(sizeof(double) * (size_t)ldi * nw, 256);
@@ -972,11 +965,10 @@ static int accumulate_w_into(spx_ctx* ctx, const double* cprod, int64_t ldc, int
   if (precision == SPX_FP64) {
     timing_mark(ctx, s, 1);
     return launch_chi0_fp64(ctx, reinterpret_cast<const double2*>(cprod), ldc, npair, nbas, W, ldi, nw,
-                            reinterpret_cast<double2*>(out), part_bytes ? sws : nullptr, part_bytes, s,
-                            launches);
+                            reinterpret_cast<double2*>(out), s, launches);
   }
   return split_chi0_slab(ctx, reinterpret_cast<const double2*>(cprod), ldc, npair, nbas, W, ldi, nw,
-                         reinterpret_cast<double2*>(out), sws, sbytes + part_bytes, s, launches, 0, 0);
+                         reinterpret_cast<double2*>(out), sws, sbytes, ctx->part, s, launches, 0, 0);
 }
 
 extern "C" int spx_chi0_accumulate_w_dev(spx_ctx* ctx, const double* cprod, int64_t ldc,
@@ -996,13 +988,12 @@ extern "C" int spx_chi0_accumulate_w_dev(spx_ctx* ctx, const double* cprod, int6
   }
   if (npair == 0 || nbas == 0 || nw == 0) return SPX_OK;
   cudaStream_t s = pick_stream(ctx, stream);
-  size_t part = part_bytes_for(ctx, npair, nbas, nw, precision);
-  if ((rc = ensure_workspace_opt(ctx, accumulate_w_scratch(npair, nbas, nw, precision), &part))) return rc;
+  if ((rc = ensure_workspace(ctx, accumulate_w_scratch(npair, nbas, nw, precision)))) return rc;
   int launches = 0;
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
   rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, w, ldw, nw, precision, susceph,
-                         (char*)ctx->ws, part, s, &launches);
+                         (char*)ctx->ws, s, &launches);
   timing_mark(ctx, s, 2);
   ctx->timing = false;
   if (rc) return rc;
@@ -1044,8 +1035,7 @@ extern "C" int spx_chi0_accumulate_c_dev(spx_ctx* ctx, const double* cprod, int6
   const int64_t npack = (int64_t)nbas * (nbas + 1) / 2;
   const size_t pbytes = align_up(sizeof(double2) * (size_t)npack * nw, 256);
   const size_t sc = accumulate_w_scratch(npair, nbas, nw, precision);
-  size_t part = part_bytes_for(ctx, npair, nbas, nw, precision);
-  if ((rc = ensure_workspace_opt(ctx, 2 * pbytes + sc, &part))) return rc;
+  if ((rc = ensure_workspace(ctx, 2 * pbytes + sc))) return rc;
   double* S1 = (double*)ctx->ws;
   double* S2 = (double*)((char*)ctx->ws + pbytes);
   char* scratch = (char*)ctx->ws + 2 * pbytes;
@@ -1053,11 +1043,9 @@ extern "C" int spx_chi0_accumulate_c_dev(spx_ctx* ctx, const double* cprod, int6
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
   if ((rc = check_cuda(ctx, cudaMemsetAsync(S1, 0, 2 * pbytes, s), "zero partial sums"))) return rc;
-  rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, wr, ldw, nw, precision, S1, scratch, part, s,
-                         &launches);
+  rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, wr, ldw, nw, precision, S1, scratch, s, &launches);
   if (!rc)
-    rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, wi, ldw, nw, precision, S2, scratch, part, s,
-                           &launches);
+    rc = accumulate_w_into(ctx, cprod, ldc, npair, nbas, wi, ldw, nw, precision, S2, scratch, s, &launches);
   if (!rc) {
     timing_mark(ctx, s, 0);
     rc = launch_suscepc_combine(ctx, nbas, nw, (const double2*)S1, (const double2*)S2,

@@ -34,15 +34,13 @@ namespace spx {
 int launch_weights(spx_ctx*, int64_t, int64_t, const double*, const double*, double, int,
                    const double*, double*, cudaStream_t);
 int launch_chi0_fp64(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
-                     int, double2*, void* part, size_t part_bytes, cudaStream_t, int*);
-size_t fp64_part_bytes(const spx_ctx*, int64_t P, int N, int nw);
+                     int, double2*, cudaStream_t, int*);
 int split_chi0_slab(spx_ctx*, const double2*, int64_t, int64_t, int, const double*, int64_t,
-                    int, double2*, void*, size_t, cudaStream_t, int*, int, int);
+                    int, double2*, void*, size_t, void* part, cudaStream_t, int*, int, int);
 int split_chi0_ediff(spx_ctx*, const double2*, int64_t, int64_t, int, const double* ediff,
                      const double* wscale, double scale_all, int nw, const double* omega, double2*, void*,
-                     size_t, cudaStream_t, int*, int variant, int slab);
+                     size_t, void* part, cudaStream_t, int*, int variant, int slab);
 size_t split_workspace_bytes(int64_t P, int N, int nw, int slab);
-size_t split_part_bytes(int num_sms, bool real);
 int launch_gen_cmatrix_rows(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, int64_t, int64_t,
                             int64_t, double, double2*, cudaStream_t);
 int launch_gen_normal(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, double, double*,
@@ -127,10 +125,10 @@ static uint64_t fnv(uint64_t h, const void* p, size_t n) {
   return h;
 }
 
-// Enqueues the whole schedule on `s`; `part` is scratch for the FP64 path's partial tiles.
+// Enqueues the whole schedule on `s`.
 static int enqueue_batch(spx_ctx* ctx, int nq, const spx_q_desc* q, const QPlan* pl, int nw,
-                         const double* omega, int precision, char* ws, void* part,
-                         size_t part_bytes, cudaStream_t s, int* launches) {
+                         const double* omega, int precision, char* ws, cudaStream_t s,
+                         int* launches) {
   for (int i = 0; i < nq; ++i) {
     const spx_q_desc& d = q[i];
     const QPlan& p = pl[i];
@@ -161,12 +159,11 @@ static int enqueue_batch(spx_ctx* ctx, int nq, const spx_q_desc* q, const QPlan*
       ++*launches;
       if (precision == SPX_SPLIT) {
         rc = split_chi0_slab(ctx, M, ldc, len, d.nbas, W, ldw, nw,
-                             reinterpret_cast<double2*>(d.susceph), sws, p.s_bytes, s, launches,
+                             reinterpret_cast<double2*>(d.susceph), sws, p.s_bytes, nullptr, s, launches,
                              p.variant, p.slab);
       } else {
         rc = launch_chi0_fp64(ctx, M, ldc, len, d.nbas, W, ldw, nw,
-                              reinterpret_cast<double2*>(d.susceph), part_bytes ? part : nullptr,
-                              part_bytes, s, launches);
+                              reinterpret_cast<double2*>(d.susceph), s, launches);
       }
       if (rc) return rc;
     }
@@ -202,20 +199,20 @@ static bool batch_by_q(const spx_ctx* ctx, int nq, const spx_q_desc* q, int nw) 
 // workspace limit is too small for the largest q.
 static int run_by_q(spx_ctx* ctx, int nq, const spx_q_desc* q, int nw, const double* omega, cudaStream_t s,
                     int* launches) {
-  size_t need = 0, part = split_part_bytes(ctx->num_sms, false);
+  size_t need = 0;
   for (int i = 0; i < nq; ++i)
     if (q[i].npair > 0 && q[i].nbas > 0)
       need = std::max(need, split_workspace_bytes(q[i].npair, q[i].nbas, nw, pb_slab_of(ctx, q[i], nw, 0)));
   if (need == 0) return SPX_OK;
   if (ctx->opt.workspace_limit > 0 && need > (size_t)ctx->opt.workspace_limit) return SPX_ENOTSUP;
-  int rc = ensure_workspace_opt(ctx, need, &part);
+  int rc = ensure_workspace(ctx, need);
   const bool timing = ctx->timing;
   ctx->timing = false;
   for (int i = 0; i < nq && !rc; ++i)
     if (q[i].npair > 0 && q[i].nbas > 0)
       rc = split_chi0_ediff(ctx, reinterpret_cast<const double2*>(q[i].cprod), q[i].ldc, q[i].npair, q[i].nbas,
                             q[i].ediff, q[i].wscale, q[i].scale_all, nw, omega,
-                            reinterpret_cast<double2*>(q[i].susceph), ctx->ws, need + part, s, launches, 0,
+                            reinterpret_cast<double2*>(q[i].susceph), ctx->ws, need, ctx->part, s, launches, 0,
                             pb_slab_of(ctx, q[i], nw, 0));
   ctx->timing = timing;
   return rc;
@@ -298,11 +295,7 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
     pl[i] = plan_q(ctx, q[i], nw, precision);
     need = std::max(need, pl[i].w_bytes + pl[i].g_bytes + pl[i].s_bytes);
   }
-  need = align_up(need + 1024, 256);
-  size_t part = 0;
-  if (precision == SPX_FP64)
-    for (int i = 0; i < nq; ++i) part = std::max(part, fp64_part_bytes(ctx, q[i].npair, q[i].nbas, nw));
-  if ((rc = ensure_workspace_opt(ctx, need, &part))) return rc;
+  if ((rc = ensure_workspace(ctx, need + 1024))) return rc;
   cudaStream_t s = pick_stream(ctx, stream);
   int launches = 0;
   cudaEvent_t e0 = ctx->ev[8], e1 = ctx->ev[9];
@@ -310,8 +303,7 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
   const bool timing = ctx->timing;
   ctx->timing = false;
   if (flags & SPX_BATCH_NOGRAPH) {
-    rc = enqueue_batch(ctx, nq, q, pl.data(), nw, omega, precision, (char*)ctx->ws, (char*)ctx->ws + need,
-                       part, s, &launches);
+    rc = enqueue_batch(ctx, nq, q, pl.data(), nw, omega, precision, (char*)ctx->ws, s, &launches);
   } else {
     uint64_t key = 1469598103934665603ull;
     key = fnv(key, &nq, sizeof(nq));
@@ -321,7 +313,7 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
     key = fnv(key, &precision, sizeof(precision));
     key = fnv(key, &ctx->ws, sizeof(ctx->ws));
     key = fnv(key, &ctx->ws_bytes, sizeof(ctx->ws_bytes));
-    key = fnv(key, &part, sizeof(part));
+    key = fnv(key, &ctx->part, sizeof(ctx->part));
     for (const QPlan& p : pl) key = fnv(key, &p, sizeof(p));
     spx_ctx::BatchGraph* hit = nullptr;
     for (auto& g : ctx->graphs)
@@ -337,8 +329,8 @@ extern "C" int spx_chi0_batched(spx_ctx* ctx, int32_t nq, const spx_q_desc* q, i
         return rc;
       }
       int cap_launches = 0;
-      rc = enqueue_batch(ctx, nq, q, pl.data(), nw, omega, precision, (char*)ctx->ws,
-                         (char*)ctx->ws + need, part, cs, &cap_launches);
+      rc = enqueue_batch(ctx, nq, q, pl.data(), nw, omega, precision, (char*)ctx->ws, cs,
+                         &cap_launches);
       cudaError_t ee = cudaStreamEndCapture(cs, &graph);
       if (!rc) rc = check_cuda(ctx, ee, "end capture");
       if (!rc) rc = check_cuda(ctx, cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
@@ -475,7 +467,8 @@ extern "C" int spx_autotune_split(spx_ctx* ctx, int32_t nbas, int64_t npair, int
           rc = pb_single(ctx, M, ld, P, nbas, E, nullptr, 1.0, nw, OM, O, kPbDefaultTile, c.slab, (char*)S,
                          sws, s, &launches);
         else
-          rc = split_chi0_slab(ctx, M, ld, P, nbas, W, ld, nw, O, S, sws, s, &launches, c.variant, c.slab);
+          rc = split_chi0_slab(ctx, M, ld, P, nbas, W, ld, nw, O, S, sws, ctx->part, s, &launches,
+                               c.variant, c.slab);
       }
       if (rc) return rc;
       cudaEventRecord(e1, s);

@@ -28,6 +28,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "spx_common.cuh"
 #include "spx_tcgen05.cuh"
 
@@ -869,23 +871,22 @@ static int f64_run(const F64Call& q, int* launches) {
   return e;
 }
 
-// Scratch for the partial tiles of a call (0 when none are used); optional: without it
-// the tiles of the last round are not cut.
-size_t fp64_part_bytes(const spx_ctx* ctx, int64_t P, int N, int nw) {
-  if (P < F64P_MINPAIR || N <= 0 || nw <= 0) return 0;
-  return f64p_part_bytes<F64P_CPLX>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
+// Bytes that hold the partial tiles of any call.
+size_t fp64_part_bytes(int num_sms) {
+  return std::max({f64p_part_bytes<F64P_CPLX>(num_sms, 3), f64p_part_bytes<F64P_HW>(num_sms, 3),
+                   f64p_part_bytes<F64P_REAL>(num_sms, 3)});
 }
 
 // Enqueues the FP64 accumulation over one slab of band pairs. W holds the weights of
 // exactly these pairs (leading dimension ldw, a multiple of 16, padding zeroed, 16-byte
-// aligned); `part` is fp64_part_bytes of scratch or NULL.
+// aligned).
 int launch_chi0_fp64(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N,
-                     const double* W, int64_t ldw, int nw, double2* out, void* part,
-                     size_t part_bytes, cudaStream_t stream, int* launches) {
+                     const double* W, int64_t ldw, int nw, double2* out, cudaStream_t stream,
+                     int* launches) {
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
   const uint64_t timeout_ns =
       (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
-  const F64Call q{ctx->num_sms, M, ldc, P, N, W, ldw, nw, out, (double2*)part, part_bytes,
+  const F64Call q{ctx->num_sms, M, ldc, P, N, W, ldw, nw, out, (double2*)ctx->part, ctx->part_bytes,
                   ctx->d_status, timeout_ns, stream};
   const int e = f64_run(q, launches);
   if (e) return set_error(ctx, SPX_ECUDA, "chi0_fp64 kernels: tensor map or attribute failed (" +
@@ -893,23 +894,16 @@ int launch_chi0_fp64(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
   return check_cuda(ctx, cudaGetLastError(), "chi0_fp64 kernel launch");
 }
 
-// Scratch for launch_headwings' partial tiles (0 when none are used), optional.
-size_t headwings_part_bytes(const spx_ctx* ctx, int64_t P, int nw) {
-  if (P < F64P_MINPAIR || nw <= 0) return 0;
-  return f64p_part_bytes<F64P_HW>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
-}
-
 // head(:, f) += sum_p dc(p, k1) conj(dc(p, k2)) w(p, f), wing(k2, i, f) += sum_p M(p, i)
 // conj(dc(p, k2)) w(p, f): M (ldc, dim), dc (ldd, 3), W (ldw, nw) with ldw even and W 16-byte
 // aligned. P < 2^30.
 int launch_headwings(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int dim,
                      const double2* dc, int64_t ldd, const double* W, int64_t ldw, int nw,
-                     double2* head, double2* wing, void* part, size_t part_bytes,
-                     cudaStream_t stream) {
+                     double2* head, double2* wing, cudaStream_t stream) {
   if (P <= 0 || nw <= 0) return SPX_OK;
   const uint64_t timeout_ns =
       (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
-  const F64Call q{ctx->num_sms, M, ldc, P, dim, W, ldw, nw, wing, (double2*)part, part_bytes,
+  const F64Call q{ctx->num_sms, M, ldc, P, dim, W, ldw, nw, wing, (double2*)ctx->part, ctx->part_bytes,
                   ctx->d_status, timeout_ns, stream};
   const F64Head hw{dc, ldd, head};
   int full = nw / 24, r = nw % 24, e = 0, launches = 0;
@@ -1127,20 +1121,14 @@ static bool f64r_takes_k1r(const F64Call& q, int n, int nt) {
   return k1 <= k1p;
 }
 
-// Scratch for the real accumulation's partial tiles (0 when none are used), optional.
-size_t fp64_real_part_bytes(const spx_ctx* ctx, int64_t P, int N, int nw) {
-  if (P < F64P_MINPAIR || N <= 0 || nw <= 0) return 0;
-  return f64p_part_bytes<F64P_REAL>(ctx->num_sms, nw > 16 ? 3 : (nw > 8 ? 2 : 1));
-}
-
 // Enqueues the FP64 accumulation over one slab of real band-pair products M (ldc, N): ldc
-// even, M 16-byte aligned; W and `part` as launch_chi0_fp64.
+// even, M 16-byte aligned; W as launch_chi0_fp64.
 int launch_chi0_fp64_real(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P, int N,
-                          const double* W, int64_t ldw, int nw, double* out, void* part,
-                          size_t part_bytes, cudaStream_t stream, int* launches) {
+                          const double* W, int64_t ldw, int nw, double* out, cudaStream_t stream,
+                          int* launches) {
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
   const F64Call q{ctx->num_sms, reinterpret_cast<const double2*>(M), ldc, P, N, W, ldw, nw,
-                  reinterpret_cast<double2*>(out), (double2*)part, part_bytes, ctx->d_status,
+                  reinterpret_cast<double2*>(out), (double2*)ctx->part, ctx->part_bytes, ctx->d_status,
                   (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull, stream};
   int e = 0;
   for (int f0 = 0; f0 < nw && !e; f0 += 24) {

@@ -1079,10 +1079,9 @@ size_t split_workspace_bytes(int64_t P, int N, int nw, int slab) {
   slab = clamp_slab(slab);
   return split_layout(P, N, nw, slab).bytes();
 }
-// Scratch for partial tiles beyond split_workspace_bytes, optional.
+// Bytes that hold the partial tiles of any call: two per CTA.
 size_t split_part_bytes(int num_sms, bool real) {
-  // two partial tiles per CTA
-  return align_up(sizeof(double) * 2 * (size_t)num_sms * split_part_elems(real, SP_WIDE_BN), 256) + 1280;
+  return align_up(sizeof(double) * 2 * (size_t)num_sms * split_part_elems(real, SP_WIDE_BN), 256);
 }
 
 size_t split_workspace_bytes(int64_t P, int N, int nw) {
@@ -1204,9 +1203,10 @@ static int split_run_steps(spx_ctx* ctx, const SplitLayout& L, int64_t P, int nb
 }
 
 // variant: 1 one CTA per 64 x 64 tile, 2 CTA pair, 5 one CTA per 64 x 80 tile, 0 the
-// context's choice; slab: pairs per exact int32 slab (0 = 32768).
+// context's choice; slab: pairs per exact int32 slab (0 = 32768); part: split_part_bytes for
+// partial tiles, or NULL.
 static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, const SplitStat& src,
-                          int nw, double2* out, void* ws, size_t ws_bytes, cudaStream_t stream,
+                          int nw, double2* out, void* ws, size_t ws_bytes, double* part, cudaStream_t stream,
                           int* launches, int variant, int slab) {
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
   slab = clamp_slab(slab);
@@ -1223,10 +1223,6 @@ static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P
   if (variant == 0) variant = split_wide(N, L.nblk) ? 5 : 1;  // untuned: one CTA per tile
   const bool pair = variant == 2;
   const bool wide = variant == 5;                  // one CTA per 64 x 80 tile (N = 160)
-  const size_t base_bytes = split_workspace_bytes(P, N, nw, slab);
-  double* part = nullptr;   // partial tiles, where the caller has room for them
-  if (!pair && ws_bytes >= base_bytes + split_part_bytes(ctx->num_sms, false))
-    part = (double*)(base + align_up(base_bytes, 256));
   // only the CTA pair needs an even number of 64-column blocks in the planes (the
   // buffers are sized for it either way)
   if (!pair) L.R = (int64_t)L.nblk * SP_ROWS;
@@ -1326,18 +1322,19 @@ static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P
 
 // The accumulation with given weights W (ldw, nw).
 int split_chi0_slab(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, const double* W,
-                    int64_t ldw, int nw, double2* out, void* ws, size_t ws_bytes,
+                    int64_t ldw, int nw, double2* out, void* ws, size_t ws_bytes, void* part,
                     cudaStream_t stream, int* launches, int variant, int slab) {
   return split_chi0_run(ctx, M, ldc, P, N, SplitStat{W, ldw, nullptr, nullptr, 0.0, nullptr}, nw, out, ws,
-                        ws_bytes, stream, launches, variant, slab);
+                        ws_bytes, (double*)part, stream, launches, variant, slab);
 }
 
 // The accumulation with the HILBERT NONE weights of ediff (the same bits as K6's).
 int split_chi0_ediff(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int N, const double* ediff,
                      const double* wscale, double scale_all, int nw, const double* omega, double2* out,
-                     void* ws, size_t ws_bytes, cudaStream_t stream, int* launches, int variant, int slab) {
+                     void* ws, size_t ws_bytes, void* part, cudaStream_t stream, int* launches, int variant,
+                     int slab) {
   return split_chi0_run(ctx, M, ldc, P, N, SplitStat{nullptr, 0, ediff, wscale, scale_all, omega}, nw, out, ws,
-                        ws_bytes, stream, launches, variant, slab);
+                        ws_bytes, (double*)part, stream, launches, variant, slab);
 }
 
 // Real layout: 128 columns per block, one plane row per column.
@@ -1358,14 +1355,11 @@ int split_chi0_real_ediff(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P,
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
   const SplitStat src{nullptr, 0, ediff, wscale, scale_all, omega};
   const SplitLayout L = split_layout_real(P, N, nw);
-  const size_t base_bytes = L.bytes();
-  if (!ws || ws_bytes < base_bytes) return set_error(ctx, SPX_EINVAL, "split workspace too small");
+  if (!ws || ws_bytes < L.bytes()) return set_error(ctx, SPX_EINVAL, "split workspace too small");
   uint8_t* base = (uint8_t*)align_up((size_t)ws, 1024);
   SplitBuf buf[2];
   const int nbuf = split_buffers(L, P, nw, base, buf);
-  double* part = ws_bytes >= base_bytes + split_part_bytes(ctx->num_sms, true)
-                     ? (double*)(base + align_up(base_bytes, 256))
-                     : nullptr;
+  double* part = (double*)ctx->part;   // partial tiles
   const bool wide = ctx->opt.split_variant != 1 && (ctx->opt.split_variant != 0 || split_wide((N + 1) / 2, L.nblk));
   CUtensorMap mapF[2], mapW[2];
   for (int b = 0; b < nbuf; ++b) {

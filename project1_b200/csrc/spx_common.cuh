@@ -25,6 +25,11 @@ struct spx_ctx {
   // grow-only device workspace, carved per call
   void* ws = nullptr;
   size_t ws_bytes = 0;
+  // partial tiles of accumulations that cut their last items, made with the context and of one
+  // size, so that no call grows the workspace for them; NULL (items stay whole) where memory or
+  // workspace_limit has no room for it
+  void* part = nullptr;
+  size_t part_bytes = 0;
   // pinned host staging for pageable host arrays
   void* pinned = nullptr;
   size_t pinned_bytes = 0;
@@ -66,9 +71,6 @@ int set_error(spx_ctx* ctx, int code, const std::string& msg);
 int check_cuda(spx_ctx* ctx, cudaError_t e, const char* what);
 // Makes sure the workspace holds `bytes`; returns SPX_OK or SPX_ENOMEM.
 int ensure_workspace(spx_ctx* ctx, size_t bytes);
-// The same for `bytes` and, if they can be had (memory, workspace_limit), `*extra` more;
-// else *extra becomes 0.
-int ensure_workspace_opt(spx_ctx* ctx, size_t bytes, size_t* extra);
 int ensure_pinned(spx_ctx* ctx, size_t bytes);
 // Reads and clears the device status word (synchronises `stream`).
 int collect_status(spx_ctx* ctx, cudaStream_t stream, const char* what);

@@ -1090,11 +1090,9 @@ extern "C" int spx_trafo_olap_dev(spx_ctx* ctx, const double* cprod, int64_t ldc
 // not start on 16 bytes, as its tensor copies need.
 
 namespace spx {
-size_t headwings_part_bytes(const spx_ctx* ctx, int64_t P, int nw);
 int launch_headwings(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int dim,
                      const double2* dc, int64_t ldd, const double* W, int64_t ldw, int nw,
-                     double2* head, double2* wing, void* part, size_t part_bytes,
-                     cudaStream_t stream);
+                     double2* head, double2* wing, cudaStream_t stream);
 }  // namespace spx
 
 extern "C" int spx_headwings_dev(spx_ctx* ctx, const double* cprod, int64_t ldc, int64_t npair,
@@ -1116,11 +1114,9 @@ extern "C" int spx_headwings_dev(spx_ctx* ctx, const double* cprod, int64_t ldc,
   const int64_t range = std::min<int64_t>(npair, realign ? (int64_t)1 << 22 : (int64_t)1 << 29);
   const int64_t ldi = (int64_t)align_up((size_t)range, 2);
   const size_t w_bytes = realign ? align_up(sizeof(double) * (size_t)ldi * nw, 256) : 0;
-  size_t part = headwings_part_bytes(ctx, range, nw);
   int rc;
-  if ((rc = ensure_workspace_opt(ctx, w_bytes + 256, &part))) return rc;
+  if ((rc = ensure_workspace(ctx, w_bytes))) return rc;
   double* W = reinterpret_cast<double*>(ctx->ws);
-  void* pt = part ? (char*)ctx->ws + w_bytes : nullptr;
   for (int64_t p0 = 0; p0 < npair; p0 += range) {
     const int64_t len = std::min<int64_t>(range, npair - p0);
     if (realign &&
@@ -1131,7 +1127,7 @@ extern "C" int spx_headwings_dev(spx_ctx* ctx, const double* cprod, int64_t ldc,
     if ((rc = launch_headwings(ctx, reinterpret_cast<const double2*>(cprod) + p0, ldc, len, dim,
                                reinterpret_cast<const double2*>(dcprod) + p0, ldd, realign ? W : w + p0,
                                realign ? ldi : ldw, nw, reinterpret_cast<double2*>(head),
-                               reinterpret_cast<double2*>(wing), pt, part, s)))
+                               reinterpret_cast<double2*>(wing), s)))
       return rc;
   }
   return SPX_OK;
