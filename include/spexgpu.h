@@ -348,15 +348,20 @@ int spx_dielec_dev(spx_ctx* ctx, int32_t nbas, int32_t nw, double* susceph,
 /* ---- many q points in one call (K7) -----------------------------------------
  * The q loop of the reference driver (src/correlation.f:293-339 calls
  * `susceptibility` once per q point) as one call: every q has its own N_MB,
- * band window and output. Each q is accumulated exactly as by
- * spx_chi0_accumulate_dev (same slabs and kernels, so the same bits). Its M is
- * a device array, or is generated on the device slab by slab from the seeded
+ * band window and output. Each q is accumulated as by spx_chi0_accumulate_dev;
+ * split sums with the same slab size are the same bits (whose default is 32768 pairs
+ * there and 16384 here), except that above 148 tiles per frequency (about 1120
+ * functions) the persistent schedule below and the separate kernels differ by the
+ * rounding of a slab's partial FP64 sums. Its M is a device array, or is generated on the device slab by slab from the seeded
  * Philox stream (cprod = NULL), so that no q's M is ever held whole.
  * With SPX_SPLIT, when every M is given, every descriptor leaves variant and slab
  * open and the batch is large (a mean of half a million nbas x npair x nw elements
- * per q), each q runs through the kernels of spx_chi0_accumulate_dev in turn, in
- * the context workspace, with slabs of the tuning table or 16384 pairs and without
- * a graph. Otherwise, and where workspace_limit is too small for that, the whole
+ * per q), each q runs through the kernels of spx_chi0_accumulate_dev in turn, with
+ * slabs of the tuning table or 16384 pairs and without a graph, in scratch that the
+ * context keeps for such batches alone: a batch may run on another stream than other
+ * calls, and batches on several streams follow one another (a graph that captured one
+ * is not ordered with others by the library). Otherwise, and where workspace_limit or
+ * the device's memory has no room for that scratch, the whole
  * batch runs as ONE persistent kernel: every SM takes
  * accumulation items (slab, tile, frequency) and operand-preparation items
  * (generation of M, weights, digit planes) from two device work queues, the q

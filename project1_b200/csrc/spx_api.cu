@@ -345,6 +345,7 @@ extern "C" int spx_ctx_create(int device, const spx_options* opt, spx_ctx** out)
   }
   for (auto& ev : ctx->ev) cudaEventCreate(&ev);
   for (auto& ev : ctx->sev) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  cudaEventCreateWithFlags(&ctx->batch_done, cudaEventDisableTiming);
   *out = ctx;
   return SPX_OK;
 }
@@ -372,6 +373,8 @@ extern "C" int spx_ctx_destroy(spx_ctx* ctx) {
   }
   if (ctx->ws) cudaFree(ctx->ws);
   if (ctx->part) cudaFree(ctx->part);
+  if (ctx->batch_ws) cudaFree(ctx->batch_ws);
+  if (ctx->batch_done) cudaEventDestroy(ctx->batch_done);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->d_prof) cudaFree(ctx->d_prof);

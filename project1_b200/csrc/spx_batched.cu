@@ -41,6 +41,7 @@ int split_chi0_ediff(spx_ctx*, const double2*, int64_t, int64_t, int, const doub
                      const double* wscale, double scale_all, int nw, const double* omega, double2*, void*,
                      size_t, void* part, cudaStream_t, int*, int variant, int slab);
 size_t split_workspace_bytes(int64_t P, int N, int nw, int slab);
+size_t split_part_bytes(int num_sms, bool real);
 int launch_gen_cmatrix_rows(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, int64_t, int64_t,
                             int64_t, double, double2*, cudaStream_t);
 int launch_gen_normal(spx_ctx*, uint64_t, uint32_t, int64_t, int64_t, double, double*,
@@ -195,8 +196,9 @@ static bool batch_by_q(const spx_ctx* ctx, int nq, const spx_q_desc* q, int nw) 
   return elems >= 5e5 * n;
 }
 
-// The batch q by q on `s`, with the slabs of the persistent schedule. SPX_ENOTSUP when the
-// workspace limit is too small for the largest q.
+// The batch q by q on `s`, with the slabs of the persistent schedule, in scratch that no other
+// call uses. SPX_ENOTSUP when the workspace limit or the device's memory is too small for the
+// largest q.
 static int run_by_q(spx_ctx* ctx, int nq, const spx_q_desc* q, int nw, const double* omega, cudaStream_t s,
                     int* launches) {
   size_t need = 0;
@@ -205,16 +207,42 @@ static int run_by_q(spx_ctx* ctx, int nq, const spx_q_desc* q, int nw, const dou
       need = std::max(need, split_workspace_bytes(q[i].npair, q[i].nbas, nw, pb_slab_of(ctx, q[i], nw, 0)));
   if (need == 0) return SPX_OK;
   if (ctx->opt.workspace_limit > 0 && need > (size_t)ctx->opt.workspace_limit) return SPX_ENOTSUP;
-  int rc = ensure_workspace(ctx, need);
+  need = align_up(need, 256);
+  size_t bytes = need + split_part_bytes(ctx->num_sms, false);
+  const bool cut = ctx->opt.workspace_limit <= 0 || bytes <= (size_t)ctx->opt.workspace_limit;
+  if (!cut) bytes = need;
+  // batches of this context follow one another in the scratch, whatever streams they are on; a
+  // captured one is ordered by whoever launches its graph
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  int rc = check_cuda(ctx, cudaStreamIsCapturing(s, &cap), "capture status");
+  if (rc) return rc;
+  const bool order = cap == cudaStreamCaptureStatusNone;
+  if (bytes > ctx->batch_ws_bytes) {
+    if (!order) return SPX_ENOTSUP;   // nothing is allocated during a capture
+    if (ctx->batch_ws) cudaFree(ctx->batch_ws);
+    ctx->batch_ws = nullptr;
+    ctx->batch_ws_bytes = 0;
+    if (cudaMalloc(&ctx->batch_ws, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      ctx->batch_ws = nullptr;
+      return SPX_ENOTSUP;
+    }
+    ctx->batch_ws_bytes = bytes;
+  }
+  if (order) rc = check_cuda(ctx, cudaStreamWaitEvent(s, ctx->batch_done, 0), "batch order");
   const bool timing = ctx->timing;
   ctx->timing = false;
   for (int i = 0; i < nq && !rc; ++i)
     if (q[i].npair > 0 && q[i].nbas > 0)
       rc = split_chi0_ediff(ctx, reinterpret_cast<const double2*>(q[i].cprod), q[i].ldc, q[i].npair, q[i].nbas,
                             q[i].ediff, q[i].wscale, q[i].scale_all, nw, omega,
-                            reinterpret_cast<double2*>(q[i].susceph), ctx->ws, need, ctx->part, s, launches, 0,
-                            pb_slab_of(ctx, q[i], nw, 0));
+                            reinterpret_cast<double2*>(q[i].susceph), ctx->batch_ws, need,
+                            cut ? (char*)ctx->batch_ws + need : nullptr, s, launches, 0, pb_slab_of(ctx, q[i], nw, 0));
   ctx->timing = timing;
+  if (order) {
+    const int er = check_cuda(ctx, cudaEventRecord(ctx->batch_done, s), "batch order");
+    if (!rc) rc = er;
+  }
   return rc;
 }
 

@@ -51,6 +51,11 @@ struct spx_ctx {
     void* mem;  // device memory the graph's persistent schedule owns (or NULL)
   };
   std::vector<BatchGraph> graphs;
+  // scratch of split batches run q by q: their own, as a graph's persistent schedule has, so
+  // that a batch may lie on another stream than other calls; `batch_done` orders batches
+  void* batch_ws = nullptr;
+  size_t batch_ws_bytes = 0;
+  cudaEvent_t batch_done = nullptr;
   uint64_t graph_clock = 0;
   void* dn = nullptr;  // dense-solver handle of the dielectric inversion, made on first use
   // role profile of the persistent schedule (spx_pb_profile_*)
