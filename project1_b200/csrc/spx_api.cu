@@ -15,7 +15,9 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <condition_variable>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -551,85 +553,93 @@ extern "C" int spx_chi0_accumulate_real_dev(spx_ctx* ctx, const double* cprod, i
 // The host threads of one host-pointer call: they gather the chunks of a pageable cprod into
 // pinned staging while earlier chunks are copied and accumulated, touch the output's pages
 // meanwhile, and add the sums at the end. One set per call (a thread costs about as much to
-// start as a megabyte to copy, so not one per chunk).
+// start as a megabyte to copy, so not one per chunk); between jobs they sleep.
 struct HostCrew {
-  struct Chunk {
-    int64_t p0, len;
+  enum Job { GATHER, TOUCH, ADD, QUIT };
+  struct Task {
+    Job job;
+    const double* src;   // GATHER: columns ldc apart, `len` pairs of `nbas` columns to dst (len, nbas)
+    double* dst;         // (TOUCH: its pages; ADD: += src)
+    int64_t ldc, len;    // TOUCH, ADD: `len` doubles
+    int nbas;
   };
-  const double* cprod = nullptr;   // NULL: nothing to gather
-  int64_t ldc = 0;
-  int nbas = 0;
-  std::vector<Chunk> chunks;
-  double* stage[3] = {};           // chunk k goes to stage[k % 3] as (len, nbas)
-  double* out = nullptr;           // susceph, `n` doubles in `pieces` parts
-  const double* sums = nullptr;
-  int64_t n = 0;
-  int pieces = 1;
-
-  std::atomic<int64_t> gather_to{-1};   // chunks up to this one may be gathered
-  std::atomic<int64_t> gathered{0};     // finished shares of chunks
-  std::atomic<int> touched{0}, add_to{-1}, added{0};
-  std::atomic<bool> stop{false};
-  std::atomic<int> size{0};             // threads and the caller; 0 until all have started
-  std::vector<std::thread> threads;
 
   ~HostCrew() {
-    stop = true;
+    if (running.load() > 0) finish();
+    post(Task{QUIT, nullptr, nullptr, 0, 0, 0});
     for (auto& t : threads) t.join();
   }
   void start(int want) {
     try {
+      threads.reserve((size_t)want);
       for (int t = 1; t < want; ++t) threads.emplace_back([this, t] { work(t); });
     } catch (...) {
       // fewer threads than wanted: the ones that started share the work
     }
-    size = (int)threads.size() + 1;
   }
-  // Columns t, t + size, ... of chunk k.
-  void gather(int t, int64_t k) {
-    const Chunk c = chunks[(size_t)k];
-    double* dst = stage[k % 3];
-    for (int i = t; i < nbas; i += size.load())
-      std::memcpy(dst + 2 * (int64_t)i * c.len, cprod + 2 * ((int64_t)i * ldc + c.p0),
-                  sizeof(double) * 2 * (size_t)c.len);
-    gathered.fetch_add(1);
-  }
-  void add(int t, int piece) {
-    const int64_t a0 = n * piece / pieces, a1 = n * (piece + 1) / pieces, w = size.load();
-    for (int64_t i = a0 + (a1 - a0) * t / w, e = a0 + (a1 - a0) * (t + 1) / w; i < e; ++i) out[i] += sums[i];
-    added.fetch_add(1);
-  }
-  // Maps this thread's share of a fresh output's pages before they are needed.
-  void touch(int t) {
-    const int64_t w = size.load();
-    for (int64_t i = n * t / w, e = n * (t + 1) / w; i < e; i += 512) {
-      volatile double* p = out + i;
-      *p = *p;
+  // Hands a task to the threads; the one before must have been finished.
+  void post(const Task& t) {
+    {
+      std::lock_guard<std::mutex> lock(m);
+      task = t;
+      running = (int)threads.size();
+      posted.fetch_add(1);
     }
-    touched.fetch_add(1);
+    go.notify_all();
   }
-  template <class Cond>
-  bool wait(Cond cond) {
-    for (int spin = 0; !cond(); ++spin) {
-      if (stop) return false;
-      if (spin < 64) std::this_thread::yield();
-      else std::this_thread::sleep_for(std::chrono::microseconds(20));
+  // Share t of the threads and the caller (share 0).
+  void share(int t, const Task& k) const {
+    const int64_t n = (int64_t)threads.size() + 1;
+    if (k.job == GATHER) {
+      for (int64_t i = t; i < k.nbas; i += n)
+        std::memcpy(k.dst + 2 * i * k.len, k.src + 2 * i * k.ldc, sizeof(double) * 2 * (size_t)k.len);
+      return;
     }
-    return true;
-  }
-  void work(int t) {
-    if (!wait([&] { return size.load() > 0; })) return;
-    if (cprod)
-      for (int64_t k = 0; k < (int64_t)chunks.size(); ++k) {
-        if (!wait([&] { return gather_to.load() >= k; })) return;
-        gather(t, k);
+    const int64_t a = k.len * t / n, e = k.len * (t + 1) / n;
+    if (k.job == TOUCH) {
+      // maps this share of a fresh output's pages before they are needed
+      for (int64_t i = a; i < e; i += 512) {
+        volatile double* p = k.dst + i;
+        *p = *p;
       }
-    touch(t);
-    for (int p = 0; p < pieces; ++p) {
-      if (!wait([&] { return add_to.load() >= p; })) return;
-      add(t, p);
+    } else {
+      for (int64_t i = a; i < e; ++i) k.dst[i] += k.src[i];
     }
   }
+  void finish() {
+    for (int spin = 0; spin < 64 && running.load() > 0; ++spin) std::this_thread::yield();
+    std::unique_lock<std::mutex> lock(m);
+    done.wait(lock, [&] { return running.load() == 0; });
+  }
+  void run(const Task& t) {
+    post(t);
+    share(0, t);
+    finish();
+  }
+
+ private:
+  void work(int t) {
+    for (int64_t seen = 0;;) {
+      for (int spin = 0; spin < 64 && posted.load() == seen; ++spin) std::this_thread::yield();
+      Task k;
+      {
+        std::unique_lock<std::mutex> lock(m);
+        go.wait(lock, [&] { return posted.load() != seen; });
+        seen = posted.load();
+        k = task;
+      }
+      if (k.job == QUIT) return;
+      share(t, k);
+      std::lock_guard<std::mutex> lock(m);
+      if (running.fetch_sub(1) == 1) done.notify_one();
+    }
+  }
+  std::mutex m;
+  std::condition_variable go, done;
+  std::atomic<int64_t> posted{0};
+  std::atomic<int> running{0};
+  Task task{};
+  std::vector<std::thread> threads;
 };
 
 extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ldc,
@@ -678,9 +688,8 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
           ? (int64_t)align_up((size_t)std::min<int64_t>(16384, std::max<int64_t>(256, (8 << 20) / (16 * (int64_t)nbas))), 256)
           : (int64_t)align_up(16384, (size_t)align);
   const int64_t first = ramp ? std::min<int64_t>(slab, first_pairs) : slab;
-  HostCrew crew;
-  int64_t longest = 0;
-  for (int64_t p0 = 0, len = 0; p0 < npair; p0 += len) {
+  // pairs of the chunk from p0 after one of `len` pairs
+  auto chunk_at = [&](int64_t p0, int64_t len) -> int64_t {
     int64_t want = first;
     if (p0 > 0 && ramp)
       want = std::min<int64_t>(slab, (int64_t)align_up((size_t)(precision == SPX_FP64 ? 2 * len : len + len / 8),
@@ -690,19 +699,20 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
     const int64_t left = npair - p0;
     if (ramp && p0 > 0 && left <= 2 * want)
       want = std::max<int64_t>(align, (int64_t)align_up((size_t)((left + 1) / 2), (size_t)align));
-    len = std::min<int64_t>(want, left);
-    crew.chunks.push_back({p0, len});
-    longest = std::max(longest, len);
-  }
-  slab = (int64_t)align_up((size_t)longest, 16);   // the buffers hold the longest chunk
+    return std::min<int64_t>(want, left);
+  };
+  int64_t longest = 0;
+  for (int64_t p0 = 0, len = 0; p0 < npair; p0 += len) longest = std::max(longest, len = chunk_at(p0, len));
+  // the buffers hold the longest chunk
+  const int64_t held = (int64_t)align_up((size_t)longest, 16);
   const int nslab_buf = 3;  // chunk k's copy waits only for chunk k-3's accumulation
   const int64_t npack = (int64_t)nbas * (nbas + 1) / 2;
   const size_t out_bytes = align_up(sizeof(double) * 2 * (size_t)npack * nw, 256);
-  const size_t slab_bytes = align_up(sizeof(double) * 2 * (size_t)slab * nbas, 256);
-  const size_t e_bytes = align_up(sizeof(double) * (size_t)slab, 256);
+  const size_t slab_bytes = align_up(sizeof(double) * 2 * (size_t)held * nbas, 256);
+  const size_t e_bytes = align_up(sizeof(double) * (size_t)held, 256);
   const size_t om_bytes = align_up(sizeof(double) * (size_t)nw, 256);
-  const size_t w_bytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)slab * nw, 256) : 0;
-  const size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, slab, nbas, nw) : 0;
+  const size_t w_bytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)held * nw, 256) : 0;
+  const size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, held, nbas, nw) : 0;
   const size_t total = out_bytes + nslab_buf * (slab_bytes + 2 * e_bytes) + om_bytes + w_bytes + s_bytes;
   if ((rc = ensure_workspace(ctx, total))) return rc;
   char* base = (char*)ctx->ws;
@@ -748,28 +758,20 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
   // rest of the call waits for the host copies
   ctx->timing = stats != nullptr;
   ctx->nmarks = 0;
-  if (!pinned) {
-    crew.cprod = cprod;
-    crew.ldc = ldc;
-    crew.nbas = nbas;
-    for (int b = 0; b < nslab_buf; ++b) crew.stage[b] = stage + (size_t)b * (slab_bytes / sizeof(double));
-  }
-  crew.out = susceph;
-  crew.sums = (const double*)ctx->pinned;
-  crew.n = 2 * npack * nw;
-  // the sums come back and are added in pieces (not worth it below a few megabytes)
-  crew.pieces = out_host_bytes > ((size_t)4 << 20) ? 4 : 1;
+  const int64_t nsum = 2 * npack * nw;
+  const HostCrew::Task touch{HostCrew::TOUCH, nullptr, susceph, 0, nsum, 0};
+  HostCrew crew;
   crew.start((int)std::max(1u, std::min(8u, std::thread::hardware_concurrency())));
-  for (int64_t k = 0; k < (int64_t)crew.chunks.size(); ++k) {
+  if (pinned) crew.post(touch);   // (nothing to gather)
+  for (int64_t p0 = 0, len = 0, k = 0; p0 < npair; p0 += len, ++k) {
+    len = chunk_at(p0, len);
     const int b = (int)(k % nslab_buf);
-    const int64_t p0 = crew.chunks[(size_t)k].p0, len = crew.chunks[(size_t)k].len;
+    double* st = pinned ? nullptr : stage + (size_t)b * (slab_bytes / sizeof(double));
     const size_t bytes = sizeof(double) * 2 * (size_t)len;
     if (!pinned) {
       // the staging part `b` is free once the copy of chunk k - 3 out of it has finished
       if (k >= nslab_buf) cudaEventSynchronize(ev_copied[b]);
-      crew.gather_to = k;
-      crew.gather(0, k);
-      crew.wait([&] { return crew.gathered.load() >= (k + 1) * crew.size.load(); });
+      crew.run({HostCrew::GATHER, cprod + 2 * p0, st, ldc, len, nbas});
     }
     cudaStreamWaitEvent(xs, ev_free[b], 0);
     if (pinned)
@@ -777,7 +779,7 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
                                              bytes, nbas, cudaMemcpyHostToDevice, xs),
                       "copy cprod slab");
     else
-      rc = check_cuda(ctx, cudaMemcpyAsync(d_slab[b], crew.stage[b], bytes * nbas, cudaMemcpyHostToDevice, xs),
+      rc = check_cuda(ctx, cudaMemcpyAsync(d_slab[b], st, bytes * nbas, cudaMemcpyHostToDevice, xs),
                       "copy cprod slab");
     if (rc) {
       ctx->timing = false;
@@ -802,13 +804,16 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
     cudaEventRecord(ev_free[b], cs);
   }
   ctx->timing = false;
-  crew.touch(0);
+  if (!pinned) crew.post(touch);
+  crew.share(0, touch);
   rc = collect_status(ctx, cs, "chi0_accumulate");   // nothing is added after a failure
   if (rc) return rc;
   cudaEvent_t ev_piece[4] = {ctx->ev[8], ctx->ev[9], ctx->ev[10], ctx->ev[11]};
   double* sums = (double*)ctx->pinned;
-  for (int i = 0; i < crew.pieces; ++i) {
-    const int64_t a0 = crew.n * i / crew.pieces, a1 = crew.n * (i + 1) / crew.pieces;
+  // the sums come back and are added in pieces (not worth it below a few megabytes)
+  const int pieces = out_host_bytes > ((size_t)4 << 20) ? 4 : 1;
+  for (int i = 0; i < pieces; ++i) {
+    const int64_t a0 = nsum * i / pieces, a1 = nsum * (i + 1) / pieces;
     if ((rc = check_cuda(ctx, cudaMemcpyAsync(sums + a0, (const double*)d_out + a0, sizeof(double) * (a1 - a0),
                                               cudaMemcpyDeviceToHost, cs),
                          "copy the sums back")) ||
@@ -816,13 +821,12 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
       return rc;
   }
   d2h += out_host_bytes;
-  crew.wait([&] { return crew.touched.load() >= crew.size.load(); });   // no page is being touched any more
-  for (int i = 0; i < crew.pieces; ++i) {
+  crew.finish();   // no page is being touched any more
+  for (int i = 0; i < pieces; ++i) {
+    const int64_t a0 = nsum * i / pieces, a1 = nsum * (i + 1) / pieces;
     if ((rc = check_cuda(ctx, cudaEventSynchronize(ev_piece[i]), "copy the sums back"))) return rc;
-    crew.add_to = i;   // susceph += sums
-    crew.add(0, i);
+    crew.run({HostCrew::ADD, sums + a0, susceph + a0, 0, a1 - a0, 0});   // susceph += sums
   }
-  crew.wait([&] { return crew.added.load() >= crew.pieces * crew.size.load(); });
   if (stats) {
     timing_collect(ctx, &stats->ms_prep, &stats->ms_gram);
     stats->h2d_bytes = h2d;
