@@ -87,13 +87,14 @@ struct SplitParams {
   double* out;            // packed complex output, as doubles
   int64_t npack;
   int whole;              // items dealt whole (all of them without `part`)
+  int ncut;               // CTAs that share the stages of the others
   double* part;           // partial tiles [CTA][2 slots][elements], or NULL
   int* status;
   uint64_t timeout_ns;
 };
 
 // The items of one CTA of the one-CTA kernels: whole items blockIdx.x, + gridDim.x, ...
-// below `whole`, then its share of the K stages of the items left over. Those would fill
+// below `whole`, then, in the first `ncut` CTAs, a share of the K stages of the items left over. Those would fill
 // a fraction of the SMs for a whole item's time; cut along K they take that fraction of
 // it. A partial sum is an exact integer (below 2^49 in magnitude), so adding the parts
 // before the scale gives the bits of an uncut item (split_gram_finish_kernel). Measured at
@@ -101,11 +102,11 @@ struct SplitParams {
 // 64 x 80 tiles, 270 us cut with 64 x 64 and 9 us for the sum.
 struct SplitSeg {
   int item, u, u1, n;
-  __device__ __forceinline__ SplitSeg(const SplitParams& p, int cta, int grid) {
+  __device__ __forceinline__ SplitSeg(const SplitParams& p, int cta) {
     item = cta;
-    const int64_t tail = (int64_t)(p.nitems - p.whole) * p.nk;   // < 2^31: fewer than `grid` items
-    u = (int)(tail * cta / grid);
-    u1 = (int)(tail * (cta + 1) / grid);
+    const int64_t tail = (int64_t)(p.nitems - p.whole) * p.nk;   // < 2^31: fewer than 148 items
+    u = cta < p.ncut ? (int)(tail * cta / p.ncut) : 0;
+    u1 = cta < p.ncut ? (int)(tail * (cta + 1) / p.ncut) : 0;
     n = 0;
   }
   // Next item and its stages [k0, k1); slot -1: the whole item.
@@ -270,7 +271,7 @@ __global__ void __maxnreg__(SP1_REGS)
       for (int s = 0; s < SP_ST; ++s) issued[s] = false, last_ph[s] = 0;
       bool ok = true;
       int item, k0, k1, slot;
-      SplitSeg seg(prm, blockIdx.x, gridDim.x);
+      SplitSeg seg(prm, blockIdx.x);
       for (int j = 0; ok && seg.next(prm, gridDim.x, &item, &k0, &k1, &slot); ++j) {
         const int f = item / prm.ntile;
         int bi, bj;
@@ -305,7 +306,7 @@ __global__ void __maxnreg__(SP1_REGS)
       uint32_t ph = 0;
       bool committed = false;
       int item, k0, k1, slot;
-      SplitSeg seg(prm, blockIdx.x, gridDim.x);
+      SplitSeg seg(prm, blockIdx.x);
       for (int j = 0; seg.next(prm, gridDim.x, &item, &k0, &k1, &slot); ++j) {
         const int f = item / prm.ntile;
         int bi, bj;
@@ -358,7 +359,7 @@ __global__ void __maxnreg__(SP1_REGS)
     const int q = warp & 3, h = (warp - 2) >> 2;
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
     int item, k0, k1, slot;
-    SplitSeg seg(prm, blockIdx.x, gridDim.x);
+    SplitSeg seg(prm, blockIdx.x);
     for (int j = 0; seg.next(prm, gridDim.x, &item, &k0, &k1, &slot); ++j) {
       if (!mbar_wait_idle(&sm.tfull, (uint32_t)(j & 1), prm.timeout_ns, prm.status)) break;
       tc_fence_after();
@@ -389,17 +390,17 @@ __global__ void __maxnreg__(SP1_REGS)
 template <bool REAL>
 constexpr int split_finish_step() { return REAL ? 16 : 8; }
 template <bool REAL, int BN>
-__global__ void __launch_bounds__(32 * SP1_EPI) split_gram_finish_kernel(SplitParams prm, int ncta) {
+__global__ void __launch_bounds__(32 * SP1_EPI) split_gram_finish_kernel(SplitParams prm, int grid) {
   await_previous();
   const int64_t tail = (int64_t)(prm.nitems - prm.whole) * prm.nk;
   const int c = blockIdx.x + 1;
-  const int64_t u = tail * c / ncta;
+  const int64_t u = tail * c / prm.ncut;
   const int64_t t0 = u / prm.nk * prm.nk, t1 = t0 + prm.nk;
-  if (u == t0 || u >= tail || tail * (c - 1) / ncta > t0) return;
+  if (u == t0 || u >= tail || tail * (c - 1) / prm.ncut > t0) return;
   const int item = prm.whole + (int)(t0 / prm.nk);
   const int f = item / prm.ntile;
   int bi, bj;
-  split_decode_tile_bn<BN>(split_item_tile(item, prm.ntile, ncta), prm.nbr, &bi, &bj);
+  split_decode_tile_bn<BN>(split_item_tile(item, prm.ntile, grid), prm.nbr, &bi, &bj);
   const int warp = (threadIdx.x >> 5) + 2, lane = threadIdx.x & 31;   // the epilogue's warp numbers
   const int q = warp & 3, h = (warp - 2) >> 2;
   constexpr int NC = BN * 4 / SP1_EPI, STEP = split_finish_step<REAL>();
@@ -407,10 +408,10 @@ __global__ void __launch_bounds__(32 * SP1_EPI) split_gram_finish_kernel(SplitPa
   double o[STEP];
 #pragma unroll
   for (int v = 0; v < STEP; ++v) o[v] = 0.0;
-  for (int k = c - 1; k < ncta; ++k) {
-    const int64_t s = tail * k / ncta;
+  for (int k = c - 1; k < prm.ncut; ++k) {
+    const int64_t s = tail * k / prm.ncut;
     if (s >= t1) break;
-    if (tail * (k + 1) / ncta == s) continue;   // an empty range
+    if (tail * (k + 1) / prm.ncut == s) continue;   // an empty range
     // the item is a CTA's first segment when its range starts inside it
     const double* pp = prm.part + ((int64_t)k * 2 + (s >= t0 ? 0 : 1)) * split_part_elems(REAL, BN) +
                        (int64_t)v0 * (32 * SP1_EPI) + threadIdx.x;
@@ -421,13 +422,20 @@ __global__ void __launch_bounds__(32 * SP1_EPI) split_gram_finish_kernel(SplitPa
   else fold_add<STEP, BN>(q, lane, bi, bj, f, prm, NC * h + v0, o);
 }
 
-// Whether cutting the last items of `nitems` pays: it saves this many of the last round's
-// `nk` stages (0.55-0.6 us each) and costs the partial tiles' way through memory and one
-// short launch: 20 us with complex tiles (403 columns, 12 frequencies: 40 of 336 items
-// left), 40 us with the twice as large real ones.
-static bool split_cuts(int nitems, int nk, int num_sms, bool real) {
-  const int left = nitems % num_sms;
-  return left > 0 && nk - (int64_t)left * nk / num_sms >= (real ? 128 : 64);
+// CTAs that share the stages of the items left over by whole rounds of `num_sms` CTAs; 0 when
+// these stay whole. A share is about the root of an item's `nk` stages at least: a stage takes
+// 0.55-0.6 us, and an item's partial tiles are added one after the other at about the same time
+// each. Cutting pays when it saves this many of the last round's stages: it costs the partial
+// tiles' way through memory and one short launch, 20 us with complex tiles (403 columns, 12
+// frequencies: 40 of 336 items left), 40 us with the twice as large real ones.
+int split_cut_ctas(int nitems, int nk, int num_sms, bool real) {
+  const int64_t left = nitems % num_sms, tail = left * nk;
+  if (left == 0) return 0;
+  int64_t share = 8;
+  while (share * share < nk) ++share;
+  const int64_t even = (tail + num_sms - 1) / num_sms;
+  if (nk - std::max(share, even) < (real ? 128 : 64)) return 0;
+  return (int)std::min<int64_t>(num_sms, tail / share);
 }
 
 // ---------------------------------------------------------------------------
@@ -1025,7 +1033,18 @@ static int split_ntile(int n, int bn, int nbr) {
 // of N = 160 takes 1.10 times the time of one of N = 128 (which is bound by the instruction
 // rate), so 64 x 80 tiles win (1.13 fewer of them at 1200 columns: 739 against 705 TFLOP/s)
 // unless their last column block is nearly empty (403 columns: 28 tiles of either shape).
-static bool split_wide(int n, int nbr) { return split_ntile(n, SP_WIDE_BN, nbr) * 110 < split_ntile(n, SP_TILE, nbr) * 100; }
+// Tiles count in rounds of the SMs, a cut last round (`cut`: partial tiles can be had) as its
+// fraction and the 36 or 72 stages that its sum takes: 320 columns, 10 frequencies are 140
+// wide tiles or 150 square ones, 110 and 114 us at 4160 pairs (65 stages), where a cut does not pay.
+static bool split_wide(int n, int nbr, int nw, int64_t nk, int num_sms, bool real, bool cut) {
+  auto rounds = [&](int bn) {
+    const int items = split_ntile(n, bn, nbr) * nw;
+    if (cut && split_cut_ctas(items, (int)nk, num_sms, real))
+      return (double)items / num_sms + (real ? 72.0 : 36.0) / (double)nk;
+    return (double)((items + num_sms - 1) / num_sms);
+  };
+  return 1.10 * rounds(SP_WIDE_BN) < rounds(SP_TILE);
+}
 
 // Most pairs of a part: a slab's scales and factors hold for all of it, but its planes are
 // written and accumulated in equal parts of at most this many pairs (the parts' FP64 adds are
@@ -1100,20 +1119,18 @@ static int split_gram_launch(spx_ctx* ctx, const CUtensorMap& mapA, const CUtens
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                       "split_gram_kernel attribute");
   if (rc) return rc;
-  const bool cut = part && split_cuts(prm.nitems, prm.nk, ctx->num_sms, REAL);
-  // a cut range is at least 8 stages long
-  const int grid = (int)std::min<int64_t>(
-      cut ? std::max<int64_t>(prm.nitems, (int64_t)prm.nitems * prm.nk / 8) : prm.nitems, ctx->num_sms);
-  prm.whole = cut ? prm.nitems / grid * grid : prm.nitems;
-  prm.part = cut ? part : nullptr;
+  prm.ncut = part ? split_cut_ctas(prm.nitems, prm.nk, ctx->num_sms, REAL) : 0;
+  prm.whole = prm.ncut ? prm.nitems / ctx->num_sms * ctx->num_sms : prm.nitems;
+  prm.part = prm.ncut ? part : nullptr;
+  const int grid = std::min(prm.whole ? prm.whole : prm.ncut, ctx->num_sms);
   if ((rc = check_cuda(ctx, launch_chained(split_gram_kernel<REAL, BN>, grid, SP1_THREADS, smem, stream, chained, mapA,
                                            mapB, prm),
                        "split_gram_kernel launch")))
     return rc;
   *launches += 1;
-  if (prm.whole < prm.nitems && grid > 1) {
+  if (prm.ncut) {
     const int ny = (REAL ? 2 : 1) * BN * 4 / SP1_EPI / split_finish_step<REAL>();
-    if ((rc = check_cuda(ctx, launch_chained(split_gram_finish_kernel<REAL, BN>, dim3(grid - 1, ny), 32 * SP1_EPI, 0,
+    if ((rc = check_cuda(ctx, launch_chained(split_gram_finish_kernel<REAL, BN>, dim3(prm.ncut - 1, ny), 32 * SP1_EPI, 0,
                                              stream, true, prm, grid),
                          "split_gram_finish_kernel launch")))
       return rc;
@@ -1220,7 +1237,8 @@ static int split_chi0_run(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P
   // planes in HBM: [plane][k-block][row][K bytes]; TMA dims (K, row, k-block, plane)
   // with increasing strides; a box (K, rows, 1, 3 planes) lands as [plane][row][K]
   if (variant == 0) variant = ctx->opt.split_variant;
-  if (variant == 0) variant = split_wide(N, L.nblk) ? 5 : 1;  // untuned: one CTA per tile
+  if (variant == 0)   // untuned: one CTA per tile
+    variant = split_wide(N, L.nblk, nw, buf[0].Pp / SP_KB, ctx->num_sms, false, part && nbuf == 1) ? 5 : 1;
   const bool pair = variant == 2;
   const bool wide = variant == 5;                  // one CTA per 64 x 80 tile (N = 160)
   // only the CTA pair needs an even number of 64-column blocks in the planes (the
@@ -1360,7 +1378,8 @@ int split_chi0_real_ediff(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P,
   SplitBuf buf[2];
   const int nbuf = split_buffers(L, P, nw, base, buf);
   double* part = (double*)ctx->part;   // partial tiles
-  const bool wide = ctx->opt.split_variant != 1 && (ctx->opt.split_variant != 0 || split_wide((N + 1) / 2, L.nblk));
+  const bool wide = ctx->opt.split_variant != 1 && (ctx->opt.split_variant != 0 || split_wide((N + 1) / 2, L.nblk, nw, buf[0].Pp / SP_KB,
+                                                                                       ctx->num_sms, true, part && nbuf == 1));
   CUtensorMap mapF[2], mapW[2];
   for (int b = 0; b < nbuf; ++b) {
     const uint64_t nkb = (uint64_t)(buf[b].Pp / SP_KB);
