@@ -847,7 +847,7 @@ int wfprod_mt_run(spx_ctx*, const spx_mt_desc*, int, int, int, const double2*, c
 int wfprod_pw_run(spx_ctx*, const spx_pw_desc*, int, int, int, const double2*, const double2*,
                   double2*, int64_t, int, void*, size_t, cudaStream_t, int*, bool, bool);
 size_t wfprod_mt_workspace(const spx_mt_desc*, int, int);
-size_t wfprod_pw_workspace(const spx_pw_desc*, int, int, int, bool);
+size_t wfprod_pw_workspace(const spx_pw_desc*, int, int, int, bool, size_t room);
 }  // namespace spx
 
 extern "C" int spx_chi0_from_coeffs_dev(spx_ctx* ctx, const spx_mt_desc* mt,
@@ -886,8 +886,10 @@ extern "C" int spx_chi0_from_coeffs_dev(spx_ctx* ctx, const spx_mt_desc* mt,
   // interstitial products on int8 slices when the accumulation is split anyway
   const bool split_products = ctx->opt.products == SPX_PRODUCTS_SPLIT ||
                               (ctx->opt.products == SPX_PRODUCTS_AUTO && precision == SPX_SPLIT);
-  const size_t prod_bytes = std::max(wfprod_mt_workspace(mt, nk, nocc),
-                                     wfprod_pw_workspace(pw, nk, nocc, nunocc, split_products));
+  const size_t limit = (size_t)std::max<int64_t>(ctx->opt.workspace_limit, 0);
+  const size_t prod_bytes = std::max(
+      wfprod_mt_workspace(mt, nk, nocc),
+      wfprod_pw_workspace(pw, nk, nocc, nunocc, split_products, limit > m_bytes ? limit - m_bytes : 0));
   const int64_t ldw = ldc;
   const size_t w_bytes = precision == SPX_FP64 ? align_up(sizeof(double) * (size_t)ldw * nw, 256) : 0;
   const size_t s_bytes = precision == SPX_SPLIT ? split_scratch_bytes(ctx, npair, nbas, nw) : 0;

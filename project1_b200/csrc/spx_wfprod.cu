@@ -698,7 +698,7 @@ static int plan_pw(spx_ctx* ctx, const spx_pw_desc* d, PwPlan* pl) {
   return SPX_OK;
 }
 
-size_t wfprod_pw_fft_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc);
+size_t wfprod_pw_fft_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc, size_t room);
 size_t sgemm_workspace_bytes(int nbatch, int M, int ncol, int K);
 int sgemm_products(spx_ctx* ctx, int nbatch, int M, int ncol, int K, const double2* A,
                    int64_t lda, int64_t a_bstride, const int* kperm, const double2* grid,
@@ -709,8 +709,10 @@ int wfprod_pw_fft_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int 
                       const double2* c1, const double2* c2, double2* cprod, int64_t ldc, int col0,
                       void* ws, size_t ws_bytes, cudaStream_t s, int* launches);
 
-size_t wfprod_pw_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc, bool split) {
-  if (d->nfft > 0) return wfprod_pw_fft_workspace(d, nk, nocc, nunocc);
+// Scratch of the products of nk k points, in chunks of k points where `room` (the most the
+// caller can have, 0 = no limit) or a budget does not hold them all.
+size_t wfprod_pw_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc, bool split, size_t room) {
+  if (d->nfft > 0) return wfprod_pw_fft_workspace(d, nk, nocc, nunocc, room);
   spx_ctx dummy;
   PwPlan pl;
   if (plan_pw(&dummy, d, &pl)) return 0;
@@ -719,7 +721,8 @@ size_t wfprod_pw_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc, b
   const size_t fixed = align_up(sizeof(int) * std::max(d->ngpt1, 1), 256) +
                        (split ? 2 : 1) * align_up(sizeof(int) * std::max(d->ngpt2, 1), 256) +
                        align_up(sizeof(int64_t) * std::max(d->ngptm, 1), 256) + 4096;
-  const size_t budget = (size_t)2 << 30;
+  size_t budget = (size_t)2 << 30;
+  if (room) budget = std::min(budget, room - std::min(room, fixed));
   const size_t kchunk = std::max<size_t>(1, std::min<size_t>((size_t)nk, budget / perk));
   return fixed + kchunk * perk;
 }
@@ -890,7 +893,8 @@ extern "C" int spx_wfprod_pw_dev(spx_ctx* ctx, const spx_pw_desc* pw, int32_t nk
   if ((int64_t)nk * nocc * nunocc == 0) return SPX_OK;
   cudaSetDevice(ctx->device);
   const bool split = ctx->opt.products == SPX_PRODUCTS_SPLIT;
-  const size_t need = wfprod_pw_workspace(pw, nk, nocc, nunocc, split);
+  const size_t need =
+      wfprod_pw_workspace(pw, nk, nocc, nunocc, split, (size_t)std::max<int64_t>(ctx->opt.workspace_limit, 0));
   if (need == 0) {
     // the plan is invalid: run it once more to report why
     if (pw->nfft > 0)

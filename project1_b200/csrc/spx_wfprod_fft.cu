@@ -767,7 +767,8 @@ static int fold_k(int v, int n) {
   return k >= -7 && k <= 7 ? k : 99;
 }
 
-static int plan_fft(spx_ctx* ctx, const spx_pw_desc* d, FftPlan* pl) {
+// fold: whether the folded passes may be taken (their padded lines need a little more scratch).
+static int plan_fft(spx_ctx* ctx, const spx_pw_desc* d, FftPlan* pl, bool fold = true) {
   const int n = d->nfft;
   if (n < 2 || n > FFT_NMAX)
     return set_error(ctx, SPX_EINVAL, "nfft must be in 2..64 for the FFT branch");
@@ -781,7 +782,7 @@ static int plan_fft(spx_ctx* ctx, const spx_pw_desc* d, FftPlan* pl) {
   pl->b2 = box_of(d->gpt2, d->ngpt2);
   // G_M alone within 7 of the origin on every axis: the folded passes, with the backfolding
   // vector in the step function (exp(2 pi i g r / n) theta(r) shifts the product's spectrum)
-  pl->sym = n >= 16;
+  pl->sym = fold && n >= 16;
   for (int i = 0; i < 3 * d->ngptm && pl->sym; ++i)
     pl->sym = fold_k(((d->gptm[i] % n) + n) % n, n) != 99;
   for (int c = 0; c < 3; ++c) {
@@ -845,27 +846,83 @@ static int plan_fft(spx_ctx* ctx, const spx_pw_desc* d, FftPlan* pl) {
   return SPX_OK;
 }
 
-static size_t fft_perk_bytes(const FftPlan& pl, int nocc, int nunocc, int nkxky) {
-  const int64_t n = pl.n;
-  const int64_t nb = std::max(nocc, nunocc);
-  const int64_t box = nb * std::max(pl.b1.size(), pl.b2.size());
-  const int64_t ta = nb * n * std::max(pl.b1.dim[1] * pl.b1.dim[2], pl.b2.dim[1] * pl.b2.dim[2]);
-  const int64_t tb = nb * n * n * std::max(pl.b1.dim[2], pl.b2.dim[2]);
-  return align_up(16 * (size_t)box, 256) + align_up(16 * (size_t)ta, 256) + align_up(16 * (size_t)tb, 256) +
-         align_up(16 * (size_t)(nocc + nunocc) * n * n * pl.ld, 256) +
-         align_up(16 * (size_t)nocc * nunocc * n * nkxky, 256) + 16 * (size_t)n * n * 9 * 2 + 2048;
+// Scratch of a call: the plan's tables, copied as one block; theta(r); and for `kchunk` k points
+// the band grids A and B and one region that first holds the passes' buffers (box, ta, tb), then
+// T2, which is written after the last of them has run.
+struct FftScratch {
+  size_t o_g1, o_g2, o_ks[3], o_gmap, o_twb, o_twf, o_cs, o_pos[3], o_tab, tables;   // bytes
+  size_t box, ta, tb, A, B, T2;   // elements per k point
+  size_t theta, theta_ta, theta_tb;
+  FftScratch() = default;
+  FftScratch(const FftPlan& pl, const spx_pw_desc* d, int nocc, int nunocc) {
+    const size_t n = (size_t)pl.n, nb = (size_t)std::max(nocc, nunocc), n2ld = n * n * (size_t)pl.ld;
+    size_t at = 0;
+    auto table = [&](size_t bytes) {
+      const size_t o = at;
+      at += align_up(std::max<size_t>(bytes, 1), 256);
+      return o;
+    };
+    o_g1 = table(4 * (size_t)d->ngpt1);
+    o_g2 = table(4 * (size_t)d->ngpt2);
+    for (int c = 0; c < 3; ++c) o_ks[c] = table(4 * pl.ks[c].size());
+    o_gmap = table(4 * (size_t)d->ngptm);
+    o_twb = table(16 * n);
+    o_twf = table(16 * n);
+    o_cs = table(16 * (size_t)pl.bs.size());
+    for (int c = 0; c < 3; ++c) o_pos[c] = table(4 * pl.pos[c].size());
+    o_tab = table(16 * pl.tab.size());
+    tables = at;
+    box = nb * (size_t)std::max(pl.b1.size(), pl.b2.size());
+    ta = nb * n * (size_t)std::max(pl.b1.dim[1] * pl.b1.dim[2], pl.b2.dim[1] * pl.b2.dim[2]);
+    tb = nb * n * n * (size_t)std::max(pl.b1.dim[2], pl.b2.dim[2]);
+    A = (size_t)nocc * n2ld;
+    B = (size_t)nunocc * n2ld;
+    T2 = (size_t)nocc * (size_t)nunocc * n * pl.ks[0].size() * pl.ks[1].size();
+    theta = n * n * n;
+    theta_ta = n * (size_t)(pl.bs.dim[1] * pl.bs.dim[2]);
+    theta_tb = n * n * (size_t)pl.bs.dim[2];
+  }
+  size_t passes(size_t k) const {   // of the region: buffers of k k points, or of theta
+    return align_up(16 * k * box, 256) + align_up(16 * std::max(k * ta, theta_ta), 256) +
+           align_up(16 * std::max(k * tb, theta_tb), 256);
+  }
+  size_t region(size_t k) const { return std::max(align_up(16 * k * T2, 256), passes(k)); }
+  size_t bytes(size_t k) const {
+    return tables + align_up(16 * theta, 256) + align_up(16 * k * A, 256) + align_up(16 * k * B, 256) + region(k);
+  }
+  // Most k points, up to nk and at least one, within `left` bytes.
+  int kchunk(int nk, size_t left) const {
+    int lo = 1, hi = nk;
+    while (lo < hi) {
+      const int mid = lo + (hi - lo + 1) / 2;
+      if (bytes((size_t)mid) <= left) lo = mid;
+      else hi = mid - 1;
+    }
+    return lo;
+  }
+};
+
+// The plan and scratch of a call within `room` bytes: folded passes where they fit.
+static int fft_plan_within(spx_ctx* ctx, const spx_pw_desc* d, int nocc, int nunocc, size_t room, FftPlan* pl,
+                           FftScratch* sc) {
+  int rc = plan_fft(ctx, d, pl);
+  if (rc) return rc;
+  *sc = FftScratch(*pl, d, nocc, nunocc);
+  if (!pl->sym || sc->bytes(1) <= room) return SPX_OK;
+  *pl = FftPlan();
+  if ((rc = plan_fft(ctx, d, pl, false))) return rc;
+  *sc = FftScratch(*pl, d, nocc, nunocc);
+  return SPX_OK;
 }
 
-size_t wfprod_pw_fft_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc) {
+// room: the most the caller can have, 0 = no limit.
+size_t wfprod_pw_fft_workspace(const spx_pw_desc* d, int nk, int nocc, int nunocc, size_t room) {
   spx_ctx dummy;
   FftPlan pl;
-  if (plan_fft(&dummy, d, &pl)) return 0;
-  const size_t perk = fft_perk_bytes(pl, nocc, nunocc, (int)(pl.ks[0].size() * pl.ks[1].size()));
-  const size_t fixed = 16 * (size_t)pl.n * pl.n * pl.n + 64 * 1024 +
-                       4 * (size_t)(d->ngpt1 + d->ngpt2 + 2 * d->ngptm) + 16 * 1024;
-  const size_t budget = (size_t)6 << 30;
-  const size_t kchunk = std::max<size_t>(1, std::min<size_t>((size_t)nk, budget / perk));
-  return fixed + kchunk * perk;
+  FftScratch sc;
+  const size_t most = room ? room - std::min<size_t>(room, 256) : SIZE_MAX;
+  if (fft_plan_within(&dummy, d, nocc, nunocc, most, &pl, &sc)) return 0;
+  return sc.bytes((size_t)sc.kchunk(std::max(nk, 1), std::min(most, (size_t)6 << 30))) + 256;
 }
 
 // Three passes G box -> r grid for nb bands: box [b][gz][gy][gx] -> out [b][z][y][ld].
@@ -903,65 +960,54 @@ int wfprod_pw_fft_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int 
                       const double2* c1, const double2* c2, double2* cprod, int64_t ldc, int col0,
                       void* ws, size_t ws_bytes, cudaStream_t s, int* launches) {
   FftPlan pl;
-  int rc = plan_fft(ctx, d, &pl);
+  FftScratch sc;
+  char* base = (char*)align_up((size_t)ws, 256);
+  const size_t left = ws_bytes - std::min(ws_bytes, (size_t)(base - (char*)ws));
+  int rc = fft_plan_within(ctx, d, nocc, nunocc, left, &pl, &sc);
   if (rc) return rc;
   if (d->ngptm == 0 || nk == 0 || nocc == 0 || nunocc == 0 || !ws) return SPX_OK;
   if ((nunocc + FFT_NP - 1) / FFT_NP > 65535)
     return set_error(ctx, SPX_EINVAL, "too many unoccupied bands for the FFT branch");
   const int n = pl.n, nkx = (int)pl.ks[0].size(), nky = (int)pl.ks[1].size(), nkz = (int)pl.ks[2].size();
-  const int64_t n3 = (int64_t)n * n * n, n2ld = (int64_t)n * n * pl.ld;
-  Carve cv{(char*)ws, ws_bytes};
-  int* d_g1 = cv.take<int>(d->ngpt1);
-  int* d_g2 = cv.take<int>(d->ngpt2);
-  int* d_ks[3];
-  for (int c = 0; c < 3; ++c) d_ks[c] = cv.take<int>(pl.ks[c].size());
-  int* d_gmap = cv.take<int>(d->ngptm);
-  double2* d_twb = cv.take<double2>(n);
-  double2* d_twf = cv.take<double2>(n);
-  double2* d_cs = cv.take<double2>((size_t)pl.bs.size());
-  double2* theta = cv.take<double2>((size_t)n3);
-  int* d_pos[3] = {};
-  double2* d_tab = nullptr;
-  if (pl.sym) {
-    for (int c = 0; c < 3; ++c) d_pos[c] = cv.take<int>(15);
-    d_tab = cv.take<double2>(pl.tab.size());
-  }
-  const size_t perk = fft_perk_bytes(pl, nocc, nunocc, nkx * nky);
-  if (!cv.ok || cv.left < perk) return set_error(ctx, SPX_ENOMEM, "FFT-branch scratch too small");
+  const int64_t n3 = (int64_t)n * n * n;
+  if (left < sc.bytes(1)) return set_error(ctx, SPX_ENOMEM, "FFT-branch scratch too small");
   // grid limit of K5c: one CTA per pair of a chunk along x
   const size_t pairs_k = (size_t)nocc * nunocc;
   if (pairs_k > 2147483647u) return set_error(ctx, SPX_EINVAL, "too many band pairs per k point");
-  const int kchunk = (int)std::min<size_t>({(size_t)nk, cv.left / perk, 2147483647u / pairs_k});
-  const int nbmax = std::max(nocc, nunocc) * kchunk;
-  // per-chunk buffers sized for kchunk k points
-  double2* box = cv.take<double2>((size_t)nbmax * std::max(pl.b1.size(), pl.b2.size()));
-  // pass buffers: the bands of a chunk, or the step-function box for theta
-  const size_t ta_n = std::max<size_t>(
-      (size_t)nbmax * n * std::max(pl.b1.dim[1] * pl.b1.dim[2], pl.b2.dim[1] * pl.b2.dim[2]),
-      (size_t)n * pl.bs.dim[1] * pl.bs.dim[2]);
-  const size_t tb_n = std::max<size_t>((size_t)nbmax * n * n * std::max(pl.b1.dim[2], pl.b2.dim[2]),
-                                       (size_t)n * n * pl.bs.dim[2]);
-  double2* ta = cv.take<double2>(ta_n);
-  double2* tb = cv.take<double2>(tb_n);
-  double2* A = cv.take<double2>((size_t)kchunk * nocc * n2ld);
-  double2* Bg = cv.take<double2>((size_t)kchunk * nunocc * n2ld);
-  double2* T2 = cv.take<double2>((size_t)kchunk * nocc * nunocc * n * nkx * nky);
-  if (!cv.ok) return set_error(ctx, SPX_ENOMEM, "FFT-branch scratch too small");
-  auto up = [&](void* dst, const void* src, size_t bytes) {
-    return bytes ? check_cuda(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s), "copy plan") : SPX_OK;
+  const int kchunk = std::min(sc.kchunk(nk, left), (int)std::min<size_t>((size_t)nk, 2147483647u / pairs_k));
+  const size_t kc = (size_t)kchunk;
+  auto at = [&](size_t o) { return base + o; };
+  const int *d_g1 = (int*)at(sc.o_g1), *d_g2 = (int*)at(sc.o_g2), *d_gmap = (int*)at(sc.o_gmap);
+  const int *d_ks[3], *d_pos[3];
+  for (int c = 0; c < 3; ++c) d_ks[c] = (int*)at(sc.o_ks[c]), d_pos[c] = (int*)at(sc.o_pos[c]);
+  const double2 *d_twb = (double2*)at(sc.o_twb), *d_twf = (double2*)at(sc.o_twf), *d_cs = (double2*)at(sc.o_cs),
+                *d_tab = (double2*)at(sc.o_tab);
+  double2* theta = (double2*)at(sc.tables);
+  double2* A = (double2*)((char*)theta + align_up(16 * sc.theta, 256));
+  double2* Bg = (double2*)((char*)A + align_up(16 * kc * sc.A, 256));
+  double2* T2 = (double2*)((char*)Bg + align_up(16 * kc * sc.B, 256));
+  double2* box = T2;
+  double2* ta = (double2*)((char*)box + align_up(16 * kc * sc.box, 256));
+  double2* tb = (double2*)((char*)ta + align_up(16 * std::max(kc * sc.ta, sc.theta_ta), 256));
+  // the tables in one copy: small calls are bound by the host's launches and copies
+  std::vector<char> tables(sc.tables);
+  auto put = [&](size_t o, const void* src, size_t bytes) {
+    if (bytes) std::memcpy(tables.data() + o, src, bytes);
   };
-  if ((rc = up(d_g1, pl.gidx1.data(), 4 * pl.gidx1.size())) || (rc = up(d_g2, pl.gidx2.data(), 4 * pl.gidx2.size())) ||
-      (rc = up(d_ks[0], pl.ks[0].data(), 4 * nkx)) || (rc = up(d_ks[1], pl.ks[1].data(), 4 * nky)) ||
-      (rc = up(d_ks[2], pl.ks[2].data(), 4 * nkz)) || (rc = up(d_gmap, pl.gmap.data(), 4 * pl.gmap.size())) ||
-      (rc = up(d_twb, pl.twb.data(), 16 * n)) || (rc = up(d_twf, pl.twf.data(), 16 * n)) ||
-      (rc = up(d_cs, d->cstep, 16 * (size_t)pl.bs.size())))
+  put(sc.o_g1, pl.gidx1.data(), 4 * pl.gidx1.size());
+  put(sc.o_g2, pl.gidx2.data(), 4 * pl.gidx2.size());
+  for (int c = 0; c < 3; ++c) {
+    put(sc.o_ks[c], pl.ks[c].data(), 4 * pl.ks[c].size());
+    put(sc.o_pos[c], pl.pos[c].data(), 4 * pl.pos[c].size());
+  }
+  put(sc.o_gmap, pl.gmap.data(), 4 * pl.gmap.size());
+  put(sc.o_twb, pl.twb.data(), 16 * (size_t)n);
+  put(sc.o_twf, pl.twf.data(), 16 * (size_t)n);
+  put(sc.o_cs, d->cstep, 16 * (size_t)pl.bs.size());
+  put(sc.o_tab, pl.tab.data(), 16 * pl.tab.size());
+  if ((rc = check_cuda(ctx, cudaMemcpyAsync(base, tables.data(), sc.tables, cudaMemcpyHostToDevice, s), "copy plan")) ||
+      (rc = check_cuda(ctx, cudaStreamSynchronize(s), "copy plan")))
     return rc;
-  if (pl.sym)
-    for (int c = 0; c < 3; ++c)
-      if ((rc = up(d_pos[c], pl.pos[c].data(), 4 * 15)) ||
-          (c == 0 && (rc = up(d_tab, pl.tab.data(), 16 * pl.tab.size()))))
-        return rc;
-  if ((rc = check_cuda(ctx, cudaStreamSynchronize(s), "copy plan"))) return rc;
   // theta(r) from the step-function box (already laid out x fastest)
   if ((rc = band_grids(ctx, pl.bs, 1, d_cs, ta, tb, theta, n, d_twb, n, 0, 1.0, nullptr, s, launches)))
     return rc;
