@@ -2,7 +2,7 @@
 //
 // Most calls run on the product-first kernels further down (K1p: complex, -DINV and the
 // q -> 0 head and wings); the two that follow the sum frequency by frequency keep calls of
-// one to four frequencies where they are faster (f64_takes_k1, f64r_takes_k1r). K1 computes,
+// few frequencies or few pairs where they are faster (f64_on_k1). K1 computes,
 // for every upper-triangle 64x64 tile (I, J) of the mixed-basis
 // matrix and every frequency f,
 //   chi_f(i, j) += sum_p M(p, i) * conj(M(p, j)) * w(p, f),      i <= j,
@@ -324,7 +324,7 @@ constexpr int F64P_MINPAIR = 256;                       // shortest p axis (pair
 // REAL, the -DINV build (src/susceptibility.f:1197): real M and chi, one product and one
 // multiply-add per frequency: 1 + 8 NT units of the pipe, four columns per warp, 16 x 16 tiles.
 // N = 1200, P = 10000, 24 frequencies: 19.4 ms on K1r, 11.2 here (0.90 of the FP64 pipe); K1r
-// keeps the shapes of f64r_takes_k1r.
+// keeps the shapes that f64_on_k1 gives it.
 constexpr int F64P_CPLX = 0, F64P_HW = 1, F64P_REAL = 2;   // MODE
 template <int MODE>
 struct F64PTile {
@@ -838,36 +838,77 @@ static int f64p_launch(const F64Call& q, const F64Head& hw, int f0, int groups, 
   return 0;
 }
 
-// Whether the last r <= 4 frequencies go to K1 rather than to one 8-wide block of K1p. Per
-// element and pair K1 takes 4 r units against 4 + 16, but on whole 64 x 64 tiles that pad
-// narrow matrices and leave SMs idle when there are few. Time of K1: its tiles per SM, two at
-// once, one alone taking 0.725 of the time of two; of K1p: its units spread over the SMs
-// (uncut: rounds of its resident tiles), 1.10 times as long per unit. Measured at 12800 pairs, K1
-// against K1p in us: 64 columns, 1 frequency 2828 / 84; 400, 4: 2866 / 1567; 600, 2: 2866 / 3454;
-// 600, 3: 3934 / 3455; 900, 3: 6802 / 7743; 900, 4: 7857 / 7745; 1200, 4: 11727 / 13587 (with
-// 16-pair chunks, 1.144; the longer ones take 0.96 of that).
-static bool f64_takes_k1(const F64Call& q, int r) {
-  const int64_t nblk = (q.N + F64_B - 1) / F64_B, sms = q.num_sms;
-  const int64_t per_sm = (nblk * (nblk + 1) / 2 * r + sms - 1) / sms;
-  const double two = 2.0 * F64_B * F64_B * 4, k1 = (double)(per_sm / 2) * two + (double)(per_sm % 2) * 0.725 * two;
-  const int64_t t2 = f64p_tiles<F64P_CPLX>(q.N);
-  const double unit = F64P_TI * F64PTile<F64P_CPLX>::TJ * (4 + 16);
-  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<F64P_CPLX>(q.num_sms, 1) && q.P >= F64P_MINPAIR;
-  const double k1p = cut ? (double)t2 * unit / (double)sms : (double)((t2 + F64PTile<F64P_CPLX>::CTAS * sms - 1) / (F64PTile<F64P_CPLX>::CTAS * sms)) * F64PTile<F64P_CPLX>::CTAS * unit;
-  return k1 <= 1.10 * k1p;
+// Which frequencies of a call go to K1 (K1r): times in us of the two forms, from a fit to both
+// over 14 widths from 17 to 1500, 1 to 12800 pairs and 1 to 48 frequencies. K1 works on whole
+// 64 x 64 tiles of one frequency, two at once per SM, 4 (real: 1) units an element and pair,
+// with pairs padded to 16; K1p on 16 x 8 (16 x 16) tiles of eight frequencies a block, 4 + 16 a
+// block (1 + 8), with pairs padded to 64 unless the last round is cut. So K1 is better for few
+// frequencies of a wide matrix, and for few pairs, which leave K1p's padding and its longer
+// epilogue. `call`, `round`: start, and a round of resident tiles; `unit`: against the pipe's 64
+// multiply-adds per clock and SM at 1.9 GHz (below and from F64P_MINPAIR pairs); `alone`: a tile
+// without a second one on its SM, of half of two; `cut`: partial tiles and their sum. us, K1 /
+// K1p (N, P, frequencies): complex 65, 80, 36: 36 / 44; 640, 16, 12: 57 / 74; 900, 80, 5:
+// 99 / 118; 1500, 16, 36: 889 / 1108; 900, 12800, 3: 6777 / 7576; 1500, 12800, 4: 18349 / 20767;
+// the other way round 150, 80, 48: 45 / 34; 640, 80, 24: 185 / 149; 1500, 80, 48: 2050 / 1714;
+// 400, 12800, 4: 2866 / 1567. Real 65, 80, 48: 26 / 36; 900, 16, 36: 228 / 309; 1500, 80, 36: 910 / 1033;
+// 1500, 12800, 4: 7643 / 9060; the other way round 300, 80, 24: 50 / 41; 300, 10000, 24: 2395 /
+// 781; 1200, 10000, 5: 4783 / 4564. Of 3807 shapes of each from 65 columns on, 41 (complex) and 78
+// (real) take over 3 % more than the better form.
+struct F64Cost {
+  double k1_call, k1_round, k1_unit, k1_alone;
+  double p_call, p_round, p_block, p_unit, p_unit_long, p_alone, p_cut;
+};
+template <int MODE>
+static double f64_us_k1(int sms, int N, int64_t P, int n, const F64Cost& c) {
+  const int64_t nblk = (N + F64_B - 1) / F64_B, per_sm = (nblk * (nblk + 1) / 2 * n + sms - 1) / sms;
+  const double tile = (MODE == F64P_REAL ? 1 : 4) * F64_B * F64_B * (double)align_up((size_t)P, 16) / (64 * 1900.0);
+  return c.k1_call + c.k1_round * (double)((per_sm + 1) / 2) +
+         c.k1_unit * tile * ((double)(per_sm / 2) * 2 + (double)(per_sm % 2) * c.k1_alone);
+}
+template <int MODE>
+static double f64_us_k1p(int sms, bool part, int N, int64_t P, int nt, int groups, const F64Cost& c) {
+  using Tile = F64PTile<MODE>;
+  const int64_t items = (int64_t)f64p_tiles<MODE>(N) * groups, per_sm = (items + sms - 1) / sms;
+  const double pair = (MODE == F64P_REAL ? 1 + 8.0 * nt : 4 + 16.0 * nt) * F64P_TI * Tile::TJ / (64 * 1900.0);
+  double us = c.p_call + (double)((per_sm + 1) / 2) * (c.p_round + c.p_block * nt);
+  if (part && P >= F64P_MINPAIR && items % (2 * sms) != 0)
+    return us + c.p_cut + c.p_unit_long * pair * (double)P * (double)items / sms;
+  return us + (P < F64P_MINPAIR ? c.p_unit : c.p_unit_long) * pair * (double)align_up((size_t)P, Tile::KC) *
+                  ((double)(per_sm / 2) * 2 + (double)(per_sm % 2) * c.p_alone);
+}
+// Frequencies of a call on K1, the last ones: all nw, the remainder of the groups of 24, or none.
+template <int MODE>
+static int f64_on_k1(int sms, bool part, int N, int64_t P, int nw) {
+  constexpr F64Cost c = MODE == F64P_REAL
+                            ? F64Cost{7.1, 11.7, 1.93, 1.8, 6.8, 1.0, 6.1, 0.91, 1.15, 1.53, 11.9}
+                            : F64Cost{6.5, 13.7, 1.17, 1.41, 6.9, 1.8, 2.5, 1.10, 1.19, 1.24, 13.3};
+  const int r = nw % 24 > 16 ? 0 : nw % 24, full = (nw - r + 23) / 24;
+  double us = full ? f64_us_k1p<MODE>(sms, part, N, P, 3, full, c) : 0.0;
+  int n = 0;
+  if (r > 0) {
+    const double k1 = f64_us_k1<MODE>(sms, N, P, r, c), k1p = f64_us_k1p<MODE>(sms, part, N, P, r > 8 ? 2 : 1, 1, c);
+    if (k1 <= k1p) n = r;
+    us += std::min(k1, k1p);
+  }
+  return f64_us_k1<MODE>(sms, N, P, nw, c) <= us ? nw : n;
+}
+int fp64_on_k1(bool real, int sms, bool part, int N, int64_t P, int nw) {
+  return real ? f64_on_k1<F64P_REAL>(sms, part, N, P, nw) : f64_on_k1<F64P_CPLX>(sms, part, N, P, nw);
 }
 
-// Frequencies go to K1p in groups of 24 (three DMMA column blocks); a remainder takes the
-// narrowest form that holds it, or K1.
+static int f64r_launch(const F64Call& q, int f0, int n, int* launches);
+
+// Frequencies go to K1p in groups of 24 (three DMMA column blocks) and a remainder in the
+// narrowest form that holds it, unless they go to K1 (K1r).
+template <int MODE>
 static int f64_run(const F64Call& q, int* launches) {
-  int full = q.nw / 24, r = q.nw % 24;
+  const int n1 = fp64_on_k1(MODE == F64P_REAL, q.num_sms, q.part != nullptr, q.N, q.P, q.nw), rest = q.nw - n1;
+  int full = rest / 24, r = rest % 24, e = 0;
   if (r > 16) ++full, r = 0;
-  int e = 0;
-  if (full) e = f64p_launch<3, F64P_CPLX>(q, {}, 0, full, launches);
-  const int f0 = 24 * full;
-  if (!e && r > 8) e = f64p_launch<2, F64P_CPLX>(q, {}, f0, 1, launches);
-  else if (!e && r > 0 && (r > 4 || !f64_takes_k1(q, r))) e = f64p_launch<1, F64P_CPLX>(q, {}, f0, 1, launches);
-  else if (!e && r > 0) e = f64_launch(q, f0, r, launches);
+  if (full) e = f64p_launch<3, MODE>(q, {}, 0, full, launches);
+  if (!e && r > 8) e = f64p_launch<2, MODE>(q, {}, 24 * full, 1, launches);
+  else if (!e && r > 0) e = f64p_launch<1, MODE>(q, {}, 24 * full, 1, launches);
+  if (!e && n1 > 0) e = MODE == F64P_REAL ? f64r_launch(q, rest, n1, launches) : f64_launch(q, rest, n1, launches);
   return e;
 }
 
@@ -888,7 +929,7 @@ int launch_chi0_fp64(spx_ctx* ctx, const double2* M, int64_t ldc, int64_t P, int
       (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull;
   const F64Call q{ctx->num_sms, M, ldc, P, N, W, ldw, nw, out, (double2*)ctx->part, ctx->part_bytes,
                   ctx->d_status, timeout_ns, stream};
-  const int e = f64_run(q, launches);
+  const int e = f64_run<F64P_CPLX>(q, launches);
   if (e) return set_error(ctx, SPX_ECUDA, "chi0_fp64 kernels: tensor map or attribute failed (" +
                                               std::to_string(e) + ")");
   return check_cuda(ctx, cudaGetLastError(), "chi0_fp64 kernel launch");
@@ -925,7 +966,7 @@ int launch_chi0_fp64_noctx(int num_sms, int* status, uint64_t timeout_ns, const 
   if (P <= 0 || N <= 0 || nw <= 0) return SPX_OK;
   const F64Call q{num_sms, M, ldc, P, N, W, ldw, nw, out, nullptr, 0, status, timeout_ns, stream};
   int launches = 0;
-  if (f64_run(q, &launches)) return SPX_ECUDA;
+  if (f64_run<F64P_CPLX>(q, &launches)) return SPX_ECUDA;
   return cudaGetLastError() == cudaSuccess ? SPX_OK : SPX_ECUDA;
 }
 
@@ -1073,7 +1114,7 @@ __global__ void __launch_bounds__(F64_THREADS, 2)
 }
 
 // K1r for the `n` frequencies from f0.
-static int f64r_launch(const F64Call& q, int f0, int n) {
+static int f64r_launch(const F64Call& q, int f0, int n, int* launches) {
   const int nblk = (q.N + F64_B - 1) / F64_B;
   F64Params prm;
   prm.P = q.P;
@@ -1097,28 +1138,8 @@ static int f64r_launch(const F64Call& q, int f0, int n) {
   const int grid = (int)std::min<int64_t>(prm.nitems, (int64_t)2 * q.num_sms);
   chi0_fp64_real_kernel<<<grid, F64_THREADS, smem, q.stream>>>(map, prm,
                                                               reinterpret_cast<double*>(q.out) + (int64_t)f0 * prm.npack);
+  ++*launches;
   return 0;
-}
-
-// Whether n <= 24 frequencies go to K1r rather than to one launch of `nt` 8-wide blocks of
-// K1p, in multiply-adds of the busiest SM: whole 64 x 64 tiles of one frequency, two at a
-// time per SM, against 1 + 8 nt for every 16 x 16 tile, spread evenly. A K1r tile costs 1.55
-// of a K1p multiply-add each (waits for its loads with two CTAs' warps), one alone on its SM
-// 0.95 of two. us, K1r / K1p: N = 300, P = 10000: 2 frequencies 1146 / 329, 24: 2395 / 781;
-// N = 20, P = 2000, 1: 235 / 38; N = 900, P = 10000, 24: 12180 / 6488; N = 1200, 24:
-// 19409 / 11155, 5: 4783 / 4564; the other way round N = 700, 3: 1230 / 1605; N = 1200, 1:
-// 1222 / 4535; N = 1300, P = 6000, 2: 1474 / 3297.
-static bool f64r_takes_k1r(const F64Call& q, int n, int nt) {
-  const int64_t nblk = (q.N + F64_B - 1) / F64_B, sms = q.num_sms;
-  const int64_t per_sm = (nblk * (nblk + 1) / 2 * n + sms - 1) / sms;
-  const double two = 2.0 * F64_B * F64_B, k1 = 1.55 * two * ((double)(per_sm / 2) + (double)(per_sm % 2) * 0.95);
-  using Tile = F64PTile<F64P_REAL>;
-  const int64_t t2 = f64p_tiles<F64P_REAL>(q.N);
-  const double unit = Tile::TI * Tile::TJ * (1 + 8.0 * nt);
-  const bool cut = q.part && q.part_bytes >= f64p_part_bytes<F64P_REAL>(q.num_sms, nt) && q.P >= F64P_MINPAIR;
-  const double k1p = cut ? (double)t2 * unit / (double)sms
-                         : (double)((t2 + Tile::CTAS * sms - 1) / (Tile::CTAS * sms)) * Tile::CTAS * unit;
-  return k1 <= k1p;
 }
 
 // Enqueues the FP64 accumulation over one slab of real band-pair products M (ldc, N): ldc
@@ -1130,14 +1151,7 @@ int launch_chi0_fp64_real(spx_ctx* ctx, const double* M, int64_t ldc, int64_t P,
   const F64Call q{ctx->num_sms, reinterpret_cast<const double2*>(M), ldc, P, N, W, ldw, nw,
                   reinterpret_cast<double2*>(out), (double2*)ctx->part, ctx->part_bytes, ctx->d_status,
                   (uint64_t)(ctx->opt.timeout_ms > 0 ? ctx->opt.timeout_ms : 4000) * 1000000ull, stream};
-  int e = 0;
-  for (int f0 = 0; f0 < nw && !e; f0 += 24) {
-    const int n = std::min(24, nw - f0), nt = (n + 7) / 8;
-    if (f64r_takes_k1r(q, n, nt)) e = f64r_launch(q, f0, n), ++*launches;
-    else if (nt == 3) e = f64p_launch<3, F64P_REAL>(q, {}, f0, 1, launches);
-    else if (nt == 2) e = f64p_launch<2, F64P_REAL>(q, {}, f0, 1, launches);
-    else e = f64p_launch<1, F64P_REAL>(q, {}, f0, 1, launches);
-  }
+  const int e = f64_run<F64P_REAL>(q, launches);
   if (e) return set_error(ctx, SPX_ECUDA, "real FP64 accumulation: tensor map or attribute failed (" +
                                               std::to_string(e) + ")");
   return check_cuda(ctx, cudaGetLastError(), "real FP64 accumulation launch");
