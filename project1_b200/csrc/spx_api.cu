@@ -761,7 +761,11 @@ extern "C" int spx_chi0_accumulate(spx_ctx* ctx, const double* cprod, int64_t ld
   const int64_t nsum = 2 * npack * nw;
   const HostCrew::Task touch{HostCrew::TOUCH, nullptr, susceph, 0, nsum, 0};
   HostCrew crew;
-  crew.start((int)std::max(1u, std::min(8u, std::thread::hardware_concurrency())));
+  // a thread per quarter of a megabyte to gather and add, up to eight: starting seven takes longer
+  // than a small call's work (20 functions, 100 pairs, pinned: 0.21 ms with eight, 0.10 with one)
+  const int64_t host_bytes = 16 * ((pinned ? 0 : npair * nbas) + npack * nw);
+  crew.start((int)std::min<int64_t>(std::max(1u, std::min(8u, std::thread::hardware_concurrency())),
+                                    1 + (host_bytes >> 18)));
   if (pinned) crew.post(touch);   // (nothing to gather)
   for (int64_t p0 = 0, len = 0, k = 0; p0 < npair; p0 += len, ++k) {
     len = chunk_at(p0, len);
