@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "spx_common.cuh"
+#include "spx_dmma.cuh"
 #include "spx_tcgen05.cuh"
 
 namespace spx {
@@ -83,37 +84,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
       "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
-}
-
-// D(16x8) += A(16xKI) * B(KIx8), f64. Fragment order: a[2q+h] = A(g+8h, t+4q),
-// b[q] = B(t+4q, g), d[r] = D(g + 8*(r>>1), 2t + (r&1)); g = lane/4, t = lane%4.
-template <int KI>
-__device__ __forceinline__ void dmma(double (&d)[4], const double* a, const double* b);
-
-template <>
-__device__ __forceinline__ void dmma<4>(double (&d)[4], const double* a, const double* b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
-      "{%0,%1,%2,%3};\n"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a[0]), "d"(a[1]), "d"(b[0]));
-}
-template <>
-__device__ __forceinline__ void dmma<8>(double (&d)[4], const double* a, const double* b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-      "{%8,%9}, {%0,%1,%2,%3};\n"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
-template <>
-__device__ __forceinline__ void dmma<16>(double (&d)[4], const double* a, const double* b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
-      "{%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};\n"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]),
-        "d"(b[0]), "d"(b[1]), "d"(b[2]), "d"(b[3]));
 }
 
 __global__ void __launch_bounds__(F64_THREADS, 2)
@@ -239,14 +209,14 @@ __global__ void __launch_bounds__(F64_THREADS, 2)
               bim[h][q] = wq * v.y;
               bneg[h][q] = -bim[h][q];
             }
-          dmma<8>(accR[mt][2 * np], ar, br[0]);
-          dmma<8>(accR[mt][2 * np + 1], ar, br[1]);
-          dmma<8>(accI[mt][2 * np], ai, br[0]);
-          dmma<8>(accI[mt][2 * np + 1], ai, br[1]);
-          dmma<8>(accR[mt][2 * np], ai, bim[0]);
-          dmma<8>(accR[mt][2 * np + 1], ai, bim[1]);
-          dmma<8>(accI[mt][2 * np], ar, bneg[0]);
-          dmma<8>(accI[mt][2 * np + 1], ar, bneg[1]);
+          dmma_16x8x8(accR[mt][2 * np], ar, br[0]);
+          dmma_16x8x8(accR[mt][2 * np + 1], ar, br[1]);
+          dmma_16x8x8(accI[mt][2 * np], ai, br[0]);
+          dmma_16x8x8(accI[mt][2 * np + 1], ai, br[1]);
+          dmma_16x8x8(accR[mt][2 * np], ai, bim[0]);
+          dmma_16x8x8(accR[mt][2 * np + 1], ai, bim[1]);
+          dmma_16x8x8(accI[mt][2 * np], ar, bneg[0]);
+          dmma_16x8x8(accI[mt][2 * np + 1], ar, bneg[1]);
         }
       }
     }
@@ -607,7 +577,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<MODE>::CTAS)
             const double b[2] = {at(sm.b[st][ks >> 1], JW * warp + jj, 0), at(sm.b[st][ks >> 1], JW * warp + jj, 1)};
             const double z[4] = {ar[0] * b[0], ar[1] * b[0], ar[2] * b[1], ar[3] * b[1]};
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.re[jj][nt], z, wf[nt]);
+            for (int nt = 0; nt < NT; ++nt) dmma_16x8x8(acc.re[jj][nt], z, wf[nt]);
           }
         } else {
           double2 a[4];   // a[2q + h] = M(pair t + 4q, row g + 8h)
@@ -628,14 +598,14 @@ __global__ void __launch_bounds__(F64_THREADS, F64PTile<MODE>::CTAS)
               z[e] = fma(a[e].x, b.x, a[e].y * b.y);
             }
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.re[jj][nt], z, wf[nt]);
+            for (int nt = 0; nt < NT; ++nt) dmma_16x8x8(acc.re[jj][nt], z, wf[nt]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const double2 b = e < 2 ? b0 : b1;
               z[e] = fma(a[e].y, b.x, -(a[e].x * b.y));
             }
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) dmma<8>(acc.im[jj][nt], z, wf[nt]);
+            for (int nt = 0; nt < NT; ++nt) dmma_16x8x8(acc.im[jj][nt], z, wf[nt]);
           }
         }
       }
@@ -1087,7 +1057,7 @@ __global__ void __launch_bounds__(F64_THREADS, 2)
           for (int h = 0; h < 2; ++h)
             a[2 * q + h] = f64r_at(A, 32 * wi + 16 * mt + g + 8 * h, 8 * ks + t + 4 * q);
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) dmma<8>(acc[mt][nt], a, bq[nt]);
+        for (int nt = 0; nt < 4; ++nt) dmma_16x8x8(acc[mt][nt], a, bq[nt]);
       }
     }
     __syncwarp();
@@ -1174,7 +1144,7 @@ __global__ void __launch_bounds__(128) dmma_peak_kernel(int iters, double* sink)
     for (int r = 0; r < 4; ++r) d[k][r] = 0.0;
   for (int it = 0; it < iters; ++it) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) dmma<8>(d[k], a, b);
+    for (int k = 0; k < 8; ++k) dmma_16x8x8(d[k], a, b);
   }
   double s = 0.0;
 #pragma unroll

@@ -58,7 +58,7 @@ constexpr int SP_THREADS = 192;        // warp 0 TMA, warp 1 MMA + TMEM, warps 2
 constexpr int SP1_EPI = 8;
 constexpr int SP_WIDE_BN = 80;  // complex columns of the wide tile (variant 5): N = 160
 constexpr int SP1_THREADS = 64 + 32 * SP1_EPI;
-constexpr int SP_SMS = 148;   // SMs of the one GPU these kernels are built for
+constexpr int SP_SMS = 148;   // a B200's SMs, for rules on sizes: scratch does not follow the device's count
 constexpr int SP1_REGS = 128;  // 40960 registers: two 96-register quantizer blocks fit beside
 
 // BROWS: real rows of the B tile (the MMA's N): 128 for 64 x 64 complex tiles, 160

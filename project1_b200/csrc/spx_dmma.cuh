@@ -1,4 +1,4 @@
-// The FP64 tensor-core product used by the FFT-branch kernels.
+// The FP64 tensor-core products of the accumulation, product and FFT-branch kernels.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -6,7 +6,7 @@ namespace spx {
 
 // D(16x8) += A(16x8) B(8x8), f64. Fragments: a[2q+h] = A(g+8h, t+4q), b[q] = B(t+4q, g),
 // d[r] = D(g + 8*(r>>1), 2t + (r&1)); g = lane/4, t = lane%4.
-__device__ __forceinline__ void dmma_16x8x8(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+__device__ __forceinline__ void dmma_16x8x8(double (&d)[4], const double* a, const double* b) {
   asm volatile(
       "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
       "{%8,%9}, {%0,%1,%2,%3};\n"

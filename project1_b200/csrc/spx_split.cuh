@@ -1,7 +1,8 @@
 // Device code shared by the split-precision accumulation kernels (one call, and the
 // persistent batched schedule): the digit-plane layout, the HILBERT NONE weight,
-// the folded factors, the quantizer task and the TMEM read-back. Both schedules use
-// these functions, so equal slabs give equal bits.
+// the folded factors, the quantizer's arithmetic and the TMEM read-back. Both schedules use
+// these (the persistent one with quantize_task, the separate kernels staging the factors in
+// shared memory), so equal slabs give equal bits.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -156,55 +157,6 @@ __device__ __forceinline__ void quantize_task(const double2* __restrict__ col, b
         *reinterpret_cast<uint4*>(F + o_re + plane * pstride) = make_uint4(br[t][0], br[t][1], br[t][2], br[t][3]);
         *reinterpret_cast<uint4*>(F + o_im + plane * pstride) = make_uint4(bim[t][0], bim[t][1], bim[t][2], bim[t][3]);
       }
-    }
-  }
-}
-
-// The real (-DINV) form of quantize_task: column i of a real M, one plane row per
-// column (`o` its byte offset in plane 0).
-__device__ __forceinline__ void quantize_task_real(const double* __restrict__ col, bool col_ok,
-                                                   int len, int p, double s, int64_t o,
-                                                   int64_t pstride, int nw,
-                                                   const int* __restrict__ wsgn,
-                                                   const double* __restrict__ G, int lenp,
-                                                   int8_t* __restrict__ F) {
-  double x[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) x[k] = (col_ok && p + k < len) ? __ldg(col + p + k) : 0.0;
-  const double inv = s > 0.0 ? 1.0 / s : 0.0;
-  for (int f = 0; f < nw; ++f) {
-    const double* gf = G + (int64_t)f * lenp + p;
-    const bool mixed = wsgn[f] == 0;
-    uint32_t a[SP_SF][4], b[SP_SF][4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      uint32_t y[4], pd[SP_SF];
-      bool neg[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const double g = gf[4 * q + e] * inv;
-        neg[e] = g < 0.0;
-        y[e] = round_mul(x[4 * q + e], fabs(g));
-      }
-      digit_planes<SP_SF>(y, pd);
-#pragma unroll
-      for (int t = 0; t < SP_SF; ++t) a[t][q] = pd[t];
-      if (mixed) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (neg[e]) y[e] = 0u - y[e];
-        digit_planes<SP_SF>(y, pd);
-#pragma unroll
-        for (int t = 0; t < SP_SF; ++t) b[t][q] = pd[t];
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < SP_SF; ++t)
-      *reinterpret_cast<uint4*>(F + o + ((int64_t)f * SP_SLOT + t) * pstride) = make_uint4(a[t][0], a[t][1], a[t][2], a[t][3]);
-    if (mixed) {
-#pragma unroll
-      for (int t = 0; t < SP_SF; ++t)
-        *reinterpret_cast<uint4*>(F + o + ((int64_t)f * SP_SLOT + SP_SF + t) * pstride) = make_uint4(b[t][0], b[t][1], b[t][2], b[t][3]);
     }
   }
 }

@@ -32,6 +32,7 @@
 
 #include "spx_chain.cuh"
 #include "spx_common.cuh"
+#include "spx_dmma.cuh"
 #include "spx_zgemm.h"
 
 namespace spx {
@@ -56,14 +57,6 @@ __device__ __forceinline__ void cp_async_commit() {
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ void dmma8(double (&d)[4], const double* a, const double* b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-      "{%8,%9}, {%0,%1,%2,%3};\n"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
 // Shared rows of 16 complex k (256 bytes); 16-byte chunk k of row r sits at
@@ -260,14 +253,14 @@ __global__ void __launch_bounds__(ZG_THREADS, 2) zgemm_gather_kernel(ZgParams pr
                 bneg[h][q] = -v.y;
               }
             // A conj(B): re += ar br + ai bi, im += ai br - ar bi
-            dmma8(accR[mt][2 * np], ar, br[0]);
-            dmma8(accR[mt][2 * np + 1], ar, br[1]);
-            dmma8(accI[mt][2 * np], ai, br[0]);
-            dmma8(accI[mt][2 * np + 1], ai, br[1]);
-            dmma8(accR[mt][2 * np], ai, bim[0]);
-            dmma8(accR[mt][2 * np + 1], ai, bim[1]);
-            dmma8(accI[mt][2 * np], ar, bneg[0]);
-            dmma8(accI[mt][2 * np + 1], ar, bneg[1]);
+            dmma_16x8x8(accR[mt][2 * np], ar, br[0]);
+            dmma_16x8x8(accR[mt][2 * np + 1], ar, br[1]);
+            dmma_16x8x8(accI[mt][2 * np], ai, br[0]);
+            dmma_16x8x8(accI[mt][2 * np + 1], ai, br[1]);
+            dmma_16x8x8(accR[mt][2 * np], ai, bim[0]);
+            dmma_16x8x8(accR[mt][2 * np + 1], ai, bim[1]);
+            dmma_16x8x8(accI[mt][2 * np], ar, bneg[0]);
+            dmma_16x8x8(accI[mt][2 * np + 1], ar, bneg[1]);
           }
         }
       }

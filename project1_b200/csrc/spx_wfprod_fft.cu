@@ -635,7 +635,7 @@ struct FoldGatherParams {
   const int* gmap;     // per ig: iz | iy << 8 | ix << 16
   double2* cprod;      // (first pair of the chunk, column col0)
   int64_t ldc, npair;
-  int n, H, nst, sl, nkz, plane, nky, ngptm;
+  int n, nst, sl, nkz, plane, nky, ngptm;
 };
 
 // The z pass and the gather: a CTA takes two consecutive pairs (32-byte runs of a cprod
@@ -1066,7 +1066,7 @@ int wfprod_pw_fft_run(spx_ctx* ctx, const spx_pw_desc* d, int nk, int nocc, int 
       if ((rc = check_cuda(ctx, cudaGetLastError(), "fft_pair_fold_kernel launch"))) return rc;
       const int64_t npair = (int64_t)kn * nocc * nunocc;
       FoldGatherParams gp{T2, d_tab, d_pos[2], d_gmap, cprod + (int64_t)k0 * nocc * nunocc + ldc * col0, ldc, npair,
-                          n, pl.H, pl.nst, pl.sl, nkz, nkx * nky, nky, d->ngptm};
+                          n, pl.nst, pl.sl, nkz, nkx * nky, nky, d->ngptm};
       fft_pair_gather_kernel<<<(unsigned)((npair + 1) / 2), 256, g_smem, s>>>(gp);
       if ((rc = check_cuda(ctx, cudaGetLastError(), "fft_pair_gather_kernel launch"))) return rc;
       *launches += 2;
