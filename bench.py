@@ -280,10 +280,21 @@ def upper_tiles(N: int, variant: int) -> int:
     return nblk * (nblk + 1) // 2
 
 
+def launch_pairs(N: int, slab: int) -> int:
+    """Pairs of one accumulation launch: a slab, or where a frequency has more than 148 tiles
+    its equal parts whose planes (3 digits) stay below 90 MB."""
+    nblk = (N + 63) // 64
+    if upper_tiles(N, 5) <= 148:
+        return slab
+    most = min(slab, max(4096, (90 << 20) // (3 * 128 * ((nblk + 1) // 2 * 2)) // 64 * 64))
+    n = -(-slab // most)
+    return -(-(-(-slab // n)) // 64) * 64
+
+
 def measured_traffic(kernel: str, nbas: int, nw: int, slab: int, npair_step: int, tiles: int = 0):
     """DRAM bytes of the dominant kernel from the committed ncu capture, scaled to one
-    launch (one slab of all frequencies) of this shape: the capture's bytes per pair,
-    frequency and 64-block tile. None when no capture of `kernel` is recorded."""
+    launch (a slab, or its part, of all frequencies) of this shape: the capture's bytes per
+    pair, frequency and 64-block tile. None when no capture of `kernel` is recorded."""
     f = ROOT / "profiles" / "roofline_traffic.json"
     if not f.exists():
         return None
@@ -293,14 +304,15 @@ def measured_traffic(kernel: str, nbas: int, nw: int, slab: int, npair_step: int
         return None
     if not rec:
         return None
+    pairs = min(launch_pairs(nbas, slab), npair_step)
     if "by_slab" in rec:
-        # the capture whose slab is nearest this one (traffic per pair falls with the slab)
-        key = min(rec["by_slab"], key=lambda k: abs(int(k) - slab))
+        # the capture whose launch is nearest this one (traffic per pair falls with its pairs)
+        key = min(rec["by_slab"], key=lambda k: abs(int(k) - pairs))
         rec = dict(rec["by_slab"][key], captured_slab=int(key))
     nblk = (nbas + 63) // 64
     tiles = tiles or nblk * (nblk + 1) // 2
-    per_launch = rec["bytes_per_pair_freq_tile"] * min(slab, npair_step) * nw * tiles
-    out = {"bytes_per_launch": per_launch, "launches_per_step": -(-npair_step // slab),
+    per_launch = rec["bytes_per_pair_freq_tile"] * pairs * nw * tiles
+    out = {"bytes_per_launch": per_launch, "launches_per_step": -(-npair_step // slab) * -(-slab // launch_pairs(nbas, slab)),
            "source": rec["source"]}
     if "captured_slab" in rec:
         out["captured_slab"] = rec["captured_slab"]
@@ -520,8 +532,8 @@ def run_ours(args):
             nblk = (N + 63) // 64
             R = ((nblk + 1) // 2 * 2 if variant == 2 else nblk) * 128   # plane rows (the pair needs even blocks)
             roof["traffic"] = tr["bytes_per_launch"]
-            roof["traffic_detail"] = dict(tr, kernel=kname, unit="bytes per launch (one slab, all frequencies)",
-                                          operand_plane_bytes_per_launch=3.0 * nw * R * min(slab, Pr))
+            roof["traffic_detail"] = dict(tr, kernel=kname, unit="bytes per launch (a slab or its part, all frequencies)",
+                                          operand_plane_bytes_per_launch=3.0 * nw * R * min(launch_pairs(N, slab), Pr))
     else:
         roof = fp64_roofline(ctx, N, nw, ach)
     if fp64 is not None:

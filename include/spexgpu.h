@@ -63,7 +63,9 @@ typedef struct spx_ctx spx_ctx;
 typedef struct spx_options {
   int32_t struct_size;      /* sizeof(spx_options), for forward compatibility   */
   int32_t verbose;          /* 0 = silent                                        */
-  int64_t workspace_limit;  /* device bytes the context may allocate, 0 = auto   */
+  int64_t workspace_limit;  /* device bytes of the workspace, and the fixed 48.5 MB for
+                               partial tiles beside it (given up first), 0 = auto; the
+                               scratch of split batches run q by q stays below it too */
   int64_t pinned_limit;     /* pinned host staging bytes, 0 = auto               */
   int32_t chunk_pairs;      /* band pairs per streamed chunk, 0 = auto           */
   int32_t timeout_ms;       /* bound on every device-side wait, 0 = 4000 ms      */

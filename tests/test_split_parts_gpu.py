@@ -35,7 +35,7 @@ def _exact(m, d, om, scale):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nbas,npair,real", [
-    (1200, 12160, False), (1200, 12161, False), (1200, 24321, False), (1200, 32768, False), (1200, 46000, False),
+    (1200, 12288, False), (1200, 12289, False), (1200, 24577, False), (1200, 32768, False), (1200, 46000, False),
     (1121, 13001, False), (2500, 13001, True), (2500, 36000, True)])
 def test_parts_against_64_bits(nbas, npair, real):
     """The stated bound: 1e-6 of sqrt(chi_ii chi_jj)."""
